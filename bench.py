@@ -450,7 +450,7 @@ def run_sky(args) -> None:
     roofline = {"bound": "fp32", "achieved": achieved_flops / 1e12,
                 "peak": (peaks["ffma_flops"] or float("nan")) / 1e12, "unit": "TFLOP/s",
                 "frac": achieved_flops / peaks["ffma_flops"] if peaks["ffma_flops"] else None,
-                "traffic": None, "kernel": "sky_warp_kernel",
+                "traffic": None, "kernel": "sky_tile_kernel",
                 "kernel_ms_per_launch": tot_ms / args.steps,
                 "work_per_pair": {"fp32_flops": F, "smem_atomic_updates": A},
                 "peak_source": "measured live in this run (FFMA microbenchmark)"}

@@ -28,7 +28,7 @@ CPP_SOURCES = ["host_helpers.cpp"]
 HOST_SOURCES = ["host/inp.cpp", "host/reader.cpp", "host/finalize.cpp", "host/outp.cpp",
                 "host/driver.cpp"]
 HEADERS = ["cpc_device.cuh", "kernels.h", "host_helpers.h", "pair_values.h", "host/host.h",
-           "df32.cuh", "pair_df.cuh", "param_check.h"]
+           "df32.cuh", "pair_df.cuh", "field_map.cuh", "param_check.h"]
 
 
 def nvcc() -> str:

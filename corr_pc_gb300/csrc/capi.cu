@@ -96,26 +96,37 @@ struct Slot {
   // redshift-ordered catalogue; these the sky-only per-galaxy quantities
   bool sky = false;
   DevBuf<double> dc, da, sd, cd, rar, decr, win;
-  DevBuf<float4> sky_su, sky_sl, sky_sw, sky_sx, sky_ss, sky_sh;  // float views (SkyFast)
-  DevBuf<float2> sky_sp;
-  double dcmax = 0;  // largest |D_C| (error bound of the float Pi)
+  // cell order (SkyFast): sorted by (region, keep flag, sky cell, redshift)
+  DevBuf<unsigned char> sky_pack;  // every array of sky_f, one allocation and one copy
+  SkyFast sky_f{};
+  bool sky_mono = false;      // the rows' redshift window bounds rise with the redshift
+  double dcmax = 0;           // largest |D_C| (error bound of the float Pi)
+  double damin = 0, damax = 0;  // range of D_A
+  double sky_mag = 0;         // largest window bound or coordinate of the float tests
+  double sky_zw = 0;          // mean width of the rows' windows in scaled redshift
+  double sky_fz = 0;          // mean share of the catalogue inside a row's redshift window
+  int sky_nkey = 0;           // (region, keep flag) keys with galaxies
+  std::vector<int> hc_zidx;   // redshift-ordered position of each cell-ordered row
+  std::vector<float> hc_z;    // scaled redshift, cell order
+  std::vector<int4> hc_bk;    // buckets
+  std::vector<SkyTileRows> hc_tiles;  // tiles over every row (built by the first count)
+  std::vector<int> hc_tile_key;       // their bucket keys
+  std::vector<float4> hc_bwin, hc_box;  // per bucket: union of its rows' RA/Dec windows; its box
   // host copies in the same order for the host edge tier
   std::vector<double> hs_ra, hs_dec, hs_dc, hs_da, hs_w, hs_e1, hs_e2, hs_phi;
   std::vector<int32_t> hs_jk;
   std::vector<uint8_t> hs_keep;
   std::vector<int64_t> hs_orig;  // input row of each redshift-ordered row (row samples)
-  // the sky kernel's outer-row order: redshift-ordered positions grouped by
-  // redshift slab (16 of equal size) and jackknife region, redshift order within
-  std::vector<int> hs_rorder;
 };
 
 // device buffers of one job of a sky launch: its histogram block, fixed-point
 // sums, counters, host-tier queue and row sample
 struct SkyJobBufs {
-  DevBuf<unsigned long long> num, fix, counters, hq_n;
+  DevBuf<unsigned long long> num, fix, counters, hq_n, xq_n;
   DevBuf<double> sums;
-  DevBuf<int2> hq;
+  DevBuf<int2> hq, xq;
   DevBuf<int> rows;
+  DevBuf<SkyTileRows> tiles;
 };
 
 struct UnitCache {
@@ -156,10 +167,10 @@ struct cpc_ctx {
   DevBuf<unsigned long long> d_num;
   DevBuf<double> d_sums;
   DevBuf<unsigned long long> d_counters;
-  // sky launches: one buffer set per job of the launch, the chunk table
+  // sky launches: one buffer set per job of the launch, the unit queue
   std::vector<std::unique_ptr<SkyJobBufs>> sky_bufs;
-  DevBuf<long long> d_chunk0;
-  DevBuf<unsigned long long> d_chunk_ctr;
+  DevBuf<SkyUnit> d_sky_units;
+  DevBuf<unsigned long long> d_sky_ctr;
   // sort scratch
   DevBuf<uint64_t> d_keys, d_ktmp;
   DevBuf<uint32_t> d_vals, d_vtmp, d_hist, d_bucket;
@@ -190,10 +201,6 @@ struct cpc_ctx {
   int twin_on = 1;
   int last_twin = 0;  // the last fast count ran a twin job
   DevBuf<unsigned> d_differ;
-  // register bound of the fast sky kernel: 2 or 3 blocks of 256 threads per SM
-  // (CPC_SKY_BLOCKS_PER_SM in the environment; the autotuner of a sky context
-  // would set it)
-  int sky_blocks_per_sm = 2;
   // CUDA graph of the fast engine's device work (zeroing, pair kernels,
   // recheck), replayed while every value baked into it stays the same
   int graph_on = 1;
@@ -1419,6 +1426,109 @@ SkyParams sky_params(const cpc_ctx *c) {
   return sp;
 }
 
+// Scaled redshift of the fast kernel's window tests: a power of two that puts
+// [0, z_max] on the scale of the angles in degrees, so that one float guard
+// serves the three window tests.
+double sky_z_scale(const cpc_params &p) {
+  return std::ldexp(1.0, (int)std::floor(std::log2(256.0 / std::max(p.z_max, 1e-6))));
+}
+
+// Cell order of a redshift-ordered sky catalogue (s.hs_*; zs its redshifts, wins
+// its row windows): rows sorted by (jackknife region, keep flag, sky cell of the
+// region, redshift), and the buckets (non-empty cells).  A region's cells divide
+// its RA x Dec box evenly, sized so that a cell holds about 96 rows (three row
+// passes of a warp) in a quarter of the redshift window, between an eighth
+// and three quarters of the mean angular window: smaller cells would only
+// shorten the candidate runs, larger ones test candidates far outside.
+void sky_cell_order(cpc_ctx *c, Slot &s, const std::vector<double> &zs,
+                    const std::vector<double> &wins) {
+  const cpc_params &p = c->p;
+  const int64_t n = s.n;
+  const int nreg = p.do_jk ? p.n_jk : 1;
+  const double zk = sky_z_scale(p);
+  struct Reg {
+    double a0 = 1e300, a1 = -1e300, d0 = 1e300, d1 = -1e300, ix = 0, iy = 0;
+    int64_t n = 0, base = 0;
+    int nx = 1, ny = 1;
+  };
+  std::vector<Reg> reg(nreg);
+  for (int64_t k = 0; k < n; k++) {
+    Reg &r = reg[p.do_jk ? s.hs_jk[k] : 0];
+    r.a0 = std::min(r.a0, s.hs_ra[k]);
+    r.a1 = std::max(r.a1, s.hs_ra[k]);
+    r.d0 = std::min(r.d0, s.hs_dec[k]);
+    r.d1 = std::max(r.d1, s.hs_dec[k]);
+    r.n++;
+  }
+  // mean window of a sample of rows: half width in Dec, width in redshift, and
+  // the share of the catalogue inside it
+  double hw = 0, zw = 0, fz = 0;
+  int64_t m = 0;
+  for (int64_t k = 0; k < n; k += std::max<int64_t>(1, n / 512), m++) {
+    const double z0 = wins[k], z1 = wins[n + k];
+    hw += 0.5 * (wins[5 * n + k] - wins[4 * n + k]);
+    zw += z1 - z0;
+    fz += (double)(std::upper_bound(zs.begin(), zs.end(), z1) -
+                   std::lower_bound(zs.begin(), zs.end(), z0)) / (double)n;
+  }
+  if (m) {
+    hw /= m;
+    zw /= m;
+    fz /= m;
+  }
+  s.sky_zw = zw * zk;
+  s.sky_fz = fz;
+  int64_t cells = 0;
+  for (Reg &r : reg) {
+    r.base = cells;
+    if (r.n > 0) {
+      const double cosd = std::cos(0.5 * (r.d0 + r.d1) * M_PI / 180.0);
+      const double ex = std::max((r.a1 - r.a0) * std::max(cosd, 1e-3), 1e-9);
+      const double ey = std::max(r.d1 - r.d0, 1e-9);
+      double sz = std::sqrt(96.0 * ex * ey / (std::max(1e-9, 0.25 * fz) * (double)r.n));
+      sz = std::min(std::max(sz, hw / 8), 0.75 * hw);
+      if (sz > 0) {
+        const double lim = std::max(1.0, std::sqrt((double)r.n / 8.0));
+        r.nx = (int)std::min(lim, std::max(1.0, std::round(ex / sz)));
+        r.ny = (int)std::min(lim, std::max(1.0, std::round(ey / sz)));
+      }
+      r.ix = r.nx / std::max(r.a1 - r.a0, 1e-30);
+      r.iy = r.ny / std::max(r.d1 - r.d0, 1e-30);
+    }
+    cells += 2ll * r.nx * r.ny;
+  }
+  std::vector<int64_t> start((size_t)cells + 1, 0);
+  std::vector<int64_t> id(n);
+  host_parallel(n, [&](int64_t b0, int64_t b1, int) {
+    for (int64_t k = b0; k < b1; k++) {
+      const Reg &r = reg[p.do_jk ? s.hs_jk[k] : 0];
+      const int cx = std::min(r.nx - 1, (int)((s.hs_ra[k] - r.a0) * r.ix));
+      const int cy = std::min(r.ny - 1, (int)((s.hs_dec[k] - r.d0) * r.iy));
+      id[k] = r.base + (s.hs_keep[k] ? (int64_t)r.nx * r.ny : 0) + (int64_t)cy * r.nx + cx;
+    }
+  });
+  for (int64_t k = 0; k < n; k++) start[id[k] + 1]++;
+  for (int64_t q = 0; q < cells; q++) start[q + 1] += start[q];
+  s.hc_bk.clear();
+  for (int g = 0; g < nreg; g++) {
+    const int64_t nc = (int64_t)reg[g].nx * reg[g].ny;
+    for (int64_t q = 0; q < 2 * nc; q++) {
+      const int64_t b = reg[g].base + q;
+      if (start[b + 1] > start[b])
+        s.hc_bk.push_back(make_int4((int)start[b], (int)start[b + 1], 2 * g + (q >= nc ? 1 : 0), 0));
+    }
+  }
+  s.sky_nkey = 0;
+  for (size_t b = 0; b < s.hc_bk.size(); b++)
+    s.sky_nkey += b == 0 || s.hc_bk[b].z != s.hc_bk[b - 1].z;
+  s.hc_zidx.resize(n);
+  s.hc_z.resize(n);
+  for (int64_t k = 0; k < n; k++) s.hc_zidx[start[id[k]]++] = (int)k;
+  host_parallel(n, [&](int64_t b0, int64_t b1, int) {
+    for (int64_t q = b0; q < b1; q++) s.hc_z[q] = (float)(zs[s.hc_zidx[q]] * zk);
+  });
+}
+
 // Upload a sky catalogue: per-galaxy windows and angles on the host (C
 // library, exactly the reference's values), redshift order from the device
 // radix sort, then every array in that order on the device and on the host.
@@ -1541,35 +1651,32 @@ cpc_status sky_upload(cpc_ctx *c, int slot, const cpc_catalog *cat) {
     }
     CK(cudaStreamSynchronize(st), "sort");
   }
-  auto take = [&](const double *src, std::vector<double> &dst) {
-    dst.resize(n);
-    host_parallel(n, [&](int64_t b0, int64_t b1, int) {
-      for (int64_t k = b0; k < b1; k++) dst[k] = src[perm[k]];
-    });
-  };
-  std::vector<double> zs, sds, cds, rars, decrs;
-  take(cat->x, s.hs_ra);
-  take(cat->y, s.hs_dec);
-  take(cat->z, zs);
-  take(cat->dc, s.hs_dc);
-  take(cat->da, s.hs_da);
-  take(w.data(), s.hs_w);
-  take(e1.data(), s.hs_e1);
-  take(e2.data(), s.hs_e2);
-  take(phi.data(), s.hs_phi);
-  take(sd.data(), sds);
-  take(cd.data(), cds);
-  take(rar.data(), rars);
-  take(decr.data(), decrs);
+  std::vector<double> zs(n), sds(n), cds(n), rars(n), decrs(n);
+  for (std::vector<double> *v : {&s.hs_ra, &s.hs_dec, &s.hs_dc, &s.hs_da, &s.hs_w, &s.hs_e1,
+                                 &s.hs_e2, &s.hs_phi})
+    v->resize(n);
   s.hs_jk.resize(n);
   s.hs_keep.resize(n);
   std::vector<int64_t> &orig = s.hs_orig;
-  orig.assign(n, 0);
+  orig.resize(n);
   std::vector<double> wins(6 * (size_t)n);
   std::vector<uint8_t> aflag(n);
   host_parallel(n, [&](int64_t b0, int64_t b1, int) {
     for (int64_t k = b0; k < b1; k++) {
       const uint32_t o = perm[k];
+      s.hs_ra[k] = cat->x[o];
+      s.hs_dec[k] = cat->y[o];
+      zs[k] = cat->z[o];
+      s.hs_dc[k] = cat->dc[o];
+      s.hs_da[k] = cat->da[o];
+      s.hs_w[k] = w[o];
+      s.hs_e1[k] = e1[o];
+      s.hs_e2[k] = e2[o];
+      s.hs_phi[k] = phi[o];
+      sds[k] = sd[o];
+      cds[k] = cd[o];
+      rars[k] = rar[o];
+      decrs[k] = decr[o];
       s.hs_jk[k] = jk[o];
       s.hs_keep[k] = keep[o];
       orig[k] = o;
@@ -1578,20 +1685,9 @@ cpc_status sky_upload(cpc_ctx *c, int slot, const cpc_catalog *cat) {
       aflag[k] = (o + 1 < (uint32_t)n && !(cat->z[o + 1] < win[o])) ? kAutoStart0 : 0;
     }
   });
-  // outer-row order of the fast sky kernel: (redshift slab, region, redshift),
-  // so that a chunk of consecutive rows usually lies in one region
-  {
-    const int kSlabs = 16;
-    const int nreg = p.do_jk ? p.n_jk : 1;
-    std::vector<int64_t> start((size_t)kSlabs * nreg + 1, 0);
-    auto key = [&](int64_t k) {
-      return (int64_t)(k * kSlabs / std::max<int64_t>(n, 1)) * nreg + (p.do_jk ? s.hs_jk[k] : 0);
-    };
-    for (int64_t k = 0; k < n; k++) start[key(k) + 1]++;
-    for (size_t q = 1; q < start.size(); q++) start[q] += start[q - 1];
-    s.hs_rorder.assign(n, 0);
-    for (int64_t k = 0; k < n; k++) s.hs_rorder[start[key(k)]++] = (int)k;
-  }
+  s.hc_tiles.clear();
+  s.hc_tile_key.clear();
+  sky_cell_order(c, s, zs, wins);
   auto put = [&](DevBuf<double> &d, const std::vector<double> &h, size_t cnt) -> cudaError_t {
     cudaError_t e = d.alloc(std::max<size_t>(cnt, 1));
     if (e != cudaSuccess || cnt == 0) return e;
@@ -1604,45 +1700,139 @@ cpc_status sky_upload(cpc_ctx *c, int slot, const cpc_catalog *cat) {
   CK(put(s.da, s.hs_da, n), "sky upload"); CK(put(s.sd, sds, n), "sky upload");
   CK(put(s.cd, cds, n), "sky upload"); CK(put(s.rar, rars, n), "sky upload");
   CK(put(s.decr, decrs, n), "sky upload"); CK(put(s.win, wins, 6 * (size_t)n), "sky upload");
-  // float views for the fast kernel: hi parts and the remainders
-  std::vector<float4> su(n), sl(n), sw(n), sx(n), ss(n), sh(n);
-  std::vector<float2> sph(n);
+  // float views for the fast kernel, in cell order: hi parts and the remainders
+  const double zk = sky_z_scale(p);
+  const size_t nbk = s.hc_bk.size();
+  size_t pack_bytes = 0;
+  auto room = [&](size_t bytes) {  // offset of an array in the packed views
+    const size_t o = pack_bytes;
+    pack_bytes += (bytes + 255) / 256 * 256;
+    return o;
+  };
+  size_t off4[9], off2[2], off1[3];
+  for (int q = 0; q < 7; q++) off4[q] = room(sizeof(float4) * n);
+  for (int q = 7; q < 9; q++) off4[q] = room(sizeof(float4) * nbk);
+  for (size_t &o : off2) o = room(sizeof(float2) * n);
+  for (size_t &o : off1) o = room(sizeof(float) * n);
+  const size_t off_bk = room(sizeof(int4) * nbk);
+  std::unique_ptr<unsigned char[]> pack(new unsigned char[std::max<size_t>(pack_bytes, 1)]);
+  auto at4 = [&](int q) { return reinterpret_cast<float4 *>(pack.get() + off4[q]); };
+  auto at2 = [&](int q) { return reinterpret_cast<float2 *>(pack.get() + off2[q]); };
+  float4 *su = at4(0), *sl = at4(1), *sw = at4(2), *sx = at4(3), *ss = at4(4), *sh = at4(5),
+         *wb = at4(6), *box = at4(7), *bwin = at4(8);
+  float2 *sph = at2(0), *wz = at2(1);
+  float *zf = reinterpret_cast<float *>(pack.get() + off1[0]);
+  float *dl = reinterpret_cast<float *>(pack.get() + off1[1]);
+  int *zidx = reinterpret_cast<int *>(pack.get() + off1[2]);
   auto hi = [](double v) { return (float)v; };
   auto lo = [](double v) { return (float)(v - (double)(float)v); };
-  std::vector<double> dcm(kMaxParts, 0.0);
+  struct Range {
+    double dc = 0, da0 = 1e300, da1 = 0, mag = 0;
+  };
+  std::vector<Range> ranges(kMaxParts);
   host_parallel(n, [&](int64_t b0, int64_t b1, int part) {
-    for (int64_t k = b0; k < b1; k++) {
+    Range &R = ranges[part];
+    for (int64_t q = b0; q < b1; q++) {
+      const int64_t k = s.hc_zidx[q];
       const double ux = cds[k] * std::cos(rars[k]), uy = cds[k] * std::sin(rars[k]), uz = sds[k];
       const double dcv = s.hs_dc[k];
-      dcm[part] = std::max(dcm[part], std::fabs(dcv));
-      su[k] = make_float4(hi(ux), hi(uy), hi(uz), (float)s.hs_da[k]);
-      sl[k] = make_float4(lo(ux), lo(uy), lo(uz), lo(dcv));
-      sw[k] = make_float4(hi(s.hs_ra[k]), hi(s.hs_dec[k]), (float)zs[k], hi(dcv));
-      sx[k] = make_float4(lo(s.hs_ra[k]), lo(s.hs_dec[k]), (float)decrs[k], (float)s.hs_w[k]);
+      R.dc = std::max(R.dc, std::fabs(dcv));
+      R.da0 = std::min(R.da0, s.hs_da[k]);
+      R.da1 = std::max(R.da1, std::fabs(s.hs_da[k]));
+      su[q] = make_float4(hi(ux), hi(uy), hi(uz), (float)s.hs_da[k]);
+      sl[q] = make_float4(lo(ux), lo(uy), lo(uz), lo(dcv));
+      dl[q] = (float)(dcv - (double)hi(dcv) - (double)lo(dcv));  // exact: at most 6 bits
+      sw[q] = make_float4(hi(s.hs_ra[k]), hi(s.hs_dec[k]), s.hc_z[q], hi(dcv));
+      sx[q] = make_float4(lo(s.hs_ra[k]), lo(s.hs_dec[k]), (float)decrs[k], (float)s.hs_w[k]);
+      zf[q] = s.hc_z[q];
+      zidx[q] = s.hc_zidx[q];
       // weighted ellipticity and the half Dec angle's cosine and sine as hi +
       // lo parts (the compensated shape terms: cos of the pair's mean Dec is
       // cos(d1/2) cos(d2/2) - sin(d1/2) sin(d2/2))
       const double we1 = s.hs_w[k] * s.hs_e1[k], we2 = s.hs_w[k] * s.hs_e2[k];
-      ss[k] = make_float4(hi(we1), hi(we2), lo(we1), lo(we2));
+      ss[q] = make_float4(hi(we1), hi(we2), lo(we1), lo(we2));
       const double ch = std::cos(decrs[k] / 2.0), sh2 = std::sin(decrs[k] / 2.0);
-      sh[k] = make_float4(hi(ch), lo(ch), hi(sh2), lo(sh2));
-      sph[k] = make_float2((float)s.hs_phi[k], lo(s.hs_w[k]));
+      sh[q] = make_float4(hi(ch), lo(ch), hi(sh2), lo(sh2));
+      sph[q] = make_float2((float)s.hs_phi[k], lo(s.hs_w[k]));
+      // windows as centre and half width; NaN bounds (lim_calc_ra_dec's acos out
+      // of range gives two) pass every candidate, as in the reference
+      float c2[3], h2[3];
+      for (int m = 0; m < 3; m++) {
+        const double f = m == 0 ? zk : 1.0;
+        const double v0 = wins[(size_t)(2 * m) * n + k] * f, v1 = wins[(size_t)(2 * m + 1) * n + k] * f;
+        if (std::isnan(v0) || std::isnan(v1)) {
+          c2[m] = 0.0f;
+          h2[m] = INFINITY;
+          continue;
+        }
+        c2[m] = (float)(0.5 * (v0 + v1));
+        h2[m] = (float)(0.5 * (v1 - v0));
+        R.mag = std::max({R.mag, std::fabs(v0), std::fabs(v1)});
+      }
+      R.mag = std::max({R.mag, std::fabs(s.hs_ra[k]), std::fabs(s.hs_dec[k]),
+                        std::fabs((double)s.hc_z[q])});
+      wz[q] = make_float2(c2[0], h2[0]);
+      wb[q] = make_float4(c2[1], h2[1], c2[2], h2[2]);
     }
   });
-  s.dcmax = 0;
-  for (double v : dcm) s.dcmax = std::max(s.dcmax, v);
-  DevBuf<float4> *fbufs[6] = {&s.sky_su, &s.sky_sl, &s.sky_sw, &s.sky_sx, &s.sky_ss, &s.sky_sh};
-  const std::vector<float4> *fsrc[6] = {&su, &sl, &sw, &sx, &ss, &sh};
-  for (int q = 0; q < 6; q++) {
-    CK(fbufs[q]->alloc(nn), "alloc");
-    if (n > 0)
-      CK(cudaMemcpyAsync(fbufs[q]->p, fsrc[q]->data(), sizeof(float4) * n, cudaMemcpyHostToDevice,
-                         st), "H2D");
+  s.dcmax = s.damax = s.sky_mag = 0;
+  s.damin = 1e300;
+  for (const Range &R : ranges) {
+    s.dcmax = std::max(s.dcmax, R.dc);
+    s.damin = std::min(s.damin, R.da0);
+    s.damax = std::max(s.damax, R.da1);
+    s.sky_mag = std::max(s.sky_mag, R.mag);
   }
-  CK(s.sky_sp.alloc(nn), "alloc");
-  if (n > 0)
-    CK(cudaMemcpyAsync(s.sky_sp.p, sph.data(), sizeof(float2) * n, cudaMemcpyHostToDevice, st),
-       "H2D");
+  // the buckets' RA and Dec ranges, and those of their rows' windows
+  s.hc_box.resize(nbk);
+  s.hc_bwin.resize(nbk);
+  host_parallel((int64_t)nbk, [&](int64_t b0, int64_t b1, int) {
+    for (int64_t b = b0; b < b1; b++) {
+      float4 r = make_float4(INFINITY, -INFINITY, INFINITY, -INFINITY), v = r;
+      for (int q = s.hc_bk[b].x; q < s.hc_bk[b].y; q++) {
+        r.x = std::min(r.x, sw[q].x);
+        r.y = std::max(r.y, sw[q].x);
+        r.z = std::min(r.z, sw[q].y);
+        r.w = std::max(r.w, sw[q].y);
+        v.x = std::min(v.x, wb[q].x - wb[q].y);
+        v.y = std::max(v.y, wb[q].x + wb[q].y);
+        v.z = std::min(v.z, wb[q].z - wb[q].w);
+        v.w = std::max(v.w, wb[q].z + wb[q].w);
+      }
+      box[b] = s.hc_box[b] = r;
+      bwin[b] = s.hc_bwin[b] = v;
+    }
+  }, 16);
+  if (nbk) std::memcpy(pack.get() + off_bk, s.hc_bk.data(), sizeof(int4) * nbk);
+  CK(s.sky_pack.alloc(std::max<size_t>(pack_bytes, 1)), "alloc");
+  if (pack_bytes)
+    CK(cudaMemcpyAsync(s.sky_pack.p, pack.get(), pack_bytes, cudaMemcpyHostToDevice, st), "H2D");
+  {
+    auto d4 = [&](int q) { return reinterpret_cast<const float4 *>(s.sky_pack.p + off4[q]); };
+    auto d2 = [&](int q) { return reinterpret_cast<const float2 *>(s.sky_pack.p + off2[q]); };
+    SkyFast &f = s.sky_f;
+    f.su = d4(0); f.sl = d4(1); f.sw = d4(2); f.sx = d4(3); f.ss = d4(4); f.sh = d4(5);
+    f.wb = d4(6); f.bk_box = d4(7); f.bk_win = d4(8);
+    f.sp = d2(0); f.wz = d2(1);
+    f.zf = reinterpret_cast<const float *>(s.sky_pack.p + off1[0]);
+    f.dl = reinterpret_cast<const float *>(s.sky_pack.p + off1[1]);
+    f.zidx = reinterpret_cast<const int *>(s.sky_pack.p + off1[2]);
+    f.bk = reinterpret_cast<const int4 *>(s.sky_pack.p + off_bk);
+    f.n_bk = (int)nbk;
+  }
+  // redshift window bounds that rise with the redshift (but for float rounding,
+  // which the kernel's guard covers) can be searched
+  s.sky_mono = true;
+  const float tol = (float)(2.0 * ulpf(std::max(s.sky_mag, 1e-30)));
+  for (const int4 &b : s.hc_bk) {
+    float top = -INFINITY, bot = -INFINITY;  // largest bounds so far
+    for (int q = b.x; q < b.y && s.sky_mono; q++) {
+      const float u = wz[q].x + wz[q].y, l = wz[q].x - wz[q].y;
+      s.sky_mono = u >= top - tol && l >= bot - tol;
+      top = std::max(top, u);
+      bot = std::max(bot, l);
+    }
+  }
   CK(s.jk.alloc(nn), "alloc"); CK(s.keep.alloc(nn), "alloc"); CK(s.orig.alloc(nn), "alloc");
   CK(s.aflag.alloc(nn), "alloc");
   if (n > 0) {
@@ -1666,6 +1856,12 @@ struct SkyPlan {
   JobDev J;
   bool empty;
   size_t cells, n_fix;
+  // the outer rows' tiles (fast engine) and their keys; own_*: of a row sample or shard
+  const std::vector<SkyTileRows> *tiles = nullptr;
+  const std::vector<int> *keys = nullptr;
+  bool all = false;  // tiles against every bucket, not region pair by region pair
+  std::vector<SkyTileRows> own_tiles;
+  std::vector<int> own_keys;
 };
 
 SkyView sky_view(Slot &s) {
@@ -1679,9 +1875,169 @@ SkyView sky_view(Slot &s) {
   return v;
 }
 
-SkyFast sky_fast(Slot &s) {
-  return SkyFast{s.sky_su.p, s.sky_sl.p, s.sky_sw.p, s.sky_sx.p, s.sky_ss.p, s.sky_sh.p,
-                 s.sky_sp.p};
+// Tiles of the fast sky kernel over the rows list[0 .. n_list) (cell positions
+// in cell order; null: every row) of slot s.  A tile holds up to kSkyTile rows
+// of one bucket within 0.35 of the mean redshift window (0.25: 5% more time on
+// 200k randoms, the candidates staged for fewer rows), or up to a whole one until
+// it has 32 rows; inside a bucket its size is a multiple of 32, so that no row
+// pass has idle lanes.
+void sky_tiles(const Slot &s, const int *list, int64_t n_list, std::vector<SkyTileRows> &tiles,
+               std::vector<int> &keys) {
+  tiles.clear();
+  keys.clear();
+  const float E = (float)(0.35 * s.sky_zw), Ehi = (float)s.sky_zw;
+  auto z = [&](int64_t k) { return s.hc_z[list ? list[k] : k]; };
+  int64_t i = 0;
+  for (const int4 &b : s.hc_bk) {
+    int64_t e = list ? i : b.y;
+    while (list && e < n_list && list[e] < b.y) e++;
+    while (i < e) {
+      const float z0 = z(i);
+      int64_t j = i + 1;
+      while (j < e && j - i < kSkyTile && (z(j) - z0 <= E || (j - i < 32 && z(j) - z0 <= Ehi))) j++;
+      if (j < e && j - i > 32) j -= (j - i) & 31;
+      tiles.push_back(SkyTileRows{(int)i, (int)(j - i)});
+      keys.push_back(b.z);
+      i = j;
+    }
+  }
+}
+
+// Work units of job m of a sky launch from its tiles (bucket keys `keys`): every
+// pair of a row key and a candidate key whose boxes meet, its tiles in `parts`
+// runs; or (all) every tile against all candidate buckets.  Returns the number
+// of (row key, candidate key) pairs.
+size_t sky_units(const Slot &g1, const Slot &g2, const std::vector<int> &keys, int m, int parts,
+                 int slices, double guard, bool flip, bool all, std::vector<SkyUnit> &units) {
+  auto runs = [](size_t n, auto key, auto &&f) {  // runs of equal keys
+    for (size_t a = 0; a < n;) {
+      size_t e = a + 1;
+      while (e < n && key(e) == key(a)) e++;
+      f(a, e);
+      a = e;
+    }
+  };
+  struct Key {
+    int key, bk0, bk1;
+    float4 box;
+  };
+  auto key_boxes = [&](const Slot &s, const std::vector<float4> &boxes) {
+    std::vector<Key> v;
+    runs(s.hc_bk.size(), [&](size_t b) { return s.hc_bk[b].z; }, [&](size_t a, size_t e) {
+      Key k{s.hc_bk[a].z, (int)a, (int)e, boxes[a]};
+      for (size_t b = a + 1; b < e; b++) {
+        k.box.x = std::min(k.box.x, boxes[b].x);
+        k.box.y = std::max(k.box.y, boxes[b].y);
+        k.box.z = std::min(k.box.z, boxes[b].z);
+        k.box.w = std::max(k.box.w, boxes[b].w);
+      }
+      v.push_back(k);
+    });
+    return v;
+  };
+  // k1: the tiles' keys, k2: the candidates'; the windows are g1's
+  const std::vector<Key> k1 = flip ? key_boxes(g2, g2.hc_box) : key_boxes(g1, g1.hc_bwin);
+  const std::vector<Key> k2 = flip ? key_boxes(g1, g1.hc_bwin) : key_boxes(g2, g2.hc_box);
+  const int nbk = (int)(flip ? g1 : g2).hc_bk.size();
+  if (flip) slices = 1;
+  size_t pairs = 0;
+  auto emit = [&](int t0, int t1, int key, int b0, int b1) {
+    for (int q = 0; q < parts; q++) {
+      const int a = t0 + (int)((int64_t)(t1 - t0) * q / parts);
+      const int e = t0 + (int)((int64_t)(t1 - t0) * (q + 1) / parts);
+      if (a < e)
+        for (int sl = 0; sl < slices; sl++)
+          units.push_back(SkyUnit{m, a, e, key, b0, b1, all ? 1 : 0, sl, slices});
+    }
+    pairs++;
+  };
+  size_t q1 = 0;
+  const float g = (float)(4 * guard);
+  runs(keys.size(), [&](size_t t) { return keys[t]; }, [&](size_t t0, size_t t1) {
+    const int key = keys[t0];
+    if (all) {
+      for (size_t t = t0; t < t1; t++) emit((int)t, (int)t + 1, key, 0, nbk);
+      return;
+    }
+    while (k1[q1].key != key) q1++;  // both in bucket order
+    const float4 w = k1[q1].box;
+    for (const Key &y : k2)
+      if (y.box.x <= w.y + g && y.box.y >= w.x - g && y.box.z <= w.w + g && y.box.w >= w.z - g)
+        emit((int)t0, (int)t1, key, y.bk0, y.bk1);
+  });
+  return pairs;
+}
+
+// Constants of the mixed-precision path of a sky job (SkyConst).  A bin index is
+// rint(s x + o) of a float x; it is certain when s x + o is farther from the next
+// half-integer (a bin edge) than the error bound E of the whole evaluation
+// against the reference's double value.
+void sky_consts(const cpc_ctx *c, const Slot &g1, const Slot &g2, JobDev &J) {
+  const cpc_params &p = c->p;
+  const int nrp = p.n_bins, npi = p.n_p_bin;
+  SkyConst &K = J.sk;
+  const double eps = std::ldexp(1.0, -24);
+  // window tests h - |x - c|: the coordinate, the centre and the half width are
+  // within half an ulp of their double values, x - c within another half (|x - c|
+  // is h there) and the last difference is exact near zero; doubled
+  K.guard = f_up(4.0 * ulpf(std::max({g1.sky_mag, g2.sky_mag, 1e-30})));
+  const double dcm = std::max(g1.dcmax, g2.dcmax);
+  const double damin = std::min(g1.damin, g2.damin), damax = std::max(g1.damax, g2.damax);
+  const double pe = 12 * eps * dcm + 1e-30;
+  K.pi_c = (float)(0.5 * (p.p_min + p.p_max));
+  K.pi_h = f_up(0.5 * (p.p_max - p.p_min) + pe + 2 * ulpf(std::fabs(p.p_min) + std::fabs(p.p_max)));
+  // Pi from hi + lo distances is within 2^-23 |Pi| + 2^-46 max D_C (doubled here)
+  {
+    const double Pm = std::max(std::fabs(p.p_min), std::fabs(p.p_max));
+    const double o = -p.p_min / c->ps - 0.5;
+    K.pi_s = (float)(1.0 / c->ps);
+    K.pi_o = (float)o;
+    const double E = (4 * eps * Pm + 4e-14 * dcm + 1e-30) / c->ps +
+                     4 * eps * (npi + std::fabs(o) + 1) + 1e-9;
+    K.pi_in = E < 0.5 ? f_down(0.5 - E) : -1.0f;
+    const double v0 = std::floor((0.0 - p.p_min) / c->ps);  // corel_bin (corels.cpp:26)
+    K.pi_zero = v0 >= 0 && v0 < npi ? (int)v0 : -1;
+  }
+  // r_p certainly outside, from t = chord^2 (D_A1 + D_A2)^2 of float unit vectors
+  // (chord within 4e-7): r_p < r_hi implies t < t_hi, r_p >= r_lo implies t >= t_lo
+  const double r_lo = c->thr_rp[0], r_hi = c->thr_rp[nrp];
+  {
+    const double h = 2 * r_hi + 8e-7 * damax;
+    K.t_hi = f_up(h * h * (1 + 1e-5));
+    // a clamped pair (theta < 1.42e-5) has r_p = 0, which bins when thr_0 <= 0
+    if (r_lo <= 0 && r_hi < 1e-4 * damax) K.t_hi = INFINITY;
+    K.t_lo = -1.0f;
+    if (r_lo > 0 && damin > 0 && r_lo < 0.5 * damin) {
+      const double th = r_lo / damin, l = 2 * r_lo * (1 - th * th / 24) - 8e-7 * damax;
+      if (l > 0) K.t_lo = f_down(l * l * (1 - 1e-5));
+    }
+  }
+  // r_p from the hi + lo chord: its series or asinf, the D_A sum (< 1.5e-6), and
+  // the reference's own sum = cos(theta) rounding through acos, at most 4e-7 for
+  // chords above 1e-4 (smaller ones take the FP64 path): 2.1e-6 relative
+  {
+    const double rel = 2.1e-6;
+    double E, o;
+    if (p.lin_bin) {
+      const double s = 1.0 / c->rsize;
+      o = -p.bin_r_min * s - 0.5;
+      K.rp_s = (float)(0.5 * s);
+      E = rel * p.bin_r_max * s + 6 * eps * (nrp + std::fabs(o) + p.bin_r_max * s + 1) + 1e-7;
+    } else {
+      // log2 of (2 r_p)^2: __log2f is within 2 ulp (4e-6 for |log2| < 32)
+      const double s = nrp / (2.0 * std::log2(p.bin_r_max / p.bin_r_min));
+      const double l0 = 2.0 + 2.0 * std::log2(p.bin_r_min);
+      o = -l0 * s - 0.5;
+      K.rp_s = (float)s;
+      E = s * (2 * rel / M_LN2 + 4e-6 + 4 * eps * (std::fabs(l0) + 32)) +
+          4 * eps * (nrp + std::fabs(o) + 1) + 1e-7;
+      // the exact thresholds must be the edges of this map
+      for (int k = 0; k <= nrp; k++)
+        if (!(std::fabs((2.0 + 2.0 * std::log2(c->thr_rp[k]) - l0) * s - k) < 1e-7)) E = 1.0;
+    }
+    K.rp_o = (float)o;
+    K.rp_in = E < 0.5 ? f_down(0.5 - E) : -1.0f;
+  }
 }
 
 // Plan job k of a sky launch: the corels2 rules, the bands and fixed-point
@@ -1746,36 +2102,7 @@ cpc_status sky_plan(cpc_ctx *c, cpc_pair_kind kind, int slot_g1, int slot_g2, in
   J.ps = c->ps;
   J.rsize = c->rsize;
   for (int q = 0; q <= p.n_bins; q++) J.thr[q] = c->thr_rp[q];
-  // float bands of the mixed-precision path.  r_p bin k is certain when
-  // [rp - tol, rp + tol] lies inside [A_k, B_k) (the exact thresholds rounded
-  // inwards; tol is per pair).  The float Pi differs from the reference's by at
-  // most 2^-23 |Pi| + 2^-46 max|D_C|; the Pi bands are shrunk by twice that.
-  {
-    const int nrp = p.n_bins, npi = p.n_p_bin;
-    for (int k = 0; k < nrp; k++) {
-      J.A[k] = f_up(c->thr_rp[k]);
-      J.B[k] = f_down(c->thr_rp[k + 1]);
-    }
-    J.rej_lo = f_down(c->thr_rp[0]);
-    J.rej_hi = f_up(c->thr_rp[nrp]);
-    const double dcm = std::max(g1.dcmax, g2.dcmax);
-    auto gp = [&](double v) { return 2.4e-7 * std::fabs(v) + 4e-14 * dcm + 1e-30; };
-    for (int k = 0; k < npi; k++) {
-      const double lo = c->thr_pi[k], hi = c->thr_pi[k + 1];
-      J.PA[k] = f_up(lo + gp(lo));
-      J.PB[k] = f_down(hi - gp(hi));
-    }
-    J.pi_out_lo = f_down(c->thr_pi[0] - gp(c->thr_pi[0]));
-    J.pi_out_hi = f_up(c->thr_pi[npi] + gp(c->thr_pi[npi]));
-    J.inv_ps_f = (float)(1.0 / c->ps);
-    J.tp0 = (float)(-p.p_min / c->ps);
-    J.rmin_f = (float)p.bin_r_min;
-    J.inv_rsize_f = (float)(1.0 / c->rsize);
-    if (!p.lin_bin) {
-      J.l2rmin2 = (float)(2.0 * std::log2(p.bin_r_min));
-      J.inv_lw = (float)(1.0 / (2.0 * std::log2(p.bin_r_max / p.bin_r_min) / nrp));
-    }
-  }
+  sky_consts(c, g1, g2, J);
   // fixed-point scales of the fast kernel: terms rint(v 2^S_f),
   // |v| 2^S_f <= 2^30 / (1 + 2^-12); the global sums keep a low and a high
   // 64-bit word per bin and field (2^48 terms per bin, checked after the count)
@@ -1808,33 +2135,69 @@ cpc_status sky_plan(cpc_ctx *c, cpc_pair_kind kind, int slot_g1, int slot_g2, in
   J.acc_fixh = Bf.fix.p + P.n_fix;
   J.sky1 = sky_view(g1);
   J.sky2 = sky_view(g2);
-  J.sf1 = sky_fast(g1);
-  J.sf2 = sky_fast(g2);
+  J.sf1 = g1.sky_f;
+  J.sf2 = g2.sky_f;
   CK(Bf.hq.alloc(kSkyHostQueue), "alloc host queue");
   CK(Bf.hq_n.alloc(1), "alloc");
   CK(cudaMemsetAsync(Bf.hq_n.p, 0, sizeof(unsigned long long), st), "memset");
+  J.sk.hist_smem = sky_hist_fits(J.corel, J.unit_w, p.n_bins * p.n_p_bin) ? 1 : 0;
   J.hq = Bf.hq.p;
   J.hq_n = Bf.hq_n.p;
-  // a row sample: the redshift-ordered positions of the g1 rows whose input
-  // index i satisfies i % rs == ro (the outer rows corels2 would count); a
-  // work shard of the fast engine (cpc_set_shard): the positions k with
-  // k % n_shards == shard
+  // the outer rows as tiles.  A row sample (input index i with i % rs == ro) or a
+  // work shard of the fast engine (cpc_set_shard: redshift-ordered positions k
+  // with k % n_shards == shard) lists its rows first.
+  // Against a g2 of at most half as many galaxies (data against randoms) the
+  // tiles hold g2's and the candidates are g1's, whose runs then fill the warps.
   J.row_list = nullptr;
-  J.n_rows = g1.n;
-  const int W = engine == CPC_ENGINE_FAST ? c->n_shards : 1;
-  if (engine == CPC_ENGINE_FAST) {  // the rows in the kernel's order (hs_rorder)
-    std::vector<int> rows;
-    rows.reserve((size_t)(g1.n / std::max<int64_t>(1, rs) / W + 1));
-    for (const int i : g1.hs_rorder)
-      if ((W <= 1 || i % W == c->shard) && (rs <= 1 || ((g1.hs_orig[i] - ro) % rs) == 0))
-        rows.push_back(i);
-    CK(Bf.rows.alloc(std::max<size_t>(rows.size(), 1)), "alloc row sample");
-    if (!rows.empty())
-      CK(cudaMemcpyAsync(Bf.rows.p, rows.data(), sizeof(int) * rows.size(),
+  const int W = c->n_shards;
+  if (engine == CPC_ENGINE_FAST) {
+    // A region pair's unit pays for itself from about 40 pairs per bin on (counts
+    // alone, whose pairs cost one global add: 300); below, and with too many keys
+    // to pair up on the host, the units are tiles against every bucket.  RsRd of
+    // 15k randoms in 100 regions (8 per bin): 0.95 ms by pairs, 0.30 by tiles; of
+    // 200k (1,400): 14.8 and 21.0.  SRd of 8k x 40k (11): 2.08 and 1.43; of 20k x
+    // 200k (140): 7.1 and 15.2.
+    {
+      const double k1 = std::max(1, g1.sky_nkey), k2 = std::max(1, g2.sky_nkey);
+      const double rows = (double)g1.n / (double)std::max<int64_t>(1, rs) / W;
+      P.all = rows / k1 * ((double)g2.n / k2) * g2.sky_fz <
+                  (J.corel == COREL_DD ? 300.0 : 40.0) * p.n_bins * p.n_p_bin ||
+              k1 * k2 > 4e6;
+    }
+    if (W <= 1 && rs <= 1) {
+      J.sk.flip = !P.all && !auto_mode && g1.sky_mono && g2.n * 2 <= g1.n ? 1 : 0;
+      Slot &gt = J.sk.flip ? g2 : g1;
+      if (gt.hc_tiles.empty()) sky_tiles(gt, nullptr, gt.n, gt.hc_tiles, gt.hc_tile_key);
+      P.tiles = &gt.hc_tiles;
+      P.keys = &gt.hc_tile_key;
+    } else {
+      std::vector<int> rows;
+      rows.reserve((size_t)(g1.n / std::max<int64_t>(1, rs) / W + 1));
+      for (int64_t q = 0; q < g1.n; q++) {
+        const int i = g1.hc_zidx[q];
+        if ((W <= 1 || i % W == c->shard) && (rs <= 1 || ((g1.hs_orig[i] - ro) % rs) == 0))
+          rows.push_back((int)q);
+      }
+      sky_tiles(g1, rows.data(), (int64_t)rows.size(), P.own_tiles, P.own_keys);
+      P.tiles = &P.own_tiles;
+      P.keys = &P.own_keys;
+      CK(Bf.rows.alloc(std::max<size_t>(rows.size(), 1)), "alloc row sample");
+      if (!rows.empty())
+        CK(cudaMemcpyAsync(Bf.rows.p, rows.data(), sizeof(int) * rows.size(),
+                           cudaMemcpyHostToDevice, st), "H2D");
+      CK(cudaStreamSynchronize(st), "sync");  // rows is a host temporary
+      J.row_list = Bf.rows.p;
+    }
+    CK(Bf.tiles.alloc(std::max<size_t>(P.tiles->size(), 1)), "alloc tiles");
+    if (!P.tiles->empty())
+      CK(cudaMemcpyAsync(Bf.tiles.p, P.tiles->data(), sizeof(SkyTileRows) * P.tiles->size(),
                          cudaMemcpyHostToDevice, st), "H2D");
-    CK(cudaStreamSynchronize(st), "sync");  // rows is a host temporary
-    J.row_list = Bf.rows.p;
-    J.n_rows = (int64_t)rows.size();
+    J.tiles = Bf.tiles.p;
+    CK(Bf.xq.alloc(kSkyExactQueue), "alloc undecided pairs");
+    CK(Bf.xq_n.alloc(1), "alloc");
+    CK(cudaMemsetAsync(Bf.xq_n.p, 0, sizeof(unsigned long long), st), "memset");
+    J.xq = Bf.xq.p;
+    J.xq_n = Bf.xq_n.p;
   }
   return CPC_OK;
 }
@@ -1911,21 +2274,17 @@ cpc_status sky_finish(cpc_ctx *c, SkyPlan &P, size_t k, cpc_engine engine, float
 // one launch of the chunked warp kernel, then the fixed-point blocks are
 // converted and each job's host edge tier runs; the FP64 engine runs the plain
 // kernel per job.
-constexpr int kSkyRowsPerChunk = 64;
 cpc_status sky_run(cpc_ctx *c, std::vector<SkyPlan> &plans, cpc_engine engine) {
   const cpc_params &p = c->p;
   cudaStream_t st = c->st;
   cpc_status st_;
   if ((st_ = ensure_scratch(c, 1, plans.size())) != CPC_OK) return st_;
   std::vector<JobDev> jd;
-  std::vector<long long> chunk0(1, 0);
   std::vector<size_t> idx;  // plan of each launched job
   for (size_t k = 0; k < plans.size(); k++) {
     if (plans[k].empty) continue;
     jd.push_back(plans[k].J);
     idx.push_back(k);
-    const long long nr = plans[k].J.n_rows;
-    chunk0.push_back(chunk0.back() + (nr + kSkyRowsPerChunk - 1) / kSkyRowsPerChunk);
   }
   // bound on |sum_gpu - sum_libm|: cos differs by <= 3 ulp (CUDA 2 + C library
   // 1), one more ulp from each of the product and the sum, doubled
@@ -1942,21 +2301,48 @@ cpc_status sky_run(cpc_ctx *c, std::vector<SkyPlan> &plans, cpc_engine engine) {
         c->launches += 1;
       }
     } else {
-      CK(c->d_chunk0.alloc(chunk0.size()), "alloc chunk table");
-      CK(c->d_chunk_ctr.alloc(1), "alloc");
-      CK(cudaMemcpyAsync(c->d_chunk0.p, chunk0.data(), sizeof(long long) * chunk0.size(),
-                         cudaMemcpyHostToDevice, st), "H2D");
-      CK(cudaMemsetAsync(c->d_chunk_ctr.p, 0, sizeof(unsigned long long), st), "memset");
-      const float rp_lo_f = f_down(c->thr_rp[0]), rp_hi_f = f_up(c->thr_rp[p.n_bins]);
-      CK(launch_sky_warp(c->d_jobs.p, c->d_chunk0.p, (int)jd.size(), chunk0.back(),
-                         kSkyRowsPerChunk, c->d_chunk_ctr.p, kSkyHostQueue, esum, rp_lo_f,
-                         rp_hi_f, c->thr_rp[0] <= 0.0 ? 1 : 0, p.n_bins, p.n_p_bin, c->sm_count,
-                         c->sky_blocks_per_sm, st), "sky kernel");
+      // the units of every job, split until each block finds about six of them:
+      // first a key pair's tiles, then the redshift range of its candidates
+      size_t hist_words = 1;
+      int set = 0;
+      std::vector<SkyUnit> units;
+      auto build = [&](int parts, int slices) {
+        size_t pairs = 0;
+        units.clear();
+        for (size_t m = 0; m < jd.size(); m++) {
+          const SkyPlan &P = plans[idx[m]];
+          pairs += sky_units(c->slots[P.s1], c->slots[P.s2], *P.keys, (int)m, parts, slices,
+                             jd[m].sk.guard, jd[m].sk.flip != 0, P.all, units);
+        }
+        return pairs;
+      };
+      for (size_t m = 0; m < jd.size(); m++) {
+        const int cl = jd[m].corel;
+        set = std::max(set, cl == COREL_DD ? 0 : cl == COREL_SD ? 1 : 2);
+        if (jd[m].sk.hist_smem)
+          hist_words = std::max(hist_words, sky_hist_words(cl, jd[m].unit_w, p.n_bins * p.n_p_bin));
+      }
+      const size_t want = (size_t)c->sm_count * 24;
+      const size_t pairs = build(1, 1);
+      if (pairs && units.size() < want) {
+        const int parts = (int)((want + pairs - 1) / pairs);
+        build(parts, 1);
+        if (units.size() < want / 2)
+          build(parts, (int)std::min<size_t>(4, want / std::max<size_t>(1, units.size())));
+      }
+      CK(c->d_sky_units.alloc(units.size()), "alloc units");
+      CK(c->d_sky_ctr.alloc(1), "alloc");
+      if (!units.empty())
+        CK(cudaMemcpyAsync(c->d_sky_units.p, units.data(), sizeof(SkyUnit) * units.size(),
+                           cudaMemcpyHostToDevice, st), "H2D");
+      CK(cudaMemsetAsync(c->d_sky_ctr.p, 0, sizeof(unsigned long long), st), "memset");
+      CK(launch_sky_tile(c->d_jobs.p, c->d_sky_units.p, (int)units.size(), set, hist_words,
+                         c->d_sky_ctr.p, kSkyHostQueue, esum, c->sm_count, st), "sky kernel");
       c->launches += 1;
       for (size_t m = 0; m < jd.size(); m++) {
         const SkyPlan &P = plans[idx[m]];
-        CK(launch_fix_to_sums((int64_t)P.n_fix, jd[m].acc_fix, jd[m].acc_fixh, jd[m].acc_sums,
-                              c->d_jobs.p + m, st), "fixed-point sums");
+        CK(launch_sky_finish((int64_t)P.n_fix, jd[m].acc_fix, jd[m].acc_fixh, jd[m].acc_sums,
+                             c->d_jobs.p + m, kSkyHostQueue, esum, st), "fixed-point sums");
         c->launches += 1;
       }
     }
@@ -2018,8 +2404,6 @@ cpc_status cpc_create(cpc_ctx **out, const cpc_params *params) try {
   if (e != cudaSuccess) return cuda_fail(nullptr, e, "cudaGetDevice");
   e = cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, c->device);
   if (e != cudaSuccess) return cuda_fail(nullptr, e, "device attribute");
-  if (const char *ev = std::getenv("CPC_SKY_BLOCKS_PER_SM"))
-    c->sky_blocks_per_sm = std::atoi(ev) >= 3 ? 3 : 2;
   if (const char *ev = std::getenv("CPC_TWIN")) c->twin_on = std::atoi(ev) != 0 ? 1 : 0;
   e = cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking);
   if (e != cudaSuccess) return cuda_fail(nullptr, e, "stream");

@@ -78,15 +78,52 @@ struct SkyView {
 };
 
 // float views of a sky catalogue for the fast kernel (hi = float(v),
-// lo = float(v - hi), so hi + lo carries about 48 bits of v)
+// lo = float(v - hi), so hi + lo carries about 48 bits of v), in cell order:
+// sorted by (jackknife region, keep flag, sky cell of the region, redshift)
 struct SkyFast {
   const float4 *su;  // unit vector (cos d cos a, cos d sin a, sin d) hi parts, D_A
   const float4 *sl;  // unit vector lo parts, D_C lo part
-  const float4 *sw;  // RA, Dec hi parts, redshift, D_C hi part
+  const float4 *sw;  // RA, Dec hi parts, scaled redshift, D_C hi part
   const float4 *sx;  // RA, Dec lo parts, Dec in radians, weight
   const float4 *ss;  // w e1, w e2 hi parts, then their lo parts
   const float4 *sh;  // cos(Dec / 2) hi, lo, sin(Dec / 2) hi, lo (Dec in radians)
   const float2 *sp;  // phi, w lo part
+  const float4 *wb;  // row window: centre and half width in RA, in Dec (NaN bounds: 0, inf)
+  const float2 *wz;  // row window: centre and half width in scaled redshift
+  const float *zf;   // scaled redshift
+  const float *dl;   // D_C - hi - lo: with it the three parts are D_C exactly
+  const int *zidx;   // redshift-ordered position of each cell-ordered row
+  const int4 *bk;    // buckets: first row, end row, 2 region + keep flag
+  const float4 *bk_box;  // their RA low, high, Dec low, high
+  const float4 *bk_win;  // the unions of their rows' windows, likewise
+  int n_bk;
+};
+
+// constants of a sky job's mixed-precision path (set-up in capi.cu)
+struct SkyConst {
+  float guard;             // a window test within it of a bound is undecided
+  float pi_c, pi_h;        // Pi certainly outside the bins beyond pi_h from pi_c
+  float t_lo, t_hi;        // c^2 (D_A1 + D_A2)^2 outside: r_p certainly outside the bins
+  float pi_s, pi_o, pi_in; // Pi bin: rint(pi_s Pi + pi_o), certain within pi_in of it
+  float rp_s, rp_o, rp_in; // r_p bin: rint(rp_s x + rp_o), x = log2 (2 r_p)^2 or 2 r_p (linear)
+  int pi_zero;             // the exact bin of Pi = 0 (-1: none)
+  int hist_smem;           // the block histogram fits shared memory
+  int flip;                // the tiles hold g2 galaxies, the candidates are g1's
+};
+// g1 rows per tile of the fast sky kernel: three row passes; 128 rows leave no
+// room for a third block per SM beside the shape histograms
+constexpr int kSkyTile = 96;
+
+// A tile of the fast sky kernel: rows start .. start + count - 1 of the job's row
+// list (or of the cell-ordered catalogue), all in one bucket.
+struct SkyTileRows {
+  int start, count;
+};
+// One work unit of the fast sky kernel: tiles [tile0, tile1) of a job, all of
+// one bucket key, against the candidate buckets [bk0, bk1) (all: of many
+// regions), redshift slice `slice` of n_slices.
+struct SkyUnit {
+  int job, tile0, tile1, key, bk0, bk1, all, slice, n_slices;
 };
 
 struct JobDev {
@@ -135,8 +172,12 @@ struct JobDev {
   unsigned long long *acc_fix, *acc_fixh;
   SkyView sky1, sky2;                  // sky catalogues g1, g2 (FP64 path of the fast kernel)
   SkyFast sf1, sf2;                    // their float views (fast sky kernel)
-  const int *row_list;                 // sky row sample: the g1 rows counted, else null
-  int64_t n_rows;                      // rows in row_list
+  SkyConst sk;
+  const int *row_list;                 // sky row sample: the g1 rows (cell positions), else null
+  const SkyTileRows *tiles;            // the fast sky kernel's row tiles of this job
+  int2 *xq;                            // sky pairs left to the FP64 path (cell positions;
+                                       // ~i1: the window test is undecided too)
+  unsigned long long *xq_n;            // their number
   int2 *hq;                            // sky host-tier queue of this job
   unsigned long long *hq_n;            // its length
 };

@@ -196,6 +196,26 @@ DF_HD void df_to_fixed15(df32 v, float qs, unsigned &lo15, unsigned &hi) {
   lo15 = (unsigned)u & 0x7FFFu;
   hi = (unsigned)(u >> 15);
 }
+// The same integer as two biased words, for |h + l| 2^S < 2^30: the float bits
+// of M + rint(t 2^-15) and of M + the signed rest, t = (h + l) 2^S.  The words are
+// summed as they are (mod 2^32); the reader of n of them subtracts n kMagicBits.
+// This saves the recombination and the split of df_to_fixed15.
+constexpr float kMagic = 12582912.0f;            // 1.5 * 2^23
+constexpr unsigned kMagicBits = 0x4B400000u;     // its bits
+DF_HD unsigned magic_bits(float x_plus_magic) { return (unsigned)magic_int(x_plus_magic) + kMagicBits; }
+DF_HD void df_to_words(df32 v, float qs, unsigned &hi, unsigned &lo) {
+  const float t = rn_mul(v.h, qs);                      // exact (power of two)
+  const float a = rn_fma(t, 3.0517578125e-05f, kMagic);
+  const float r = rn_fma(rn_sub(a, kMagic), -32768.0f, t);  // exact, |r| <= 2^14
+  hi = magic_bits(a);
+  lo = magic_bits(rn_add(rn_fma(v.l, qs, r), kMagic));
+}
+DF_HD void f_to_words(float v, float qs, unsigned &hi, unsigned &lo) {
+  const float t = rn_mul(v, qs);
+  const float a = rn_fma(t, 3.0517578125e-05f, kMagic);
+  hi = magic_bits(a);
+  lo = magic_bits(rn_add(rn_fma(rn_sub(a, kMagic), -32768.0f, t), kMagic));
+}
 // the same for a float term (one rounding conversion)
 DF_HD void f_to_fixed15(float v, float qs, unsigned &lo15, unsigned &hi) {
 #ifdef __CUDA_ARCH__

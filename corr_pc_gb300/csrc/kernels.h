@@ -112,19 +112,21 @@ cudaError_t launch_plain_fp64(const JobDev *job, const DCat &a, const DCat &b, c
 // Sky pairs (coordinates 0) in FP64; pairs whose r_p may bin differently with
 // the C library's trigonometry are appended to hq (host edge tier).
 constexpr unsigned long long kSkyHostQueue = 1ull << 22;
-// (SkyFast, the float views of a sky catalogue, is declared in cpc_device.cuh)
-// The fast sky kernel over n_jobs jobs (pair types) in one launch: job k's rows
-// are dealt in chunks chunk0[k] .. chunk0[k+1]-1 of rows_per_chunk rows;
-// chunk_ctr (zeroed) is the chunk queue.  Every job has the same binning.
-// blocks_per_sm: the register bound the kernel is compiled for (2 or 3).
-cudaError_t launch_sky_warp(const JobDev *jobs, const long long *chunk0, int n_jobs,
-                            long long n_chunks, int rows_per_chunk,
-                            unsigned long long *chunk_ctr, unsigned long long hq_cap, double esum,
-                            float rp_lo_f, float rp_hi_f, int zero_bin, int nrp, int npi,
-                            int sm_count, int blocks_per_sm, cudaStream_t st);
-cudaError_t launch_fix_to_sums(int64_t n, const unsigned long long *lo,
-                               const unsigned long long *hi, double *sums, const JobDev *job,
-                               cudaStream_t st);
+constexpr unsigned long long kSkyExactQueue = 1ull << 20;  // undecided pairs of a job
+// (SkyFast, SkyConst and SkyUnit are declared in cpc_device.cuh)
+// The fast sky kernel over the units of every job (pair types) of one launch;
+// ctr (zeroed) is the unit queue.  set: 0 every job counts (density_density),
+// 1 shape_density too, 2 shape_shape too; hist_words: the largest block
+// histogram of the jobs that keep one in shared memory.
+cudaError_t launch_sky_tile(const JobDev *jobs, const SkyUnit *units, int n_units, int set,
+                            size_t hist_words, unsigned long long *ctr,
+                            unsigned long long hq_cap, double esum, int sm_count,
+                            cudaStream_t st);
+size_t sky_hist_words(int corel, int unit_w, int ncell);
+bool sky_hist_fits(int corel, int unit_w, int ncell);
+cudaError_t launch_sky_finish(int64_t n, const unsigned long long *lo,
+                              const unsigned long long *hi, double *sums, const JobDev *job,
+                              unsigned long long hq_cap, double esum, cudaStream_t st);
 cudaError_t launch_sky_fp64(const JobDev *job, const SkyView &a, const SkyView &b, int2 *hq,
                             unsigned long long *hq_n, unsigned long long hq_cap, double esum,
                             cudaStream_t st);

@@ -19,24 +19,34 @@
 // within esum of the reference's clamp at 0.9999999999, is appended to a host
 // queue and binned there with the C library.  All other pairs are binned here
 // against the exact host-derived thresholds, so the integer counts equal the
-// reference's.  Shape sums use CUDA's atan/cos/sin (within 1e-6).
+// reference's.  D_C is a row of the distance table, so 0.2% of the pairs have
+// Pi = 0 exactly, often a bin edge: the fast kernel recognises them by equal
+// D_C (three float parts) and takes their bin from the host.  Shape sums use CUDA's atan/cos/sin (within 1e-6).
 //
 // Two kernels:
 //  * sky_fp64_kernel -- the plain FP64 kernel: one thread per g1 row, every
 //    window pair through the FP64 path, global atomics (CPC_ENGINE_FP64).
-//  * sky_warp_kernel -- the fast kernel (CPC_ENGINE_FAST): one warp per g1 row
-//    (dynamic row queue), lanes take consecutive candidates of the row's
-//    redshift range, their float views prefetched into per-warp shared stages
-//    with asynchronous copies one 32-candidate stage ahead; FP32 definite-in/definite-out
-//    window tests (ambiguous ones re-tested in double); FP32 prefilters that
-//    reject pairs certainly outside the Pi range or certainly outside
-//    [thr_0, thr_nrp) in r_p (the chord |u1 - u2| of float unit vectors with a
-//    rigorous error bound); survivors are compacted into a per-warp queue and
+//  * sky_tile_kernel -- the fast kernel (CPC_ENGINE_FAST).  Catalogues are held
+//    in cell order (jackknife region, keep flag, sky cell of the region,
+//    redshift).  A unit is a run of row tiles of one region against the buckets
+//    of one partner region: whole buckets outside the tile's windows are
+//    skipped, a run of the others is cut to the tile's redshift range, and the
+//    block histogram holds one region pair, so the jackknife attribution costs
+//    a flush and nothing per pair.  Each warp stages its own candidates,
+//    broadcasts them to 32 rows at a time (one per lane) and keeps a bit per
+//    test; the surviving pairs are queued by a prefix sum of the bit counts and
 //    evaluated 32 at a time with every lane busy: Pi and r_p in FP32 from hi+lo
-//    floats with per-pair error bounds, FP32 shape values when both bins are
-//    certain, the FP64 path (and behind it the host tier) otherwise.  The main
-//    histogram lives in shared memory (FP64 atomics) and is flushed once per
-//    block.
+//    floats, their bins from the linear maps of Pi and log2 r_p with one error
+//    bound each (no table lookups), compensated shape terms (pair_df.cuh).
+//    Undecided windows and bins go to a queue that sky_finish_kernel evaluates
+//    in FP64 (behind it the host tier).
+//
+//    Bound by instruction issue (77% of issue slots on counts: 34 instructions
+//    per 32 window tests, 120 per 32 binned pairs) with the shared-memory pipe
+//    at 46%.  Four terms of 20k data and 200k randoms, 100 regions, 1.44e9
+//    binned pairs: 111.6 ms before (a warp per row scanning its whole redshift
+//    range, every corel in one 128-register kernel, the partner's region by
+//    global atomics per pair), 32.6 ms now; counts alone (RsRd) 8.0e10 pairs/s.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -44,6 +54,7 @@
 #include <climits>
 
 #include "cpc_device.cuh"
+#include "field_map.cuh"
 #include "kernels.h"
 #include "pair_df.cuh"
 
@@ -139,14 +150,19 @@ sky_fp64_kernel(const JobDev *__restrict__ jobp, SkyView a, SkyView b, int2 *hq,
 
 constexpr int kSkyThreads = 256;
 constexpr int kSkyWarps = kSkyThreads / 32;
-constexpr int kSkyQ = 64;
-constexpr int kSkyAhead = 1;  // candidate stages copied ahead of the tested one
-
-struct SkyRow {
-  int64_t i;
-  double ra, dec, dc, da, sd, cd, rar, decr, w, e1, e2, phi;
-  int jk, keep;
-};
+// candidate slots per warp: 32 for launches of counts alone; with shapes 16, and
+// 24 for the counts beside them, so that three blocks fit an SM
+__host__ __device__ constexpr int sky_cand(int set, bool shapes) {
+  return set == 0 ? 32 : shapes ? 16 : 24;
+}
+constexpr int kSkySeg = 256;            // candidate buckets taken at a time
+// per-warp ring of pairs awaiting the heavy step: a pass over cand - 1 candidates
+// adds at most 32 of them each to fewer than 32 left over
+__host__ __device__ constexpr int sky_ring(int cand) { return 32 * cand; }
+// pairs a block may add to a bin between flushes: |u| < 2^30 splits into words
+// of at most 2^15, so 2^16 of them stay within a signed 32-bit word
+constexpr int kSkyFlushPairs = 1 << 16;
+constexpr unsigned kSkyEdge = 0x8000u;  // queue entry: the window test is undecided
 
 // Jackknife attribution of a sky pair: jk_check_sky (jk.cpp:53-57), each
 // region whose galaxy has jk_prob >= 0.5 (same region: g1's only).
@@ -181,12 +197,11 @@ __device__ __forceinline__ void sky_accumulate_exact(const JobDev &J, int r1, in
   }
 }
 
-// Terms of a pair from the mixed-precision path as fixed-point integers
-// Add x (a term rint(v 2^S_f), or a block's partial sum of terms) to the
-// global fixed-point sum of one bin and field: its low 15 bits (0 .. 2^15 - 1)
-// into word lo, its arithmetic shift x >> 15 into word hi.  Terms have
-// |x| < 2^30 and a block's partial sum holds fewer than 2^33 of them, so a bin
-// takes 2^48 terms before either word can overflow; the value is
+// Add x (a term rint(v 2^S_f), |v| 2^S_f < 2^30, or a block's partial sum of
+// terms) to the global fixed-point sum of one bin and field: its low 15 bits
+// (0 .. 2^15 - 1) into word lo, its arithmetic shift x >> 15 into word hi.
+// Terms have |x| < 2^30 and a block's partial sum holds fewer than 2^33 of them,
+// so a bin takes 2^48 terms before either word can overflow; the value is
 // hi 2^15 + lo (fix_to_sums_kernel).
 __device__ __forceinline__ void fix_add(unsigned long long *lo, unsigned long long *hi,
                                         long long x) {
@@ -196,549 +211,773 @@ __device__ __forceinline__ void fix_add(unsigned long long *lo, unsigned long lo
   if (h) atomicAdd(hi, (unsigned long long)h);
 }
 
-// rint(v 2^S_f), |v| 2^S_f < 2^30 (S_f from bounds on |v|): the fields whose
-// sums cancel from double-float terms vd, the others from float terms v; added
-// as 64-bit integers: the main histogram in shared memory (SMEM) or in the
-// global fixed-point block, the regions in the global fixed-point block.
-// Field 0 (the weight) is skipped when every weight is 1 (wt_num = count).
-template <bool SMEM>
-__device__ __forceinline__ void sky_accumulate_fixed(const JobDev &J, int r1, int keep1, int r2,
-                                                     int keep2, int64_t cell, const float *v,
-                                                     const df32 *vd, int nf, const float *s_qs,
-                                                     unsigned long long *s_num,
-                                                     unsigned long long *s_fix) {
-  const int f0 = J.unit_w ? 1 : 0;
-  const int corel = J.corel;
-  auto fx = [&](int q) {
-    return (long long)(df_field(corel, q) ? df_to_int(vd[q], s_qs[q])
-                                          : __float2int_rn(v[q] * s_qs[q]));
-  };
-  auto nz = [&](int q) { return df_field(corel, q) ? vd[q].h != 0.0f : v[q] != 0.0f; };
-  atomicAdd(SMEM ? &s_num[cell] : &J.acc_num[cell], 1ull);
-#pragma unroll
-  for (int q = 0; q < kNF; q++) {  // constant indices: v stays in registers
-    if (q < f0 || q >= nf || !nz(q)) continue;
-    const int64_t o = cell * kNF + q;
-    if (SMEM) atomicAdd(&s_fix[o], (unsigned long long)fx(q));
-    else fix_add(&J.acc_fix[o], &J.acc_fixh[o], fx(q));
-  }
-  if (!J.do_jk) return;
-  const int64_t hstride = (int64_t)J.nrp * J.npi;
-  int rs[2];
-  const int nr = sky_regions(r1, keep1, r2, keep2, rs);
-  for (int t = 0; t < nr; t++) {
-    const int64_t hc = (int64_t)(1 + rs[t]) * hstride + cell;
-    atomicAdd(&J.acc_num[hc], 1ull);
-    unsigned long long *sj = J.acc_fix + hc * kNF, *sh = J.acc_fixh + hc * kNF;
-    if (f0 == 0 && v[0] != 0.0f) fix_add(&sj[0], &sh[0], fx(0));
-    if (J.which_corr == 0 || nf == 1) continue;
-#pragma unroll
-    for (int q = 1; q < kNF; q += 2)
-      if (nz(q)) fix_add(&sj[q], &sh[q], fx(q));
-  }
-}
-
 // FP64 path of one window pair whose Pi and r_p may fall in the bins: exact
-// Pi bin, great-circle r_p, ambiguity test, values and accumulation.
-__device__ __noinline__ void sky_pair_fp64(const JobDev &J, int64_t i, int64_t j, int2 *hq,
-                                           unsigned long long *hq_n, unsigned long long hq_cap,
-                                           double esum) {
+// Pi bin, great-circle r_p, ambiguity test, values and accumulation.  i, j:
+// redshift-ordered positions.
+__device__ __noinline__ void sky_pair_fp64(const JobDev &J, int64_t i, int64_t j,
+                                           unsigned long long hq_cap, double esum) {
   const SkyView &a = J.sky1, &b = J.sky2;
-  SkyRow r;
-  r.i = i;
-  r.ra = a.d.x[i]; r.dec = a.d.y[i]; r.dc = a.dc[i]; r.da = a.da[i];
-  r.sd = a.sd[i]; r.cd = a.cd[i]; r.rar = a.rar[i]; r.decr = a.decr[i];
-  r.w = a.d.w[i]; r.e1 = a.d.e1[i]; r.e2 = a.d.e2[i]; r.phi = a.d.phi[i];
-  r.jk = a.d.jk[i]; r.keep = a.d.keep[i];
-  const double dP = __dsub_rn(b.dc[j], r.dc);
+  const double dP = __dsub_rn(b.dc[j], a.dc[i]);
   const double v2 = floor(__ddiv_rn(__dsub_rn(dP, J.pmin), J.ps));
   if (!(v2 >= 0.0) || v2 >= (double)J.npi) return;
-  const double cdel = cos(__dsub_rn(r.rar, b.rar[j]));
-  const double sum = __dadd_rn(__dmul_rn(r.sd, b.sd[j]), __dmul_rn(__dmul_rn(r.cd, b.cd[j]), cdel));
+  const double cdel = cos(__dsub_rn(a.rar[i], b.rar[j]));
+  const double sum =
+      __dadd_rn(__dmul_rn(a.sd[i], b.sd[j]), __dmul_rn(__dmul_rn(a.cd[i], b.cd[j]), cdel));
   const double kClamp = 0.9999999999;
   const double kEps = 2.220446049250313e-16;
   bool amb = fabs(sum - kClamp) <= esum;
   double daR = 0.0, tol = 0.0;
   if (!(sum > kClamp)) {
     const double th = acos(sum);
-    daR = __ddiv_rn(__dmul_rn(th, __dadd_rn(r.da, b.da[j])), 2.0);
+    daR = __ddiv_rn(__dmul_rn(th, __dadd_rn(a.da[i], b.da[j])), 2.0);
     const double rel = esum / fmax(sin(th) * th, 1e-300) + 8.0 * kEps;
     tol = 2.0 * daR * rel;
   }
   const int k = thr_count(J, daR);
   if (!amb && tol > 0.0) amb = thr_count(J, daR - tol) != k || thr_count(J, daR + tol) != k;
   if (amb) {
-    const unsigned long long q = atomicAdd(hq_n, 1ull);
-    if (q < hq_cap) hq[q] = make_int2((int)r.i, (int)j);
+    const unsigned long long q = atomicAdd(J.hq_n, 1ull);
+    if (q < hq_cap) J.hq[q] = make_int2((int)i, (int)j);
     return;
   }
   if (k < 1 || k > J.nrp) return;
-  const double wt = __dmul_rn(r.w, b.d.w[j]);
+  const double wt = __dmul_rn(a.d.w[i], b.d.w[j]);
   double theta = 0.0;
   if (J.corel != COREL_DD)
-    theta = atan((b.d.y[j] - r.dec) / ((b.d.x[j] - r.ra) * cos((r.decr + b.decr[j]) / 2.0)));
+    theta = atan((b.d.y[j] - a.d.y[i]) /
+                 ((b.d.x[j] - a.d.x[i]) * cos((a.decr[i] + b.decr[j]) / 2.0)));
   double f[kNF];
-  pair_values(J.corel, J.gws, wt, theta, PairGal{r.e1, r.e2, r.phi},
+  pair_values(J.corel, J.gws, wt, theta, PairGal{a.d.e1[i], a.d.e2[i], a.d.phi[i]},
               PairGal{b.d.e1[j], b.d.e2[j], b.d.phi[j]}, f);
-  sky_accumulate_exact(J, r.jk, r.keep, b.d.jk[j], b.d.keep[j], (int64_t)(k - 1) * J.npi + (int)v2,
-                       f);
+  sky_accumulate_exact(J, a.d.jk[i], a.d.keep[i], b.d.jk[j], b.d.keep[j],
+                       (int64_t)(k - 1) * J.npi + (int)v2, f);
 }
 
-// the row's float quantities for the mixed-precision path
-struct SkyRowF {
-  float4 u, ul, w, x, s, h;  // su, sl, sw, sx, ss, sh of the row
-  float2 p;                  // sp of the row
+// A pair the mixed-precision path leaves undecided (cell positions i1, j2): the
+// exact double window first when that test is the undecided one (edge), then
+// the FP64 path.
+__device__ __noinline__ void sky_pair_exact(const JobDev &J, int i1, int j2, bool edge,
+                                            unsigned long long hq_cap, double esum) {
+  const int64_t i = J.sf1.zidx[i1], j = J.sf2.zidx[j2];
+  if (edge) {
+    const double *win = J.sky1.win;
+    const int64_t n1 = J.sky1.d.n;
+    const double z2 = J.sky2.d.z[j], dec2 = J.sky2.d.y[j], ra2 = J.sky2.d.x[j];
+    if (z2 < win[i] || z2 > win[n1 + i]) return;
+    if (dec2 > win[5 * n1 + i] || dec2 < win[4 * n1 + i]) return;
+    if (ra2 < win[2 * n1 + i] || ra2 > win[3 * n1 + i]) return;  // NaN bounds pass
+    atomicAdd(&J.counters[1], 1ull);
+  }
+  sky_pair_fp64(J, i, j, hq_cap, esum);
+}
+
+// Undecided pairs (about 1 in 10^4) are queued and evaluated by
+// sky_finish_kernel with every lane busy: evaluated here, one lane of a warp at
+// a time, they kept the FP64 pipe 62% busy and took half of the kernel's time.
+// Past the queue's end they are evaluated here all the same.
+__device__ __forceinline__ void sky_undecided(const JobDev &J, int i1, int j2, bool edge,
+                                              unsigned long long hq_cap, double esum) {
+  const unsigned long long pos = atomicAdd(J.xq_n, 1ull);
+  if (pos < kSkyExactQueue) J.xq[pos] = make_int2(edge ? ~i1 : i1, j2);
+  else sky_pair_exact(J, i1, j2, edge, hq_cap, esum);
+}
+
+// first index in [lo, hi) that is not below (below(i): true, then false)
+template <class P>
+__device__ __forceinline__ int sky_lower_bound(const P &below, int lo, int hi) {
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (below(mid)) lo = mid + 1; else hi = mid;
+  }
+  return lo;
+}
+
+// Static shared memory of a block.
+struct SkyShared {
+  int unit;
+  int wcnt[kSkyWarps];
+  float red[kSkyTile / 32][6];
+  int seg_a[kSkySeg], seg_key[kSkySeg], seg_pre[kSkySeg + 1];
+  int key[kSkyThreads];     // bucket key of each staged candidate
+  // tile rows, then candidate slots: cell position, third part of D_C (SkyFast::dl)
+  int pos[kSkyTile + kSkyThreads];
+  float d3[kSkyTile + kSkyThreads];
+  int rorig[kSkyTile];      // corels1: input row of each tile row
+  float qs[kNF];            // fixed-point scales of the unit's job
+  SkyConst k;               // and its constants
 };
 
-// estimated bin index confirmed against definite bands: the bin, -1 certainly
-// outside, -2 undecided.  band k is [lo_k, hi_k) in the estimate's units.
-__device__ __forceinline__ int band_bin(float v, float tol, int est, int n, const float *lo,
-                                        const float *hi, float rej_lo, float rej_hi) {
-  if (v + tol < rej_lo || v - tol >= rej_hi) return -1;
-  est = min(max(est, 0), n - 1);
-  for (int d = 0; d < 3; d++) {
-    const int k = d == 0 ? est : d == 1 ? est - 1 : est + 1;
-    if (k < 0 || k >= n) continue;
-    if (v - tol >= lo[k] && v + tol < hi[k]) return k;
-  }
-  return -2;
+// Dynamic shared memory before the histogram: the views of the tile rows and of
+// the candidate slots (16-byte views su, sw, sl, sx; the windows; with shapes ss,
+// sh, sp) and the pair queues
+__host__ __device__ constexpr size_t sky_stage_bytes(int set, bool shapes) {
+  return (size_t)(kSkyTile + kSkyWarps * sky_cand(set, shapes)) *
+             (5 * 16 + 8 + (shapes ? 2 * 16 + 8 : 0)) +
+         (size_t)kSkyWarps * sky_ring(sky_cand(set, shapes)) * 2;
 }
+// Offset of the block histogram: behind the staging of every corel of the launch,
+// so that a block that goes from one job's unit to another's finds it zero.
+__host__ __device__ constexpr size_t sky_hist_off(int set) {
+  return set > 0 && sky_stage_bytes(set, true) > sky_stage_bytes(set, false)
+             ? sky_stage_bytes(set, true) : sky_stage_bytes(set, false);
+}
+// 32-bit words of a bin of the block histogram: the count, then a high and a
+// low word per field
+__host__ __device__ constexpr int sky_bin_words(int fm, int f0) { return 1 + 2 * (fm - f0); }
 
-// Mixed-precision evaluation of a pair that may bin.  Pi from hi+lo float
-// comoving distances, r_p = 2 asin(|u1 - u2| / 2) (D_A1 + D_A2) / 2 from hi+lo
-// float unit vectors, each with a bound on its difference from the
-// reference's double value; when both bins are certain the shape values are
-// computed in FP32 and accumulated, otherwise the pair takes the FP64 path.
-template <bool SMEM>
-__device__ __forceinline__ void sky_pair_mixed(const JobDev &J, const SkyRow &r, const SkyRowF &rf,
-                                               const SkyView &b, const SkyFast &fb, int64_t j,
-                                               unsigned long long *s_num,
-                                               unsigned long long *s_fix, const float *s_qs,
-                                               int2 *hq, unsigned long long *hq_n,
-                                               unsigned long long hq_cap, double esum,
-                                               const float *s_A, const float *s_B,
-                                               const float *s_PA, const float *s_PB) {
-  const float4 w2 = fb.sw[j], l2 = fb.sl[j], u2 = fb.su[j];
-  // every load of the pair issued before the first test: one memory round trip
-  // instead of three (most queued pairs bin)
-  const float4 x2 = fb.sx[j];
-  const int jk2 = b.d.jk[j], keep2 = b.d.keep[j];
-  float4 se2 = make_float4(0.f, 0.f, 0.f, 0.f), sh2 = se2;
-  float2 sp2 = make_float2(0.f, 0.f);
-  if (J.corel != COREL_DD) {
-    se2 = fb.ss[j];
-    sh2 = fb.sh[j];
-    sp2 = fb.sp[j];
-  }
-  // Pi: (dc2_hi - dc1_hi) + (dc2_lo - dc1_lo); the bands carry the error bound
-  const float pf = (w2.w - rf.w.w) + (l2.w - rf.ul.w);
-  const int k2 = band_bin(pf, 0.0f, (int)floorf(fmaf(pf, J.inv_ps_f, J.tp0)), J.npi, s_PA, s_PB,
-                          J.pi_out_lo, J.pi_out_hi);
-  if (k2 == -1) return;
-  // chord of the unit vectors, then theta and r_p
-  const float dx = (rf.u.x - u2.x) + (rf.ul.x - l2.x);
-  const float dy = (rf.u.y - u2.y) + (rf.ul.y - l2.y);
-  const float dz = (rf.u.z - u2.z) + (rf.ul.z - l2.z);
-  const float c2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-  const float c = sqrtf(c2);
-  int k1 = -2;
-  if (k2 >= 0 && c > 1.5e-5f) {  // below: near the clamp of dA_calc
-    // |rp - rp_ref| / rp: float chord, asinf and D_A sum (< 6e-7), the double
-    // unit vectors (3e-16 / c), and the reference's own sum = cos(theta)
-    // rounding through acos (< 1.2e-15 / theta^2), each with margin
-    const float rp = asinf(0.5f * c) * (rf.u.w + u2.w);
-    // (approximate reciprocal: the factor 1.001 covers its few-ulp error)
-    const float rc = __fdividef(1.0f, c);
-    const float tol = rp * fmaf(4e-15f * rc, rc, fmaf(3e-14f, rc, 1.5e-6f)) * 1.001f;
-    const int est = J.lin_bin ? (int)floorf((rp - J.rmin_f) * J.inv_rsize_f)
-                              : (int)floorf((__log2f(rp * rp) - J.l2rmin2) * J.inv_lw);
-    k1 = band_bin(rp, tol, est, J.nrp, s_A, s_B, J.rej_lo, J.rej_hi);
-    if (k1 == -1) return;
-  }
-  if (k1 < 0 || k2 < 0) {
-    sky_pair_fp64(J, r.i, j, hq, hq_n, hq_cap, esum);
-    return;
-  }
-  // values: theta = atan(dDec / (dRA cos(mean Dec))) (sky_calcs.cpp:13-22)
-  const float wt = rf.x.w * x2.w;
-  const int64_t cell = (int64_t)k1 * J.npi + k2;
-  if (J.corel == COREL_DD) {
-    const float f0[1] = {wt};
-    sky_accumulate_fixed<SMEM>(J, r.jk, r.keep, jk2, keep2, cell, f0, nullptr, 1, s_qs, s_num,
-                               s_fix);
-  } else {
-    // the separation in RA and Dec (hi + lo degrees) and cos of the mean Dec,
-    // cos(d1/2 + d2/2), as double-floats; X = dRA cos(mean Dec), Y = dDec
-    const df32 dra = df_diff_hl(w2.x, x2.x, rf.w.x, rf.x.x);
-    const df32 ddec = df_diff_hl(w2.y, x2.y, rf.w.y, rf.x.y);
-    const df32 cm = df_sub(df_mul(df32{rf.h.x, rf.h.y}, df32{sh2.x, sh2.y}),
-                           df_mul(df32{rf.h.z, rf.h.w}, df32{sh2.z, sh2.w}));
-    const df32 X = df_mul(dra, cm);
-    float v[kNF];
-    df32 vd[kNF];
-    for (int q = 0; q < kNF; q++) {
-      v[q] = 0.0f;
-      vd[q] = df32{0.0f, 0.0f};
+// Add the block histogram to the job's global fixed-point block -- the full
+// sample, region xreg (the tile's, when its rows are kept) and the partner
+// region yreg (each -1: none) -- and zero it.
+template <int C>
+__device__ __noinline__ void sky_flush(const JobDev &J, unsigned *H, int xreg, int yreg) {
+  using F = FieldMap<C>;
+  const int ncell = J.nrp * J.npi, f0 = J.unit_w ? 1 : 0;
+  const int SW = sky_bin_words(F::FM, f0);
+  const bool regf = J.which_corr != 0 && C != COREL_DD;
+  const int64_t hx = xreg >= 0 ? (int64_t)(1 + xreg) * ncell : -1;
+  const int64_t hy = yreg >= 0 ? (int64_t)(1 + yreg) * ncell : -1;
+  for (int c = threadIdx.x; c < ncell; c += kSkyThreads) {
+    unsigned *h = H + c * SW;
+    const unsigned n = h[0];
+    if (!n) continue;
+    h[0] = 0u;
+    atomicAdd(&J.acc_num[c], (unsigned long long)n);
+    if (hx >= 0) atomicAdd(&J.acc_num[hx + c], (unsigned long long)n);
+    if (hy >= 0) atomicAdd(&J.acc_num[hy + c], (unsigned long long)n);
+    const unsigned bias = n * kMagicBits;
+    for (int f = f0; f < F::FM; f++) {
+      const int o = 1 + 2 * (f - f0), fld = F::m(f);
+      const long long x = (long long)(int)(h[o] - bias) * 32768ll + (int)(h[o + 1] - bias);
+      h[o] = 0u;
+      h[o + 1] = 0u;
+      if (x == 0) continue;
+      const bool rf = fld == 0 || ((fld & 1) && regf);
+      const int64_t m = (int64_t)c * kNF + fld;
+      fix_add(&J.acc_fix[m], &J.acc_fixh[m], x);
+      if (rf && hx >= 0) fix_add(&J.acc_fix[hx * kNF + m], &J.acc_fixh[hx * kNF + m], x);
+      if (rf && hy >= 0) fix_add(&J.acc_fix[hy * kNF + m], &J.acc_fixh[hy * kNF + m], x);
     }
-    v[0] = wt;
-    if (X.h == 0.0f && ddec.h == 0.0f) {  // coincident on the sky: atan(0/0), the FP64 path
-      sky_pair_fp64(J, r.i, j, hq, hq_n, hq_cap, esum);
-      return;
-    }
-    df32 c, sn;
-    df_cos_sin_2theta(X, ddec, c, sn);
-    const float theta = atanf(__fdividef(ddec.h, X.h));
-    const DfGal g1{{rf.s.x, rf.s.z}, {rf.s.y, rf.s.w}, {rf.x.w, rf.p.y}, rf.p.x};
-    const DfGal g2{{se2.x, se2.z}, {se2.y, se2.w}, {x2.w, sp2.y}, sp2.x};
-    const bool uw = J.unit_w != 0;
-    if (J.corel == COREL_SD) df_pair_terms<COREL_SD>(c, sn, theta, g1, g2, J.gws, uw, vd, v);
-    else if (J.corel == COREL_SS) df_pair_terms<COREL_SS>(c, sn, theta, g1, g2, J.gws, uw, vd, v);
-    else df_pair_terms<COREL_SSA>(c, sn, theta, g1, g2, J.gws, uw, vd, v);
-    sky_accumulate_fixed<SMEM>(J, r.jk, r.keep, jk2, keep2, cell, v, vd, kNF, s_qs, s_num,
-                               s_fix);
   }
 }
 
-// 16-byte asynchronous copy global -> shared (the candidate prefetch below)
-__device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-// all but the newest kSkyAhead groups complete: the current stage has landed
-__device__ __forceinline__ void cp_async_wait_prev() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(kSkyAhead) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-}
-
-// window membership of x in [lo, hi] from the float value: 1 in, 0 out,
-// -1 undecided (x within a float ulp of a bound, or a NaN bound)
-__device__ __forceinline__ int fwin(float x, float lo_ru, float hi_rd, float lo_rd, float hi_ru) {
-  if (x > lo_ru && x < hi_rd) return 1;
-  if (x < lo_rd || x > hi_ru) return 0;
-  return -1;
-}
-
-// Rows are dealt in chunks of consecutive rows of one job (a pair type of the
-// batch): a block takes a chunk, its warps take the chunk's rows one at a time,
-// and the block meets at a barrier between chunks.  The block-private main
-// histogram belongs to one job; when the next chunk belongs to another job
-// (the chunks are numbered job after job, so a block switches at most
-// n_jobs - 1 times) the block adds it to the previous job's global block and
-// starts the next from zero.  A job's rows are every row of g1 or, for a row
-// sample, the listed rows.
-template <bool SMEM, int MINB>
-__global__ void __launch_bounds__(kSkyThreads, MINB)
-sky_warp_kernel(const JobDev *__restrict__ jobs, const long long *__restrict__ chunk0, int n_jobs,
-                int rows_per_chunk, unsigned long long *chunk_ctr, unsigned long long hq_cap,
-                double esum, float rp_lo_f, float rp_hi_f, int zero_bin) {
-  extern __shared__ __align__(16) unsigned char sky_smem[];
-  __shared__ int s_q[kSkyWarps][kSkyQ];
-  // per warp, kSkyAhead + 1 stages of 32 candidates' sw and su views: the next
-  // kSkyAhead stages are copied asynchronously while the current one is tested
-  __shared__ float4 s_pw[kSkyWarps][kSkyAhead + 1][32], s_pu[kSkyWarps][kSkyAhead + 1][32];
-  __shared__ SkyRowF s_rowf[kSkyWarps];
-  __shared__ float s_A[kMaxRp], s_B[kMaxRp], s_PA[kMaxPi], s_PB[kMaxPi];
-  __shared__ float s_qs[kNF];
-  __shared__ long long s_chunk;
-  __shared__ int s_rowctr, s_xmin, s_xmax;
-  __shared__ unsigned long long s_red[kSkyWarps];
-  const int ncell = jobs[0].nrp * jobs[0].npi;  // one binning for every job of a launch
-  unsigned long long *s_num = reinterpret_cast<unsigned long long *>(sky_smem);
-  unsigned long long *s_fix = s_num + ncell;
+// One unit: a run of row tiles of one (jackknife region, keep flag), up to
+// kSkyTile g1 rows each, against the candidate buckets [bk0, bk1) that a tile's
+// windows reach, or one of n_slices redshift slices of them.  The buckets are
+// those of one partner region where the host can pair the regions up: the
+// block histogram then holds one (region, partner region) pair, whose
+// attribution is done once per flush instead of per pair.
+template <int C, int SET>
+__device__ __forceinline__ void sky_unit(const SkyUnit &U, const JobDev &J, unsigned char *smem,
+                                         unsigned *H, SkyShared &S, unsigned long long hq_cap,
+                                         double esum) {
+  using F = FieldMap<C>;
+  constexpr bool kShapes = C != COREL_DD;
+  constexpr int kCand = sky_cand(SET, kShapes);
   const unsigned FULL = 0xffffffffu;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int *q = s_q[warp];
-  int cur = -1;                 // the job whose histogram the block holds
-  unsigned long long nwin = 0;  // window pairs of this thread's rows of job cur
-  for (;;) {
-    __syncthreads();  // every warp is done with the previous chunk
-    if (threadIdx.x == 0) {
-      s_chunk = (long long)atomicAdd(chunk_ctr, 1ull);
-      s_rowctr = 0;
-      s_xmin = INT_MAX;
-      s_xmax = INT_MIN;
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  const unsigned lt_mask = (1u << lane) - 1u;
+  // views, the tile rows' at [0, kSkyTile), the candidate slots' behind them
+  constexpr int kRec = kSkyTile + kSkyWarps * kCand;
+  float4 *v_u = reinterpret_cast<float4 *>(smem);
+  float4 *v_w = v_u + kRec, *v_l = v_w + kRec, *v_x = v_l + kRec, *v_b = v_x + kRec;
+  float4 *v_s = v_b + kRec, *v_h = v_s + (kShapes ? kRec : 0);
+  float2 *v_z = reinterpret_cast<float2 *>(v_h + (kShapes ? kRec : 0));
+  float2 *v_p = v_z + kRec;
+  constexpr int kRing = sky_ring(kCand);
+  unsigned short *wq =
+      reinterpret_cast<unsigned short *>(v_p + (kShapes ? kRec : 0)) + wid * kRing;
+
+  // the tile rows' catalogue and the candidates' (flip: g2 and g1)
+  const bool flip = J.sk.flip != 0;
+  const SkyFast &fa = flip ? J.sf2 : J.sf1, &fb = flip ? J.sf1 : J.sf2;
+  const float guard = J.sk.guard, pi_c = J.sk.pi_c, pi_h = J.sk.pi_h, t_hi = J.sk.t_hi;
+  if (t < kNF) S.qs[t] = J.qscale[t];
+  if (t == 0) S.k = J.sk;
+  const int nrp = J.nrp, npi = J.npi, ncell = nrp * npi;
+  const int f0 = J.unit_w ? 1 : 0;
+  const int SW = sky_bin_words(F::FM, f0);
+  const bool jk = J.do_jk != 0, regf = J.which_corr != 0 && kShapes;
+  const bool hsm = J.sk.hist_smem != 0;
+  const int auto_mode = J.auto_mode;
+  const int gws = J.gws;
+  const bool uw = J.unit_w != 0, lin = J.lin_bin != 0;
+  const int xreg = U.key >> 1;
+  const bool xkeep = (U.key & 1) != 0;
+  unsigned nwin = 0;
+  // an upper bound of the pairs in the histogram, and the regions that take
+  // them at the flush (the tile's, the candidates'; -1: none)
+  int pending = 0, cur_x = -1, cur_y = -1;
+  // counts alone cannot overflow their words: only the fixed-point words can
+  const int flush_pairs = (F::FM > f0) ? kSkyFlushPairs : 1 << 30;
+  for (int ti = U.tile0; ti < U.tile1; ti++) {
+  const SkyTileRows T = J.tiles[ti];
+  const int W = (T.count + 31) >> 5;
+  // tiles of at most 16 (8) rows: 2 (4) candidate streams per warp
+  const int rlanes = T.count <= 8 ? 8 : T.count <= 16 ? 16 : 32;
+  const int nsub = 32 / rlanes, sub = lane / rlanes, rl = lane & (rlanes - 1);
+  // ---- the tile's rows; slot tr = s * 32 + l holds tile row l * W + s, so the
+  // lanes of a pass are spread over the tile ----
+  float un[6] = {INFINITY, INFINITY, INFINITY, INFINITY, INFINITY, INFINITY};
+  if (t < kSkyTile) {
+    const int q = (t & 31) * W + (t >> 5);
+    // no row: every window test fails
+    float4 b = make_float4(0.f, 0.f, 0.f, 0.f), w = make_float4(0.f, 0.f, INFINITY, 0.f);
+    float2 z = make_float2(0.f, -INFINITY);
+    if ((t >> 5) < W && q < T.count) {
+      int i1 = T.start + q;
+      if (J.row_list) i1 = J.row_list[i1];
+      v_u[t] = fa.su[i1];
+      w = fa.sw[i1];
+      v_l[t] = fa.sl[i1];
+      v_x[t] = fa.sx[i1];
+      S.pos[t] = i1;
+      S.d3[t] = fa.dl[i1];
+      if (kShapes) {
+        v_s[t] = fa.ss[i1];
+        v_h[t] = fa.sh[i1];
+        v_p[t] = fa.sp[i1];
+      }
+      bool ok = true;
+      if (auto_mode) {
+        const int zi = fa.zidx[i1];
+        S.rorig[t] = (int)J.sky1.d.orig[zi];
+        // corels1, sorted: the scan from row i + 1 must pass the lower bound
+        if (auto_mode == 2) ok = (J.sky1.d.aflag[zi] & kAutoStart0) != 0;
+      }
+      if (flip) {
+        un[0] = w.x; un[1] = -w.x; un[2] = w.y; un[3] = -w.y; un[4] = w.z; un[5] = -w.z;
+      } else if (ok) {
+        b = fa.wb[i1];
+        z = fa.wz[i1];
+        un[0] = b.x - b.y; un[1] = -(b.x + b.y);
+        un[2] = b.z - b.w; un[3] = -(b.z + b.w);
+        un[4] = z.x - z.y; un[5] = -(z.x + z.y);
+      }
+    } else {
+      v_u[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    v_w[t] = w;
+    v_b[t] = b;
+    v_z[t] = z;
+#pragma unroll
+    for (int q6 = 0; q6 < 6; q6++) {
+      for (int o = 16; o > 0; o >>= 1) un[q6] = fminf(un[q6], __shfl_xor_sync(FULL, un[q6], o));
+      if (lane == 0) S.red[wid][q6] = un[q6];
+    }
+  }
+  __syncthreads();
+  // the union of the rows' windows (flip: the range of the rows), widened by the
+  // guard
+  auto uni = [&](int q6) {
+    float v = S.red[0][q6];
+    for (int w = 1; w < kSkyTile / 32; w++) v = fminf(v, S.red[w][q6]);
+    return v;
+  };
+  const float g2 = 4.0f * guard;
+  const float ra_lo = uni(0) - g2, ra_hi = g2 - uni(1), de_lo = uni(2) - g2, de_hi = g2 - uni(3);
+  float z_lo = uni(4) - g2, z_hi = g2 - uni(5);
+  {  // this unit's redshift slice, half-open (the last one closed by the guard)
+    const float d = (z_hi - z_lo) / (float)U.n_slices, z0 = z_lo;
+    if (U.slice > 0) z_lo = z0 + d * (float)U.slice;
+    if (U.slice + 1 < U.n_slices) z_hi = z0 + d * (float)(U.slice + 1);
+  }
+
+  int b0 = U.bk0;
+  while (b0 < U.bk1) {
+    // ---- the next candidate buckets (in region order) and their runs inside
+    // the redshift range ----
+    int ns = 0;
+    while (b0 < U.bk1 && ns + kSkyThreads <= kSkySeg) {
+      const int b = b0 + t;
+      int a = 0, e = 0, key = 0;
+      if (b < U.bk1) {
+        // the bucket's box (flip: the union of its rows' windows)
+        const float4 bx = flip ? fb.bk_win[b] : fb.bk_box[b];
+        const int4 bk = fb.bk[b];
+        key = bk.z;
+        if (bx.x <= ra_hi && bx.y >= ra_lo && bx.z <= de_hi && bx.w >= de_lo) {
+          if (!flip) {
+            a = sky_lower_bound([&](int i) { return fb.zf[i] < z_lo; }, bk.x, bk.y);
+            e = sky_lower_bound([&](int i) { return fb.zf[i] < z_hi; }, a, bk.y);
+          } else {  // rows whose redshift window reaches the tile (monotone bounds)
+            a = sky_lower_bound([&](int i) { return fb.wz[i].x + fb.wz[i].y < z_lo; }, bk.x, bk.y);
+            e = sky_lower_bound([&](int i) { return fb.wz[i].x - fb.wz[i].y <= z_hi; }, a, bk.y);
+          }
+        }
+      }
+      const unsigned m = __ballot_sync(FULL, e > a);
+      if (lane == 0) S.wcnt[wid] = __popc(m);
+      __syncthreads();
+      int pos = ns + __popc(m & lt_mask), tot = 0;
+      for (int w = 0; w < kSkyWarps; w++) {
+        const int v = S.wcnt[w];
+        if (w < wid) pos += v;
+        tot += v;
+      }
+      if (e > a) {
+        S.seg_a[pos] = a;
+        S.seg_pre[pos] = e - a;
+        S.seg_key[pos] = key;
+      }
+      ns += tot;
+      b0 += kSkyThreads;
+      __syncthreads();
+    }
+    if (wid == 0) {  // exclusive prefix of the run lengths
+      int run = 0;
+      for (int k0 = 0; k0 < ns; k0 += 32) {
+        const int v = k0 + lane < ns ? S.seg_pre[k0 + lane] : 0;
+        int s = v;
+        for (int o = 1; o < 32; o <<= 1) {
+          const int u = __shfl_up_sync(FULL, s, o);
+          if (lane >= o) s += u;
+        }
+        if (k0 + lane < ns) S.seg_pre[k0 + lane] = run + s - v;
+        run += __shfl_sync(FULL, s, 31);
+      }
+      if (lane == 0) S.seg_pre[ns] = run;
     }
     __syncthreads();
-    const long long ch = s_chunk;
+
     int k = 0;
-    while (k < n_jobs && ch >= chunk0[k + 1]) k++;  // block-uniform
-    if (k != cur) {
-      if (cur >= 0) {  // the previous job's window count (its histogram is flushed)
-        const JobDev &P = jobs[cur];
-        unsigned long long v = nwin;
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(FULL, v, o);
-        if (lane == 0 && v) atomicAdd(&P.counters[1], v);
-        nwin = 0;
+    while (k < ns) {  // groups of one (region, keep flag); U.all: one of every bucket
+      const int key = S.seg_key[k];
+      int g = k + 1;
+      while (g < ns && (U.all || S.seg_key[g] == key)) g++;
+      const int yreg = key >> 1;
+      const int gN = S.seg_pre[g] - S.seg_pre[k];
+      // jk_check_sky (jk.cpp:53-57): g1's region takes the pair when g1 is kept,
+      // g2's when g2 is kept and in another region
+      const bool other = yreg != xreg;
+      const bool xj = jk && xkeep && (other || !flip);  // (U.all is never flipped)
+      const bool yj = jk && (key & 1) != 0 && (other || flip);
+      // Where the candidates' region gets its pairs: from the histogram at its
+      // flush; or (U.all: few pairs per region pair) each pair adds its own terms
+      // to the global block, the candidates of every region in one group.  A
+      // flush touches up to ncell bins and a pair's own update a third of one, but
+      // a region pair's unit has its fixed cost too (sky_run's choice).
+      const bool ydir = !hsm || U.all != 0;
+      const int want_x = xj ? xreg : -1, want_y = yj && !ydir ? yreg : -1;
+      const int cap = max(kSkyThreads, flush_pairs / T.count);
+      for (int base = 0; base < gN; base += cap) {
+        const int nc = min(cap, gN - base);
+        if (pending &&
+            (want_x != cur_x || want_y != cur_y || pending + T.count * nc > flush_pairs)) {
+          __syncthreads();
+          sky_flush<C>(J, H, cur_x, cur_y);
+          pending = 0;
+          __syncthreads();
+        }
+        cur_x = want_x;
+        cur_y = want_y;
+        if (hsm) pending += T.count * nc;
+        // this warp's candidates: positions p = wid (mod nw) of the chunk, in
+        // nbw batches of at most kCand - 1 strided over its share (columns and
+        // redshifts mixed, so that a warp's pairs fall in different bins)
+        const int nw = min(kSkyWarps, max(1, nc >> 3));
+        const int share = wid < nw ? (nc - wid + nw - 1) / nw : 0;
+        const int nbw = (share + kCand - 2) / (kCand - 1);
+        const int c0 = kSkyTile + wid * kCand;
+        for (int bw = 0; bw < nbw; bw++) {
+          const int nk = (share - bw + nbw - 1) / nbw;
+          const int slot = c0 + lane;
+          if (lane < nk) {
+            const int p = S.seg_pre[k] + base + (lane * nbw + bw) * nw + wid;
+            int lo = k, hi = g;  // run lo with pre[lo] <= p < pre[lo + 1]
+            while (hi - lo > 1) {
+              const int mid = (lo + hi) >> 1;
+              if (S.seg_pre[mid] <= p) lo = mid; else hi = mid;
+            }
+            const int j2 = S.seg_a[lo] + (p - S.seg_pre[lo]);
+            S.key[slot - kSkyTile] = S.seg_key[lo];
+            S.pos[slot] = j2;
+            S.d3[slot] = fb.dl[j2];
+            v_u[slot] = fb.su[j2];
+            v_w[slot] = fb.sw[j2];
+            v_l[slot] = fb.sl[j2];
+            if (kShapes || !uw) v_x[slot] = fb.sx[j2];
+            if (kShapes) {
+              v_s[slot] = fb.ss[j2];
+              v_h[slot] = fb.sh[j2];
+              v_p[slot] = fb.sp[j2];
+            }
+            if (flip) {
+              v_b[slot] = fb.wb[j2];
+              v_z[slot] = fb.wz[j2];
+            }
+            if (auto_mode)  // corels1 (never flipped): the candidate's input row
+              v_z[slot].x = __int_as_float((int)J.sky2.d.orig[fb.zidx[j2]]);
+          } else if (lane < kCand) {  // no candidate: outside every redshift window
+            v_u[slot] = make_float4(0.f, 0.f, 0.f, 0.f);
+            v_w[slot] = make_float4(0.f, 0.f, INFINITY, 0.f);
+            v_b[slot] = make_float4(0.f, 0.f, 0.f, 0.f);
+            v_z[slot] = make_float2(0.f, -INFINITY);  // (as an input row: 0)
+          }
+          __syncwarp();
+          // ---- window tests of every (row, candidate), 32 rows at a time: a
+          // candidate is broadcast to the rows of the lanes, a bit per step marks
+          // the pairs that may bin.  After a pass each lane queues its pairs
+          // (a prefix sum of the bit counts gives its place): one row against
+          // candidates spread over the group, which fall in different bins ----
+          const int nks = (nk + nsub - 1) / nsub;
+          int pass = 0, qhead = 0, qtail = 0;
+          for (;;) {
+            if (qtail - qhead < 32 && pass < W) {
+              const int tr = pass * 32 + rl;
+              unsigned mask = 0u, emask = 0u;
+              const float4 u1 = v_u[tr], w1 = v_w[tr];
+              unsigned bit = 1u;
+              if (!flip) {
+                const float4 wb = v_b[tr];
+                const float2 wz = v_z[tr];
+                const float dc1 = w1.w + pi_c;
+                const int ro = auto_mode ? S.rorig[tr] : 0;
+                const float4 *cp = v_w + c0 + sub;
+#pragma unroll 4
+                for (int s = 0; s < nks; s++) {
+                  const float4 a = cp[0], v = cp[-kRec];  // v_w, v_u
+                  // distance inside the window, the smallest of the three
+                  const float da = wb.y - fabsf(a.x - wb.x), dd = wb.w - fabsf(a.y - wb.z);
+                  const float dr = wz.y - fabsf(a.z - wz.x);
+                  const float d = fminf(fminf(da, dd), dr);
+                  const float dx = u1.x - v.x, dy = u1.y - v.y, dz = u1.z - v.z;
+                  const float c2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                  const float ds = u1.w + v.w;
+                  const float tt = c2 * (ds * ds);
+                  const float pf = a.w - dc1;
+                  bool in = d > guard, edge = fabsf(d) <= guard;
+                  if (auto_mode) {  // corels1: partners after the row
+                    const bool ord = __float_as_int(v_z[c0 + sub + s * nsub].x) > ro;
+                    in = in && ord;
+                    edge = edge && ord;
+                  }
+                  if (in) nwin++;
+                  if (in && fabsf(pf) <= pi_h && tt < t_hi) mask |= bit;
+                  if (edge) emask |= bit;
+                  bit += bit;
+                  cp += nsub;
+                }
+              } else {  // the candidates' windows against the row
+                const float dc2 = w1.w - pi_c;
+                const float4 *cp = v_u + c0 + sub;
+                const float2 *zp = v_z + c0 + sub;
+#pragma unroll 4
+                for (int s = 0; s < nks; s++) {
+                  const float4 v = cp[0], wb = cp[4 * kRec];  // v_u, v_b
+                  const float2 wz = zp[0];
+                  const float dc1 = cp[kRec].w;               // v_w
+                  const float da = wb.y - fabsf(w1.x - wb.x), dd = wb.w - fabsf(w1.y - wb.z);
+                  const float dr = wz.y - fabsf(w1.z - wz.x);
+                  const float d = fminf(fminf(da, dd), dr);
+                  const float dx = u1.x - v.x, dy = u1.y - v.y, dz = u1.z - v.z;
+                  const float c2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                  const float ds = u1.w + v.w;
+                  const float tt = c2 * (ds * ds);
+                  const float pf = dc2 - dc1;
+                  const bool in = d > guard;
+                  if (in) nwin++;
+                  if (in && fabsf(pf) <= pi_h && tt < t_hi) mask |= bit;
+                  if (fabsf(d) <= guard) emask |= bit;
+                  bit += bit;
+                  cp += nsub;
+                  zp += nsub;
+                }
+              }
+              const int cnt = __popc(mask) + __popc(emask);
+              int sum = cnt;
+              for (int o = 1; o < 32; o <<= 1) {
+                const int u = __shfl_up_sync(FULL, sum, o);
+                if (lane >= o) sum += u;
+              }
+              unsigned pos = (unsigned)(qtail + sum - cnt);  // qtail < 2 kRing
+              if (pos >= kRing) pos -= kRing;
+              const unsigned en = (unsigned)tr | (unsigned)(sub << 7);
+              while (mask) {
+                const int s = 31 - __clz(mask);
+                mask ^= 1u << s;
+                wq[pos] = (unsigned short)(en + ((unsigned)(s * nsub) << 7));
+                if (++pos == kRing) pos = 0;
+              }
+              while (emask) {
+                const int s = 31 - __clz(emask);
+                emask ^= 1u << s;
+                wq[pos] = (unsigned short)((en + ((unsigned)(s * nsub) << 7)) | kSkyEdge);
+                if (++pos == kRing) pos = 0;
+              }
+              qtail += __shfl_sync(FULL, sum, 31);
+              pass++;
+              __syncwarp();
+              continue;
+            }
+            const int take = min(32, qtail - qhead);
+            if (take == 0) break;
+            if (lane < take) {
+              // ---- heavy step for one queued pair ----
+              const int qp = qhead + lane;
+              const unsigned en = wq[qp >= kRing ? qp - kRing : qp];
+              const int er = en & 127, ec = c0 + ((en >> 7) & 31);
+              const int a1 = flip ? ec : er, a2 = flip ? er : ec;  // g1, g2
+              const float4 u1 = v_u[a1], l1 = v_l[a1], u2 = v_u[a2], l2 = v_l[a2];
+              const float4 w1 = v_w[a1], w2 = v_w[a2];
+              // Pi from hi + lo comoving distances, its bin from the linear map
+              const float pf = (w2.w - w1.w) + (l2.w - l1.w);
+              const float v2 = fmaf(pf, S.k.pi_s, S.k.pi_o);
+              const float m2 = v2 + kMagic;
+              int n2 = __float_as_int(m2) - (int)kMagicBits;
+              bool pi_ok = fabsf(v2 - (m2 - kMagic)) <= S.k.pi_in;
+              // equal D_C (all three parts: common, as D_C is a distance-table row):
+              // Pi is exactly 0, here a bin edge
+              const bool zero_pi =
+                  !pi_ok && pf == 0.0f && w1.w == w2.w && l1.w == l2.w && S.d3[a1] == S.d3[a2];
+              if (zero_pi) {
+                n2 = S.k.pi_zero;
+                pi_ok = true;
+              }
+              // chord of the hi + lo unit vectors; (2 asin(c / 2))^2 as its series
+              // (c^2 <= 1/16: the first omitted term is 5e-9 of the sum)
+              const float dx = (u1.x - u2.x) + (l1.x - l2.x);
+              const float dy = (u1.y - u2.y) + (l1.y - l2.y);
+              const float dz = (u1.z - u2.z) + (l1.z - l2.z);
+              const float c2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+              float th2 = fmaf(c2, fmaf(c2, fmaf(c2, 1.0f / 560.0f, 1.0f / 90.0f), 1.0f / 12.0f),
+                               1.0f) * c2;
+              if (c2 > 0.0625f) {
+                const float th = 2.0f * asinf(0.5f * sqrtf(c2));
+                th2 = th * th;
+              }
+              const float ds = u1.w + u2.w;
+              const float r4 = th2 * (ds * ds);  // (2 r_p)^2
+              const float v1 = lin ? fmaf(sqrtf(r4), S.k.rp_s, S.k.rp_o)
+                                   : fmaf(__log2f(r4), S.k.rp_s, S.k.rp_o);
+              const float m1 = v1 + kMagic;
+              const int n1 = __float_as_int(m1) - (int)kMagicBits;
+              // undecided: near a Pi or r_p edge, or a separation so small that
+              // the reference's own rounding of cos theta matters
+              const float tt = c2 * (ds * ds);
+              const bool amb =
+                  !(pi_ok && fabsf(v1 - (m1 - kMagic)) <= S.k.rp_in && c2 >= 1e-8f) &&
+                  tt >= S.k.t_lo;
+              bool bin = tt >= S.k.t_lo && (unsigned)n1 < (unsigned)nrp && (unsigned)n2 < (unsigned)npi;
+              bool exact = amb || (en & kSkyEdge);
+              df32 X{0.f, 0.f}, ddec{0.f, 0.f};
+              float4 x1, x2;
+              if (kShapes || !uw) {
+                x1 = v_x[a1];
+                x2 = v_x[a2];
+              }
+              float4 h1, h2;
+              if (kShapes && bin && !exact) {
+                // tangent-plane separation: X = dRA cos(mean Dec), Y = dDec (hi + lo
+                // degrees; the cosine from the half angles), as double-floats
+                h1 = v_h[a1];
+                h2 = v_h[a2];
+                const df32 dra = df_diff_hl(w2.x, x2.x, w1.x, x1.x);
+                ddec = df_diff_hl(w2.y, x2.y, w1.y, x1.y);
+                const df32 cm = df_sub(df_mul(df32{h1.x, h1.y}, df32{h2.x, h2.y}),
+                                       df_mul(df32{h1.z, h1.w}, df32{h2.z, h2.w}));
+                X = df_mul(dra, cm);
+                // coincident on the sky: atan(0/0), the FP64 path
+                exact = X.h == 0.0f && ddec.h == 0.0f;
+              }
+              if (exact) {
+                sky_undecided(J, S.pos[a1], S.pos[a2], (en & kSkyEdge) != 0, hq_cap, esum);
+              } else if (bin) {
+                const int cell = n1 * npi + n2;
+                float v[kNF];
+                df32 vd[kNF];
+                if (!uw) v[0] = x1.w * x2.w;
+                if (kShapes) {
+                  // theta = atan(dDec / (dRA cos(mean Dec))) (sky_calcs.cpp:13-22)
+                  df32 c, sn;
+                  df_cos_sin_2theta(X, ddec, c, sn);
+                  const float theta = atanf(__fdividef(ddec.h, X.h));
+                  const float4 e1 = v_s[a1], e2 = v_s[a2];
+                  const float2 p1 = v_p[a1], p2 = v_p[a2];
+                  const DfGal g1{{e1.x, e1.z}, {e1.y, e1.w}, {x1.w, p1.y}, p1.x};
+                  const DfGal g2{{e2.x, e2.z}, {e2.y, e2.w}, {x2.w, p2.y}, p2.x};
+                  // (pairs at Pi = 0, one bin's share of which is large, would reach the
+                  // FP64 path but for their exact bin: their phi terms stay as exact)
+                  df_pair_terms<C>(c, sn, theta, g1, g2, gws, uw, vd, v, nullptr, nullptr, zero_pi);
+                }
+                unsigned wh[F::FM], wl[F::FM];
+#pragma unroll
+                for (int f = 0; f < F::FM; f++) {
+                  if (f < f0) continue;
+                  const int q = F::m(f);
+                  if (df_field(C, q)) df_to_words(vd[q], S.qs[q], wh[f], wl[f]);
+                  else f_to_words(v[q], S.qs[q], wh[f], wl[f]);
+                }
+                auto term = [&](int f) {  // the integer rint(v 2^S)
+                  return (long long)((int)(wh[f] - kMagicBits) * 32768 + (int)(wl[f] - kMagicBits));
+                };
+                if (hsm) {
+                  unsigned *h = H + cell * SW;
+                  atomicAdd(h, 1u);
+                  // even lanes add the high word first, odd lanes the low word, so
+                  // lanes that hit one bin split over two banks
+                  const bool odd = (lane & 1) != 0;
+                  unsigned *ha = h + 1 - 2 * f0 + (odd ? 1 : 0), *hb = h + 2 - 2 * f0 - (odd ? 1 : 0);
+#pragma unroll
+                  for (int f = 0; f < F::FM; f++) {
+                    if (f < f0) continue;
+                    atomicAdd(ha + 2 * f, odd ? wl[f] : wh[f]);
+                    atomicAdd(hb + 2 * f, odd ? wh[f] : wl[f]);
+                  }
+                }
+                // straight to the global block: the partner's region of a sparse
+                // group; with no room for a block histogram, everything
+                auto direct = [&](int64_t h0, bool all) {
+                  atomicAdd(&J.acc_num[h0 + cell], 1ull);
+#pragma unroll
+                  for (int f = 0; f < F::FM; f++) {
+                    const int q = F::m(f);
+                    if (f < f0 || !(all || q == 0 || ((q & 1) && regf))) continue;
+                    const int64_t o = (h0 + cell) * kNF + q;
+                    fix_add(&J.acc_fix[o], &J.acc_fixh[o], term(f));
+                  }
+                };
+                if (!hsm) {
+                  direct(0, true);
+                  if (xj) direct((int64_t)(1 + xreg) * ncell, false);
+                }
+                if (ydir && jk) {
+                  const int ky = S.key[ec - kSkyTile], yr = ky >> 1;
+                  if ((ky & 1) && (yr != xreg || flip)) direct((int64_t)(1 + yr) * ncell, false);
+                }
+              }
+            }
+            qhead += take;
+            if (qhead >= kRing) {
+              qhead -= kRing;
+              qtail -= kRing;
+            }
+            __syncwarp();
+          }
+          __syncwarp();  // every lane is done with the slots before restaging
+        }
       }
-      if (k >= n_jobs) break;
-      cur = k;
-      const JobDev &N = jobs[k];
-      for (int c = threadIdx.x; c < N.nrp; c += blockDim.x) { s_A[c] = N.A[c]; s_B[c] = N.B[c]; }
-      for (int c = threadIdx.x; c < N.npi; c += blockDim.x) { s_PA[c] = N.PA[c]; s_PB[c] = N.PB[c]; }
-      if (threadIdx.x < kNF) s_qs[threadIdx.x] = N.qscale[threadIdx.x];
-      if (SMEM) {
-        for (int c = threadIdx.x; c < ncell; c += blockDim.x) s_num[c] = 0ull;
-        for (int c = threadIdx.x; c < ncell * kNF; c += blockDim.x) s_fix[c] = 0ull;
-      }
-      __syncthreads();  // bands, scales, zeroed histogram
+      k = g;
     }
-    const JobDev &J = jobs[k];
-    const SkyView &a = J.sky1, &b = J.sky2;
-    const SkyFast &fa = J.sf1, &fb = J.sf2;
-    const int64_t n1 = a.d.n, n2 = b.d.n;
-    const int64_t n_rows = J.row_list ? J.n_rows : n1;
-    const int64_t r0 = (ch - chunk0[k]) * rows_per_chunk;
-    const int64_t r1 = min(r0 + (int64_t)rows_per_chunk, n_rows);
-    const float pmin_f = (float)J.pmin, pmax_f = (float)J.pmax;
-    int2 *hq = J.hq;
-    unsigned long long *hq_n = J.hq_n;
-    // When every outer row of the chunk lies in one jackknife region xreg and is
-    // kept (jk_prob >= 0.5), that region takes every pair the chunk adds to the
-    // block histogram (jk_check_sky, jk.cpp:53-57): it receives the histogram
-    // when the chunk ends, and the rows' pairs skip their own region update.
-    // (The rows are ordered by redshift slab and region, so most chunks are.)
-    int xreg = -1;
-    if (SMEM && J.do_jk) {
-      for (int64_t t = r0 + threadIdx.x; t < r1; t += blockDim.x) {
-        const int64_t ii = J.row_list ? J.row_list[t] : t;
-        const int reg = a.d.keep[ii] ? a.d.jk[ii] : -1;
-        atomicMin(&s_xmin, reg);
-        atomicMax(&s_xmax, reg);
-      }
-      __syncthreads();
-      xreg = (s_xmin == s_xmax && s_xmin >= 0) ? s_xmin : -1;
-    }
+    __syncthreads();  // the run tables are free
+  }
+  __syncthreads();  // the row slots are free
+  }
+  if (pending) sky_flush<C>(J, H, cur_x, cur_y);
+  {
+    unsigned v = nwin;
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(FULL, v, o);
+    if (lane == 0 && v) atomicAdd(&J.counters[1], (unsigned long long)v);
+  }
+}
+
+// Every job of a launch: the units of all jobs in one queue.  SET: the corels
+// the instantiation holds (0 density_density; 1 also shape_density; 2 also
+// shape_shape), so that a run of counts alone keeps few registers.
+template <int SET, int MINB>
+__global__ void __launch_bounds__(kSkyThreads, MINB)
+sky_tile_kernel(const JobDev *__restrict__ jobs, const SkyUnit *__restrict__ units, int n_units,
+                unsigned long long *ctr, unsigned long long hq_cap, double esum, int hist_off,
+                int hist_words) {
+  extern __shared__ __align__(16) unsigned char sky_smem[];
+  __shared__ SkyShared S;
+  unsigned *H = reinterpret_cast<unsigned *>(sky_smem + hist_off);
+  for (int k = threadIdx.x; k < hist_words; k += kSkyThreads) H[k] = 0u;
   for (;;) {
-    int64_t i = 0;
-    if (lane == 0) i = r0 + atomicAdd(&s_rowctr, 1);
-    i = __shfl_sync(FULL, i, 0);
-    if (i >= r1) break;
-    if (J.row_list) i = J.row_list[i];
-    if (J.auto_mode == 2 && !(a.d.aflag[i] & kAutoStart0)) continue;  // corels1, sorted
-    const int64_t oi = a.d.orig[i];
-    // the mixed path reads the row's index, region and keep flag; the FP64 path
-    // reloads the rest by index
-    SkyRow r;
-    r.i = i;
-    r.jk = a.d.jk[i];
-    r.keep = xreg >= 0 ? 0 : a.d.keep[i];  // xreg: the region takes the chunk's histogram
-    const double z_min = a.win[i], z_max = a.win[n1 + i];
-    // RA / Dec windows: float bounds rounded both ways here; the exact double
-    // bounds are reloaded in the rare undecided case (fewer live registers)
-    const double *w_ra_min = a.win + 2 * n1 + i, *w_ra_max = a.win + 3 * n1 + i;
-    const double *w_de_min = a.win + 4 * n1 + i, *w_de_max = a.win + 5 * n1 + i;
-    const float ra_lru = __double2float_ru(*w_ra_min), ra_hrd = __double2float_rd(*w_ra_max);
-    const float ra_lrd = __double2float_rd(*w_ra_min), ra_hru = __double2float_ru(*w_ra_max);
-    const float de_lru = __double2float_ru(*w_de_min), de_hrd = __double2float_rd(*w_de_max);
-    const float de_lrd = __double2float_rd(*w_de_min), de_hru = __double2float_ru(*w_de_max);
-    const float4 u1 = fa.su[i];
-    const float dc1f = fa.sw[i].w;
-    // the row's float views for the heavy step, in this warp's shared slot
-    SkyRowF &rf = s_rowf[warp];
-    if (lane == 0) {
-      rf.u = u1;
-      rf.ul = fa.sl[i];
-      rf.w = fa.sw[i];
-      rf.x = fa.sx[i];
-      rf.s = fa.ss[i];
-      rf.h = fa.sh[i];
-      rf.p = fa.sp[i];
+    __syncthreads();
+    if (threadIdx.x == 0) S.unit = (int)atomicAdd(ctr, 1ull);
+    __syncthreads();
+    const int u = S.unit;
+    if (u >= n_units) break;
+    const SkyUnit U = units[u];
+    const JobDev &J = jobs[U.job];
+    const int C = J.corel;
+    if (SET == 0 || C == COREL_DD) {
+      sky_unit<COREL_DD, SET>(U, J, sky_smem, H, S, hq_cap, esum);
+    } else if (SET >= 1 && C == COREL_SD) {
+      sky_unit<COREL_SD, SET>(U, J, sky_smem, H, S, hq_cap, esum);
+    } else if (SET >= 2) {
+      if (C == COREL_SS) sky_unit<COREL_SS, SET>(U, J, sky_smem, H, S, hq_cap, esum);
+      else sky_unit<COREL_SSA, SET>(U, J, sky_smem, H, S, hq_cap, esum);
     }
-    __syncwarp();
-    // redshift range [lo, hi): z_min <= z <= z_max
-    int64_t lo = 0, hi = n2;
-    while (lo < hi) {
-      const int64_t mid = (lo + hi) >> 1;
-      if (b.d.z[mid] < z_min) lo = mid + 1; else hi = mid;
-    }
-    int64_t end = n2, l2 = lo;
-    while (l2 < end) {
-      const int64_t mid = (l2 + end) >> 1;
-      if (b.d.z[mid] > z_max) end = mid; else l2 = mid + 1;
-    }
-    int count = 0;
-    // each lane prefetches its own candidate slot (no cross-lane reads of the
-    // stage buffers): stage 0 now, stage k+1 while stage k is tested
-    for (int a0 = 0; a0 < kSkyAhead; a0++) {
-      const int64_t jp = lo + 32 * a0 + lane;
-      if (jp < end) {
-        cp_async16(&s_pw[warp][a0][lane], fb.sw + jp);
-        cp_async16(&s_pu[warp][a0][lane], fb.su + jp);
-      }
-      cp_async_commit();
-    }
-    int stage = 0;
-    for (int64_t base = lo; base < end; base += 32, stage = (stage + 1) % (kSkyAhead + 1)) {
-      const int64_t j = base + lane;
-      const int64_t jn = j + 32 * kSkyAhead;
-      const int sn = (stage + kSkyAhead) % (kSkyAhead + 1);
-      if (jn < end) {
-        cp_async16(&s_pw[warp][sn][lane], fb.sw + jn);
-        cp_async16(&s_pu[warp][sn][lane], fb.su + jn);
-      }
-      cp_async_commit();
-      cp_async_wait_prev();  // this lane's copies of the current stage are done
-      bool need = false;
-      if (j < end && (!J.auto_mode || b.d.orig[j] > oi)) {  // corels1: partners after i
-        const float4 w2 = s_pw[warp][stage][lane];
-        int in = fwin(w2.y, de_lru, de_hrd, de_lrd, de_hru);
-        if (in < 0) {
-          const double d2 = b.d.y[j];
-          in = !(d2 > *w_de_max || d2 < *w_de_min);
-        }
-        if (in) {
-          int ir = fwin(w2.x, ra_lru, ra_hrd, ra_lrd, ra_hru);
-          if (ir < 0) {
-            const double a2 = b.d.x[j];
-            ir = !(a2 < *w_ra_min || a2 > *w_ra_max);
-          }
-          in = ir;
-        }
-        if (in) {
-          nwin++;
-          // Pi certainly outside [p_min, p_max): float dc carry <= 1 ulp each
-          const float pf = w2.w - dc1f;
-          const float pe = 4.0f * 5.96e-8f * (fabsf(w2.w) + fabsf(dc1f)) + 1e-30f;
-          const bool pi_out = (pf < pmin_f - pe) || (pf > pmax_f + pe);
-          if (!pi_out) {
-            // r_p bounds from the chord of float unit vectors
-            const float4 u2 = s_pu[warp][stage][lane];
-            const float dx = u1.x - u2.x, dy = u1.y - u2.y, dz = u1.z - u2.z;
-            const float c2 = dx * dx + dy * dy + dz * dz;
-            const float ch = sqrtf(c2);
-            const float dsum = 0.5f * (u1.w + u2.w);
-            const float ch_lo = fmaxf(ch * (1.0f - 1e-6f) - 4e-7f, 0.0f);
-            const float ch_hi = ch * (1.0f + 1e-6f) + 4e-7f;
-            const float rlo = ch_lo * dsum * (1.0f - 1e-6f);
-            const float rhi = ch_hi * (1.0f + ch_hi * ch_hi * (1.0f / 6.0f)) * dsum * (1.0f + 1e-6f);
-            // a clamped pair (theta < 1.41421e-5, r_p = 0) can bin when
-            // thr_0 <= 0: never reject it as "above the range" then
-            const bool above = rlo >= rp_hi_f && (!zero_bin || ch_lo > 1.5e-5f);
-            need = !(above || rhi < rp_lo_f);
-          }
-        }
-      }
-      const unsigned m = __ballot_sync(FULL, need);
-      if (need) q[count + __popc(m & ((1u << lane) - 1u))] = (int)j;
-      count += __popc(m);
-      __syncwarp();
-      if (count >= 32) {
-        sky_pair_mixed<SMEM>(J, r, rf, b, fb, q[lane], s_num, s_fix, s_qs, hq, hq_n, hq_cap, esum, s_A,
-                             s_B, s_PA, s_PB);
-        __syncwarp();
-        if (lane < count - 32) q[lane] = q[lane + 32];
-        count -= 32;
-        __syncwarp();
-      }
-    }
-    cp_async_wait_all();  // no copy in flight into the stage buffers of the next row
-    if (lane < count)
-      sky_pair_mixed<SMEM>(J, r, rf, b, fb, q[lane], s_num, s_fix, s_qs, hq, hq_n, hq_cap, esum, s_A,
-                           s_B, s_PA, s_PB);
-    __syncwarp();
-  }  // rows of the chunk
-    if (SMEM) {  // the chunk's block histogram into the job's main block (and region xreg)
-      __syncthreads();
-      const int64_t hx = xreg >= 0 ? (int64_t)(1 + xreg) * ncell : -1;
-      const bool regf = J.which_corr != 0 && J.corel != COREL_DD;
-      const bool wf = !J.unit_w;
-      for (int c = threadIdx.x; c < ncell; c += blockDim.x) {
-        const unsigned long long v = s_num[c];
-        if (!v) continue;
-        s_num[c] = 0ull;
-        atomicAdd(&J.acc_num[c], v);
-        if (hx >= 0) atomicAdd(&J.acc_num[hx + c], v);
-        for (int f = 0; f < kNF; f++) {
-          const long long x = (long long)s_fix[c * kNF + f];
-          if (x == 0) continue;
-          s_fix[c * kNF + f] = 0ull;
-          const int64_t o = c * kNF + f, ox = (hx + c) * kNF + f;
-          fix_add(&J.acc_fix[o], &J.acc_fixh[o], x);
-          if (hx >= 0 && ((f == 0 && wf) || ((f & 1) && regf)))
-            fix_add(&J.acc_fix[ox], &J.acc_fixh[ox], x);
-        }
-      }
-    }
-  }  // chunks
+  }
 }
 
-size_t sky_warp_smem_bytes(int nrp, int npi) {
-  return (size_t)nrp * npi * (1 + kNF) * sizeof(unsigned long long);
-}
-
-// fixed-point block -> FP64 sums: sums[i] += (hi[i] 2^15 + lo[i]) 2^-S_f,
-// f = i mod kNF (fix_add)
-__global__ void fix_to_sums_kernel(int64_t n, const unsigned long long *__restrict__ lo,
-                                   const unsigned long long *__restrict__ hi,
-                                   double *__restrict__ sums, const JobDev *__restrict__ jobp) {
+// Per job, after the pair kernel: the undecided pairs on the FP64 path, and
+// the fixed-point block added to the FP64 sums, sums[i] += (hi[i] 2^15 + lo[i])
+// 2^-S_f, f = i mod kNF (fix_add).
+__global__ void sky_finish_kernel(int64_t n, const unsigned long long *__restrict__ lo,
+                                  const unsigned long long *__restrict__ hi,
+                                  double *__restrict__ sums, const JobDev *__restrict__ jobp,
+                                  unsigned long long hq_cap, double esum) {
   const JobDev &J = *jobp;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned long long nx = min(*J.xq_n, kSkyExactQueue);
+  for (int64_t i = i0; i < (int64_t)nx; i += step) {
+    const int2 e = J.xq[i];
+    const bool edge = e.x < 0;
+    sky_pair_exact(J, edge ? ~e.x : e.x, e.y, edge, hq_cap, esum);
+  }
+  for (int64_t i = i0; i < n; i += step) {
     const unsigned long long l = lo[i];
     const long long h = (long long)hi[i];
     if (l != 0 || h != 0)
-      sums[i] += fma((double)h, 32768.0, (double)l) * J.inv_qscale[i % kNF];
+      atomicAdd(&sums[i], fma((double)h, 32768.0, (double)l) * J.inv_qscale[i % kNF]);
   }
 }
 
-cudaError_t launch_fix_to_sums(int64_t n, const unsigned long long *lo,
-                               const unsigned long long *hi, double *sums, const JobDev *job,
-                               cudaStream_t st) {
+cudaError_t launch_sky_finish(int64_t n, const unsigned long long *lo,
+                              const unsigned long long *hi, double *sums, const JobDev *job,
+                              unsigned long long hq_cap, double esum, cudaStream_t st) {
   if (n == 0) return cudaSuccess;
   const int64_t blocks = std::min<int64_t>((n + 255) / 256, 4096);
-  fix_to_sums_kernel<<<(unsigned)blocks, 256, 0, st>>>(n, lo, hi, sums, job);
+  sky_finish_kernel<<<(unsigned)blocks, 256, 0, st>>>(n, lo, hi, sums, job, hq_cap, esum);
   return cudaGetLastError();
 }
 
-template <int MINB>
-static cudaError_t launch_sky_warp_t(const JobDev *jobs, const long long *chunk0, int n_jobs,
-                                     long long n_chunks, int rows_per_chunk,
-                                     unsigned long long *chunk_ctr, unsigned long long hq_cap,
-                                     double esum, float rp_lo_f, float rp_hi_f, int zero_bin,
-                                     size_t smem, bool use_smem, int sm_count, cudaStream_t st) {
-  int bps = 0;
-  cudaError_t e;
-  if (use_smem) {
-    e = cudaFuncSetAttribute(sky_warp_kernel<true, MINB>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, sky_warp_kernel<true, MINB>,
-                                                      kSkyThreads, smem);
-  } else {
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, sky_warp_kernel<false, MINB>,
-                                                      kSkyThreads, 0);
-  }
+// Words of the block histogram a job of this corel needs, and whether the
+// histogram (behind the staging buffers) fits a block at two blocks per SM.
+size_t sky_hist_words(int corel, int unit_w, int ncell) {
+  const int fm = corel == COREL_DD ? FieldMap<COREL_DD>::FM
+                 : corel == COREL_SD ? FieldMap<COREL_SD>::FM
+                 : corel == COREL_SS ? FieldMap<COREL_SS>::FM : FieldMap<COREL_SSA>::FM;
+  return (size_t)sky_bin_words(fm, unit_w ? 1 : 0) * ncell;
+}
+bool sky_hist_fits(int corel, int unit_w, int ncell) {
+  return sky_hist_off(corel == COREL_DD ? 0 : 1) + 4 * sky_hist_words(corel, unit_w, ncell) +
+             sizeof(SkyShared) + 1024 <= (size_t)(228 * 1024) / 2;
+}
+
+template <int SET, int MINB>
+static cudaError_t launch_sky_t(const JobDev *jobs, const SkyUnit *units, int n_units,
+                                size_t hist_words, unsigned long long *ctr,
+                                unsigned long long hq_cap, double esum, int sm_count,
+                                cudaStream_t st) {
+  auto kern = sky_tile_kernel<SET, MINB>;
+  const size_t off = sky_hist_off(SET), smem = off + 4 * hist_words;
+  cudaError_t e =
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  if (bps < 1) bps = 1;
-  const int grid = (int)std::min<long long>((long long)sm_count * bps, n_chunks);
-  if (use_smem)
-    sky_warp_kernel<true, MINB><<<grid, kSkyThreads, smem, st>>>(
-        jobs, chunk0, n_jobs, rows_per_chunk, chunk_ctr, hq_cap, esum, rp_lo_f, rp_hi_f,
-        zero_bin);
-  else
-    sky_warp_kernel<false, MINB><<<grid, kSkyThreads, 0, st>>>(
-        jobs, chunk0, n_jobs, rows_per_chunk, chunk_ctr, hq_cap, esum, rp_lo_f, rp_hi_f,
-        zero_bin);
+  int bps = 0;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, kSkyThreads, smem);
+  if (e != cudaSuccess) return e;
+  if (bps < 1) return cudaErrorInvalidConfiguration;
+  const int grid = (int)std::min<long long>((long long)sm_count * bps, n_units);
+  kern<<<grid, kSkyThreads, smem, st>>>(jobs, units, n_units, ctr, hq_cap, esum, (int)off,
+                                        (int)hist_words);
   return cudaGetLastError();
 }
 
-cudaError_t launch_sky_warp(const JobDev *jobs, const long long *chunk0, int n_jobs,
-                            long long n_chunks, int rows_per_chunk,
-                            unsigned long long *chunk_ctr, unsigned long long hq_cap, double esum,
-                            float rp_lo_f, float rp_hi_f, int zero_bin, int nrp, int npi,
-                            int sm_count, int blocks_per_sm, cudaStream_t st) {
-  if (n_jobs <= 0 || n_chunks <= 0) return cudaSuccess;
-  const size_t smem = sky_warp_smem_bytes(nrp, npi);
-  const bool use_smem = smem <= 100 * 1024;
-  if (blocks_per_sm >= 3)  // 80 registers: more warps, a few spills
-    return launch_sky_warp_t<3>(jobs, chunk0, n_jobs, n_chunks, rows_per_chunk, chunk_ctr,
-                                hq_cap, esum, rp_lo_f, rp_hi_f, zero_bin, smem, use_smem,
-                                sm_count, st);
-  return launch_sky_warp_t<2>(jobs, chunk0, n_jobs, n_chunks, rows_per_chunk, chunk_ctr, hq_cap,
-                              esum, rp_lo_f, rp_hi_f, zero_bin, smem, use_smem, sm_count, st);
+cudaError_t launch_sky_tile(const JobDev *jobs, const SkyUnit *units, int n_units, int set,
+                            size_t hist_words, unsigned long long *ctr,
+                            unsigned long long hq_cap, double esum, int sm_count,
+                            cudaStream_t st) {
+  if (n_units <= 0) return cudaSuccess;
+  if (set == 0)
+    return launch_sky_t<0, 4>(jobs, units, n_units, hist_words, ctr, hq_cap, esum, sm_count, st);
+  if (set == 1)
+    return launch_sky_t<1, 3>(jobs, units, n_units, hist_words, ctr, hq_cap, esum, sm_count, st);
+  return launch_sky_t<2, 2>(jobs, units, n_units, hist_words, ctr, hq_cap, esum, sm_count, st);
 }
 
 cudaError_t launch_sky_fp64(const JobDev *job, const SkyView &a, const SkyView &b, int2 *hq,
