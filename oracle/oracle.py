@@ -42,8 +42,8 @@ REF_DIR = os.environ.get("CPC_REFERENCE_DIR", "/root/reference")
 
 def build_reference() -> str | None:
     """Build the reference harness from the reference sources (no-op where the
-    reference tree is absent)."""
-    if not os.path.isdir(REF_DIR):
+    reference tree is absent or empty)."""
+    if not os.path.isdir(REF_DIR) or not os.listdir(REF_DIR):
         return None
     subprocess.run(["make", "-s", "-C", HERE, "ref", f"REF_DIR={REF_DIR}"], check=True)
     return REF_BIN
