@@ -72,7 +72,7 @@ struct Slot {
   uint64_t version = 0;
   // grid this cell list was built with
   int ncx = 0, ncy = 0, n_reg = 1, kcells = 0;
-  double cw_x = 0, cw_y = 0;
+  double cw_x = 0, cw_y = 0, row_density = 0;
   // device, cell order
   DevBuf<float4> pos, shp, ewt, aux;
   DevBuf<float> zlo, zf;
@@ -131,7 +131,7 @@ struct SkyJobBufs {
 
 struct UnitCache {
   uint64_t v1 = 0, v2 = 0;
-  int s1 = -1, s2 = -1, wpi = 0, tile = 0, twin = 0;
+  int s1 = -1, s2 = -1, wpi = 0, tile = 0, twin = 0, variant = 0;
   std::vector<UnitDesc> units;  // job field filled at launch
 };
 
@@ -142,6 +142,8 @@ struct JobPlan;  // one planned count (below)
 }  // namespace
 
 struct cpc_ctx {
+  int64_t pref_n = -1;  // preferred_cells for a largest catalogue of pref_n rows
+  int pref_k = 2;
   cpc_params p{};
   std::vector<double> H, dA;
   std::string err;
@@ -410,6 +412,7 @@ struct JobPlan {
   int s1, s2;  // after the swap
   JobRule rule;
   int wpi, tile;
+  int variant;  // of the fast kernel (kernels.h)
   int64_t row_stride, row_offset;
   cpc_accum *out;
   JobDev jd;
@@ -505,6 +508,194 @@ bool twin_job(cpc_ctx *c, const JobRule &rule, int s1, int s2, int64_t rs, int64
   return slots_twin(c, s1, s2);
 }
 
+// Constants of the mixed-precision path of a box job (BoxConst): error bounds of
+// the float separations (ea: the absolute error of a coordinate difference, from
+// positions that are not float32 values or image shifts that round) against the
+// reference's double values.
+void box_consts(const cpc_ctx *c, const Slot &g1, const Slot &g2, JobDev &J) {
+  const cpc_params &p = c->p;
+  const int nrp = p.n_bins, npi = p.n_p_bin;
+  const bool rmu = p.coordinates == 7;
+  const double L = p.periodic_box_size, eps = std::ldexp(1.0, -24);
+  const double ea = eps_abs(c, g1, g2);
+  const double z0 = J.wz_lo, z1 = J.wz_hi, zm = std::max(std::fabs(z0), std::fabs(z1));
+  const double dtiny = 1e-12 * (L + std::max({p.bin_r_max, z1, -z0}));
+  BoxConst &K = J.bc;
+  // window: one rounding per difference, one of xyc - m or zh - |dz|, those of
+  // the bounds, and of z1 + zc where the z window is not symmetric; doubled
+  const double z_mid = 0.5 * (z0 + z1), cmax = std::max({g1.cmax, g2.cmax, L});
+  // (a window symmetric but for rounding is taken as symmetric)
+  const double zc = std::fabs(z_mid) <= std::ldexp(zm, -20) ? 0.0 : z_mid;
+  K.xyc = (float)p.bin_r_max;
+  K.zc = (float)zc;
+  K.zh = (float)(0.5 * (z1 - z0));
+  K.guard = f_up(2 * (ea + 4 * eps * std::max(p.bin_r_max, zm) +
+                      (zc != 0 ? ulpf(cmax + std::fabs(zc)) : std::fabs(z_mid)) + dtiny));
+  // r^2: each squared difference within (2 eps + 2 ea / r) of its share, two more
+  // roundings; relative 2^-21 and twice the absolute part
+  const double nterm = rmu ? 3.0 : 2.0;
+  auto gr = [&](double T) {
+    return 8 * eps * T * T + 2.0 * std::sqrt(nterm) * T * ea + nterm * ea * ea + 1e-12 * T * T;
+  };
+  const double lo = c->thr_rp[0], hi = c->thr_rp[nrp];
+  K.rej_lo = f_down(lo * lo - gr(lo));
+  K.rej_hi = f_up(hi * hi + gr(hi));
+  auto certain = [](double E) { return E < 0.5 ? f_down(0.5 - E) : -1.0f; };
+  {
+    const double s = 1.0 / c->ps, o = -p.p_min * s - 0.5;
+    const double map = 3 * eps * (npi + std::fabs(o) + 1) + 1e-9;  // roundings of the map
+    K.pi_s = (float)s;
+    K.pi_o = (float)o;
+    K.pi_abs = 0.0f;
+    if (!rmu) {
+      K.pi_in = certain((2 * eps * zm + 2 * ea + dtiny) * s + map);
+    } else {  // mu = dz / r, |mu| <= 1: relative 2^-21 (rsqrtf 2 ulp) and 3 ea / r
+      const double tmax = std::max({1.0, std::fabs(p.p_min), std::fabs(p.p_max)});
+      K.pi_in = certain(8 * eps * tmax * s + map);
+      K.pi_abs = f_up((4 * ea * tmax + dtiny + 1e-30) * s);
+    }
+  }
+  {
+    double E, o;
+    K.rp_abs = 0.0f;
+    if (p.lin_bin) {
+      const double s = 1.0 / c->rsize;
+      o = -p.bin_r_min * s - 0.5;
+      K.rp_s = (float)s;
+      E = (6 * eps * p.bin_r_max + std::sqrt(nterm) * 2 * ea + dtiny) * s +
+          4 * eps * (nrp + std::fabs(o) + p.bin_r_max * s + 1) + 1e-7;
+    } else {
+      const double s = nrp / (2.0 * std::log2(p.bin_r_max / p.bin_r_min));
+      const double l0 = 2.0 * std::log2(p.bin_r_min);
+      const double lm = std::max(std::fabs(l0), std::fabs(2.0 * std::log2(p.bin_r_max)));
+      o = -l0 * s - 0.5;
+      K.rp_s = (float)s;
+      // log2 r^2: relative 8 eps of r^2; __log2f within 2 ulp (2^-21.4 near 1)
+      E = s * (8 * eps / M_LN2 + std::max(4 * eps * lm, 8e-7) + 2 * eps * lm) +
+          3 * eps * (nrp + std::fabs(o) + 1) + 1e-7;
+      K.rp_abs = f_up(s * 1.01 * (2 * std::sqrt(nterm) * ea + 1e-30) / M_LN2 * 1.05);
+      if (!(ea > 0)) K.rp_abs = 0.0f;
+      // the exact thresholds must be the edges of this map
+      for (int k = 0; k <= nrp; k++)
+        if (!(std::fabs((2.0 * std::log2(c->thr_rp[k]) - l0) * s - k) < 1e-7)) E = 1.0;
+    }
+    K.rp_o = (float)o;
+    K.rp_in = certain(E);
+  }
+}
+
+// Model of the kernel's time, by which a job's cell width, kernel variant and the
+// z extent of its chunks of rows are chosen.  Per row of a chunk of r rows (of
+// lam rows per unit of z): r / 32 + 1/4 rounds of lanes over r on each candidate of the
+// chunk's z range, kap of them per unit of z (the quarter is the staging and the
+// lanes left idle); four rounds of 32 lanes per 32 pairs that bin; and each unit's set-up
+// and flush, about 500 such rounds of a 256-thread block.  With fewer units than
+// the GPU holds blocks, blocks wait.
+// Measured against fixed rules (the smallest blocks of at least 11 bins, chunks of
+// half the window or a quarter of the z range, k = 2 but for sparse tiles) over
+// drawn boxes: the kernel with fixed rules 1.38 times as fast as before it was
+// rewritten, with the model 1.7 to 1.9; kappa of 20,000 rows in 288 buckets 0.86 ->
+// 0.17 ms, a batch of w++ boxes of up to 9,000 rows 4.0 -> 1.3; the 200k wg+ box,
+// whose tiles are full either way, 13.8 -> 13.5.
+struct ChunkModel {
+  double kap, heavy, zw, ps, n, slots, unit, scale;
+  int npi, wpi;
+  bool rmu, narrow;
+  ChunkModel(const cpc_ctx *c, double n1, double n2, double cell, int twin, int variant, int w) {
+    const cpc_params &p = c->p;
+    const double L = p.periodic_box_size, r = p.bin_r_max, d = n2 / (L * L * L);
+    const double side = std::min(L, 2 * r + 2 * cell);
+    zw = wz_hi(p) - (twin ? 0.0 : wz_lo(p));
+    kap = d * side * side;
+    heavy = 4.0 / 32 * d * M_PI * r * r * zw;
+    ps = c->ps;
+    n = n1;
+    npi = p.n_p_bin;
+    wpi = w;
+    rmu = p.coordinates == 7;
+    narrow = !rmu && wpi < npi;
+    slots = (double)c->sm_count * fast_variant_blocks(variant);
+    unit = 500.0 * 4 / fast_variant_blocks(variant);
+    scale = variant == 1 ? 1.0 : variant == 2 ? 1.05 : 1.1;  // wider blocks wait for one another
+  }
+  // Pi range that the pairs of a narrow unit may cover: it starts anywhere in the
+  // window's first bin and ends anywhere in its last.
+  double window() const { return (wpi - 2) * ps; }
+  double cost(double lam, double *extent = nullptr) const {
+    double best = INFINITY;
+    for (const double f : {0.125, 0.1875, 0.25, 0.375, 0.5, 0.625, 0.75}) {
+      const double E = narrow ? std::min({f * window(), window() - ps, zw}) : f * zw;
+      const double r0 = std::max(1.0, lam * E), r = r0 / std::ceil(r0 / kTileThreads);
+      const double units =
+          narrow ? std::max(1.0, (zw + E) / std::max(ps, window() - E)) : 1.0;
+      const double t = kap * (zw + E) * (1.0 / 32 + 0.25 / r) + heavy + unit * units / r;
+      const double slices = rmu ? std::ceil((double)npi / wpi) : 1.0;  // all of it, per mu slice
+      const double idle = slots / std::max(1.0, n / r * units * slices);
+      const double total = scale * t * slices * std::max(1 + 0.2 * idle, idle);
+      if (total < best) {
+        best = total;
+        if (extent) *extent = E;
+      }
+    }
+    return best;
+  }
+};
+
+// Smallest window worth a kernel of its own (coordinates 7: any mu slice).
+int min_window(const cpc_params &p, int twin) { return p.coordinates == 7 ? 1 : twin ? 5 : 8; }
+
+struct Variant {
+  int variant = 0, wpi = 0;  // 0: the smallest window fits no variant's share of an SM
+  double cost = 0;
+};
+// The variant for a job of n1 x n2 rows: of the widest window that each holds,
+// the one the model finds fastest.
+Variant choose_variant(const cpc_ctx *c, int corel, int auto_mode, int unit_w, int twin, double n1,
+                       double n2, double cell, double lam) {
+  const cpc_params &p = c->p;
+  const int jk = p.do_jk ? 1 : 0, wmin = min_window(p, twin);
+  Variant best;
+  for (int v = 1; v <= 3; v++) {
+    const size_t budget = fast_block_smem(v) - fast_static_smem_bytes(corel, jk, v, twin) - 1024;
+    auto bytes = [&](int w) {
+      return fast_smem_bytes(corel, jk, p.n_bins, w, auto_mode, unit_w, twin, v);
+    };
+    // (the bytes are linear in the window)
+    const size_t b0 = bytes(0), bin = bytes(1) - b0;
+    const int w = std::min(p.n_p_bin, std::max(wmin, budget > b0 ? (int)((budget - b0) / bin) : 0));
+    if (bytes(w) > budget || (best.variant && w <= best.wpi)) continue;
+    const double t = ChunkModel(c, n1, n2, cell, twin, v, w).cost(lam);
+    if (!best.variant || t < best.cost) best = Variant{v, w, t};
+  }
+  return best;
+}
+
+// Cell width (r_max / k) when none is set, from the largest catalogue of the
+// context (or the n rows of an upload), so that every count of the context uses
+// one width and a catalogue is rebuilt at most when a larger one comes: 2, or 1
+// where the model finds it as fast within a tenth, with the rows spread evenly
+// over the columns and jackknife cubes (k = 1 quadruples a bucket's rows, for
+// 16 / 9 of the candidates).  Measured, k = 1 over 2: wgg of 20,000 points 0.71, 12
+// boxes of L = 3.3 r_max 1.0, w++ boxes of 9,000 rows 0.5; 200k wg+ box 1.07, ED 1.14.
+int preferred_cells(cpc_ctx *c, int64_t n = 0) {
+  const cpc_params &p = c->p;
+  for (const Slot &s : c->slots)
+    if (s.valid && !s.sky) n = std::max(n, s.n);
+  if (c->pref_n == n) return c->pref_k;
+  const double L = p.periodic_box_size;
+  const int corel = p.which_corr < 3 ? COREL_DD + p.which_corr : COREL_DK + (p.which_corr - 3);
+  auto cost = [&](int k) {
+    const double cols = std::max(1.0, std::floor(L / (p.bin_r_max / k)));
+    const double cuts = cols + (p.do_jk ? std::cbrt((double)p.n_jk) - 1 : 0);
+    return choose_variant(c, corel, 0, 0, 0, (double)n, (double)n, L / cols, n / (cuts * cuts * L)).cost;
+  };
+  c->pref_n = n;
+  c->pref_k = cost(1) < 1.1 * cost(2) ? 1 : 2;
+  return c->pref_k;
+}
+
+cpc_status rebuild_cells(cpc_ctx *c, Slot &s, int k);
+
 // allow_twin: false for the cell-list FP64 comparison engine, which counts every
 // order and keeps the plain job's window
 cpc_status plan_job(cpc_ctx *c, cpc_pair_kind kind, int slot_g1, int slot_g2, int64_t rs,
@@ -526,12 +717,20 @@ cpc_status plan_job(cpc_ctx *c, cpc_pair_kind kind, int slot_g1, int slot_g2, in
   jp.s1 = jp.rule.swapped ? slot_g2 : slot_g1;
   jp.s2 = jp.rule.swapped ? slot_g1 : slot_g2;
   Slot &g1 = c->slots[jp.s1], &g2 = c->slots[jp.s2];
+  if (c->tune_k == 0 && !g1.sky && !g2.sky) {
+    const int k = preferred_cells(c);
+    for (Slot *s : {&g1, &g2})
+      if (s->kcells != k) {
+        const cpc_status st = rebuild_cells(c, *s, k);
+        if (st != CPC_OK) return st;
+      }
+  }
   if (g1.ncx != g2.ncx || g1.ncy != g2.ncy || g1.n_reg != g2.n_reg)
     return fail(c, CPC_ERR_STATE, "catalogues were uploaded with different cell grids");
   jp.empty = (A.n == 0 || B.n == 0);
   const int nrp = p.n_bins, npi = p.n_p_bin;
   const int jk = p.do_jk ? 1 : 0;
-  // block-local Pi window: as many Pi bins as fit kFastBlocksPerSM blocks per SM.  With
+  // block-local Pi window: as many Pi bins as fit a block's shared memory.  With
   // coordinates 7 the mu bins have no locality in z: a block holds every mu bin
   // when they fit (else the units are repeated over slices of wpi mu bins)
   const bool rmu = p.coordinates == 7;
@@ -540,27 +739,35 @@ cpc_status plan_job(cpc_ctx *c, cpc_pair_kind kind, int slot_g1, int slot_g2, in
   // the pair order with g2 ahead, whose units span half the Pi range)
   const int twin =
       (allow_twin && !jp.empty && twin_job(c, jp.rule, jp.s1, jp.s2, rs, ro, auto_mode)) ? 1 : 0;
-  const int wmin = rmu ? 1 : twin ? 5 : 8;
-  // Automatic window: the largest that fits 4 blocks per SM when it holds at
-  // least 12 Pi bins (or all of them), else the largest for 3 blocks.
-  const size_t static_b = fast_static_smem_bytes(twin);
-  auto fit = [&](int blocks) {
-    const size_t budget = (size_t)(228 * 1024) / blocks - static_b - 1024;
-    int w = npi;
-    while (w > wmin && fast_smem_bytes(jp.rule.corel, jk, nrp, w, auto_mode,
-                                       unit_weights(g1, g2), twin) > budget)
-      w--;
-    return w;
-  };
-  int wpi = npi;
+  const int wmin = min_window(p, twin);
+  // The kernel variant (block size) and its window.  A window set by
+  // cpc_set_tuning takes the smallest blocks whose share of an SM it fits.
+  const int uw = unit_weights(g1, g2);
+  int wpi = 0, variant = 0;
   if (c->tune_wpi > 0 && !rmu) {
     wpi = std::min(npi, c->tune_wpi);
+    auto bytes = [&](int v, int w) {
+      return fast_smem_bytes(jp.rule.corel, jk, nrp, w, auto_mode, uw, twin, v);
+    };
+    auto fixed = [&](int v) { return fast_static_smem_bytes(jp.rule.corel, jk, v, twin); };
+    for (variant = 1; variant <= 3; variant++)
+      if (bytes(variant, wpi) <= fast_block_smem(variant) - fixed(variant) - 1024) break;
+    if (variant > 3) {  // fewer blocks per SM, of the variant with the least staging
+      variant = 1;
+      // histograms of up to 200 KB are accepted, and narrowed beside the staging
+      const size_t room = 227 * 1024 - fixed(1);
+      if (bytes(1, wpi) - bytes(1, 0) <= 200 * 1024)
+        while (wpi > 1 && bytes(1, wpi) > room) wpi--;
+    }
   } else {
-    wpi = fit(kFastBlocksPerSM);
-    if (wpi < npi && wpi < 12) wpi = std::max(wpi, fit(kFastBlocksPerSM - 1));
+    const Variant b = choose_variant(c, jp.rule.corel, auto_mode, uw, twin, (double)g1.n,
+                                     (double)g2.n, g1.cw_x, g1.row_density);
+    variant = b.variant ? b.variant : 3;  // (else the smallest window in the largest blocks)
+    wpi = b.variant ? b.wpi : wmin;
   }
   if (!rmu && wpi < npi && wpi < wmin) wpi = std::min(npi, wmin);
   jp.wpi = wpi;
+  jp.variant = variant;
   jp.tile = kTileThreads;
 
   JobDev &J = jp.jd;
@@ -600,62 +807,7 @@ cpc_status plan_job(cpc_ctx *c, cpc_pair_kind kind, int slot_g1, int slot_g2, in
   J.ps = c->ps;
   J.rsize = c->rsize;
   for (int k = 0; k <= nrp; k++) J.thr[k] = c->thr_rp[k];
-  // ---- guard bands (see pair_fast.cu): relative 2^-21 per coordinate
-  // difference, 2^-20 on r^2, plus the absolute representation/wrap error.
-  const double ea = eps_abs(c, g1, g2);
-  const double crel = std::ldexp(1.0, -21);
-  const double zlo_w = J.wz_lo, zhi_w = J.wz_hi;
-  const double dtiny = 1e-12 * (L + std::max({p.bin_r_max, zhi_w, -zlo_w}));
-  const double gxy = crel * p.bin_r_max + 2 * ea + dtiny;
-  J.xy_in = f_down(p.bin_r_max - gxy);
-  J.xy_out = f_up(p.bin_r_max + gxy);
-  auto gp = [&](double v) { return crel * std::fabs(v) + 2 * ea + dtiny + 1e-30; };
-  J.pi_in_lo = f_up(zlo_w + gp(zlo_w));
-  J.pi_out_lo = f_down(zlo_w - gp(zlo_w));
-  J.pi_in_hi = f_down(zhi_w - gp(zhi_w));
-  J.pi_out_hi = f_up(zhi_w + gp(zhi_w));
-  if (!rmu) {
-    for (int k = 0; k < npi; k++) {
-      const double lo = c->thr_pi[k], hi = c->thr_pi[k + 1];
-      J.PA[k] = f_up(lo + gp(lo));
-      J.PB[k] = f_down(hi - gp(hi));
-    }
-  } else {
-    // mu bins: the edges themselves (nearest float); a pair is inside bin k when
-    // dz - PA[k] r >= mu_rel r + mu_abs and PB[k] r - dz > mu_rel r + mu_abs,
-    // which covers the float errors of dz, r, the edge and the products
-    for (int k = 0; k < npi; k++) {
-      J.PA[k] = (float)c->thr_pi[k];
-      J.PB[k] = (float)c->thr_pi[k + 1];
-    }
-    const double tmax = std::max({1.0, std::fabs(p.p_min), std::fabs(p.p_max)});
-    J.mu_rel = (float)(std::ldexp(1.0, -19) * tmax);
-    J.mu_abs = (float)(8 * ea * tmax + dtiny + 1e-30);
-  }
-  J.inv_ps_f = (float)(1.0 / c->ps);
-  J.tp0 = (float)(-p.p_min / c->ps);
-  // r^2 error bound: two squared differences (r_p), three for coordinates 7 (r)
-  const double nterm = rmu ? 3.0 : 2.0;
-  auto gr = [&](double T) {
-    return std::ldexp(1.0, -20) * T * T + 2.0 * std::sqrt(nterm) * T * ea + nterm * ea * ea +
-           1e-12 * T * T;
-  };
-  for (int k = 0; k < nrp; k++) {
-    const double lo = c->thr_rp[k], hi = c->thr_rp[k + 1];
-    J.A[k] = f_up(lo * lo + gr(lo));
-    J.B[k] = f_down(hi * hi - gr(hi));
-  }
-  J.rej_lo = f_down(c->thr_rp[0] * c->thr_rp[0] - gr(c->thr_rp[0]));
-  J.rej_hi = f_up(c->thr_rp[nrp] * c->thr_rp[nrp] + gr(c->thr_rp[nrp]));
-  J.rmin_f = (float)p.bin_r_min;
-  J.inv_rsize_f = (float)(1.0 / c->rsize);
-  if (p.lin_bin) {  // linear bins: estimate index from r, bands still decide
-    J.l2rmin2 = 0.f;
-    J.inv_lw = 0.f;
-  } else {
-    J.l2rmin2 = (float)(2.0 * std::log2(p.bin_r_min));
-    J.inv_lw = (float)(1.0 / (2.0 * std::log2(p.bin_r_max / p.bin_r_min) / nrp));
-  }
+  box_consts(c, g1, g2, J);
   // fixed-point scales: field f's terms are rint(v 2^S_f) with
   // |v_f| 2^S_f <= 2^29 / (1 + 2^-12) < 2^29 - 2^17 (see pair_fast.cu); S_f
   // from a bound on |v_f| (emax bounds |e|, so every rotated ellipticity)
@@ -697,7 +849,7 @@ const std::vector<UnitDesc> &build_units(JobPlan &jp) {
   for (auto &uc : c->unit_cache)
     if (uc.s1 == jp.s1 && uc.s2 == jp.s2 && uc.v1 == c->slots[jp.s1].version &&
         uc.v2 == c->slots[jp.s2].version && uc.wpi == jp.wpi && uc.tile == jp.tile &&
-        uc.twin == jp.jd.twin)
+        uc.twin == jp.jd.twin && uc.variant == jp.variant)
       return uc.units;
   if (c->unit_cache.size() >= 8) c->unit_cache.erase(c->unit_cache.begin());
   c->unit_cache.emplace_back();
@@ -709,6 +861,7 @@ const std::vector<UnitDesc> &build_units(JobPlan &jp) {
   uc.wpi = jp.wpi;
   uc.tile = jp.tile;
   uc.twin = jp.jd.twin;
+  uc.variant = jp.variant;
   const cpc_params &p = c->p;
   const Slot &g1 = c->slots[jp.s1];
   const double L = p.periodic_box_size;
@@ -719,18 +872,13 @@ const std::vector<UnitDesc> &build_units(JobPlan &jp) {
   const bool rmu = p.coordinates == 7;
   const double zw0 = wz_lo(p), zw1 = wz_hi(p);
   const double guard = 4 * ulpf(2 * cmax) + 2 * ea + std::ldexp(1.0, -20) * (std::fabs(zw0) + std::fabs(zw1) + p.bin_r_max);
-  // tile z-extent: wide enough that the 32 lanes of a warp (spread over the
-  // tile) see different Pi bins, small enough to fit the block-local window
-  double Emax = 0.25 * (zw1 - zw0);
-  if (!rmu) {
-    if (wpi < npi) Emax = std::min(Emax, (wpi - 6) * ps / 2.0);
-    Emax = std::max(Emax, std::min(2.0 * ps, 0.25 * (p.p_max - p.p_min)));
-  }
-  // sparse buckets: a chunk of extent Emax may hold fewer rows than a warp has
-  // lanes (the other lanes then test rows that do not exist); such a chunk grows
-  // up to Ehi, the widest extent whose units still fit the window
-  // ((wpi - 4) ps - extent >= ps), until it holds 32 rows
-  const double Ehi = (!rmu && wpi < npi) ? std::max(Emax, (wpi - 5) * ps) : Emax;
+  // chunk extents by the bucket's rows per unit of z, in steps of a quarter octave
+  const Slot &g2 = c->slots[jp.s2];
+  const ChunkModel model(c, (double)g1.n, (double)g2.n, g1.cw_x, jp.jd.twin, jp.variant, wpi);
+  constexpr int kOne = 64;  // entry of one row per z range
+  double extents[2 * kOne + 1];
+  for (int q = 0; q <= 2 * kOne; q++)
+    model.cost(std::exp2(0.25 * (q - kOne)) / model.zw, &extents[q]);
   const int ncx = g1.ncx, ncy = g1.ncy;
   const double inv_cwx = 1.0 / g1.cw_x, inv_cwy = 1.0 / g1.cw_y;
   std::vector<UnitDesc> &units = uc.units;
@@ -744,18 +892,20 @@ const std::vector<UnitDesc> &build_units(JobPlan &jp) {
     for (int b = (int)b_lo; b < (int)b_hi; b++) {
       const int s = g1.h_bk_start[b], e = g1.h_bk_end[b];
       int i = s;
+      const double ext = std::max<double>((double)g1.h_pos[e - 1].z - g1.h_pos[s].z, ps);
+      const double lq = 4 * std::log2((e - s) / ext * model.zw) + kOne;
+      const double extent = extents[(int)std::lrint(std::min(std::max(lq, 0.0), 2.0 * kOne))];
       while (i < e) {
-        // z-chunk of extent <= Emax, dealt round-robin into tiles of <= tile rows
+        // z-chunk, dealt round-robin into tiles of <= tile rows
         const float z0 = g1.h_pos[i].z;
-        int j = i;
+        int j = i + 1;
+        while (j < e && (double)g1.h_pos[j].z - z0 <= extent) j++;
         float bx0 = INFINITY, bx1 = -INFINITY, by0 = INFINITY, by1 = -INFINITY;
-        while (j < e && ((double)g1.h_pos[j].z - z0 <= Emax ||
-                         (j - i < 32 && (double)g1.h_pos[j].z - z0 <= Ehi))) {
-          bx0 = std::min(bx0, g1.h_pos[j].x);
-          bx1 = std::max(bx1, g1.h_pos[j].x);
-          by0 = std::min(by0, g1.h_pos[j].y);
-          by1 = std::max(by1, g1.h_pos[j].y);
-          j++;
+        for (int k = i; k < j; k++) {
+          bx0 = std::min(bx0, g1.h_pos[k].x);
+          bx1 = std::max(bx1, g1.h_pos[k].x);
+          by0 = std::min(by0, g1.h_pos[k].y);
+          by1 = std::max(by1, g1.h_pos[k].y);
         }
         const int m = j - i;
         const int nt = (m + jp.tile - 1) / jp.tile;
@@ -781,29 +931,22 @@ const std::vector<UnitDesc> &build_units(JobPlan &jp) {
           u.g1_count = (m - k + nt - 1) / nt;
           u.region = g1.h_bk_region[b];
           u.cx_lo = cx0; u.cx_hi = cx1; u.cy_lo = cy0; u.cy_hi = cy1;
-          if (wpi >= npi || rmu) {
-            // coordinates 7: one unit per slice of wpi mu bins; each pair is
-            // taken by the slice holding its estimated bin (pair_fast.cu)
-            u.zlo = Zlo;
-            u.zhi = Zhi;
-            for (int base = 0; base < npi; base += wpi) {
-              u.n2_base = base;
-              units.push_back(u);
-            }
-          } else {
-            const double span = std::max(ps, (wpi - 4) * ps - (zt1 - zt0));
-            const int U = std::max(1, (int)std::ceil((Zhi - Zlo) / span));
+          int U = 1;
+          if (model.narrow)
+            U = std::max(1, (int)std::ceil((Zhi - Zlo) /
+                                           std::max(ps, model.window() - (zt1 - zt0))));
+          // coordinates 7: one unit per slice of wpi mu bins; each pair is taken by
+          // the slice holding its bin (pair_fast.cu)
+          for (int base = 0; base < (rmu ? npi : 1); base += wpi)
             for (int q = 0; q < U; q++) {
-              const double a = (q == 0) ? Zlo : Zlo + (Zhi - Zlo) * q / U;
-              const double bnd = (q == U - 1) ? Zhi : Zlo + (Zhi - Zlo) * (q + 1) / U;
-              int base = (int)std::floor((a - zt1 - p.p_min) / ps) - 1;
-              base = std::max(0, std::min(base, npi - wpi));
+              u.zlo = (q == 0) ? Zlo : Zlo + (Zhi - Zlo) * q / U;
+              u.zhi = (q == U - 1) ? Zhi : Zlo + (Zhi - Zlo) * (q + 1) / U;
               u.n2_base = base;
-              u.zlo = a;
-              u.zhi = bnd;
+              if (model.narrow)
+                u.n2_base = std::max(
+                    0, std::min((int)std::floor((u.zlo - zt1 - guard - p.p_min) / ps), npi - wpi));
               units.push_back(u);
             }
-          }
         }
         i = j;
       }
@@ -979,7 +1122,7 @@ cpc_status run_fast(std::vector<JobPlan> &jobs, int grow_attempt = 0);
 
 // one persistent launch of the fast kernel over a range of the unit list
 struct FastGroup {
-  int corel, jk, minb, grid;
+  int corel, jk, variant, grid;
   size_t first, n_units, smem;
   FastScales sc;
   int auto_pairs;  // the group holds corels1 jobs (their rules in shared memory)
@@ -1007,7 +1150,7 @@ cpc_status fast_body(cpc_ctx *c0, std::vector<JobPlan> &jobs, const std::vector<
   CK(cudaEventRecordWithFlags(c0->e0, st, rec_flags), "event");
   for (const FastGroup &g : gs) {
     CK(cudaMemsetAsync(c0->d_unit_ctr.p, 0, sizeof(unsigned int), st), "memset");
-    CK(launch_fast(g.corel, g.jk, g.minb, g.twin, c0->d_jobs.p, c0->d_units.p + g.first,
+    CK(launch_fast(g.corel, g.jk, g.variant, g.twin, c0->d_jobs.p, c0->d_units.p + g.first,
                    (int)g.n_units,
                    c0->d_unit_ctr.p, c0->d_queue.p, c0->d_qcount.p, c0->qcap, g.sc, g.smem,
                    g.grid, g.auto_pairs, st),
@@ -1045,7 +1188,7 @@ std::vector<uint64_t> fast_graph_key(cpc_ctx *c0, const std::vector<JobPlan> &jo
   for (const FastGroup &g : gs) {
     put((uint64_t)g.corel);
     put((uint64_t)g.jk);
-    put((uint64_t)g.minb);
+    put((uint64_t)g.variant);
     put((uint64_t)g.grid);
     put(g.first);
     put(g.n_units);
@@ -1122,15 +1265,16 @@ cpc_status enqueue_fast(std::vector<JobPlan> &jobs) {
     jobs[k].jd.acc_sums = jobs[k].c->d_sums.p;
     jobs[k].jd.counters = jobs[k].c->d_counters.p;
   }
-  // group by kernel template
-  // group by kernel instantiation: corel, jackknife, twin
-  std::map<std::tuple<int, int, int>, std::vector<int>> groups;
+  // group by kernel instantiation: corel, jackknife, twin, variant
+  using Inst = std::tuple<int, int, int, int>;
+  std::map<Inst, std::vector<int>> groups;
   for (size_t k = 0; k < jobs.size(); k++)
     if (!jobs[k].empty)
-      groups[std::make_tuple(jobs[k].jd.corel, jobs[k].jd.do_jk, jobs[k].jd.twin)].push_back((int)k);
+      groups[Inst(jobs[k].jd.corel, jobs[k].jd.do_jk, jobs[k].jd.twin,
+                  jobs[k].jd.all_exact ? 0 : jobs[k].variant)].push_back((int)k);
   size_t total_units = 0;
   std::vector<std::pair<size_t, size_t>> ranges;
-  std::vector<std::tuple<int, int, int>> gkeys;
+  std::vector<Inst> gkeys;
   for (auto &g : groups) {
     const size_t b = all.size();
     for (int k : g.second) {
@@ -1177,7 +1321,8 @@ cpc_status enqueue_fast(std::vector<JobPlan> &jobs) {
     CK(cudaMemcpyAsync(c0->d_units.p, all.data(), sizeof(UnitDesc) * total_units, cudaMemcpyHostToDevice, st), "H2D units");
   std::vector<FastGroup> gs;
   for (size_t g = 0; g < ranges.size(); g++) {
-    const int corel = std::get<0>(gkeys[g]), jk = std::get<1>(gkeys[g]), twin = std::get<2>(gkeys[g]);
+    const int corel = std::get<0>(gkeys[g]), jk = std::get<1>(gkeys[g]), twin = std::get<2>(gkeys[g]),
+              variant = std::get<3>(gkeys[g]);
     size_t smem = 0;  // the largest any job of the group needs
     FastScales sc;    // per field the smallest scale of the group's jobs
     int auto_pairs = 0;
@@ -1190,22 +1335,20 @@ cpc_status enqueue_fast(std::vector<JobPlan> &jobs) {
     for (size_t k = ranges[g].first; k < ranges[g].second; k++) {
       const JobPlan &jp = jobs[all[k].job];
       smem = std::max(smem, fast_smem_bytes(corel, jk, jp.jd.nrp, jp.wpi, auto_pairs,
-                                            jp.jd.unit_w, jp.jd.twin));
+                                            jp.jd.unit_w, jp.jd.twin, variant));
       for (int f = 0; f < kNF; f++)
         if (jp.jd.qscale[f] < sc.qs[f]) {
           sc.qs[f] = jp.jd.qscale[f];
           sc.iqs[f] = jp.jd.inv_qscale[f];
         }
     }
-    int bps = 0;
-    const int minb = fast_variant(corel, jk, smem, &bps,
-                                  jobs[all[ranges[g].first].job].jd.all_exact, twin);
+    const int bps = fast_blocks(corel, jk, variant, smem, twin);
     if (bps <= 0) return fail(c, CPC_ERR_INVALID, "fast kernel does not fit on an SM with these bins");
     const size_t n_units = ranges[g].second - ranges[g].first;
     if (n_units == 0) continue;
     const int grid = (int)std::min<int64_t>((int64_t)c0->sm_count * bps, (int64_t)n_units);
     gs.push_back(
-        FastGroup{corel, jk, minb, grid, ranges[g].first, n_units, smem, sc, auto_pairs, twin});
+        FastGroup{corel, jk, variant, grid, ranges[g].first, n_units, smem, sc, auto_pairs, twin});
   }
   return launch_fast_body(c0, jobs, gs);
 }
@@ -1369,6 +1512,13 @@ cpc_status build_cells(cpc_ctx *c, Slot &s, int64_t n, int k, const int64_t *ori
   CK(cudaMemcpyAsync(s.col_begin.p, cb.data(), 4 * ncol, cudaMemcpyHostToDevice, st), "H2D");
   CK(cudaMemcpyAsync(s.col_end.p, ce.data(), 4 * ncol, cudaMemcpyHostToDevice, st), "H2D");
   CK(cudaStreamSynchronize(st), "upload");
+  // rows per unit of z that the buckets' rows see, on average
+  double dens = 0;
+  for (size_t b = 0; b < nb; b++) {
+    const double m = s.h_bk_end[b] - s.h_bk_start[b];
+    dens += m * m / std::max<double>((double)bz1[b] - bz0[b], c->ps);
+  }
+  s.row_density = dens / (double)nn;
   s.valid = true;
   return CPC_OK;
 }
@@ -2532,7 +2682,7 @@ cpc_status cpc_upload(cpc_ctx *c, int slot, const cpc_catalog *cat) try {
     CK(cudaMemcpyAsync(&c->h_ustats, c->d_ustats.p, sizeof(UploadStats), cudaMemcpyDeviceToHost,
                        st), "D2H");
   }
-  return build_cells(c, s, n, c->tune_k > 0 ? c->tune_k : 2, nullptr, true);
+  return build_cells(c, s, n, c->tune_k > 0 ? c->tune_k : preferred_cells(c, n), nullptr, true);
 } catch (...) {
   return host_exception(c);
 }
@@ -2636,7 +2786,7 @@ cpc_status cpc_count_auto(cpc_ctx *c, cpc_pair_kind kind, int slot, cpc_engine e
   return host_exception(c);
 }
 
-// Pi windows the autotuner tries: for 4, 3 and 2 blocks per SM the largest
+// Pi windows the autotuner tries: for 256, 512 and 1024 threads per block the largest
 // window whose histograms fit, and three quarters of it (more, narrower units).
 // With coordinates 7 the mu window is automatic (every mu bin when they fit):
 // only the cell width is tuned.
@@ -2645,17 +2795,17 @@ std::vector<int> tune_windows(const cpc_params &p, int corel, int unit_w, int tw
   if (p.coordinates == 7) return {0};
   const int wmin = twin ? 5 : 8;
   const int jk = p.do_jk ? 1 : 0, nrp = p.n_bins, npi = p.n_p_bin;
-  const size_t static_b = fast_static_smem_bytes(twin);
-  for (int b = 4; b >= 2; b--) {
-    const size_t budget = (size_t)(228 * 1024) / b - static_b - 1024;
+  for (int v = 1; v <= 3; v++) {
+    const size_t budget =
+        fast_block_smem(v) - fast_static_smem_bytes(corel, jk, v, twin) - 1024;
     int w = npi;
-    while (w > 1 && fast_smem_bytes(corel, jk, nrp, w, 0, unit_w, twin) > budget) w--;
-    if (fast_smem_bytes(corel, jk, nrp, w, 0, unit_w, twin) > budget) continue;
+    while (w > 1 && fast_smem_bytes(corel, jk, nrp, w, 0, unit_w, twin, v) > budget) w--;
+    if (fast_smem_bytes(corel, jk, nrp, w, 0, unit_w, twin, v) > budget) continue;
     for (int cand : {w, (3 * w + 3) / 4}) {
       if (cand < std::min(npi, wmin)) continue;
       if (std::find(ws.begin(), ws.end(), cand) == ws.end()) ws.push_back(cand);
     }
-    if (w == npi) break;  // every Pi bin fits: fewer blocks gain nothing
+    if (w == npi) break;  // every Pi bin fits: larger blocks gain nothing
   }
   if (ws.empty()) ws.push_back(0);
   return ws;
@@ -2700,6 +2850,7 @@ cpc_status cpc_autotune(cpc_ctx *c, cpc_pair_kind kind, int slot_g1, int slot_g2
   int bk = c->slots[slot_g1].kcells, bw = c->tune_wpi;
   for (int k : ks) {
     cpc_status s;
+    c->tune_k = k;  // (a count would choose its own width)
     if (c->slots[slot_g1].kcells != k && (s = rebuild_cells(c, c->slots[slot_g1], k)) != CPC_OK)
       return s;
     if (slot_g2 != slot_g1 && c->slots[slot_g2].kcells != k &&
@@ -2814,6 +2965,7 @@ cpc_status cpc_autotune_batch(int n_jobs, cpc_ctx *const *ctxs, const cpc_pair_k
   }
   // every slot a job reads, on cells r_max / kc
   auto regrid = [&](int kc) -> cpc_status {
+    for (int k = 0; k < n_jobs; k++) ctxs[k]->tune_k = kc;  // (a count would choose its own)
     for (int k = 0; k < n_jobs; k++)
       for (int sl : {slots_g1[k], slots_g2[k]}) {
         Slot &s = ctxs[k]->slots[sl];

@@ -126,6 +126,17 @@ struct SkyUnit {
   int job, tile0, tile1, key, bk0, bk1, all, slice, n_slices;
 };
 
+// constants of a box job's mixed-precision path (set-up in capi.cu): a bin index
+// is rint(s x + o), certain when within `in` of it, less abs / r where the error
+// of the separation has an absolute part
+struct BoxConst {
+  float xyc, zc, zh;       // window: |dx|, |dy| <= xyc, |dz - zc| <= zh
+  float guard;             // a window test within it of a bound is undecided
+  float rej_lo, rej_hi;    // r_p^2 (r^2) certainly below or above the bins
+  float pi_s, pi_o, pi_in, pi_abs;  // Pi bin of Pi (coordinates 7: mu bin of mu)
+  float rp_s, rp_o, rp_in, rp_abs;  // r_p bin of log2 r_p^2 (linear bins: of r_p)
+};
+
 struct JobDev {
   FCat f1, f2;  // g1 (outer rows) and g2 after the swap rule
   DCat d1, d2;  // same catalogues, FP64, cell order
@@ -145,18 +156,10 @@ struct JobDev {
   int64_t row_stride, row_offset;
   // ---- fast-path single precision constants ----
   float Lf;
-  float xy_in, xy_out;                 // definite window bounds on max(|dx|,|dy|)
-  float pi_in_lo, pi_in_hi, pi_out_lo, pi_out_hi;
-  float inv_ps_f, tp0;                 // approximate Pi bin: floor(dz*inv_ps + tp0)
-  float l2rmin2, inv_lw;               // log2(r_min^2), 1/(log2 width in r^2)
-  float rmin_f, inv_rsize_f;           // linear-bin estimate
-  float rej_lo, rej_hi;                // definite r^2 rejection bounds
-  float mu_rel, mu_abs;                // coordinates 7: mu-bin margin mu_rel r + mu_abs (dz units)
+  BoxConst bc;
   float qscale[kNF];                   // per-field fixed-point scale 2^S_f
   int qbias;                           // fixed-point bound: |v_f| 2^S_f <= qbias
   int unit_w;                          // every weight is 1: wt_num = count
-  float A[kMaxRp], B[kMaxRp];          // definite r^2 band of r_p bin k
-  float PA[kMaxPi], PB[kMaxPi];        // definite Pi band of Pi bin k
   // ---- FP64 exact constants ----
   double L, rmin, rmax, pmin, pmax, ps, rsize;
   double wz_lo, wz_hi;                 // z window offsets: p_min, p_max (coordinates 6)

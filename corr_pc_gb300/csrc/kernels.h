@@ -72,22 +72,23 @@ double from_orderable_key(unsigned long long k);
 
 // pair_fast.cu
 constexpr int kTileThreads = 128;  // g1 rows per tile (a warp tests them in passes of 32)
-constexpr int kFastBlocksPerSM = 4;  // occupancy target: registers and shared memory sized for it
 // Per work unit: at most kFastMaxCols neighbour columns (the host rejects units
 // with more; (2k + 3)^2 columns for cells r_max / k wide, so k <= 9) and
 // candidate slots taken kFastMaxSeg at a time.
 constexpr int kFastMaxCols = 512;
 constexpr int kFastMaxSeg = 256;
 constexpr int kMaxCellsPerRmax = 9;
-// auto_pairs: the launch holds corels1 (auto-pair) jobs, whose rules take
-// another kBatch + 3 kTile ints of shared memory
+// variant: 1 blocks of 256 threads, 4 per SM; 2 of 512, 2 per SM; 3 of 1024, 1
+// per SM; 0 the cell-list FP64 comparison engine (all_exact jobs).  auto_pairs:
+// the launch holds corels1 (auto-pair) jobs, whose rules take more shared
+// memory.  twin: the twin kernels (density_density and shape_shape jobs whose
+// slots hold the same galaxies).
 size_t fast_smem_bytes(int corel, int do_jk, int nrp, int wpi, int auto_pairs, int unit_w,
-                       int twin);
-size_t fast_static_smem_bytes(int twin);
-// minb 4 or 3: the register bound (blocks per SM) of the fast kernel; 1: the
-// cell-list FP64 comparison engine (all_exact jobs).  twin: the twin kernels
-// (density_density and shape_shape jobs whose slots hold the same galaxies)
-int fast_variant(int corel, int jk, size_t smem, int *blocks_per_sm, int all_exact, int twin);
+                       int twin, int variant);
+size_t fast_static_smem_bytes(int corel, int jk, int variant, int twin);
+int fast_variant_blocks(int variant);  // blocks per SM
+size_t fast_block_smem(int variant);  // a block's share of an SM's shared memory
+int fast_blocks(int corel, int jk, int variant, size_t smem, int twin);
 // Fixed-point scales of one fast-kernel launch (kernel parameters, read from
 // the constant bank): field f's terms are rint(v qs[f]), summed back with
 // iqs[f] = 1 / qs[f].  A launch over several jobs takes, per field, the smallest
@@ -97,7 +98,7 @@ struct FastScales {
   float qs[kNF];
   double iqs[kNF];
 };
-cudaError_t launch_fast(int corel, int jk, int minb, int twin, const JobDev *jobs,
+cudaError_t launch_fast(int corel, int jk, int variant, int twin, const JobDev *jobs,
                         const UnitDesc *units, int n_units, unsigned int *unit_ctr, QEntry *q,
                         unsigned long long *qcount, unsigned long long qcap,
                         const FastScales &sc, size_t smem, int grid, int auto_pairs,

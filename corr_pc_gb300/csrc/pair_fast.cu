@@ -3,19 +3,31 @@
 // One persistent launch drains a device work queue of "units".  A unit is a
 // tile of up to kTile g1 rows from one (column, jackknife region) bucket and
 // z-chunk, paired with every g2 candidate of the neighbouring columns inside
-// the unit's shifted-z range.  A block of 8 warps keeps the tile's rows in
-// shared memory; each warp stages its own batches of up to 32 candidates and
-// tests them against every row, in W passes of 32 rows for a tile of up to
-// 32 W rows (one row per lane; the lanes of a warp are spread over the tile).
-// Candidates are drawn in chunks of a coprime-stride permutation of the
-// (partner region, image shift) group, so simultaneous pairs of a warp fall in
-// different bins; the block meets at a barrier once per chunk.
+// the unit's shifted-z range.  A block keeps the tile's rows in shared memory;
+// each warp stages its own batches of candidates and tests them against every
+// row, in W passes of 32 rows (one row per lane; the lanes of a warp are spread
+// over the tile).  Candidates are strided over their (partner region, image
+// shift) group, so that a batch mixes columns and redshifts.
 //
-// Light pass (every candidate): FP32 separations with the image shift applied
-// exactly, definite in / definite out tests of the reference's window, r^2
-// range test; binned pairs go to a per-warp queue.  Heavy step (32 queued
-// pairs, all lanes busy): exact r_p and Pi bins from an estimated index checked
-// against definite bands, shape values, histogram updates.
+// Light pass (every candidate, broadcast to 32 rows): FP32 separations with the
+// image shift applied exactly; the distance inside the reference's window is
+// one number, compared with a guard both ways, and a bit per step keeps the
+// pairs that may bin.  After a pass each lane queues its pairs (a prefix sum of
+// the bit counts).  Heavy step (32 queued pairs, all lanes busy): r_p and Pi bins
+// from linear maps of Pi and log2 r^2 with an error bound each, shape values,
+// histogram updates.
+//
+// Measured (GB300, before -> now): kernel of the 200k wg+ box 17.9 -> 13.5 ms,
+// kappa 11.6 -> 7.6, ED 7.0 -> 4.1; w++ twin of 2M points 567 -> 420, weighted w++
+// (60k x 151k) 6.9 -> 5.2, 12 uneven w++ boxes 58 -> 25; wgg of 20,000 points
+// 0.36 -> 0.12.  What gave it: one bit per test instead of a queue push per step
+// (67 -> 24 instructions a step), maps instead of band tables, records of words
+// at constant offsets added with their bias (no split of the fixed-point term),
+// four-way order of the reductions, unit set-up by scans instead of serial
+// loops, no barrier per thousand candidates, blocks of 512 and 1024 threads
+// that share a wider histogram, and units cut by a model of their cost (capi.cu).  Bound now by the shared-memory reductions for
+// the shape corels (74-78% of the pipe: a bin's pairs are serialised, see
+// order4) and by instruction issue (87%) for kappa, ED and counts.
 //
 // Precision: a pair is resolved on this path only when it is farther than a
 // rigorous error bound from every decision boundary (the r_p / Pi window,
@@ -38,6 +50,7 @@
 // about 1e-9 of the field's bound.
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <atomic>
 #include <climits>
 
 #include "cpc_device.cuh"
@@ -48,67 +61,54 @@
 namespace cpc {
 
 constexpr int kTile = kTileThreads;          // g1 rows per tile
-constexpr int kThreads = 256;                 // block size: 8 warps
-constexpr int kBatch = kThreads;              // staging slots: 32 per warp
+// Kernel variants: block size and blocks per SM (32 warps per SM at 64 registers;
+// the FP64 comparison engine 16 at 128).  Wider blocks share a histogram among
+// more warps, which widens its Pi window (choose_variant chooses).
+__host__ __device__ constexpr int variant_threads(int v) { return v == 3 ? 1024 : v == 2 ? 512 : 256; }
+__host__ __device__ constexpr int variant_blocks(int v) { return v == 3 ? 1 : v == 1 ? 4 : 2; }
 constexpr int kMaxSeg = kFastMaxSeg;
 constexpr int kMaxCols = kFastMaxCols;
-// candidates of a group per block barrier: a chunk adds at most kTile * kChunk
-// = 2^17 terms to any word, so the flush test below runs once per chunk
-constexpr int kChunk = 4 * kThreads;
-
-// Padding that puts the high-word array (FW * NB words after the low words)
-// 16 banks away from the low-word array.
-__host__ __device__ constexpr int hi_pad(int words) { return (16 - (words & 31) + 32) & 31; }
-
-// Replicas of the hot r_p bins (a build option, off by default).  Most pairs
-// fall in the few largest r_p bins (their count grows as r_p^2), so the lanes of
-// one heavy-step instruction often add into the same main-histogram bins, and
-// same-address shared reductions are serialised.  With CPC_HOT_REP > 1 the top
-// kHotBins r_p bins of the main histogram get kHotRep copies each, the copy
-// picked by lane bits 1-2 (bit 0 already splits lanes over the low and high
-// words), and the flush adds the copies together in exact integer arithmetic.
-// Measured on GB300: 4 copies of the top 4 bins gain 2% on the 200k wg+ box and
-// lose 3-4% on the kappa and ED workloads (the copies take shared memory from
-// the Pi window); on the 2M w++ box 2 copies of the top one or two rows or 4
-// of the top row gain nothing (777, 773 and 786 ms against 773 ms), so the
-// default is one copy.
-#ifndef CPC_HOT_REP
-#define CPC_HOT_REP 1
-#endif
-#ifndef CPC_HOT_BINS
-#define CPC_HOT_BINS 4
-#endif
-constexpr int kHotRep = CPC_HOT_REP, kHotBins = CPC_HOT_BINS;
-static_assert(kHotRep == 1 || kHotRep == 2 || kHotRep == 4 || kHotRep == 8, "replicas: 1, 2, 4 or 8");
-// main-histogram bins of a block: nrp * wpi, plus the hot bins' extra copies
-__host__ __device__ __forceinline__ int hot_rows(int nrp) { return nrp < kHotBins ? nrp : kHotBins; }
-__host__ __device__ __forceinline__ int main_bins(int nrp, int wpi) {
-  return nrp * wpi + (kHotRep - 1) * hot_rows(nrp) * wpi;
+static_assert(kMaxSeg == 256, "one candidate slot per thread");
+// Candidate slots per warp: 32; 16 for the corels with many fields, whose
+// staging and queue come out of the Pi window's shared memory (kappa with 32
+// instead of 16: 8.6 -> 7.6 ms on the 200k box; weighted w++: 5.4 -> 6.0).  A
+// warp's queue takes a pass over cand - 1 candidates, at most 32 pairs each, and
+// fewer than 32 left over.
+__host__ __device__ constexpr int cand_slots(int corel) {
+  return corel == COREL_SD || corel == COREL_SS || corel == COREL_SSA ? 16 : 32;
 }
-// bin of copy r (1 <= r < kHotRep) of hot bin (n1, elk), n1 >= nrp - hot_rows(nrp)
-__host__ __device__ __forceinline__ int rep_bin(int r, int n1, int elk, int nrp, int wpi) {
-  const int h = hot_rows(nrp);
-  return nrp * wpi + ((r - 1) * h + (n1 - (nrp - h))) * wpi + elk;
-}
+__host__ __device__ constexpr int ring_size(int corel) { return 32 * cand_slots(corel); }
 
 // Dynamic shared memory of the candidate staging: positions, then (for the
 // corels with values) the weighted ellipticities or orientation and the aux
-// view (x lo, y lo, phi, w lo) of each staged candidate.
-__host__ __device__ constexpr size_t stage_bytes(int corel) {
-  return sizeof(float4) * (corel == COREL_DD ? 2 : 3) * kBatch +
-         (corel == COREL_ED ? sizeof(float) * (kBatch + kTile) : 0);  // ED: z lo parts
+// view (x lo, y lo, phi, w lo) of each staged candidate, and the pair queues.
+__host__ __device__ constexpr size_t stage_bytes(int corel, int warps) {
+  return sizeof(float4) * (corel == COREL_DD ? 1 : 3) * warps * cand_slots(corel) +
+         (corel == COREL_ED ? sizeof(float) * (warps * cand_slots(corel) + kTile) : 0) +  // z lo
+         sizeof(unsigned short) * warps * ring_size(corel);
 }
 // Dynamic shared memory of the corels1 (auto pair) rules, after the staging:
 // each staged candidate's input index and each row's thresholds per z image.
-constexpr size_t kAutoBytes = sizeof(int) * (kBatch + 3 * kTile);
+__host__ __device__ constexpr size_t auto_bytes(int corel, int warps) {
+  return sizeof(int) * (warps * cand_slots(corel) + 3 * kTile);
+}
+
+// Block histograms: one record of 32-bit words per (r_p bin, window Pi bin) --
+// the pair count, then per field a high and a low word (df_to_words) -- so that a
+// pair's words are at compile-time offsets from one address.  Records have an
+// odd number of words: the records' banks spread like their indices.  Twin jobs
+// append the other order's order-dependent fields to the main record.  Unit
+// weights (f0 = 1): field 0, equal to the count, has no words.
+__host__ __device__ constexpr int rec_words(int fields, int f0, int fa) {
+  return 1 + 2 * (fields - f0 + fa);
+}
 
 // Shared-memory bytes a block needs for a job with nrp r_p bins and a wpi-bin
-// Pi window.  With unit weights (unit_w) field 0 (the weight sum, equal to the
-// count) is not accumulated and has no words.  A twin job adds the other
-// order's order-dependent main fields and its two region histograms.
+// Pi window: the staging, the main histogram, with jackknife the two region
+// histograms, in a twin job the other order's two.
 size_t fast_smem_bytes(int corel, int do_jk, int nrp, int wpi, int auto_pairs, int unit_w,
-                       int twin) {
-  const int NB = nrp * wpi, NBm = main_bins(nrp, wpi);
+                       int twin, int variant) {
+  const int NB = nrp * wpi;
   int FM = 1, FJ = 1;
   if (corel == COREL_SD) { FM = 7; FJ = 4; }
   if (corel == COREL_SS) { FM = 11; FJ = 6; }
@@ -116,54 +116,48 @@ size_t fast_smem_bytes(int corel, int do_jk, int nrp, int wpi, int auto_pairs, i
   if (corel == COREL_DK) { FM = 2; FJ = 2; }
   if (corel == COREL_SK) { FM = 4; FJ = 4; }
   if (corel == COREL_ED) { FM = 3; FJ = 2; }
-  const int FA = corel == COREL_SS ? FieldMap<COREL_SS>::FA : 0;
+  const int FA = twin && corel == COREL_SS ? FieldMap<COREL_SS>::FA : 0;
   const int f0 = unit_w ? 1 : 0;
-  FM -= f0;
-  FJ -= f0;
-  size_t b = stage_bytes(corel) + (auto_pairs ? kAutoBytes : 0);  // staging
-  b += 8ull * FM * NBm + 4ull * NBm + 4ull * hi_pad(FM * NBm);
-  if (do_jk) b += 2 * (8ull * FJ * NB + 4ull * NB + 4ull * hi_pad(FJ * NB));
-  if (twin) {
-    b += 8ull * FA * NB + 4ull * hi_pad(FA * NB);
-    if (do_jk) b += 2 * (8ull * FJ * NB + 4ull * NB + 4ull * hi_pad(FJ * NB));
-  }
+  const int warps = variant_threads(variant) / 32;
+  size_t b = stage_bytes(corel, warps) + (auto_pairs ? auto_bytes(corel, warps) : 0);
+  b += 4ull * NB * rec_words(FM, f0, FA);
+  if (do_jk) b += 4ull * NB * rec_words(FJ, f0, 0) * (twin ? 4 : 2);
   return b;
 }
 
 // Fixed-point sums in 32-bit shared words.  A term v of field f becomes the
-// integer u = rint(v * 2^S_f), |u| < 2^29 (S_f from a bound on |v|); u is split
-// into its low 15 bits (0..32767) and the arithmetic shift u >> 15
-// (-2^14..2^14 - 1), each added to its own 32-bit word with a plain reduction
-// (no return value: no scoreboard wait; lanes of one instruction that hit the
-// same word are serialised, which red_pair halves).  A block counts the pairs
-// its warps queued since the last flush and flushes before a chunk that could
-// take the count past 2^17 (a chunk adds at most kTile * kChunk = 2^17 pairs),
-// so a bin takes at most 2^17 terms between flushes: the low word stays below
-// 2^32 and the high word, read as a signed integer, within [-2^31, 2^31).
-constexpr unsigned kFlushTerms = 1u << 17;
-static_assert((unsigned)kTile * kChunk <= kFlushTerms, "a chunk fits between flushes");
-// The two reductions of one term, even lanes taking the low word first and odd
-// lanes the high word first: lanes of one instruction that hit the same bin then
-// split over two addresses 16 banks apart (same-address shared reductions are
-// serialised), halving those collisions.
-// wa, wb: the lane's two words in that order (low, high for even lanes).
-__device__ __forceinline__ void red_pair(unsigned *lo, unsigned *hi, unsigned wa, unsigned wb,
-                                         bool odd) {
-  atomicAdd(odd ? hi : lo, wa);
-  atomicAdd(odd ? lo : hi, wb);
+// integer u = rint(v * 2^S_f), |u| < 2^29 (S_f from a bound on |v|), split into
+// a high part of at most 2^14 and a signed low part of at most 2^14 + 1, each
+// added with its bias (df_to_words) to its own 32-bit word with a plain
+// reduction (no return value: no scoreboard wait).  A bin takes at most kBinTerms
+// pairs between flushes, so that a word, read as a signed integer after its
+// bin's count of biases is taken off, stays within 2^31: a block keeps a bound
+// on the fullest bin (its last known maximum plus every pair tested since),
+// finds the maximum when the bound could pass kBinTerms and flushes when the
+// maximum itself could.  (Bounding the block's pair total instead flushed
+// almost every thousand candidates.)
+constexpr int kBinTerms = (1 << 17) - 64;
+// candidates a bin bound takes at a time: half of kBinTerms for a full tile
+constexpr int kChunkTests = 1 << 16;
+__device__ __forceinline__ long long fixed_sum(const unsigned *w, unsigned bias) {
+  return (long long)(int)(w[0] - bias) * 32768ll + (int)(w[1] - bias);
 }
-__device__ __forceinline__ double fixed_total(unsigned lw, unsigned hw, double inv_scale) {
-  const long long tot = (long long)(int)hw * 32768ll + (long long)lw;
-  return (double)tot * inv_scale;
-}
-
-__device__ __forceinline__ int gcd_int(int a, int b) {
-  while (b) {
-    const int r = a % b;
-    a = b;
-    b = r;
-  }
-  return a;
+// Order of a lane's reductions.  Lanes of one instruction that hit the same bin
+// are serialised (a cycle each), and the pairs of a tile concentrate on a few
+// r_p bins: 32 pairs drawn from a (tile, group) of the 200k wg+ box put 6.2 on
+// the fullest bank when every lane adds the same word, 4.7 when odd lanes take
+// the two words of a field in the other order, 3.9 when the four words of two
+// fields go in the order k ^ (lane & 3).  (Eight words: 3.5, for a third select
+// per word.)
+// The four words h0 l0 h1 l1 of two fields as this lane's 1st .. 4th.
+__device__ __forceinline__ void order4(unsigned h0, unsigned l0, unsigned h1, unsigned l1, int lane,
+                                       unsigned o[4]) {
+  const bool a = lane & 1, b = lane & 2;
+  const unsigned x0 = a ? l0 : h0, x1 = a ? h0 : l0, x2 = a ? l1 : h1, x3 = a ? h1 : l1;
+  o[0] = b ? x2 : x0;
+  o[1] = b ? x3 : x1;
+  o[2] = b ? x0 : x2;
+  o[3] = b ? x1 : x3;
 }
 
 __device__ __forceinline__ int floordiv(int a, int b) {
@@ -198,208 +192,184 @@ __device__ __forceinline__ void enqueue(int job, int64_t i1, int64_t j2, int cod
   }
 }
 
-// ephi_calc (calcs.cpp:97-105) in FP32
-__device__ __forceinline__ float ephi_f(float phi, float theta) {
-  float t = fabsf(phi - theta);
-  return t > 1.5707963267948966f ? 3.14159265358979f - t : t;
-}
-
-// Flush the partner-region histogram (jackknife fields) into the global FP64
-// block at histogram index h, and zero it.  mirror: the histogram holds the
-// other order of twin pairs, whose Pi bin is npi - 1 - (the window's bin).
+// Flush a region histogram (jackknife fields) into the global FP64 block at
+// histogram index h, and zero it.  mirror: the histogram holds the other order
+// of twin pairs, whose Pi bin is npi - 1 - (the window's bin).
 template <class FMAP>
-__device__ __forceinline__ void flush_region(unsigned *cnt, unsigned *lo, unsigned *hi, int NB,
-                                             int wpi, int npi, int nrp, int n2_base, int h, int f0,
-                                             const double *s_iqs, const JobDev &J,
-                                             bool mirror = false) {
+__device__ __noinline__ void flush_region(unsigned *H, int NB, int wpi, int npi, int nrp,
+                                          int n2_base, int h, int f0, const double *s_iqs,
+                                          const JobDev &J, bool mirror) {
   const int64_t hb = (int64_t)h * nrp * npi;
-  for (int lb = threadIdx.x; lb < NB; lb += kThreads) {
-    const unsigned n = cnt[lb];
+  const int S = rec_words(FMAP::FJ, f0, 0);
+  for (int lb = threadIdx.x; lb < NB; lb += blockDim.x) {
+    unsigned *r = H + lb * S;
+    const unsigned n = r[0];
     if (!n) continue;
     const int n2 = n2_base + lb % wpi;
     const int64_t cell = hb + (int64_t)(lb / wpi) * npi + (mirror ? npi - 1 - n2 : n2);
     atomicAdd(&J.acc_num[cell], (unsigned long long)n);
-    cnt[lb] = 0u;
+    r[0] = 0u;
+    const unsigned bias = n * kMagicBits;
 #pragma unroll
     for (int g = 0; g < FMAP::FJ; g++) {
       if (g < f0) continue;  // field 0 of unit weights: no words
-      const size_t o = (size_t)g * NB + lb;
+      unsigned *w = r + 1 + 2 * (g - f0);
       const int fld = FMAP::j(g);
-      const double v = fixed_total(lo[o], hi[o], s_iqs[fld]);
-      if (v != 0.0) atomicAdd(&J.acc_sums[cell * kNF + fld], v);
-      lo[o] = 0u;
-      hi[o] = 0u;
+      const long long v = fixed_sum(w, bias);
+      if (v != 0) atomicAdd(&J.acc_sums[cell * kNF + fld], (double)v * s_iqs[fld]);
+      w[0] = 0u;
+      w[1] = 0u;
     }
   }
 }
 
-// The histograms of the other order of twin pairs (a twin job's block): its
-// order-dependent main fields (FA words per bin, low and high) and its two
-// region histograms (the tile's region: the pairs it does not take; the
-// partner's region), all indexed by the window bin of the pair's own order.
-struct TwinHist {
-  bool on;
-  unsigned *alo, *ahi;              // order-dependent main fields [FA][NB]
-  unsigned *ncnt, *nlo, *nhi;       // tile's region, pairs it does not take
-  unsigned *ycnt, *ylo, *yhi;       // partner's region
+// A block's histograms: main; with jackknife the pairs the tile's own region
+// does not take (nx) and the partner's region (y); in a twin job the same two of
+// the other order, indexed by the window bin of the pair's own order.
+struct BlockHist {
+  unsigned *main, *nx, *y, *tnx, *ty;
 };
 
 // Flush the main histogram (into h = 0) and the tile's region (into hx): the
-// region takes main minus NX, in exact integer arithmetic; zero both.
-// Main bins are strided by NBm (main_bins: the hot bins' copies after the NB
-// plain bins); the copies of a hot bin are summed into it.  Twin blocks also
-// add the other order of each bin's pairs to the mirrored Pi bin
+// region takes main minus NX, in exact integer arithmetic; zero both.  Twin
+// blocks also add the other order of each bin's pairs to the mirrored Pi bin
 // npi - 1 - n2: the same count and order-independent sums, its own
 // order-dependent sums, and its own tile-region exclusions.
-template <int FM, int FJ, class FMAP>
-__device__ __forceinline__ void flush_main_x(unsigned *mcnt, unsigned *mlo, unsigned *mhi,
-                                             unsigned *ncnt, unsigned *nlo, unsigned *nhi, int NB,
-                                             int NBm, int wpi, int npi, int nrp, int n2_base,
-                                             int hx, bool jk, int f0, const double *s_iqs,
-                                             const JobDev &J, const TwinHist &tw) {
+template <class FMAP, bool TW>
+__device__ __noinline__ void flush_main_x(const BlockHist &B, int NB, int wpi, int npi, int nrp,
+                                          int n2_base, int hx, bool jk, int f0,
+                                          const double *s_iqs, const JobDev &J) {
+  constexpr int FM = FMAP::FM, FJ = FMAP::FJ, FA = TW ? FMAP::FA : 0;
   const int64_t hsz = (int64_t)nrp * npi;
-  const int hot0 = nrp - hot_rows(nrp);
-  constexpr int FA = FMAP::FA > 0 ? FMAP::FA : 1;
-  for (int lb = threadIdx.x; lb < NB; lb += kThreads) {
-    const int n1 = lb / wpi, elk = lb - n1 * wpi;
-    const int nrep = (kHotRep > 1 && n1 >= hot0) ? kHotRep : 1;
-    unsigned n = mcnt[lb];
-    for (int r = 1; r < nrep; r++) n += mcnt[rep_bin(r, n1, elk, nrp, wpi)];
+  const int S = rec_words(FM, f0, FA), SJ = rec_words(FJ, f0, 0);
+  for (int lb = threadIdx.x; lb < NB; lb += blockDim.x) {
+    unsigned *r = B.main + lb * S;
+    const unsigned n = r[0];
     if (!n) continue;  // no pair in this bin since the last flush: every word is 0
+    const int n1 = lb / wpi, elk = lb - n1 * wpi;
     const int64_t cell = (int64_t)n1 * npi + n2_base + elk;
     atomicAdd(&J.acc_num[cell], (unsigned long long)n);
-    mcnt[lb] = 0u;
-    for (int r = 1; r < nrep; r++) mcnt[rep_bin(r, n1, elk, nrp, wpi)] = 0u;
+    r[0] = 0u;
+    const unsigned bias = n * kMagicBits;
     long long tm[FM];
 #pragma unroll
     for (int f = 0; f < FM; f++) {
       tm[f] = 0;
       if (f < f0) continue;  // field 0 of unit weights: no words
-      for (int r = 0; r < nrep; r++) {
-        const size_t o = (size_t)f * NBm + (r == 0 ? lb : rep_bin(r, n1, elk, nrp, wpi));
-        tm[f] += (long long)(int)mhi[o] * 32768ll + (long long)mlo[o];
-        mlo[o] = 0u;
-        mhi[o] = 0u;
-      }
+      unsigned *w = r + 1 + 2 * (f - f0);
+      tm[f] = fixed_sum(w, bias);
+      w[0] = 0u;
+      w[1] = 0u;
       const int fld = FMAP::m(f);
       if (tm[f] != 0) atomicAdd(&J.acc_sums[cell * kNF + fld], (double)tm[f] * s_iqs[fld]);
     }
-    long long ta[FA];
+    long long ta[FA > 0 ? FA : 1];
     const int64_t cm = (int64_t)n1 * npi + (npi - 1 - (n2_base + elk));
-    if (tw.on) {
+    if (TW) {
       atomicAdd(&J.acc_num[cm], (unsigned long long)n);
 #pragma unroll
-      for (int i = 0; i < FMAP::FA; i++) {
-        const size_t o = (size_t)i * NB + lb;
-        ta[i] = (long long)(int)tw.ahi[o] * 32768ll + (long long)tw.alo[o];
-        tw.alo[o] = 0u;
-        tw.ahi[o] = 0u;
+      for (int i = 0; i < FA; i++) {
+        unsigned *w = r + 1 + 2 * (FM - f0 + i);
+        ta[i] = fixed_sum(w, bias);
+        w[0] = 0u;
+        w[1] = 0u;
       }
 #pragma unroll
       for (int f = 0; f < FM; f++) {
         if (f < f0) continue;
-        const int ap = asym_pos<FMAP>(f);
+        const int ap = FA > 0 ? asym_pos<FMAP>(f) : -1;
         const long long v = ap >= 0 ? ta[ap] : tm[f];
         const int fld = FMAP::m(f);
         if (v != 0) atomicAdd(&J.acc_sums[cm * kNF + fld], (double)v * s_iqs[fld]);
       }
     }
     if (!jk) continue;
-    const int64_t xc = (int64_t)hx * hsz + cell;
-    const unsigned nx = ncnt[lb];
-    ncnt[lb] = 0u;
-    if (n - nx) atomicAdd(&J.acc_num[xc], (unsigned long long)(n - nx));
 #pragma unroll
-    for (int g = 0; g < FJ; g++) {
-      if (g < f0) continue;
-      const size_t o = (size_t)g * NB + lb;
-      const long long tn = (long long)(int)nhi[o] * 32768ll + (long long)nlo[o];
-      nlo[o] = 0u;
-      nhi[o] = 0u;
-      const long long tx = tm[FMAP::jm(g)] - tn;
-      const int fld = FMAP::j(g);
-      if (tx != 0) atomicAdd(&J.acc_sums[xc * kNF + fld], (double)tx * s_iqs[fld]);
-    }
-    if (!tw.on) continue;
-    const int64_t xm = (int64_t)hx * hsz + cm;
-    const unsigned nxm = tw.ncnt[lb];
-    tw.ncnt[lb] = 0u;
-    if (n - nxm) atomicAdd(&J.acc_num[xm], (unsigned long long)(n - nxm));
+    for (int o = 0; o < (TW ? 2 : 1); o++) {  // the pair's own order, then the other
+      unsigned *x = (o == 0 ? B.nx : B.tnx) + lb * SJ;
+      const int64_t xc = (int64_t)hx * hsz + (o == 0 ? cell : cm);
+      const unsigned nx = x[0], xb = nx * kMagicBits;
+      x[0] = 0u;
+      if (n - nx) atomicAdd(&J.acc_num[xc], (unsigned long long)(n - nx));
 #pragma unroll
-    for (int g = 0; g < FJ; g++) {
-      if (g < f0) continue;
-      const size_t o = (size_t)g * NB + lb;
-      const long long tn = (long long)(int)tw.nhi[o] * 32768ll + (long long)tw.nlo[o];
-      tw.nlo[o] = 0u;
-      tw.nhi[o] = 0u;
-      const int ap = asym_pos<FMAP>(FMAP::jm(g));
-      const long long tx = (ap >= 0 ? ta[ap] : tm[FMAP::jm(g)]) - tn;
-      const int fld = FMAP::j(g);
-      if (tx != 0) atomicAdd(&J.acc_sums[xm * kNF + fld], (double)tx * s_iqs[fld]);
+      for (int g = 0; g < FJ; g++) {
+        if (g < f0) continue;
+        unsigned *w = x + 1 + 2 * (g - f0);
+        const long long tn = fixed_sum(w, xb);
+        w[0] = 0u;
+        w[1] = 0u;
+        const int ap = (FA > 0 && o == 1) ? asym_pos<FMAP>(FMAP::jm(g)) : -1;
+        const long long tx = (ap >= 0 ? ta[ap] : tm[FMAP::jm(g)]) - tn;
+        const int fld = FMAP::j(g);
+        if (tx != 0) atomicAdd(&J.acc_sums[xc * kNF + fld], (double)tx * s_iqs[fld]);
+      }
     }
   }
 }
 
-constexpr int kQCap = 64;  // per-warp ring of binned pairs awaiting the heavy step
 constexpr unsigned kEdgeFlag = 0x8000u;  // queue entry: near the window edge
 
-// MINB: blocks per SM the registers are bounded for (4 when the job's
-// histograms fit a quarter of shared memory, else 3).  TW: twin jobs (every job
+// VAR: the variant (variant_threads; 0: the FP64 comparison engine).  TW: twin jobs (every job
 // of the launch), compiled apart so that the other jobs' kernel carries none of
 // the twin code.
-template <int C, bool JK, int MINB, bool TW>
-__global__ void __launch_bounds__(kThreads, MINB == 1 ? 2 : MINB)
+template <int C, bool JK, int VAR, bool TW>
+__global__ void __launch_bounds__(variant_threads(VAR), variant_blocks(VAR))
 fast_pairs_kernel(const JobDev *__restrict__ jobs, const UnitDesc *__restrict__ units,
                   int n_units, unsigned int *__restrict__ unit_ctr, QEntry *__restrict__ queue,
                   unsigned long long *__restrict__ qcount, unsigned long long qcap,
                   const __grid_constant__ FastScales sc, int zero_words, int auto_smem) {
   using F = FieldMap<C>;
+  constexpr int kThreads = variant_threads(VAR), kWarps = kThreads / 32;
+  constexpr int kCand = cand_slots(C), kSlots = kWarps * kCand, kRing = ring_size(C);
+  constexpr int FA = TW ? F::FA : 0;
+  const unsigned FULL = 0xffffffffu;
   extern __shared__ __align__(16) unsigned char smem[];
   float4 *s_pos = reinterpret_cast<float4 *>(smem);
-  float4 *s_shp = s_pos + kBatch;
-  float4 *s_aux = s_shp + kBatch;  // x lo, y lo, phi, w lo of each staged candidate
+  // s_rshp / s_shp hold the weighted ellipticities (ewt) for the corels with
+  // shape terms and the orientation (shp) for ED; s_aux: x lo, y lo, phi, w lo
+  float4 *s_shp = s_pos + kSlots, *s_aux = s_shp + kSlots;
   // ED: z lo parts of the staged candidates and of the tile's rows
-  float *s_zlo = reinterpret_cast<float *>(smem + sizeof(float4) * 3 * kBatch);
-  float *s_rzlo = s_zlo + kBatch;
+  float *s_zlo = reinterpret_cast<float *>(s_pos + (C == COREL_DD ? 1 : 3) * kSlots);
+  float *s_rzlo = s_zlo + kSlots;
+  unsigned short *wq =
+      reinterpret_cast<unsigned short *>(C == COREL_ED ? s_rzlo + kTile : s_zlo) +
+      (threadIdx.x >> 5) * kRing;
   // corels1 rules (launches with auto-pair jobs only): the input index of each
   // staged candidate; per row and z image (index sz + 1) a threshold on the
   // partner's input index: -1 every partner (and every pair outside corels1),
   // the row's own index: partners after it, INT_MAX: none
-  int *s_orig = auto_smem ? reinterpret_cast<int *>(smem + stage_bytes(C)) : nullptr;
-  int *s_rothr = auto_smem ? s_orig + kBatch : nullptr;
-  unsigned char *hist_base = smem + stage_bytes(C) + (auto_smem ? kAutoBytes : 0);
+  int *s_orig = auto_smem ? reinterpret_cast<int *>(smem + stage_bytes(C, kWarps)) : nullptr;
+  int *s_rothr = auto_smem ? s_orig + kSlots : nullptr;
+  unsigned *hist = reinterpret_cast<unsigned *>(smem + stage_bytes(C, kWarps) +
+                                                (auto_smem ? auto_bytes(C, kWarps) : 0));
   // the candidate slots of a unit, used only while the staging buffer is idle
   // (between the unit's slot set-up barriers, before any candidate is staged)
   int *s_slot_b = reinterpret_cast<int *>(s_pos);
   int *s_slot_info = s_slot_b + kMaxSeg;
-  static_assert(2 * kMaxSeg * sizeof(int) <= kBatch * sizeof(float4), "slot tables fit the staging buffer");
+  static_assert(2 * kMaxSeg * sizeof(int) <= kSlots * sizeof(float4), "slot tables fit the staging");
 
-  __shared__ int s_unit;
+  __shared__ int s_unit, s_nseg, s_ngrp;
+  __shared__ float s_zr[2][3];  // the unit's candidate z range per z image
   __shared__ int s_cnt[kMaxCols + 1];
-  __shared__ int s_seg_a[kMaxSeg], s_seg_len[kMaxSeg], s_seg_key[kMaxSeg];
-  __shared__ int s_order[kMaxSeg], s_pre[kMaxSeg + 1];
-  __shared__ int s_jidx[kBatch];
-  __shared__ unsigned char s_keep[kBatch];
+  // candidate runs sorted by (partner region, image): start, prefix of the
+  // lengths, key; s_grp: first run of each group of one key
+  __shared__ int s_run_a[kMaxSeg], s_pre[kMaxSeg + 1], s_key[kMaxSeg], s_grp[kMaxSeg + 1];
+  __shared__ __align__(16) int s_comp[kMaxSeg];
+  __shared__ int s_jidx[kSlots];
+  __shared__ unsigned char s_keep[kSlots];
   // twin jobs: the other role's keep flag of each staged candidate (g1's) and of
   // each tile row (g2's)
-  __shared__ unsigned char s_keep2[TW ? kBatch : 1];
-  __shared__ unsigned long long s_red[kThreads / 32];
-  __shared__ unsigned s_nbin;  // pairs queued by the block's warps since the last flush
-  __shared__ float s_A[kMaxRp], s_B[kMaxRp], s_PA[kMaxPi], s_PB[kMaxPi];
+  __shared__ unsigned char s_keep2[TW ? kSlots : 1];
+  __shared__ unsigned long long s_red[kWarps];
+  __shared__ int s_max[2];  // pairs in the fullest bin, by turns
   // the tile's g1 rows, for the heavy step (any lane may process any row)
-  // s_rshp / s_shp hold the weighted ellipticities (ewt) for the corels with
-  // shape terms and the orientation (shp) for ED
-  __shared__ float4 s_rpos[kTile], s_rshp[kTile], s_raux[kTile];
+  __shared__ float4 s_rpos[kTile], s_rshp[C == COREL_DD ? 1 : kTile], s_raux[C == COREL_DD ? 1 : kTile];
   __shared__ unsigned char s_rkeep[kTile], s_rkeep2[TW ? kTile : 1];
-  __shared__ unsigned s_wq[kThreads / 32][kQCap];
 
   const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
-  const unsigned lt_mask = (1u << lane) - 1u;
-  {
-    unsigned int *z = reinterpret_cast<unsigned int *>(hist_base);
-    for (int k = t; k < zero_words; k += kThreads) z[k] = 0u;
-    if (t == 0) s_nbin = 0u;
-  }
+  for (int k = t; k < zero_words; k += kThreads) hist[k] = 0u;
+  if (t < 2) s_max[t] = 0;
+  int bound = 0, turn = 0;  // bound of the pairs in any bin; the s_max in use
   __syncthreads();
 
   for (;;) {
@@ -410,683 +380,623 @@ fast_pairs_kernel(const JobDev *__restrict__ jobs, const UnitDesc *__restrict__ 
     const UnitDesc U = units[u];
     const JobDev &J = jobs[U.job];
     const int nrp = J.nrp, wpi = J.wpi, npi = J.npi, NB = nrp * wpi;
-    const int NBm = main_bins(nrp, wpi), hot0 = nrp - hot_rows(nrp);
-    // per histogram: count[NB], low words [F][NB], high words [F][NB] (main:
-    // NBm bins, the hot bins' copies included).  Unit weights: wt_num = count,
-    // field 0 is not accumulated and gets no words; the word arrays are indexed
-    // by field f >= f0 from a base f0 rows before their first stored row (which
-    // then coincides with the count array, never read through it).
     const int f0 = J.unit_w ? 1 : 0;
-    const int FMs = F::FM - f0, FJs = F::FJ - f0;  // stored fields
-    unsigned *s_mnum = reinterpret_cast<unsigned *>(hist_base);
-    // the high words sit hi_pad words after a 32-word-aligned offset from the low
-    // words, so the low and high word of one bin are 16 banks apart (red_pair)
-    unsigned *s_mlo0 = s_mnum + NBm;
-    unsigned *s_mhi0 = s_mlo0 + (size_t)FMs * NBm + hi_pad(FMs * NBm);
-    unsigned *s_nxnum = s_mhi0 + (size_t)FMs * NBm;
-    unsigned *s_nxlo0 = s_nxnum + NB;
-    unsigned *s_nxhi0 = s_nxlo0 + (size_t)FJs * NB + hi_pad(FJs * NB);
-    unsigned *s_ynum = s_nxhi0 + (size_t)FJs * NB;
-    unsigned *s_ylo0 = s_ynum + NB;
-    unsigned *s_yhi0 = s_ylo0 + (size_t)FJs * NB + hi_pad(FJs * NB);
-    unsigned *s_mlo = s_mlo0 - (size_t)f0 * NBm, *s_mhi = s_mhi0 - (size_t)f0 * NBm;
-    unsigned *s_nxlo = s_nxlo0 - (size_t)f0 * NB, *s_nxhi = s_nxhi0 - (size_t)f0 * NB;
-    unsigned *s_ylo = s_ylo0 - (size_t)f0 * NB, *s_yhi = s_yhi0 - (size_t)f0 * NB;
-    // twin jobs: the other order's histograms after the region histograms
-    constexpr bool twin = TW;
-    constexpr int FA = F::FA;
-    TwinHist tw;
-    {
-      unsigned *base = JK ? s_yhi0 + (size_t)FJs * NB : s_nxnum;
-      tw.on = twin;
-      tw.alo = base;
-      tw.ahi = tw.alo + (size_t)FA * NB + hi_pad(FA * NB);
-      tw.ncnt = tw.ahi + (size_t)FA * NB;
-      unsigned *nlo0 = tw.ncnt + NB;
-      unsigned *nhi0 = nlo0 + (size_t)FJs * NB + hi_pad(FJs * NB);
-      tw.ycnt = nhi0 + (size_t)FJs * NB;
-      unsigned *ylo0 = tw.ycnt + NB;
-      unsigned *yhi0 = ylo0 + (size_t)FJs * NB + hi_pad(FJs * NB);
-      tw.nlo = nlo0 - (size_t)f0 * NB;
-      tw.nhi = nhi0 - (size_t)f0 * NB;
-      tw.ylo = ylo0 - (size_t)f0 * NB;
-      tw.yhi = yhi0 - (size_t)f0 * NB;
-    }
+    const int S = rec_words(F::FM, f0, FA), SJ = rec_words(F::FJ, f0, 0);
+    BlockHist B;
+    B.main = hist;
+    B.nx = B.main + NB * S;
+    B.y = B.nx + NB * SJ;
+    B.tnx = B.y + NB * SJ;
+    B.ty = B.tnx + NB * SJ;
 
     // ---- the tile's g1 rows, in shared memory.  Row slot tr = s * 32 + l holds
     // tile row q = l * W + s (s < W): a warp holds slots s * 32 .. s * 32 + 31 in
     // its pass s, so its lanes are spread over the whole tile and simultaneous
     // pairs of a warp fall in different Pi bins.  Every warp tests its own
-    // candidates against every row, one pass of 32 rows at a time. ----
+    // candidates against every row, one pass of 32 rows at a time; tiles of at
+    // most 16 (8) rows take 2 (4) candidates per step. ----
     const int W = (U.g1_count + 31) >> 5;
+    const int rlanes = U.g1_count <= 8 ? 8 : U.g1_count <= 16 ? 16 : 32;
+    const int nsub = 32 / rlanes, sub = lane / rlanes, rl = lane & (rlanes - 1);
     // hi + lo positions for the orientation angle (raw separations) and the ED
     // separation
     constexpr bool kTheta = C == COREL_SD || C == COREL_SS || C == COREL_SSA || C == COREL_SK;
     const bool has_lo = (kTheta || C == COREL_ED) && J.has_lo;
-    const int rmu = J.rmu;
-    // MINB == 1: the cell-list FP64 comparison engine (CPC_ENGINE_CELL_FP64): every
+    const bool rmu = J.rmu != 0, lin = J.lin_bin != 0;
+    // VAR == 0: the cell-list FP64 comparison engine (CPC_ENGINE_CELL_FP64): every
     // candidate inside the outer window bounds is evaluated by the FP64 path,
     // inline, with global atomics (no FP32 value, no shared histogram)
-    constexpr bool all_exact = MINB == 1;
+    constexpr bool all_exact = VAR == 0;
     // jackknife attribution: jk_check_PB (the box's rule; this kernel runs box
     // jobs only)
-    const int gws = J.gws, lin_bin = J.lin_bin;
-    const float rmin_f = J.rmin_f, inv_rsize_f = J.inv_rsize_f;
-    for (int tr = t; tr < 32 * W; tr += kThreads) {
-      const int q = (tr & 31) * W + (tr >> 5);
-      float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
-      unsigned char ok = 0, af = 0;
+    const int gws = J.gws;
+    if (t < kTile && (t >> 5) < W) {
+      const int q = (t & 31) * W + (t >> 5);
+      // a row that is not counted is infinitely far: every window test fails
+      float4 p = make_float4(0.f, 0.f, INFINITY, 0.f);
+      unsigned char af = 0;
       int oi = 0;
       if (q < U.g1_count) {
         const int64_t i1 = (int64_t)U.g1_start + (int64_t)q * U.g1_stride;
         p = J.f1.pos[i1];
-        ok = 1;
         if (J.auto_mode) {
           oi = (int)J.d1.orig[i1];  // input index (corels1)
           af = J.f1.aflag[i1];      // corels1 scan-start flags
         }
-        if (J.row_stride > 1) {
-          const int64_t o = J.d1.orig[i1] - J.row_offset;
-          ok = (o % J.row_stride) == 0;
-        }
+        if (J.row_stride > 1 && (J.d1.orig[i1] - J.row_offset) % J.row_stride != 0) p.z = INFINITY;
         if (C != COREL_DD) {
-          s_rshp[tr] = C == COREL_ED ? J.f1.shp[i1] : J.f1.ewt[i1];
-          s_raux[tr] = J.f1.aux[i1];
+          s_rshp[t] = C == COREL_ED ? J.f1.shp[i1] : J.f1.ewt[i1];
+          s_raux[t] = J.f1.aux[i1];
         }
-        if (C == COREL_ED && has_lo) s_rzlo[tr] = J.f1.zlo[i1];
-        if (JK) s_rkeep[tr] = J.f1.keep[i1];
-        if (JK && TW) s_rkeep2[tr] = J.f2.keep[i1];
+        if (C == COREL_ED && has_lo) s_rzlo[t] = J.f1.zlo[i1];
+        if (JK) s_rkeep[t] = J.f1.keep[i1];
+        if (JK && TW) s_rkeep2[t] = J.f2.keep[i1];
       }
-      // a row that is not counted gets z = NaN: every window test fails
-      if (!ok) p.z = __int_as_float(0x7fc00000);
-      s_rpos[tr] = p;
+      s_rpos[t] = p;
       if (auto_smem)
         for (int z = -1; z <= 1; z++)
-          s_rothr[(z + 1) * kTile + tr] = auto_image_all(J.auto_mode, z, af) ? -1
-                                          : auto_image_gt(J.auto_mode, z, af) ? oi : INT_MAX;
+          s_rothr[(z + 1) * kTile + t] = auto_image_all(J.auto_mode, z, af) ? -1
+                                         : auto_image_gt(J.auto_mode, z, af) ? oi : INT_MAX;
     }
+    if (t < 6) s_zr[t / 3][t % 3] = (float)((t < 3 ? U.zlo : U.zhi) - J.L * (t % 3 - 1));
     const float Lf = J.Lf;
-    const float xy_in = J.xy_in, xy_out = J.xy_out;
-    const float pi_in_lo = J.pi_in_lo, pi_in_hi = J.pi_in_hi;
-    const float pi_out_lo = J.pi_out_lo, pi_out_hi = J.pi_out_hi;
-    const float inv_ps = J.inv_ps_f, tp0 = J.tp0;
-    const float mu_rel = J.mu_rel, mu_abs = J.mu_abs;
-    for (int k = t; k < nrp; k += kThreads) { s_A[k] = J.A[k]; s_B[k] = J.B[k]; }
-    for (int k = t; k < npi; k += kThreads) { s_PA[k] = J.PA[k]; s_PB[k] = J.PB[k]; }
-    const float l2rmin2 = J.l2rmin2, inv_lw = J.inv_lw, rej_lo = J.rej_lo, rej_hi = J.rej_hi;
+    const float xyc = J.bc.xyc, zc = J.bc.zc, zh = J.bc.zh, gd = J.bc.guard;
+    const float rej_hi = J.bc.rej_hi;
     const int n2_base = U.n2_base;
-    unsigned nwin = 0;  // window pairs of this thread's row in this unit
+    unsigned nwin = 0, nself = 0;  // window pairs of this thread's rows; pairs of a row with itself
+    __syncthreads();
 
     // ---- enumerate candidate slots: (column, bucket, sz) overlapping the unit's z range ----
     const int ncxu = U.cx_hi - U.cx_lo + 1;
     const int ncol = ncxu * (U.cy_hi - U.cy_lo + 1);
     const int nsz_lo = J.periodic ? -1 : 0, nsz_hi = J.periodic ? 1 : 0;
-    for (int c = t; c < ncol; c += kThreads) {
+    // f(bucket, sz, code) for every slot of column c, in order
+    auto slots = [&](int c, auto &&f) {
       const int cx = U.cx_lo + c % ncxu, cy = U.cy_lo + c / ncxu;
       const int sx = J.periodic ? floordiv(cx, J.ncx) : 0, sy = J.periodic ? floordiv(cy, J.ncy) : 0;
-      int cnt = 0;
-      if (sx >= -1 && sx <= 1 && sy >= -1 && sy <= 1) {
-        const int col = (cy - sy * J.ncy) * J.ncx + (cx - sx * J.ncx);
-        const int b0 = J.f2.col_begin[col], b1 = J.f2.col_end[col];
-        for (int b = b0; b < b1; b++) {
-          const float bz0 = J.f2.bk_zmin[b], bz1 = J.f2.bk_zmax[b];
-          for (int sz = nsz_lo; sz <= nsz_hi; sz++) {
-            const float lo = (float)(U.zlo - J.L * sz), hi = (float)(U.zhi - J.L * sz);
-            if (bz1 >= lo && bz0 < hi) cnt++;
-          }
-        }
+      if (sx < -1 || sx > 1 || sy < -1 || sy > 1) return;
+      const int col = (cy - sy * J.ncy) * J.ncx + (cx - sx * J.ncx);
+      const int b1 = J.f2.col_end[col];
+      for (int b = J.f2.col_begin[col]; b < b1; b++) {
+        const float bz0 = J.f2.bk_zmin[b], bz1 = J.f2.bk_zmax[b];
+        for (int sz = nsz_lo; sz <= nsz_hi; sz++)
+          if (bz1 >= s_zr[0][sz + 1] && bz0 < s_zr[1][sz + 1]) f(b, shift_code(sx, sy, sz));
       }
+    };
+    for (int c = t; c < ncol; c += kThreads) {
+      int cnt = 0;
+      slots(c, [&](int, int) { cnt++; });
       s_cnt[c] = cnt;
     }
     __syncthreads();
-    if (t == 0) {
+    if (wid == 0) {  // exclusive prefix over the columns
       int run = 0;
-      for (int c = 0; c < ncol; c++) {
-        const int v = s_cnt[c];
-        s_cnt[c] = run;
-        run += v;
+      for (int c0 = 0; c0 < ncol; c0 += 32) {
+        const int v = c0 + lane < ncol ? s_cnt[c0 + lane] : 0;
+        int p = v;
+        for (int o = 1; o < 32; o <<= 1) {
+          const int w = __shfl_up_sync(FULL, p, o);
+          if (lane >= o) p += w;
+        }
+        if (c0 + lane < ncol) s_cnt[c0 + lane] = run + p - v;
+        run += __shfl_sync(FULL, p, 31);
       }
-      s_cnt[ncol] = run;
+      if (lane == 0) s_cnt[ncol] = run;
     }
     __syncthreads();
     const int total_slots = s_cnt[ncol];
     int cur_y = -1;        // region held in the Y histogram
-    unsigned wbin = 0;     // pairs this warp queued in its current batch
 
     for (int chunk0 = 0; chunk0 < total_slots; chunk0 += kMaxSeg) {
       const int nslot = min(kMaxSeg, total_slots - chunk0);
       for (int c = t; c < ncol; c += kThreads) {
-        int pos = s_cnt[c];
-        if (pos >= chunk0 + kMaxSeg || s_cnt[c + 1] <= chunk0) continue;
-        const int cx = U.cx_lo + c % ncxu, cy = U.cy_lo + c / ncxu;
-        const int sx = J.periodic ? floordiv(cx, J.ncx) : 0, sy = J.periodic ? floordiv(cy, J.ncy) : 0;
-        const int col = (cy - sy * J.ncy) * J.ncx + (cx - sx * J.ncx);
-        const int b0 = J.f2.col_begin[col], b1 = J.f2.col_end[col];
-        for (int b = b0; b < b1; b++) {
-          const float bz0 = J.f2.bk_zmin[b], bz1 = J.f2.bk_zmax[b];
-          for (int sz = nsz_lo; sz <= nsz_hi; sz++) {
-            const float lo = (float)(U.zlo - J.L * sz), hi = (float)(U.zhi - J.L * sz);
-            if (!(bz1 >= lo && bz0 < hi)) continue;
-            const int k = pos - chunk0;
-            if (k >= 0 && k < kMaxSeg) {
-              s_slot_b[k] = b;
-              s_slot_info[k] = shift_code(sx, sy, sz);
-            }
-            pos++;
+        int pos = s_cnt[c] - chunk0;
+        if (pos >= kMaxSeg || s_cnt[c + 1] <= chunk0) continue;
+        slots(c, [&](int b, int code) {
+          if (pos >= 0 && pos < kMaxSeg) {
+            s_slot_b[pos] = b;
+            s_slot_info[pos] = code;
+          }
+          pos++;
+        });
+      }
+      __syncthreads();
+      {  // a run per thread of the first kMaxSeg, ranked by (partner region, image)
+        int a = 0, len = 0, comp = INT_MAX;
+        if (t < nslot) {
+          const int b = s_slot_b[t], code = s_slot_info[t];
+          const int sz = code / 9 - 1;
+          // twin jobs test each unordered pair once, in the order whose g2 is
+          // ahead of g1: image -1 candidates are the other order of image +1
+          // pairs of their own tiles
+          if (!(TW && sz < 0)) {
+            const int bs = J.f2.bk_start[b], be = J.f2.bk_end[b];
+            a = lower_bound_f(J.f2.zf, bs, be, s_zr[0][sz + 1]);
+            len = lower_bound_f(J.f2.zf, a, be, s_zr[1][sz + 1]) - a;
+            if (len > 0) comp = (J.f2.bk_region[b] * 27 + code) * kMaxSeg + t;
           }
         }
-      }
-      __syncthreads();
-      for (int k = t; k < nslot; k += kThreads) {
-        const int b = s_slot_b[k], code = s_slot_info[k];
-        const int sz = code / 9 - 1;
-        const float lo = (float)(U.zlo - J.L * sz), hi = (float)(U.zhi - J.L * sz);
-        const int bs = J.f2.bk_start[b], be = J.f2.bk_end[b];
-        const int a = lower_bound_f(J.f2.zf, bs, be, lo);
-        const int e = lower_bound_f(J.f2.zf, a, be, hi);
-        s_seg_a[k] = a;
-        s_seg_len[k] = e - a;
-        s_seg_key[k] = (e > a) ? J.f2.bk_region[b] * 27 + code : INT_MAX;
-      }
-      __syncthreads();
-      for (int k = t; k < nslot; k += kThreads) {  // stable rank sort by key
-        const int key = s_seg_key[k];
+        if (t < kMaxSeg) s_comp[t] = comp;
+        const unsigned any = __ballot_sync(FULL, comp != INT_MAX);
+        __syncthreads();
         int r = 0;
-        for (int m = 0; m < nslot; m++) {
-          const int km = s_seg_key[m];
-          r += (km < key) || (km == key && m < k);
+        if (any) {
+          const int n4 = (nslot + 3) >> 2;
+          for (int m = 0; m < n4; m++) {
+            const int4 v = reinterpret_cast<const int4 *>(s_comp)[m];
+            r += (v.x < comp) + (v.y < comp) + (v.z < comp) + (v.w < comp);
+          }
         }
-        s_order[r] = k;
+        if (comp != INT_MAX) {
+          s_run_a[r] = a;
+          s_pre[r] = len;
+          s_key[r] = comp / kMaxSeg;
+        }
+        if (t == 0) s_nseg = 0;
+        __syncthreads();
+        if (lane == 0 && any) atomicAdd(&s_nseg, __popc(any));
       }
       __syncthreads();
-      if (t == 0) {
-        int run = 0;
-        for (int k = 0; k < nslot; k++) {
-          s_pre[k] = run;
-          run += s_seg_len[s_order[k]];
+      if (wid == 0) {  // prefix of the run lengths, first run of each group
+        const int n = s_nseg;
+        int run = 0, ng = 0;
+        for (int k0 = 0; k0 < n; k0 += 32) {
+          const int k = k0 + lane;
+          const int v = k < n ? s_pre[k] : 0;
+          int p = v;
+          for (int o = 1; o < 32; o <<= 1) {
+            const int w = __shfl_up_sync(FULL, p, o);
+            if (lane >= o) p += w;
+          }
+          const bool first = k < n && (k == 0 || s_key[k] != s_key[k - 1]);
+          const unsigned m = __ballot_sync(FULL, first);
+          if (k < n) s_pre[k] = run + p - v;
+          if (first) s_grp[ng + __popc(m & ((1u << lane) - 1u))] = k;
+          ng += __popc(m);
+          run += __shfl_sync(FULL, p, 31);
         }
-        s_pre[nslot] = run;
+        if (lane == 0) {
+          s_pre[n] = run;
+          s_grp[ng] = n;
+          s_ngrp = ng;
+        }
       }
       __syncthreads();
 
-      int k = 0;
-      while (k < nslot) {
-        const int key = s_seg_key[s_order[k]];
-        if (key == INT_MAX) break;
-        int g = k + 1;
-        while (g < nslot && s_seg_key[s_order[g]] == key) g++;
+      for (int gi = 0; gi < s_ngrp; gi++) {
+        const int k = s_grp[gi], g = s_grp[gi + 1];
+        const int key = s_key[k];
         const int region2 = key / 27, code = key % 27;
         int sx, sy, sz;
         shift_decode(code, sx, sy, sz);
         const bool same_region = region2 == U.region;
-        // twin jobs test each unordered pair once, in the order whose g2 is
-        // ahead of g1: z image +1, or image 0 with a larger z (ties: the image
-        // shift in y, then x, then the index).  Image -1 candidates are the
-        // other order of image +1 pairs of their own tiles.
-        if (twin && sz < 0) {
-          k = g;
-          continue;
-        }
-        const int tie_dir = sy != 0 ? sy : sx;  // z ties within image 0
-        // staging order: position (i * ks) mod N over the group's N candidates,
-        // ks coprime with N and ~0.618 N, so a batch is a spread-out sample of
-        // the group's columns and z range (decorrelated bins, fewer collisions)
         const int gN = s_pre[g] - s_pre[k];
-        int ks = 1;
-        if (gN > 2) {
-          ks = max(1, (int)(0.6180339887f * gN));
-          while (gcd_int(ks, gN) != 1) ks++;
-        }
         if (JK && !same_region && cur_y != region2) {
           if (cur_y >= 0) {
             __syncthreads();
-            flush_region<F>(s_ynum, s_ylo, s_yhi, NB, wpi, npi, nrp, n2_base,
-                                       1 + cur_y, f0, sc.iqs, J);
-            if (twin)
-              flush_region<F>(tw.ycnt, tw.ylo, tw.yhi, NB, wpi, npi, nrp, n2_base, 1 + cur_y, f0,
-                              sc.iqs, J, true);
+            flush_region<F>(B.y, NB, wpi, npi, nrp, n2_base, 1 + cur_y, f0, sc.iqs, J, false);
+            if (TW)
+              flush_region<F>(B.ty, NB, wpi, npi, nrp, n2_base, 1 + cur_y, f0, sc.iqs, J, true);
             __syncthreads();
           }
           cur_y = region2;
         }
         // g2-side shift for -1 images (x2 - L exact for the candidates that can
-        // reach the window); the g1-side shift for +1 images (x1 - L exact for
-        // x1 >= L/2) is applied per row below
+        // reach the window), g1-side shift for +1 images (x1 - L exact for
+        // x1 >= L/2)
         const float g2sx = sx == -1 ? Lf : 0.f, g2sy = sy == -1 ? Lf : 0.f, g2sz = sz == -1 ? Lf : 0.f;
+        const float g1sx = sx == 1 ? Lf : 0.f, g1sy = sy == 1 ? Lf : 0.f, g1sz = sz == 1 ? Lf : 0.f;
+        // twin jobs, image 0: the order with the larger z of g2 (the sign of a
+        // float difference is exact; ties by the image shift in y, then x, then
+        // the index)
+        const int tie_dir = sy != 0 ? sy : sx;
+        const float zmin = !TW || sz != 0 ? -INFINITY : tie_dir > 0 ? -1e-45f : 0.0f;
+        const bool tie0 = TW && sz == 0 && tie_dir == 0;
 
-        for (int base = 0; base < gN; base += kChunk) {
-          const int nc = min(kChunk, gN - base);
-          // s_nbin is read after a barrier and changed only after the next one
-          if (s_nbin + (unsigned)(kTile * nc) > kFlushTerms) {  // keep every word below 2^32
+        const int chunk = kChunkTests / 32 / W;
+        for (int base = 0; base < gN; base += chunk) {
+          const int nc = min(chunk, gN - base);
+          if (!all_exact && bound + 32 * W * nc > kBinTerms) {  // (block-uniform)
+            int m = 0;
             __syncthreads();
-            flush_main_x<F::FM, F::FJ, F>(s_mnum, s_mlo, s_mhi, s_nxnum, s_nxlo, s_nxhi, NB, NBm,
-                                          wpi, npi, nrp, n2_base, 1 + U.region, JK, f0, sc.iqs,
-                                          J, tw);
-            if (JK && cur_y >= 0) {
-              flush_region<F>(s_ynum, s_ylo, s_yhi, NB, wpi, npi, nrp, n2_base,
-                                         1 + cur_y, f0, sc.iqs, J);
-              if (twin)
-                flush_region<F>(tw.ycnt, tw.ylo, tw.yhi, NB, wpi, npi, nrp, n2_base, 1 + cur_y,
-                                f0, sc.iqs, J, true);
+            for (int lb = t; lb < NB; lb += kThreads) m = max(m, (int)hist[lb * S]);
+            m = __reduce_max_sync(FULL, m);
+            if (lane == 0 && m > 0) atomicMax(&s_max[turn], m);
+            if (t == 0) s_max[turn ^ 1] = 0;
+            __syncthreads();
+            bound = s_max[turn];
+            turn ^= 1;
+            if (bound + 32 * W * nc > kBinTerms) {
+              flush_main_x<F, TW>(B, NB, wpi, npi, nrp, n2_base, 1 + U.region, JK, f0, sc.iqs, J);
+              if (JK && cur_y >= 0) {
+                flush_region<F>(B.y, NB, wpi, npi, nrp, n2_base, 1 + cur_y, f0, sc.iqs, J, false);
+                if (TW)
+                  flush_region<F>(B.ty, NB, wpi, npi, nrp, n2_base, 1 + cur_y, f0, sc.iqs, J, true);
+              }
+              bound = 0;
+              __syncthreads();
             }
-            if (t == 0) s_nbin = 0u;
-            __syncthreads();
           }
-          // this warp's share of the chunk, positions [wlo, wlo + wlen) (an
-          // eighth of it), in nbw batches of at most 32 candidates of even size,
-          // staged in the warp's own slots c0 .. c0 + 31 (read by this warp
-          // only: no block barrier)
-          const int c0 = wid * 32;
-          const int wlo = (wid * nc) / (kThreads / 32);
-          const int wlen = ((wid + 1) * nc) / (kThreads / 32) - wlo;
-          const int nbw = (wlen + 31) >> 5;
+          bound += 32 * W * nc;
+          // this warp's share of the chunk, positions p = wid (mod nw), in nbw
+          // batches of at most kCand - 1 candidates strided over it (columns and
+          // redshifts mixed, so that a warp's pairs fall in different bins),
+          // staged in the warp's own slots c0 .. (read by this warp only: no block
+          // barrier)
+          const int c0 = wid * kCand;
+          const int nw = min(kWarps, max(1, nc >> 3));
+          const int share = wid < nw ? (nc - wid + nw - 1) / nw : 0;
+          const int nbw = (share + kCand - 2) / (kCand - 1);
           for (int bw = 0; bw < nbw; bw++) {
-          const int s0 = wlo + (bw * wlen) / nbw;
-          const int nk = wlo + ((bw + 1) * wlen) / nbw - s0;  // 1 .. 32
-          if (lane < nk) {
-            const int p = s_pre[k] + (int)(((long long)(base + s0 + lane) * ks) % gN);
-            int lo = k, hi = g;  // segment s_order[lo] with s_pre[lo] <= p < s_pre[lo+1]
-            while (hi - lo > 1) {
-              const int mid = (lo + hi) >> 1;
-              if (s_pre[mid] <= p) lo = mid; else hi = mid;
+            const int nk = (share - bw + nbw - 1) / nbw;  // 1 .. kCand - 1
+            if (lane < kCand) {
+              const int slot = c0 + lane;
+              // no candidate: infinitely far from every row (absent rows too)
+              float4 q2 = make_float4(0.f, 0.f, -INFINITY, 0.f);
+              if (lane < nk) {
+                const int p = s_pre[k] + base + (lane * nbw + bw) * nw + wid;
+                int lo = k, hi = g;  // run lo with s_pre[lo] <= p < s_pre[lo + 1]
+                while (hi - lo > 1) {
+                  const int mid = (lo + hi) >> 1;
+                  if (s_pre[mid] <= p) lo = mid; else hi = mid;
+                }
+                const int j2 = s_run_a[lo] + (p - s_pre[lo]);
+                q2 = J.f2.pos[j2];
+                q2.x -= g2sx;
+                q2.y -= g2sy;
+                q2.z -= g2sz;
+                if (C != COREL_DD) {
+                  s_shp[slot] = C == COREL_ED ? J.f2.shp[j2] : J.f2.ewt[j2];
+                  s_aux[slot] = J.f2.aux[j2];
+                }
+                if (C == COREL_ED && has_lo) s_zlo[slot] = J.f2.zlo[j2];
+                s_jidx[slot] = j2;
+                if (auto_smem && J.auto_mode) s_orig[slot] = (int)J.d2.orig[j2];
+                if (JK) s_keep[slot] = J.f2.keep[j2];
+                if (JK && TW) s_keep2[slot] = J.f1.keep[j2];
+              }
+              s_pos[slot] = q2;
             }
-            const int sg = s_order[lo];
-            const int j2 = s_seg_a[sg] + (p - s_pre[lo]);
-            float4 q2 = J.f2.pos[j2];
-            q2.x -= g2sx;
-            q2.y -= g2sy;
-            q2.z -= g2sz;
-            s_pos[t] = q2;
-            if (C != COREL_DD) {
-              s_shp[t] = C == COREL_ED ? J.f2.shp[j2] : J.f2.ewt[j2];
-              s_aux[t] = J.f2.aux[j2];
-            }
-            if (C == COREL_ED && has_lo) s_zlo[t] = J.f2.zlo[j2];
-            s_jidx[t] = j2;
-            if (auto_smem && J.auto_mode) s_orig[t] = (int)J.d2.orig[j2];
-            if (JK) s_keep[t] = J.f2.keep[j2];
-            if (JK && twin) s_keep2[t] = J.f1.keep[j2];
-          }
-          __syncwarp();
+            __syncwarp();
 
-          // ---- light pass over the warp's candidates, row pass by row pass;
-          // binned pairs are queued per warp and the heavy step runs whenever
-          // 32 are queued (all lanes busy).  Lane l at step s takes slot
-          // c0 + (s + l) mod nk, so a warp works on 32 different candidates. ----
-          // row registers of pass `pass` (row slot pass * 32 + lane): the
-          // shifted position and othr, the row's corels1 threshold for this image
-          int pass = 0;
-          float x1s, y1s, z1s;
-          int othr;
-#define CPC_SET_ROW()                                                         \
-  {                                                                           \
-    const int tr_ = pass * 32 + lane;                                         \
-    const float4 p1 = s_rpos[tr_];                                            \
-    x1s = sx == 1 ? p1.x - Lf : p1.x;                                         \
-    y1s = sy == 1 ? p1.y - Lf : p1.y;                                         \
-    z1s = sz == 1 ? p1.z - Lf : p1.z;                                         \
-    othr = auto_smem ? s_rothr[(sz + 1) * kTile + tr_] : -1;                  \
-  }
-          CPC_SET_ROW();
-          int step = 0;
-          int qhead = 0, qtail = 0;
-          int cr = lane % nk;  // (step + lane) mod nk, kept incrementally
-          for (;;) {
-            while (pass < W && (qtail - qhead) < 32) {
-              const int c = c0 + cr;
-              const float4 p2 = s_pos[c];
-              const float dz = p2.z - z1s;
-              const float dx = x1s - p2.x;
-              const float dy = y1s - p2.y;
-              const float m = fmaxf(fabsf(dx), fabsf(dy));
-              bool binned = false, edge = false;
-              // twin jobs, image 0: the order with g2 ahead of g1 (the sign of a
-              // float difference is exact); a pair of a row with itself counts once
-              bool canon = true, tself = false;
-              if (twin && sz == 0 && !(dz > 0.0f)) {
-                canon = false;
-                if (dz == 0.0f) {
-                  if (tie_dir > 0) {
-                    canon = true;
-                  } else if (tie_dir == 0) {
-                    const int gi = U.g1_start + (lane * W + pass) * U.g1_stride;
-                    canon = s_jidx[c] >= gi;
-                    tself = s_jidx[c] == gi;
+            // ---- window tests: a candidate at a time against the lanes' rows, a
+            // bit per step for the pairs that may bin and one for those near the
+            // window's edge; after a pass each lane queues its pairs (a prefix
+            // sum of the bit counts gives its place) and the heavy step runs
+            // while 32 are queued (all lanes busy) ----
+            const int nks = (nk + nsub - 1) / nsub;
+            int pass = 0, qhead = 0, qtail = 0;
+            for (;;) {
+              if (qtail - qhead < 32 && pass < W) {
+                const int tr = pass * 32 + rl;
+                unsigned mask = 0u, emask = 0u;
+                {
+                  const float4 p1 = s_rpos[tr];
+                  const float x1 = p1.x - g1sx, y1 = p1.y - g1sy, z1 = (p1.z - g1sz) + zc;
+                  const int othr = auto_smem ? s_rothr[(sz + 1) * kTile + tr] : -1;
+                  const float4 *cp = s_pos + c0 + sub;
+                  unsigned bit = 1u;
+#pragma unroll 4
+                  for (int st = 0; st < nks; st++) {
+                    const float4 p2 = cp[0];
+                    const float dz = p2.z - z1, dx = x1 - p2.x, dy = y1 - p2.y;
+                    // distance inside the window, the smaller of the two
+                    const float d =
+                        fminf(zh - fabsf(dz), xyc - fmaxf(fabsf(dx), fabsf(dy)));
+                    float r2 = fmaf(dx, dx, dy * dy);
+                    if (rmu) r2 = fmaf(dz, dz, r2);
+                    bool in = d > gd, edge = fabsf(d) <= gd;
+                    if (TW) {
+                      bool ahead = dz > zmin;
+                      if (tie0 && dz == 0.0f) {
+                        const int j2 = s_jidx[c0 + sub + st * nsub];
+                        const int i1 = U.g1_start + (rl * W + pass) * U.g1_stride;
+                        ahead = j2 >= i1;
+                        if (j2 == i1 && d > gd) nself++;
+                      }
+                      in = in && ahead;
+                      edge = edge && ahead;
+                    }
+                    if (auto_smem && othr >= 0) {
+                      const bool ord = s_orig[c0 + sub + st * nsub] > othr;
+                      in = in && ord;
+                      edge = edge && ord;
+                    }
+                    if (all_exact) {
+                      edge = edge || in;
+                    } else {
+                      if (in) nwin++;
+                      // r_p^2 (or r^2 of coordinates 7) certainly above the bins?
+                      if (in && r2 < rej_hi) mask |= bit;
+                    }
+                    if (edge) emask |= bit;
+                    bit += bit;
+                    cp += nsub;
                   }
                 }
+                const int cnt = __popc(mask) + __popc(emask);
+                int sum = cnt;
+                for (int o = 1; o < 32; o <<= 1) {
+                  const int v = __shfl_up_sync(FULL, sum, o);
+                  if (lane >= o) sum += v;
+                }
+                unsigned pos = (unsigned)(qtail + sum - cnt);  // qtail < 2 kRing
+                if (pos >= kRing) pos -= kRing;
+                const unsigned en = (unsigned)tr | (unsigned)(sub << 7);
+                while (mask) {
+                  const int st = 31 - __clz(mask);
+                  mask ^= 1u << st;
+                  wq[pos] = (unsigned short)(en + ((unsigned)(st * nsub) << 7));
+                  if (++pos == kRing) pos = 0;
+                }
+                while (emask) {
+                  const int st = 31 - __clz(emask);
+                  emask ^= 1u << st;
+                  wq[pos] = (unsigned short)((en + ((unsigned)(st * nsub) << 7)) | kEdgeFlag);
+                  if (++pos == kRing) pos = 0;
+                }
+                qtail += __shfl_sync(FULL, sum, 31);
+                pass++;
+                __syncwarp();
+                continue;
               }
-              if (canon && (othr < 0 || s_orig[c] > othr) && dz >= pi_out_lo &&
-                  dz <= pi_out_hi && m <= xy_out) {
-                if (all_exact || !(dz >= pi_in_lo && dz <= pi_in_hi && m <= xy_in)) {
-                  // near the window edge: queued with a flag, the heavy step hands
-                  // it to the exact FP64 evaluation of the whole pair
-                  edge = true;
+              const int take = min(32, qtail - qhead);
+              if (take == 0) break;
+              if (lane < take) {
+                // ---- heavy step for one queued pair ----
+                const int qp = qhead + lane;
+                const unsigned en = wq[qp >= kRing ? qp - kRing : qp];
+                const int er = en & 127, ec = c0 + ((en >> 7) & 31);
+                const bool edge = (en & kEdgeFlag) != 0;
+                const float4 r1 = s_rpos[er];
+                const float4 p2 = s_pos[ec];
+                const float hdz = p2.z - (r1.z - g1sz);
+                const float hdx = (r1.x - g1sx) - p2.x;
+                const float hdy = (r1.y - g1sy) - p2.y;
+                float r2 = fmaf(hdx, hdx, hdy * hdy);
+                // the bins from the linear maps of Pi (or mu) and log2 r^2 (or r):
+                // the nearest integer, certain when farther from the next
+                // half-integer than the error bound (BoxConst)
+                float lim2 = J.bc.pi_in, lim1 = J.bc.rp_in, v2;
+                if (rmu) {
+                  // coordinates 7: r = |(dx, dy, dz)|, mu = dz / r (r_mu_calc)
+                  r2 = fmaf(hdz, hdz, r2);
+                  const float ri = rsqrtf(r2);
+                  v2 = fmaf(hdz * ri, J.bc.pi_s, J.bc.pi_o);
+                  lim2 -= J.bc.pi_abs * ri;
+                  lim1 -= J.bc.rp_abs * ri;
                 } else {
-                  nwin += (twin && !tself) ? 2u : 1u;
-                  // r_p^2, or r^2 = r_p^2 + dz^2 for coordinates 7
-                  float r2 = fmaf(dx, dx, dy * dy);
-                  if (rmu) r2 = fmaf(dz, dz, r2);
-                  binned = r2 >= rej_lo && r2 < rej_hi;
+                  v2 = fmaf(hdz, J.bc.pi_s, J.bc.pi_o);
+                  if (J.bc.rp_abs > 0.0f) lim1 -= J.bc.rp_abs * rsqrtf(r2);
                 }
-              }
-              const bool push = binned || edge;
-              const unsigned bm = __ballot_sync(0xffffffffu, push);
-              if (push)
-                s_wq[wid][(qtail + __popc(bm & lt_mask)) & (kQCap - 1)] =
-                    (unsigned)(pass * 32 + lane) | ((unsigned)c << 7) | (edge ? kEdgeFlag : 0u);
-              qtail += __popc(bm);
-              if (++step == nk) {  // next row pass
-                step = 0;
-                cr = lane % nk;
-                if (++pass < W) CPC_SET_ROW();
-              } else {
-                cr = (cr + 1 == nk) ? 0 : cr + 1;
-              }
-            }
-            const int avail = qtail - qhead;
-            if (avail == 0) break;
-            __syncwarp();
-            const int take = min(avail, 32);
-            if (lane < take) {
-              // ---- heavy step for one queued pair ----
-              const unsigned e = s_wq[wid][(qhead + lane) & (kQCap - 1)];
-              const int er = e & 127, ec = (e >> 7) & 255;
-              const bool edge = (e & kEdgeFlag) != 0;
-              const float4 r1 = s_rpos[er];
-              const float4 p2 = s_pos[ec];
-              // exact bins: approximate index confirmed against the definite bands
-              const float hdz = p2.z - (sz == 1 ? r1.z - Lf : r1.z);
-              const float hdx = (sx == 1 ? r1.x - Lf : r1.x) - p2.x;
-              const float hdy = (sy == 1 ? r1.y - Lf : r1.y) - p2.y;
-              float r2 = fmaf(hdx, hdx, hdy * hdy);
-              bool amb = false, own = true;
-              int n2;
-              if (!rmu) {
-                n2 = (int)floorf(fmaf(hdz, inv_ps, tp0));
-                n2 = min(max(n2, 0), npi - 1);
-                if (!(hdz >= s_PA[n2] && hdz < s_PB[n2])) {
-                  if (n2 > 0 && hdz >= s_PA[n2 - 1] && hdz < s_PB[n2 - 1]) n2--;
-                  else if (n2 + 1 < npi && hdz >= s_PA[n2 + 1] && hdz < s_PB[n2 + 1]) n2++;
-                  else amb = true;
+                const float m2 = v2 + kMagic;
+                const int n2 = __float_as_int(m2) - (int)kMagicBits;
+                const float v1 = lin ? fmaf(sqrtf(r2), J.bc.rp_s, J.bc.rp_o)
+                                     : fmaf(__log2f(r2), J.bc.rp_s, J.bc.rp_o);
+                const float m1 = v1 + kMagic;
+                const int n1 = __float_as_int(m1) - (int)kMagicBits;
+                bool amb = !(fabsf(v2 - (m2 - kMagic)) <= lim2 && fabsf(v1 - (m1 - kMagic)) <= lim1);
+                // a block holds the bins [n2_base, n2_base + wpi) of Pi; of mu, each
+                // pair belongs to the unit whose slice holds its estimated bin
+                // (clamped), the others skip it
+                const int elk = n2 - n2_base;
+                const int n2c = min(max(n2, 0), npi - 1) - n2_base;
+                const bool own = !rmu || (unsigned)n2c < (unsigned)wpi;
+                bool bin = r2 >= J.bc.rej_lo;  // else certainly below the bins
+                if (!amb) {
+                  bin = bin && (unsigned)n1 < (unsigned)nrp && (unsigned)n2 < (unsigned)npi;
+                  amb = (unsigned)elk >= (unsigned)wpi;
                 }
-              } else {
-                // coordinates 7: r = |(dx, dy, dz)|, mu = dz / r (r_mu_calc); the
-                // mu bin is certain when dz is farther than mu_rel r + mu_abs from
-                // both edges scaled by r.  A block holds the mu bins
-                // [n2_base, n2_base + wpi): each pair belongs to the unit whose
-                // slice holds its estimated bin, the others skip it
-                r2 = fmaf(hdz, hdz, r2);
-                const float r = sqrtf(r2);
-                n2 = r2 > 0.0f ? (int)floorf(fmaf(__fdividef(hdz, r), inv_ps, tp0)) : 0;
-                n2 = min(max(n2, 0), npi - 1);
-                own = n2 >= n2_base && n2 < n2_base + wpi;
-                const float mg = fmaf(r, mu_rel, mu_abs);
-                auto in_mu = [&](int k) {
-                  return hdz - s_PA[k] * r >= mg && s_PB[k] * r - hdz > mg;
-                };
-                if (!in_mu(n2)) {
-                  if (n2 > 0 && in_mu(n2 - 1)) n2--;
-                  else if (n2 + 1 < npi && in_mu(n2 + 1)) n2++;
-                  else amb = true;
-                }
-              }
-              int n1 = lin_bin ? (int)floorf((sqrtf(r2) - rmin_f) * inv_rsize_f)
-                               : (int)floorf((__log2f(r2) - l2rmin2) * inv_lw);
-              n1 = min(max(n1, 0), nrp - 1);
-              if (!(r2 >= s_A[n1] && r2 < s_B[n1])) {
-                if (n1 > 0 && r2 >= s_A[n1 - 1] && r2 < s_B[n1 - 1]) n1--;
-                else if (n1 + 1 < nrp && r2 >= s_A[n1 + 1] && r2 < s_B[n1 + 1]) n1++;
-                else amb = true;
-              }
-              const int elk = n2 - n2_base;
-              if ((unsigned)elk >= (unsigned)wpi) amb = true;
-              // raw (un-shifted) separation for the orientation angle
-              // (angle_orient_axis_PB); coincident positions give atan(0/0) in
-              // the reference: those pairs take the exact path
-              // The separation is a double-float: the exact difference of the
-              // float hi parts, plus the lo parts for inputs that are not
-              // float32 values (renormalised); it is zero only when the
-              // positions coincide.
-              df32 dxr{0.f, 0.f}, dyr{0.f, 0.f};
-              if (kTheta) {
-                const float x2r = p2.x + g2sx, y2r = p2.y + g2sy;  // x2, y2 restored exactly
-                if (has_lo) {
-                  const float4 a1 = s_raux[er], a2 = s_aux[ec];
-                  dxr = df_diff_hl(x2r, a2.x, r1.x, a1.x);
-                  dyr = df_diff_hl(y2r, a2.y, r1.y, a1.y);
-                } else {
-                  dxr = two_diff(x2r, r1.x);
-                  dyr = two_diff(y2r, r1.y);
-                }
-                if (dxr.h == 0.0f && dyr.h == 0.0f) amb = true;
-              }
-              // ED: the shifted separation g1 - (g2 + L*PB) (ED_calc_PB) from
-              // hi + lo positions; a zero separation gives 0/0 in the reference
-              float sxe = 0.f, sye = 0.f, sze = 0.f, see = 1.f;
-              if (C == COREL_ED) {
-                sxe = hdx;
-                sye = hdy;
-                sze = -hdz;
-                if (has_lo) {
-                  const float4 a1 = s_raux[er], a2 = s_aux[ec];
-                  sxe += a1.x - a2.x;
-                  sye += a1.y - a2.y;
-                  sze += s_rzlo[er] - s_zlo[ec];
-                }
-                see = fmaf(sxe, sxe, fmaf(sye, sye, sze * sze));
-                if (!(see > 0.0f)) amb = true;
-              }
-              // twin jobs: a row paired with itself has no other order; it takes
-              // the exact path (its count is not mirrored)
-              bool tself = false;
-              if (twin && sx == 0 && sy == 0 && sz == 0 && hdz == 0.0f) {
-                const int gi = U.g1_start + (((er & 31) * W) + (er >> 5)) * U.g1_stride;
-                tself = s_jidx[ec] == gi;
-                if (tself) amb = true;
-              }
-              if (all_exact) {
-                // the comparison engine: the reference's double arithmetic for
-                // every candidate (window, bins, values), global FP64 atomics.
-                // With coordinates 7 every mu slice visits the pair: the window
-                // count is kept from slice 0 only, the pair's values go in by the
-                // slice that holds its exact mu bin
-                const int64_t gi1 = (int64_t)U.g1_start +
-                                    (int64_t)(((er & 31) * W) + (er >> 5)) * U.g1_stride;
-                const int64_t gj2 = s_jidx[ec];
-                int xn1, xn2;
-                const int r = exact_classify(J, J.d1, gi1, J.d2, gj2, sx, sy, sz, xn1, xn2);
-                if (r >= 1) nwin++;
-                if (r == 2 && (!rmu || (xn2 >= n2_base && xn2 < n2_base + wpi))) {
-                  double f[kNF];
-                  exact_values(J, J.d1, gi1, J.d2, gj2, sx, sy, sz, f);
-                  exact_accumulate(J, J.d1, gi1, J.d2, gj2, xn1, xn2, f);
-                }
-              } else if (!own) {
-                // another mu slice's pair
-              } else if (amb || edge) {
-                // near the window edge (not yet counted) or a bin edge (window
-                // counted): exact FP64 evaluation
-                const int64_t gi1 = (int64_t)U.g1_start +
-                                    (int64_t)(((er & 31) * W) + (er >> 5)) * U.g1_stride;
-                enqueue(U.job, gi1, s_jidx[ec], edge ? code : (code | kWindowCounted), queue,
-                        qcount, qcap);
-                // twin jobs: the other order, (g1 = the candidate, g2 = the row)
-                // at the opposite image
-                if (twin && !tself) {
-                  const int mcode = shift_code(-sx, -sy, -sz);
-                  enqueue(U.job, s_jidx[ec], gi1, edge ? mcode : (mcode | kWindowCounted), queue,
-                          qcount, qcap);
-                }
-              } else {
-              const int lb = n1 * wpi + elk;
-              // per-field terms: v (float) for every field, vd (double-float)
-              // for the fields whose sums cancel (df_field)
-              float v[kNF];
-              df32 vd[kNF];
-              // twin jobs: the other order's order-dependent terms (shape_shape)
-              constexpr bool kMir = F::FA > 0;
-              float vm[kMir ? kNF : 1];
-              df32 vdm[kMir ? kNF : 1];
-              const float w = r1.w * p2.w;
-              v[0] = w;
-              if (C == COREL_ED) {
-                const float4 es = gws == 2 ? s_shp[ec] : s_rshp[er];
-                const float dot = fmaf(es.x, sxe, fmaf(es.y, sye, es.w * sze));
-                v[11] = __fdividef(dot * dot, see);
-                v[12] = v[11] * v[11];
-              } else if (C != COREL_DD) {
-                // (w e1, w e2) hi and lo parts, the weight's lo part and phi
-                const float4 ea = s_rshp[er], eb = s_shp[ec];
-                const float4 xa = s_raux[er], xb = s_aux[ec];
-                const DfGal g1{{ea.x, ea.z}, {ea.y, ea.w}, {r1.w, xa.w}, xa.z};
-                const DfGal g2{{eb.x, eb.z}, {eb.y, eb.w}, {p2.w, xb.w}, xb.z};
-                df32 c2{0.f, 0.f}, s2v{0.f, 0.f};
-                float theta = 0.f;
+                // raw (un-shifted) separation for the orientation angle
+                // (angle_orient_axis_PB); coincident positions give atan(0/0) in
+                // the reference: those pairs take the exact path
+                // The separation is a double-float: the exact difference of the
+                // float hi parts, plus the lo parts for inputs that are not
+                // float32 values (renormalised); it is zero only when the
+                // positions coincide.
+                df32 dxr{0.f, 0.f}, dyr{0.f, 0.f};
                 if (kTheta) {
-                  df_cos_sin_2theta(dxr, dyr, c2, s2v);
-                  if (C != COREL_SK) theta = atanf(__fdividef(dyr.h, dxr.h));
-                }
-                if constexpr (kMir)
-                  df_pair_terms<C>(c2, s2v, theta, g1, g2, gws, J.unit_w != 0, vd, v,
-                                   twin ? vdm : nullptr, twin ? vm : nullptr);
-                else
-                  df_pair_terms<C>(c2, s2v, theta, g1, g2, gws, J.unit_w != 0, vd, v);
-              }
-              // fixed-point words of the main fields, in this lane's order (even
-              // lanes low word first, odd lanes high word first: red_pair); the
-              // region histograms reuse them
-              const bool odd_lane = (lane & 1) != 0;
-              unsigned wa[F::FM], wb[F::FM];
-#pragma unroll
-              for (int f = 0; f < F::FM; f++) {
-                const int q = F::m(f);
-                unsigned lo15, hi;
-                if (df_field(C, q)) df_to_fixed15(vd[q], sc.qs[q], lo15, hi);
-                else f_to_fixed15(v[q], sc.qs[q], lo15, hi);
-                wa[f] = odd_lane ? hi : lo15;
-                wb[f] = odd_lane ? lo15 : hi;
-              }
-              // the main bin, or one of its copies for a hot r_p bin
-              const int rep = (lane >> 1) & (kHotRep - 1);
-              const int lbm = (kHotRep > 1 && n1 >= hot0 && rep != 0)
-                                  ? rep_bin(rep, n1, elk, nrp, wpi) : lb;
-              atomicAdd(&s_mnum[lbm], 1u);
-#pragma unroll
-              for (int f = 0; f < F::FM; f++)
-                if (f >= f0)
-                  red_pair(&s_mlo[(size_t)f * NBm + lbm], &s_mhi[(size_t)f * NBm + lbm], wa[f],
-                           wb[f], odd_lane);
-              if (JK) {
-                // jk_check_PB (jk.cpp:64-71): the tile's region takes a same-region
-                // pair and a cross-region pair whose row is kept (main - NX); the
-                // partner's region takes a cross-region pair whose partner is kept
-                const bool nxc = !same_region && !s_rkeep[er];
-                const bool yc = !same_region && s_keep[ec];
-                if (nxc) {
-                  atomicAdd(&s_nxnum[lb], 1u);
-#pragma unroll
-                  for (int g = 0; g < F::FJ; g++)
-                    if (g >= f0)
-                      red_pair(&s_nxlo[(size_t)g * NB + lb], &s_nxhi[(size_t)g * NB + lb],
-                               wa[F::jm(g)], wb[F::jm(g)], odd_lane);
-                }
-                if (yc) {
-                  atomicAdd(&s_ynum[lb], 1u);
-#pragma unroll
-                  for (int g = 0; g < F::FJ; g++)
-                    if (g >= f0)
-                      red_pair(&s_ylo[(size_t)g * NB + lb], &s_yhi[(size_t)g * NB + lb],
-                               wa[F::jm(g)], wb[F::jm(g)], odd_lane);
-                }
-              }
-              if (twin) {
-                // the other order (g1 = the candidate, g2 = the row): the same bin
-                // count and order-independent terms (added at the flush), its
-                // order-dependent terms here, and its own region attribution:
-                // the tile's region takes it when the row is kept in the g2 role,
-                // the partner's region when the candidate is kept in the g1 role
-                unsigned xa[kMir ? F::FA : 1], xb[kMir ? F::FA : 1];
-                if constexpr (kMir) {
-#pragma unroll
-                  for (int i = 0; i < F::FA; i++) {
-                    const int q = F::m(F::a(i));
-                    unsigned lo15, hi;
-                    if (df_field(C, q)) df_to_fixed15(vdm[q], sc.qs[q], lo15, hi);
-                    else f_to_fixed15(vm[q], sc.qs[q], lo15, hi);
-                    xa[i] = odd_lane ? hi : lo15;
-                    xb[i] = odd_lane ? lo15 : hi;
-                    red_pair(&tw.alo[(size_t)i * NB + lb], &tw.ahi[(size_t)i * NB + lb], xa[i],
-                             xb[i], odd_lane);
+                  const float x2r = p2.x + g2sx, y2r = p2.y + g2sy;  // x2, y2 restored exactly
+                  if (has_lo) {
+                    const float4 a1 = s_raux[er], a2 = s_aux[ec];
+                    dxr = df_diff_hl(x2r, a2.x, r1.x, a1.x);
+                    dyr = df_diff_hl(y2r, a2.y, r1.y, a1.y);
+                  } else {
+                    dxr = two_diff(x2r, r1.x);
+                    dyr = two_diff(y2r, r1.y);
                   }
+                  if (dxr.h == 0.0f && dyr.h == 0.0f) amb = true;
                 }
-                if (JK) {
-                  const bool nxm = !same_region && !s_rkeep2[er];
-                  const bool ym = !same_region && s_keep2[ec];
-                  if (nxm) {
-                    atomicAdd(&tw.ncnt[lb], 1u);
+                // ED: the shifted separation g1 - (g2 + L*PB) (ED_calc_PB) from
+                // hi + lo positions; a zero separation gives 0/0 in the reference
+                float sxe = 0.f, sye = 0.f, sze = 0.f, see = 1.f;
+                if (C == COREL_ED) {
+                  sxe = hdx;
+                  sye = hdy;
+                  sze = -hdz;
+                  if (has_lo) {
+                    const float4 a1 = s_raux[er], a2 = s_aux[ec];
+                    sxe += a1.x - a2.x;
+                    sye += a1.y - a2.y;
+                    sze += s_rzlo[er] - s_zlo[ec];
+                  }
+                  see = fmaf(sxe, sxe, fmaf(sye, sye, sze * sze));
+                  if (!(see > 0.0f)) amb = true;
+                }
+                // twin jobs: a row paired with itself has no other order; it takes
+                // the exact path (its count is not mirrored)
+                bool tself = false;
+                if (TW && tie0 && hdz == 0.0f) {
+                  const int i1 = U.g1_start + (((er & 31) * W) + (er >> 5)) * U.g1_stride;
+                  tself = s_jidx[ec] == i1;
+                  if (tself) amb = true;
+                }
+                if (all_exact) {
+                  // the comparison engine: the reference's double arithmetic for
+                  // every candidate (window, bins, values), global FP64 atomics.
+                  // With coordinates 7 every mu slice visits the pair: the window
+                  // count is kept from slice 0 only, the pair's values go in by the
+                  // slice that holds its exact mu bin
+                  const int64_t gi1 = (int64_t)U.g1_start +
+                                      (int64_t)(((er & 31) * W) + (er >> 5)) * U.g1_stride;
+                  const int64_t gj2 = s_jidx[ec];
+                  int xn1, xn2;
+                  const int r = exact_classify(J, J.d1, gi1, J.d2, gj2, sx, sy, sz, xn1, xn2);
+                  if (r >= 1) nwin++;
+                  if (r == 2 && (!rmu || (xn2 >= n2_base && xn2 < n2_base + wpi))) {
+                    double f[kNF];
+                    exact_values(J, J.d1, gi1, J.d2, gj2, sx, sy, sz, f);
+                    exact_accumulate(J, J.d1, gi1, J.d2, gj2, xn1, xn2, f);
+                  }
+                } else if (own && (edge || (bin && amb))) {
+                  // near the window edge (not yet counted) or a bin edge (window
+                  // counted): exact FP64 evaluation
+                  const int64_t gi1 = (int64_t)U.g1_start +
+                                      (int64_t)(((er & 31) * W) + (er >> 5)) * U.g1_stride;
+                  enqueue(U.job, gi1, s_jidx[ec], edge ? code : (code | kWindowCounted), queue,
+                          qcount, qcap);
+                  // twin jobs: the other order, (g1 = the candidate, g2 = the row)
+                  // at the opposite image
+                  if (TW && !tself) {
+                    const int mcode = shift_code(-sx, -sy, -sz);
+                    enqueue(U.job, s_jidx[ec], gi1, edge ? mcode : (mcode | kWindowCounted), queue,
+                            qcount, qcap);
+                  }
+                } else if (own && bin) {
+                  const int lb = n1 * wpi + elk;
+                  // per-field terms: v (float) for every field, vd (double-float)
+                  // for the fields whose sums cancel (df_field)
+                  float v[kNF];
+                  df32 vd[kNF];
+                  // twin jobs: the other order's order-dependent terms (shape_shape)
+                  float vm[FA > 0 ? kNF : 1];
+                  df32 vdm[FA > 0 ? kNF : 1];
+                  v[0] = r1.w * p2.w;
+                  if (C == COREL_ED) {
+                    const float4 es = gws == 2 ? s_shp[ec] : s_rshp[er];
+                    const float dot = fmaf(es.x, sxe, fmaf(es.y, sye, es.w * sze));
+                    v[11] = __fdividef(dot * dot, see);
+                    v[12] = v[11] * v[11];
+                  } else if (C != COREL_DD) {
+                    // (w e1, w e2) hi and lo parts, the weight's lo part and phi
+                    const float4 ea = s_rshp[er], eb = s_shp[ec];
+                    const float4 xa = s_raux[er], xb = s_aux[ec];
+                    const DfGal g1{{ea.x, ea.z}, {ea.y, ea.w}, {r1.w, xa.w}, xa.z};
+                    const DfGal g2{{eb.x, eb.z}, {eb.y, eb.w}, {p2.w, xb.w}, xb.z};
+                    df32 c2{0.f, 0.f}, s2v{0.f, 0.f};
+                    float theta = 0.f;
+                    if (kTheta) {
+                      df_cos_sin_2theta(dxr, dyr, c2, s2v);
+                      if (C != COREL_SK) theta = atanf(__fdividef(dyr.h, dxr.h));
+                    }
+                    if constexpr (FA > 0)
+                      df_pair_terms<C>(c2, s2v, theta, g1, g2, gws, J.unit_w != 0, vd, v, vdm, vm);
+                    else
+                      df_pair_terms<C>(c2, s2v, theta, g1, g2, gws, J.unit_w != 0, vd, v);
+                  }
+                  // the words of the main fields; those of two fields at a time go in
+                  // this lane's order (order4), a single field's by lane parity
+                  unsigned wh[F::FM], wl[F::FM];
 #pragma unroll
-                    for (int g = 0; g < F::FJ; g++) {
-                      if (g < f0) continue;
-                      const int ap = asym_pos<F>(F::jm(g));
-                      red_pair(&tw.nlo[(size_t)g * NB + lb], &tw.nhi[(size_t)g * NB + lb],
-                               ap >= 0 ? xa[ap] : wa[F::jm(g)], ap >= 0 ? xb[ap] : wb[F::jm(g)],
-                               odd_lane);
+                  for (int f = 0; f < F::FM; f++) {
+                    const int q = F::m(f);
+                    if (df_field(C, q)) df_to_words(vd[q], sc.qs[q], wh[f], wl[f]);
+                    else f_to_words(v[q], sc.qs[q], wh[f], wl[f]);
+                  }
+                  const int odd = lane & 1, r4 = lane & 3;
+                  auto add1 = [&](unsigned *w, unsigned h, unsigned l) {
+                    atomicAdd(w + odd, odd ? l : h);
+                    atomicAdd(w + 1 - odd, odd ? h : l);
+                  };
+                  auto add2 = [&](unsigned *w, unsigned h0, unsigned l0, unsigned h1, unsigned l1) {
+                    unsigned o[4];
+                    order4(h0, l0, h1, l1, lane, o);
+                    atomicAdd(w + r4, o[0]);
+                    atomicAdd(w + (1 ^ r4), o[1]);
+                    atomicAdd(w + (2 ^ r4), o[2]);
+                    atomicAdd(w + (3 ^ r4), o[3]);
+                  };
+                  // field f's words are at r0 + 2 f
+                  unsigned *rec = hist + lb * S, *r0 = rec + 1 - 2 * f0;
+                  atomicAdd(rec, 1u);
+                  if (f0 == 0) add1(r0, wh[0], wl[0]);
+#pragma unroll
+                  for (int f = 1; f + 1 < F::FM; f += 2)
+                    add2(r0 + 2 * f, wh[f], wl[f], wh[f + 1], wl[f + 1]);
+                  if constexpr (F::FM > 1 && F::FM % 2 == 0)
+                    add1(r0 + 2 * (F::FM - 1), wh[F::FM - 1], wl[F::FM - 1]);
+                  unsigned xh[FA > 0 ? FA : 1], xl[FA > 0 ? FA : 1];
+                  if constexpr (FA > 0) {
+                    // the other order's order-dependent terms
+                    static_assert(FA % 2 == 0, "order-dependent fields in pairs");
+#pragma unroll
+                    for (int i = 0; i < FA; i++) {
+                      const int q = F::m(F::a(i));
+                      if (df_field(C, q)) df_to_words(vdm[q], sc.qs[q], xh[i], xl[i]);
+                      else f_to_words(vm[q], sc.qs[q], xh[i], xl[i]);
+                    }
+#pragma unroll
+                    for (int i = 0; i < FA; i += 2)
+                      add2(r0 + 2 * (F::FM + i), xh[i], xl[i], xh[i + 1], xl[i + 1]);
+                  }
+                  if (JK && !same_region) {
+                    // jk_check_PB (jk.cpp:64-71): the tile's region takes a same-region
+                    // pair and a cross-region pair whose row is kept (main - NX); the
+                    // partner's region takes a cross-region pair whose partner is kept
+                    auto region = [&](unsigned *h, bool other) {
+                      unsigned *q = h + lb * SJ, *q0 = q + 1 - 2 * f0;
+                      atomicAdd(q, 1u);
+#pragma unroll
+                      for (int j = 0; j < F::FJ; j++) {
+                        if (j < f0) continue;
+                        const int ap = (FA > 0 && other) ? asym_pos<F>(F::jm(j)) : -1;
+                        if (ap >= 0) add1(q0 + 2 * j, xh[ap < 0 ? 0 : ap], xl[ap < 0 ? 0 : ap]);
+                        else add1(q0 + 2 * j, wh[F::jm(j)], wl[F::jm(j)]);
+                      }
+                    };
+                    if (!s_rkeep[er]) region(B.nx, false);
+                    if (s_keep[ec]) region(B.y, false);
+                    if (TW) {
+                      // the other order (g1 = the candidate, g2 = the row): the tile's
+                      // region takes it when the row is kept in the g2 role, the
+                      // partner's region when the candidate is kept in the g1 role
+                      if (!s_rkeep2[er]) region(B.tnx, true);
+                      if (s_keep2[ec]) region(B.ty, true);
                     }
                   }
-                  if (ym) {
-                    atomicAdd(&tw.ycnt[lb], 1u);
-#pragma unroll
-                    for (int g = 0; g < F::FJ; g++) {
-                      if (g < f0) continue;
-                      const int ap = asym_pos<F>(F::jm(g));
-                      red_pair(&tw.ylo[(size_t)g * NB + lb], &tw.yhi[(size_t)g * NB + lb],
-                               ap >= 0 ? xa[ap] : wa[F::jm(g)], ap >= 0 ? xb[ap] : wb[F::jm(g)],
-                               odd_lane);
-                    }
-                  }
                 }
               }
+              qhead += take;
+              if (qhead >= kRing) {
+                qhead -= kRing;
+                qtail -= kRing;
               }
+              __syncwarp();
             }
-            qhead += take;
-            wbin += (unsigned)take;
-            __syncwarp();
-            if (pass >= W && qtail == qhead) break;
+            __syncwarp();  // every lane is done with the staged slots before restaging
           }
-          if (lane == 0 && wbin) atomicAdd(&s_nbin, wbin);
-          wbin = 0;
-          __syncwarp();  // every lane is done with the staged slots before restaging
-          }
-#undef CPC_SET_ROW
-          // s_nbin complete before the next chunk's flush test
-          __syncthreads();
         }
-        k = g;
       }
-      __syncthreads();
+      __syncthreads();  // the run tables and staging are free
     }
 
     // ---- flush main, X and the last Y ----
-    __syncthreads();
-    flush_main_x<F::FM, F::FJ, F>(s_mnum, s_mlo, s_mhi, s_nxnum, s_nxlo, s_nxhi, NB, NBm, wpi, npi,
-                                  nrp, n2_base, 1 + U.region, JK, f0, sc.iqs, J, tw);
+    flush_main_x<F, TW>(B, NB, wpi, npi, nrp, n2_base, 1 + U.region, JK, f0, sc.iqs, J);
     if (JK && cur_y >= 0) {
-      flush_region<F>(s_ynum, s_ylo, s_yhi, NB, wpi, npi, nrp, n2_base, 1 + cur_y, f0,
-                                 sc.iqs, J);
-      if (twin)
-        flush_region<F>(tw.ycnt, tw.ylo, tw.yhi, NB, wpi, npi, nrp, n2_base, 1 + cur_y, f0,
-                        sc.iqs, J, true);
+      flush_region<F>(B.y, NB, wpi, npi, nrp, n2_base, 1 + cur_y, f0, sc.iqs, J, false);
+      if (TW) flush_region<F>(B.ty, NB, wpi, npi, nrp, n2_base, 1 + cur_y, f0, sc.iqs, J, true);
     }
-    if (t == 0) s_nbin = 0u;
+    bound = 0;
     // window-pair counter (once per pair: mu slices other than the first skip it)
     {
-      unsigned long long v = (rmu && n2_base != 0) ? 0ull : (unsigned long long)nwin;
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+      unsigned long long v =
+          (rmu && n2_base != 0) ? 0ull : (TW ? 2ull * nwin - nself : (unsigned long long)nwin);
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(FULL, v, o);
       if (lane == 0) s_red[wid] = v;
       __syncthreads();
       if (t == 0) {
         unsigned long long sm = 0;
-        for (int w = 0; w < kThreads / 32; w++) sm += s_red[w];
+        for (int w = 0; w < kWarps; w++) sm += s_red[w];
         if (sm) atomicAdd(&J.counters[0], sm);
       }
     }
@@ -1118,42 +1028,33 @@ __global__ void recheck_kernel(const JobDev *__restrict__ jobs, const QEntry *__
 }
 
 // ---- host-side launchers (called from capi.cu) ----
-// Calls fn.run<C, JK, MINB>() for the runtime corel, jackknife flag and bound.
+// Calls fn.run<C, JK, VAR, TW>() for the runtime corel, jackknife flag and variant.
+template <int C, bool TW, class Fn>
+static auto dispatch_var(int jk, int var, const Fn &fn) -> decltype(fn.template run<C, true, 1, TW>()) {
+  if (var == 3) return jk ? fn.template run<C, true, 3, TW>() : fn.template run<C, false, 3, TW>();
+  if (var == 2) return jk ? fn.template run<C, true, 2, TW>() : fn.template run<C, false, 2, TW>();
+  if constexpr (!TW)
+    if (var == 0) return jk ? fn.template run<C, true, 0, TW>() : fn.template run<C, false, 0, TW>();
+  return jk ? fn.template run<C, true, 1, TW>() : fn.template run<C, false, 1, TW>();
+}
 template <class Fn>
-static auto dispatch(int corel, int jk, int minb, int twin, const Fn &fn)
-    -> decltype(fn.template run<0, false, 3, false>()) {
-  // twin jobs: density_density and shape_shape, 4 or 3 blocks per SM
-#define CPC_TCASE(CC)                                                                 \
-  if (corel == CC) {                                                                  \
-    if (jk) return minb == 4 ? fn.template run<CC, true, 4, true>()                  \
-                             : fn.template run<CC, true, 3, true>();                  \
-    return minb == 4 ? fn.template run<CC, false, 4, true>()                          \
-                     : fn.template run<CC, false, 3, true>();                         \
+static auto dispatch(int corel, int jk, int var, int twin, const Fn &fn)
+    -> decltype(fn.template run<0, false, 1, false>()) {
+  // twin jobs: density_density and shape_shape
+  if (twin && var != 0) {
+    if (corel == COREL_SS) return dispatch_var<COREL_SS, true>(jk, var, fn);
+    if (corel == COREL_SSA) return dispatch_var<COREL_SSA, true>(jk, var, fn);
+    return dispatch_var<COREL_DD, true>(jk, var, fn);
   }
-  if (twin && minb != 1) {
-    CPC_TCASE(COREL_DD)
-    CPC_TCASE(COREL_SS)
-    CPC_TCASE(COREL_SSA)
+  switch (corel) {
+    case COREL_SD: return dispatch_var<COREL_SD, false>(jk, var, fn);
+    case COREL_SS: return dispatch_var<COREL_SS, false>(jk, var, fn);
+    case COREL_SSA: return dispatch_var<COREL_SSA, false>(jk, var, fn);
+    case COREL_DK: return dispatch_var<COREL_DK, false>(jk, var, fn);
+    case COREL_SK: return dispatch_var<COREL_SK, false>(jk, var, fn);
+    case COREL_ED: return dispatch_var<COREL_ED, false>(jk, var, fn);
+    default: return dispatch_var<COREL_DD, false>(jk, var, fn);
   }
-#undef CPC_TCASE
-#define CPC_CASE(CC)                                                                  \
-  if (corel == CC) {                                                                  \
-    if (jk) return minb == 4 ? fn.template run<CC, true, 4, false>()                 \
-                  : minb == 1 ? fn.template run<CC, true, 1, false>()                 \
-                              : fn.template run<CC, true, 3, false>();                \
-    return minb == 4 ? fn.template run<CC, false, 4, false>()                         \
-           : minb == 1 ? fn.template run<CC, false, 1, false>()                       \
-                       : fn.template run<CC, false, 3, false>();                      \
-  }
-  CPC_CASE(COREL_DD)
-  CPC_CASE(COREL_SD)
-  CPC_CASE(COREL_SS)
-  CPC_CASE(COREL_SSA)
-  CPC_CASE(COREL_DK)
-  CPC_CASE(COREL_SK)
-  CPC_CASE(COREL_ED)
-#undef CPC_CASE
-  return fn.template run<COREL_DD, false, 3, false>();  // unreachable for valid corels
 }
 
 struct LaunchFast {
@@ -1168,57 +1069,68 @@ struct LaunchFast {
   int grid;
   int auto_pairs;
   cudaStream_t st;
-  template <int C, bool JK, int MINB, bool TW>
+  template <int C, bool JK, int VAR, bool TW>
   cudaError_t run() const {
-    auto kern = fast_pairs_kernel<C, JK, MINB, TW>;
+    auto kern = fast_pairs_kernel<C, JK, VAR, TW>;
     cudaError_t err =
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return err;
-    const int zero_words =
-        (int)((smem - stage_bytes(C) - (auto_pairs ? kAutoBytes : 0)) / 4);
-    kern<<<grid, kThreads, smem, st>>>(jobs, units, n_units, unit_ctr, q, qcount, qcap, *sc,
-                                       zero_words, auto_pairs);
+    constexpr int kThr = variant_threads(VAR);
+    const int zero_words = (int)((smem - stage_bytes(C, kThr / 32) -
+                                  (auto_pairs ? auto_bytes(C, kThr / 32) : 0)) / 4);
+    kern<<<grid, kThr, smem, st>>>(jobs, units, n_units, unit_ctr, q, qcount, qcap, *sc,
+                                   zero_words, auto_pairs);
     return cudaGetLastError();
   }
 };
 
 struct Occupancy {
   size_t smem;
-  template <int C, bool JK, int MINB, bool TW>
+  template <int C, bool JK, int VAR, bool TW>
   int run() const {
-    auto kern = fast_pairs_kernel<C, JK, MINB, TW>;
+    auto kern = fast_pairs_kernel<C, JK, VAR, TW>;
     int nb = 0;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
             cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, kThreads, smem) != cudaSuccess)
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, variant_threads(VAR), smem) !=
+            cudaSuccess)
       return 0;
     return nb;
   }
 };
 
-cudaError_t launch_fast(int corel, int jk, int minb, int twin, const JobDev *jobs,
+cudaError_t launch_fast(int corel, int jk, int variant, int twin, const JobDev *jobs,
                         const UnitDesc *units, int n_units, unsigned int *unit_ctr, QEntry *q,
                         unsigned long long *qcount, unsigned long long qcap,
                         const FastScales &sc, size_t smem, int grid, int auto_pairs,
                         cudaStream_t st) {
   if (corel < COREL_DD || corel > COREL_ED) return cudaErrorInvalidValue;
-  return dispatch(corel, jk, minb, twin,
+  return dispatch(corel, jk, variant, twin,
                   LaunchFast{jobs, units, n_units, unit_ctr, q, qcount, qcap, &sc, smem, grid,
                              auto_pairs, st});
 }
 
-// The register-bound variant for this shared-memory size and its blocks per SM:
-// the 4-block variant when 4 blocks fit, else the 3-block one.
-int fast_variant(int corel, int jk, size_t smem, int *blocks_per_sm, int all_exact, int twin) {
-  if (corel < COREL_DD || corel > COREL_ED) { *blocks_per_sm = 0; return 3; }
-  if (all_exact) {  // the cell-list FP64 comparison engine
-    *blocks_per_sm = dispatch(corel, jk, 1, 0, Occupancy{smem});
-    return 1;
+struct StaticSmem {
+  template <int C, bool JK, int VAR, bool TW>
+  size_t run() const {
+    cudaFuncAttributes a;
+    const cudaError_t e = cudaFuncGetAttributes(&a, fast_pairs_kernel<C, JK, VAR, TW>);
+    return e == cudaSuccess ? a.sharedSizeBytes : 24 * 1024;
   }
-  const int b4 = dispatch(corel, jk, 4, twin, Occupancy{smem});
-  if (b4 >= 4) { *blocks_per_sm = b4; return 4; }
-  *blocks_per_sm = dispatch(corel, jk, 3, twin, Occupancy{smem});
-  return 3;
+};
+// Static shared memory of a block, asked of the runtime once per kernel.
+size_t fast_static_smem_bytes(int corel, int jk, int variant, int twin) {
+  static std::atomic<size_t> known[COREL_ED + 1][2][4][2];
+  std::atomic<size_t> &k = known[corel][jk ? 1 : 0][variant][twin ? 1 : 0];
+  size_t b = k.load(std::memory_order_relaxed);
+  if (!b) k.store(b = dispatch(corel, jk, variant, twin, StaticSmem{}), std::memory_order_relaxed);
+  return b;
+}
+
+// Blocks per SM of a variant with this much dynamic shared memory (0: none fit).
+int fast_blocks(int corel, int jk, int variant, size_t smem, int twin) {
+  if (corel < COREL_DD || corel > COREL_ED) return 0;
+  return dispatch(corel, jk, variant, twin, Occupancy{smem});
 }
 
 cudaError_t launch_recheck(const JobDev *jobs, const QEntry *q, const unsigned long long *qcount,
@@ -1227,14 +1139,6 @@ cudaError_t launch_recheck(const JobDev *jobs, const QEntry *q, const unsigned l
   return cudaGetLastError();
 }
 
-}  // namespace cpc
-
-namespace cpc {
-size_t fast_static_smem_bytes(int twin) {
-  cudaFuncAttributes a;
-  const cudaError_t e = twin ? cudaFuncGetAttributes(&a, fast_pairs_kernel<COREL_SS, true, 4, true>)
-                             : cudaFuncGetAttributes(&a, fast_pairs_kernel<COREL_SS, true, 4, false>);
-  if (e != cudaSuccess) return 24 * 1024;
-  return a.sharedSizeBytes;
-}
+int fast_variant_blocks(int variant) { return variant_blocks(variant); }
+size_t fast_block_smem(int variant) { return (size_t)(228 * 1024) / variant_blocks(variant); }
 }  // namespace cpc
