@@ -1708,6 +1708,8 @@ cpc_status sky_upload(cpc_ctx *c, int slot, const cpc_catalog *cat) {
     double wmax = 0, wmin = 1e300, emax = 0, phimax = 0;
   };
   const int kMaxParts = 64;
+  // rows worth a thread: about 0.1 us each of trigonometry and window tables
+  const int64_t kSkyRows = 1024;
   std::vector<Part> parts(kMaxParts);
   host_parallel(n, [&](int64_t b0, int64_t b1, int part) {
     Part &P = parts[part];
@@ -1768,7 +1770,7 @@ cpc_status sky_upload(cpc_ctx *c, int slot, const cpc_catalog *cat) {
       }
       for (int q = 0; q < 6; q++) win[(size_t)q * n + i] = wv[q];
     }
-  });
+  }, kSkyRows);
   s.wmax = 0;
   s.wmin = n > 0 ? 1e300 : 1.0;
   s.emax = 0;
@@ -1834,7 +1836,7 @@ cpc_status sky_upload(cpc_ctx *c, int slot, const cpc_catalog *cat) {
       // corels1 scan start: row o + 1 (input order) against z_min of row o
       aflag[k] = (o + 1 < (uint32_t)n && !(cat->z[o + 1] < win[o])) ? kAutoStart0 : 0;
     }
-  });
+  }, 4 * kSkyRows);
   s.hc_tiles.clear();
   s.hc_tile_key.clear();
   sky_cell_order(c, s, zs, wins);
@@ -1924,7 +1926,7 @@ cpc_status sky_upload(cpc_ctx *c, int slot, const cpc_catalog *cat) {
       wz[q] = make_float2(c2[0], h2[0]);
       wb[q] = make_float4(c2[1], h2[1], c2[2], h2[2]);
     }
-  });
+  }, kSkyRows);
   s.dcmax = s.damax = s.sky_mag = 0;
   s.damin = 1e300;
   for (const Range &R : ranges) {

@@ -213,7 +213,7 @@ cpc_status cpc_set_tuning(cpc_ctx *ctx, int cells_per_rmax, int pi_window, int t
  * full count; twin counts run as twins) of this pair type, the faster of two
  * timed runs per candidate, for cell widths r_max / k (k = 2 .. 6; the cell lists are
  * rebuilt on the device) and block-local Pi windows (for 256, 512 and 1024 threads a
- * SM, the largest window that fits and three quarters of it), keeps the
+ * block, the largest window that fits and three quarters of it), keeps the
  * fastest for this context (as cpc_set_tuning would) and returns it.  Results
  * never depend on the choice.  With coordinates 7 (r-mu) only the cell width is
  * tuned and pi_window returns 0 (the mu window stays automatic).  Box runs only
