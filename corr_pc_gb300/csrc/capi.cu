@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -132,6 +133,7 @@ struct SkyJobBufs {
 struct UnitCache {
   uint64_t v1 = 0, v2 = 0;
   int s1 = -1, s2 = -1, wpi = 0, tile = 0, twin = 0, variant = 0;
+  uint64_t id = 0;  // of this list's contents: never given twice in the process
   std::vector<UnitDesc> units;  // job field filled at launch
 };
 
@@ -160,6 +162,7 @@ struct cpc_ctx {
   // scratch
   DevBuf<JobDev> d_jobs;
   DevBuf<UnitDesc> d_units;
+  std::vector<uint64_t> units_key;  // what d_units holds (enqueue_fast)
   DevBuf<unsigned int> d_unit_ctr;
   DevBuf<QEntry> d_queue;
   DevBuf<unsigned long long> d_qcount;
@@ -844,13 +847,13 @@ cpc_status plan_job(cpc_ctx *c, cpc_pair_kind kind, int slot_g1, int slot_g2, in
 }
 
 // tiles of g1 rows and their units (cached per slot versions and window)
-const std::vector<UnitDesc> &build_units(JobPlan &jp) {
+const UnitCache &build_units(JobPlan &jp) {
   cpc_ctx *c = jp.c;
   for (auto &uc : c->unit_cache)
     if (uc.s1 == jp.s1 && uc.s2 == jp.s2 && uc.v1 == c->slots[jp.s1].version &&
         uc.v2 == c->slots[jp.s2].version && uc.wpi == jp.wpi && uc.tile == jp.tile &&
         uc.twin == jp.jd.twin && uc.variant == jp.variant)
-      return uc.units;
+      return uc;
   if (c->unit_cache.size() >= 8) c->unit_cache.erase(c->unit_cache.begin());
   c->unit_cache.emplace_back();
   UnitCache &uc = c->unit_cache.back();
@@ -862,6 +865,8 @@ const std::vector<UnitDesc> &build_units(JobPlan &jp) {
   uc.tile = jp.tile;
   uc.twin = jp.jd.twin;
   uc.variant = jp.variant;
+  static std::atomic<uint64_t> next_id{1};
+  uc.id = next_id++;
   const cpc_params &p = c->p;
   const Slot &g1 = c->slots[jp.s1];
   const double L = p.periodic_box_size;
@@ -956,7 +961,7 @@ const std::vector<UnitDesc> &build_units(JobPlan &jp) {
   for (const auto &v : part_units) total += v.size();
   units.reserve(total);
   for (const auto &v : part_units) units.insert(units.end(), v.begin(), v.end());
-  return units;
+  return uc;
 }
 
 cpc_status ensure_scratch(cpc_ctx *c, size_t n_units, size_t n_jobs) {
@@ -1257,7 +1262,6 @@ cpc_status enqueue_fast(std::vector<JobPlan> &jobs) {
   cpc_ctx *c0 = jobs[0].c;
   cpc_ctx *c = c0;
   cudaStream_t st = c0->st;
-  std::vector<UnitDesc> all;
   for (size_t k = 0; k < jobs.size(); k++) {
     cpc_status s;
     if ((s = alloc_accum(jobs[k].c)) != CPC_OK) return s;
@@ -1272,32 +1276,54 @@ cpc_status enqueue_fast(std::vector<JobPlan> &jobs) {
     if (!jobs[k].empty)
       groups[Inst(jobs[k].jd.corel, jobs[k].jd.do_jk, jobs[k].jd.twin,
                   jobs[k].jd.all_exact ? 0 : jobs[k].variant)].push_back((int)k);
+  // the launches' unit ranges, and what identifies the list that they make up: a
+  // context that counts the same pairs again finds it on the device (copying the
+  // units of the 2M w++ box took 6 ms a call, of the 200k wg+ box 0.5 of 14.3)
   size_t total_units = 0;
   std::vector<std::pair<size_t, size_t>> ranges;
   std::vector<Inst> gkeys;
+  std::vector<std::vector<int>> members;
+  std::vector<uint64_t> key;
   for (auto &g : groups) {
-    const size_t b = all.size();
+    const size_t b = total_units;
     for (int k : g.second) {
-      const std::vector<UnitDesc> &u = build_units(jobs[k]);
+      const UnitCache &uc = build_units(jobs[k]);
       // this context's shard of the units (cpc_set_shard): every n_shards-th
       // unit from `shard`; the units partition the pairs, so the shards' blocks
       // sum to the whole count
-      const int nsh = jobs[k].c->n_shards, sh = jobs[k].c->shard;
-      for (size_t ui = (size_t)sh; ui < u.size(); ui += (size_t)nsh) {
-        UnitDesc d = u[ui];
-        d.job = k;
-        const int64_t ncol = (int64_t)(d.cx_hi - d.cx_lo + 1) * (d.cy_hi - d.cy_lo + 1);
-        if (ncol < 1 || ncol > kFastMaxCols || d.g1_count < 1 || d.g1_count > kTileThreads)
-          return fail(c, CPC_ERR_INVALID, "work unit outside kernel limits (too many neighbour columns)");
-        all.push_back(d);
-      }
+      const size_t nsh = (size_t)jobs[k].c->n_shards, sh = (size_t)jobs[k].c->shard;
+      key.insert(key.end(), {uc.id, (uint64_t)k, nsh, sh});
+      total_units += uc.units.size() > sh ? (uc.units.size() - sh + nsh - 1) / nsh : 0;
     }
-    ranges.push_back({b, all.size()});
+    ranges.push_back({b, total_units});
     gkeys.push_back(g.first);
+    members.push_back(g.second);
   }
-  total_units = all.size();
   cpc_status s;
+  const UnitDesc *held = c0->d_units.p;
   if ((s = ensure_scratch(c0, std::max<size_t>(1, total_units), jobs.size())) != CPC_OK) return s;
+  if (held != c0->d_units.p || key != c0->units_key) {
+    c0->units_key.clear();
+    std::vector<UnitDesc> all;
+    all.reserve(total_units);
+    for (const auto &m : members)
+      for (int k : m) {
+        const std::vector<UnitDesc> &u = build_units(jobs[k]).units;
+        const size_t nsh = (size_t)jobs[k].c->n_shards;
+        for (size_t ui = (size_t)jobs[k].c->shard; ui < u.size(); ui += nsh) {
+          UnitDesc d = u[ui];
+          d.job = k;
+          const int64_t ncol = (int64_t)(d.cx_hi - d.cx_lo + 1) * (d.cy_hi - d.cy_lo + 1);
+          if (ncol < 1 || ncol > kFastMaxCols || d.g1_count < 1 || d.g1_count > kTileThreads)
+            return fail(c, CPC_ERR_INVALID, "work unit outside kernel limits (too many neighbour columns)");
+          all.push_back(d);
+        }
+      }
+    if (total_units)
+      CK(cudaMemcpyAsync(c0->d_units.p, all.data(), sizeof(UnitDesc) * total_units,
+                         cudaMemcpyHostToDevice, st), "H2D units");
+    c0->units_key = std::move(key);
+  }
   // size the edge queue from the rate earlier counts of this context queued
   // (per unit): a count whose queue overflows is run again, which a full count
   // after sharded or sampled ones would otherwise pay
@@ -1317,8 +1343,6 @@ cpc_status enqueue_fast(std::vector<JobPlan> &jobs) {
   std::vector<JobDev> jds(jobs.size());
   for (size_t k = 0; k < jobs.size(); k++) jds[k] = jobs[k].jd;
   CK(cudaMemcpyAsync(c0->d_jobs.p, jds.data(), sizeof(JobDev) * jds.size(), cudaMemcpyHostToDevice, st), "H2D jobs");
-  if (total_units)
-    CK(cudaMemcpyAsync(c0->d_units.p, all.data(), sizeof(UnitDesc) * total_units, cudaMemcpyHostToDevice, st), "H2D units");
   std::vector<FastGroup> gs;
   for (size_t g = 0; g < ranges.size(); g++) {
     const int corel = std::get<0>(gkeys[g]), jk = std::get<1>(gkeys[g]), twin = std::get<2>(gkeys[g]),
@@ -1330,10 +1354,9 @@ cpc_status enqueue_fast(std::vector<JobPlan> &jobs) {
       sc.qs[f] = INFINITY;
       sc.iqs[f] = 0.0;
     }
-    for (size_t k = ranges[g].first; k < ranges[g].second; k++)
-      auto_pairs |= jobs[all[k].job].jd.auto_mode ? 1 : 0;
-    for (size_t k = ranges[g].first; k < ranges[g].second; k++) {
-      const JobPlan &jp = jobs[all[k].job];
+    for (int k : members[g]) auto_pairs |= jobs[k].jd.auto_mode ? 1 : 0;
+    for (int k : members[g]) {
+      const JobPlan &jp = jobs[k];
       smem = std::max(smem, fast_smem_bytes(corel, jk, jp.jd.nrp, jp.wpi, auto_pairs,
                                             jp.jd.unit_w, jp.jd.twin, variant));
       for (int f = 0; f < kNF; f++)
@@ -1342,10 +1365,10 @@ cpc_status enqueue_fast(std::vector<JobPlan> &jobs) {
           sc.iqs[f] = jp.jd.inv_qscale[f];
         }
     }
-    const int bps = fast_blocks(corel, jk, variant, smem, twin);
-    if (bps <= 0) return fail(c, CPC_ERR_INVALID, "fast kernel does not fit on an SM with these bins");
     const size_t n_units = ranges[g].second - ranges[g].first;
     if (n_units == 0) continue;
+    const int bps = fast_blocks(corel, jk, variant, smem, twin);
+    if (bps <= 0) return fail(c, CPC_ERR_INVALID, "fast kernel does not fit on an SM with these bins");
     const int grid = (int)std::min<int64_t>((int64_t)c0->sm_count * bps, (int64_t)n_units);
     gs.push_back(
         FastGroup{corel, jk, variant, grid, ranges[g].first, n_units, smem, sc, auto_pairs, twin});
