@@ -644,7 +644,7 @@ struct ChunkModel {
   }
 };
 
-// Smallest window worth a kernel of its own (coordinates 7: any mu slice).
+// Smallest window (coordinates 7: any mu slice): what always fits a block.
 int min_window(const cpc_params &p, int twin) { return p.coordinates == 7 ? 1 : twin ? 5 : 8; }
 
 struct Variant {
@@ -759,7 +759,7 @@ cpc_status plan_job(cpc_ctx *c, cpc_pair_kind kind, int slot_g1, int slot_g2, in
       variant = 1;
       // histograms of up to 200 KB are accepted, and narrowed beside the staging
       const size_t room = 227 * 1024 - fixed(1);
-      if (bytes(1, wpi) - bytes(1, 0) <= 200 * 1024)
+      if (fast_window_bytes(jp.rule.corel, jk, nrp, wpi, uw, twin) <= 200 * 1024)
         while (wpi > 1 && bytes(1, wpi) > room) wpi--;
     }
   } else {

@@ -86,6 +86,7 @@ constexpr int kMaxCellsPerRmax = 9;
 size_t fast_smem_bytes(int corel, int do_jk, int nrp, int wpi, int auto_pairs, int unit_w,
                        int twin, int variant);
 size_t fast_static_smem_bytes(int corel, int jk, int variant, int twin);
+size_t fast_window_bytes(int corel, int do_jk, int nrp, int wpi, int unit_w, int twin);
 int fast_variant_blocks(int variant);  // blocks per SM
 size_t fast_block_smem(int variant);  // a block's share of an SM's shared memory
 int fast_blocks(int corel, int jk, int variant, size_t smem, int twin);

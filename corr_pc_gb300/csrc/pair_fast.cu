@@ -18,7 +18,7 @@
 // histogram updates.
 //
 // Measured (GB300, before -> now): kernel of the 200k wg+ box 17.9 -> 13.5 ms,
-// kappa 11.6 -> 7.6, ED 7.0 -> 4.1; w++ twin of 2M points 567 -> 420, weighted w++
+// kappa 11.6 -> 7.3, ED 7.0 -> 4.1; w++ twin of 2M points 567 -> 420, weighted w++
 // (60k x 151k) 6.9 -> 5.2, 12 uneven w++ boxes 58 -> 25; wgg of 20,000 points
 // 0.36 -> 0.12.  What gave it: one bit per test instead of a queue push per step
 // (67 -> 24 instructions a step), maps instead of band tables, records of words
@@ -39,7 +39,8 @@
 // in shared memory -- the full sample ("main"), the cross-region pairs that the
 // tile's own jackknife region does NOT take ("NX": that region's sums are main
 // minus NX, so the pairs it takes, most of them, cost no update of their own) and
-// one other region ("Y", the partner's region for cross-region pairs) -- with
+// one other region ("Y", the partner's region for cross-region pairs); the corels
+// of few fields keep a main histogram per attribution instead (by_class) -- with
 // 32-bit counts and fixed-point sums split over two 32-bit words per field
 // (exact integer addition, order independent), flushed to the FP64 global
 // histogram block when the pairs added since the last flush could overflow a
@@ -103,26 +104,48 @@ __host__ __device__ constexpr int rec_words(int fields, int f0, int fa) {
   return 1 + 2 * (fields - f0 + fa);
 }
 
-// Shared-memory bytes a block needs for a job with nrp r_p bins and a wpi-bin
-// Pi window: the staging, the main histogram, with jackknife the two region
-// histograms, in a twin job the other order's two.
+// With jackknife, the corels of few fields keep four main histograms a block, by
+// which of its two regions take the pair (the tile's 1, the partner's 2): a pair adds one
+// record instead of up to three, and pairs of one bin fall on four.  200k box:
+// kappa 7.6 -> 7.3 ms, ED 4.27 -> 4.14.  Where the records are long the window
+// pays: with the four, auto pairs of shapes 6.3 -> 6.9, weighted w++ 5.15 -> 5.07, wg+
+// 13.5 -> 13.3; twin jobs would need sixteen.
+__host__ __device__ constexpr bool by_class(int corel, int jk, int twin) {
+  return jk && !twin && corel != COREL_SD && corel != COREL_SS && corel != COREL_SSA;
+}
+// Words from one class's record of a bin to the next class's: 8 banks on.
+__host__ __device__ constexpr int class_stride(int words) { return words + ((8 - words) & 31); }
+
+// Fields of a corel's main and region records.
+static void record_fields(int corel, int *FM, int *FJ) {
+  *FM = 1, *FJ = 1;
+  if (corel == COREL_SD) { *FM = 7; *FJ = 4; }
+  if (corel == COREL_SS) { *FM = 11; *FJ = 6; }
+  if (corel == COREL_SSA) { *FM = 13; *FJ = 7; }
+  if (corel == COREL_DK) { *FM = 2; *FJ = 2; }
+  if (corel == COREL_SK) { *FM = 4; *FJ = 4; }
+  if (corel == COREL_ED) { *FM = 3; *FJ = 2; }
+}
+// Bytes of a wpi-bin window of nrp r_p bins as one main record and two (twin: four)
+// region records a bin: the measure by which a set window is too wide.
+size_t fast_window_bytes(int corel, int do_jk, int nrp, int wpi, int unit_w, int twin) {
+  int FM, FJ;
+  record_fields(corel, &FM, &FJ);
+  const int f0 = unit_w ? 1 : 0, FA = twin && corel == COREL_SS ? FieldMap<COREL_SS>::FA : 0;
+  return 4ull * nrp * wpi *
+         (rec_words(FM, f0, FA) + (do_jk ? rec_words(FJ, f0, 0) * (twin ? 4 : 2) : 0));
+}
+// Shared-memory bytes a block needs for a job: the staging, then the histograms
+// (linear in wpi).
 size_t fast_smem_bytes(int corel, int do_jk, int nrp, int wpi, int auto_pairs, int unit_w,
                        int twin, int variant) {
-  const int NB = nrp * wpi;
-  int FM = 1, FJ = 1;
-  if (corel == COREL_SD) { FM = 7; FJ = 4; }
-  if (corel == COREL_SS) { FM = 11; FJ = 6; }
-  if (corel == COREL_SSA) { FM = 13; FJ = 7; }
-  if (corel == COREL_DK) { FM = 2; FJ = 2; }
-  if (corel == COREL_SK) { FM = 4; FJ = 4; }
-  if (corel == COREL_ED) { FM = 3; FJ = 2; }
-  const int FA = twin && corel == COREL_SS ? FieldMap<COREL_SS>::FA : 0;
-  const int f0 = unit_w ? 1 : 0;
   const int warps = variant_threads(variant) / 32;
-  size_t b = stage_bytes(corel, warps) + (auto_pairs ? auto_bytes(corel, warps) : 0);
-  b += 4ull * NB * rec_words(FM, f0, FA);
-  if (do_jk) b += 4ull * NB * rec_words(FJ, f0, 0) * (twin ? 4 : 2);
-  return b;
+  const size_t b = stage_bytes(corel, warps) + (auto_pairs ? auto_bytes(corel, warps) : 0);
+  if (!by_class(corel, do_jk, twin))
+    return b + fast_window_bytes(corel, do_jk, nrp, wpi, unit_w, twin);
+  int FM, FJ;
+  record_fields(corel, &FM, &FJ);
+  return b + 16ull * (nrp * wpi * rec_words(FM, unit_w ? 1 : 0, 0) + 31);
 }
 
 // Fixed-point sums in 32-bit shared words.  A term v of field f becomes the
@@ -307,6 +330,67 @@ __device__ __noinline__ void flush_main_x(const BlockHist &B, int NB, int wpi, i
   }
 }
 
+// Flush of a block with class histograms (by_class; CS: class_stride): the pairs
+// that the partner's region hy takes, whose classes are then folded into those that
+// it does not take, and when `all` is set the full sample and the tile's region hx.
+// Integer sums throughout; zeroes what it flushes.
+template <class FMAP>
+__device__ __noinline__ void flush_classes(unsigned *H, int CS, int NB, int wpi, int npi, int nrp,
+                                           int n2_base, int hx, int hy, bool all, int f0,
+                                           const double *s_iqs, const JobDev &J) {
+  constexpr int FM = FMAP::FM, FJ = FMAP::FJ;
+  const int64_t hsz = (int64_t)nrp * npi;
+  const int S = rec_words(FM, f0, 0);
+  for (int lb = threadIdx.x; lb < NB; lb += blockDim.x) {
+    unsigned *r0 = H + lb * S, *r1 = r0 + CS, *r2 = r1 + CS, *r3 = r2 + CS;
+    const int64_t cell = (int64_t)(lb / wpi) * npi + n2_base + lb % wpi;
+    const unsigned n2 = r2[0], n3 = r3[0];
+    if (n2 | n3) {
+      const int64_t yc = (int64_t)hy * hsz + cell;
+      atomicAdd(&J.acc_num[yc], (unsigned long long)(n2 + n3));
+#pragma unroll
+      for (int g = 0; g < FJ; g++) {
+        if (g < f0) continue;
+        const int o = 1 + 2 * (FMAP::jm(g) - f0), fld = FMAP::j(g);
+        const long long v = fixed_sum(r2 + o, n2 * kMagicBits) + fixed_sum(r3 + o, n3 * kMagicBits);
+        if (v != 0) atomicAdd(&J.acc_sums[yc * kNF + fld], (double)v * s_iqs[fld]);
+      }
+      for (int w = 0; w < S; w++) {
+        r0[w] += r2[w];
+        r1[w] += r3[w];
+        r2[w] = 0u;
+        r3[w] = 0u;
+      }
+    }
+    if (!all) continue;
+    const unsigned n0 = r0[0], n1 = r1[0];
+    if (!(n0 | n1)) continue;
+    const int64_t xc = (int64_t)hx * hsz + cell;
+    atomicAdd(&J.acc_num[cell], (unsigned long long)(n0 + n1));
+    if (n1) atomicAdd(&J.acc_num[xc], (unsigned long long)n1);
+    r0[0] = 0u;
+    r1[0] = 0u;
+    long long tx[FM];
+#pragma unroll
+    for (int f = 0; f < FM; f++) {
+      tx[f] = 0;
+      if (f < f0) continue;  // field 0 of unit weights: no words
+      const int o = 1 + 2 * (f - f0), fld = FMAP::m(f);
+      tx[f] = fixed_sum(r1 + o, n1 * kMagicBits);
+      const long long v = fixed_sum(r0 + o, n0 * kMagicBits) + tx[f];
+      if (v != 0) atomicAdd(&J.acc_sums[cell * kNF + fld], (double)v * s_iqs[fld]);
+      r0[o] = r0[o + 1] = r1[o] = r1[o + 1] = 0u;
+    }
+#pragma unroll
+    for (int g = 0; g < FJ; g++) {
+      if (g < f0) continue;
+      const long long v = tx[FMAP::jm(g)];
+      const int fld = FMAP::j(g);
+      if (v != 0) atomicAdd(&J.acc_sums[xc * kNF + fld], (double)v * s_iqs[fld]);
+    }
+  }
+}
+
 constexpr unsigned kEdgeFlag = 0x8000u;  // queue entry: near the window edge
 
 // VAR: the variant (variant_threads; 0: the FP64 comparison engine).  TW: twin jobs (every job
@@ -382,6 +466,8 @@ fast_pairs_kernel(const JobDev *__restrict__ jobs, const UnitDesc *__restrict__ 
     const int nrp = J.nrp, wpi = J.wpi, npi = J.npi, NB = nrp * wpi;
     const int f0 = J.unit_w ? 1 : 0;
     const int S = rec_words(F::FM, f0, FA), SJ = rec_words(F::FJ, f0, 0);
+    constexpr bool kClasses = by_class(C, JK, TW);
+    const int CS = class_stride(NB * S);
     BlockHist B;
     B.main = hist;
     B.nx = B.main + NB * S;
@@ -486,6 +572,21 @@ fast_pairs_kernel(const JobDev *__restrict__ jobs, const UnitDesc *__restrict__ 
     __syncthreads();
     const int total_slots = s_cnt[ncol];
     int cur_y = -1;        // region held in the Y histogram
+    // y: what the region in Y took; all: the rest too
+    auto flush = [&](bool y, bool all) {
+      if constexpr (kClasses) {
+        flush_classes<F>(hist, CS, NB, wpi, npi, nrp, n2_base, 1 + U.region, 1 + cur_y, all, f0,
+                         sc.iqs, J);
+      } else {
+        if (all)
+          flush_main_x<F, TW>(B, NB, wpi, npi, nrp, n2_base, 1 + U.region, JK, f0, sc.iqs, J);
+        if (JK && y) {
+          flush_region<F>(B.y, NB, wpi, npi, nrp, n2_base, 1 + cur_y, f0, sc.iqs, J, false);
+          if (TW)
+            flush_region<F>(B.ty, NB, wpi, npi, nrp, n2_base, 1 + cur_y, f0, sc.iqs, J, true);
+        }
+      }
+    };
 
     for (int chunk0 = 0; chunk0 < total_slots; chunk0 += kMaxSeg) {
       const int nslot = min(kMaxSeg, total_slots - chunk0);
@@ -574,9 +675,7 @@ fast_pairs_kernel(const JobDev *__restrict__ jobs, const UnitDesc *__restrict__ 
         if (JK && !same_region && cur_y != region2) {
           if (cur_y >= 0) {
             __syncthreads();
-            flush_region<F>(B.y, NB, wpi, npi, nrp, n2_base, 1 + cur_y, f0, sc.iqs, J, false);
-            if (TW)
-              flush_region<F>(B.ty, NB, wpi, npi, nrp, n2_base, 1 + cur_y, f0, sc.iqs, J, true);
+            flush(true, false);
             __syncthreads();
           }
           cur_y = region2;
@@ -599,7 +698,10 @@ fast_pairs_kernel(const JobDev *__restrict__ jobs, const UnitDesc *__restrict__ 
           if (!all_exact && bound + 32 * W * nc > kBinTerms) {  // (block-uniform)
             int m = 0;
             __syncthreads();
-            for (int lb = t; lb < NB; lb += kThreads) m = max(m, (int)hist[lb * S]);
+            for (int lb = t; lb < NB; lb += kThreads) {
+              const unsigned *r = hist + lb * S;
+              m = max(m, (int)(kClasses ? r[0] + r[CS] + r[2 * CS] + r[3 * CS] : r[0]));
+            }
             m = __reduce_max_sync(FULL, m);
             if (lane == 0 && m > 0) atomicMax(&s_max[turn], m);
             if (t == 0) s_max[turn ^ 1] = 0;
@@ -607,12 +709,7 @@ fast_pairs_kernel(const JobDev *__restrict__ jobs, const UnitDesc *__restrict__ 
             bound = s_max[turn];
             turn ^= 1;
             if (bound + 32 * W * nc > kBinTerms) {
-              flush_main_x<F, TW>(B, NB, wpi, npi, nrp, n2_base, 1 + U.region, JK, f0, sc.iqs, J);
-              if (JK && cur_y >= 0) {
-                flush_region<F>(B.y, NB, wpi, npi, nrp, n2_base, 1 + cur_y, f0, sc.iqs, J, false);
-                if (TW)
-                  flush_region<F>(B.ty, NB, wpi, npi, nrp, n2_base, 1 + cur_y, f0, sc.iqs, J, true);
-              }
+              flush(cur_y >= 0, true);
               bound = 0;
               __syncthreads();
             }
@@ -917,7 +1014,13 @@ fast_pairs_kernel(const JobDev *__restrict__ jobs, const UnitDesc *__restrict__ 
                     atomicAdd(w + (3 ^ r4), o[3]);
                   };
                   // field f's words are at r0 + 2 f
-                  unsigned *rec = hist + lb * S, *r0 = rec + 1 - 2 * f0;
+                  unsigned *rec = hist + lb * S;
+                  // jk_check_PB (jk.cpp:64-71): the tile's region takes a same-region
+                  // pair and a cross-region pair whose row is kept; the partner's
+                  // region takes a cross-region pair whose partner is kept
+                  if (kClasses)
+                    rec += (same_region ? 1 : (s_rkeep[er] ? 1 : 0) + (s_keep[ec] ? 2 : 0)) * CS;
+                  unsigned *r0 = rec + 1 - 2 * f0;
                   atomicAdd(rec, 1u);
                   if (f0 == 0) add1(r0, wh[0], wl[0]);
 #pragma unroll
@@ -939,10 +1042,8 @@ fast_pairs_kernel(const JobDev *__restrict__ jobs, const UnitDesc *__restrict__ 
                     for (int i = 0; i < FA; i += 2)
                       add2(r0 + 2 * (F::FM + i), xh[i], xl[i], xh[i + 1], xl[i + 1]);
                   }
-                  if (JK && !same_region) {
-                    // jk_check_PB (jk.cpp:64-71): the tile's region takes a same-region
-                    // pair and a cross-region pair whose row is kept (main - NX); the
-                    // partner's region takes a cross-region pair whose partner is kept
+                  if (JK && !kClasses && !same_region) {
+                    // (the tile's region: main - NX)
                     auto region = [&](unsigned *h, bool other) {
                       unsigned *q = h + lb * SJ, *q0 = q + 1 - 2 * f0;
                       atomicAdd(q, 1u);
@@ -981,11 +1082,7 @@ fast_pairs_kernel(const JobDev *__restrict__ jobs, const UnitDesc *__restrict__ 
     }
 
     // ---- flush main, X and the last Y ----
-    flush_main_x<F, TW>(B, NB, wpi, npi, nrp, n2_base, 1 + U.region, JK, f0, sc.iqs, J);
-    if (JK && cur_y >= 0) {
-      flush_region<F>(B.y, NB, wpi, npi, nrp, n2_base, 1 + cur_y, f0, sc.iqs, J, false);
-      if (TW) flush_region<F>(B.ty, NB, wpi, npi, nrp, n2_base, 1 + cur_y, f0, sc.iqs, J, true);
-    }
+    flush(cur_y >= 0, true);
     bound = 0;
     // window-pair counter (once per pair: mu slices other than the first skip it)
     {

@@ -95,15 +95,16 @@ def test_windows_and_blocks(which, twin, window):
     ctx.close()
 
 
-@pytest.mark.parametrize("corr", [0, 2])
+@pytest.mark.parametrize("corr", [0, 2, 3])
 def test_a_bin_past_its_words(corr):
-    """A clump whose tiles put more than 2^17 pairs in one bin, each term near its
-    bound: the block's histogram is flushed inside a unit; and the auto pairs."""
+    """A clump over eight jackknife regions whose tiles put more than 2^17 pairs in one
+    bin, each term near its bound: the block's histogram is flushed inside a unit;
+    and the auto pairs."""
     rng = np.random.default_rng(9)
     n = 3000
     x, y, z = 30.0 + rng.uniform(-0.4, 0.4, (3, n))
     e1, e2 = synth.shapes(rng, n)
-    c = synth.Catalog(x, y, z, np.full(n, 1.99), e1 if corr else None, e2 if corr else None,
+    c = synth.Catalog(x, y, z, np.full(n, 1.99), e1 if corr else None, e2 if corr == 2 else None,
                       synth.jk_cubes(x, y, z, 60.0, 2)).sorted_by_z()
     p = _params(corr, n, rmin=0.0, rmax=2.0, nrp=2, npi=1, pmax=2.0, lin_bin=1)
     ctx = _context(p, [("S", c), ("D", c)])
