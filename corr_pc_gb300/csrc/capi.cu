@@ -2052,15 +2052,16 @@ SkyView sky_view(Slot &s) {
 
 // Tiles of the fast sky kernel over the rows list[0 .. n_list) (cell positions
 // in cell order; null: every row) of slot s.  A tile holds up to kSkyTile rows
-// of one bucket within 0.35 of the mean redshift window (0.25: 5% more time on
-// 200k randoms, the candidates staged for fewer rows), or up to a whole one until
-// it has 32 rows; inside a bucket its size is a multiple of 32, so that no row
-// pass has idle lanes.
+// of one bucket within half the mean redshift window, or up to two of them until it
+// has 64 rows: a tile's bucket searches and staging cost more than the tests of a
+// wide redshift range (data x randoms of 20k x 200k, up to one window until 32 rows
+// 7.08 ms, two and 64 6.42, three and 96 6.65; half a window and 32 rows 8.3).  Inside
+// a bucket its size is a multiple of 32, so that no row pass has idle lanes.
 void sky_tiles(const Slot &s, const int *list, int64_t n_list, std::vector<SkyTileRows> &tiles,
                std::vector<int> &keys) {
   tiles.clear();
   keys.clear();
-  const float E = (float)(0.35 * s.sky_zw), Ehi = (float)s.sky_zw;
+  const float E = (float)(0.5 * s.sky_zw), Ehi = (float)(2 * s.sky_zw);
   auto z = [&](int64_t k) { return s.hc_z[list ? list[k] : k]; };
   int64_t i = 0;
   for (const int4 &b : s.hc_bk) {
@@ -2069,7 +2070,7 @@ void sky_tiles(const Slot &s, const int *list, int64_t n_list, std::vector<SkyTi
     while (i < e) {
       const float z0 = z(i);
       int64_t j = i + 1;
-      while (j < e && j - i < kSkyTile && (z(j) - z0 <= E || (j - i < 32 && z(j) - z0 <= Ehi))) j++;
+      while (j < e && j - i < kSkyTile && (z(j) - z0 <= E || (j - i < 64 && z(j) - z0 <= Ehi))) j++;
       if (j < e && j - i > 32) j -= (j - i) & 31;
       tiles.push_back(SkyTileRows{(int)i, (int)(j - i)});
       keys.push_back(b.z);
