@@ -157,6 +157,7 @@ struct cpc_ctx {
   int tune_k = 0, tune_wpi = 0, tune_tile = 0;
   int device = 0, sm_count = 152;
   cudaStream_t st = nullptr;
+  cudaStream_t st2 = nullptr;  // beside st, for launches that may overlap (sky_run)
   cudaEvent_t e0 = nullptr, e1 = nullptr, e2 = nullptr;
   cudaEvent_t e_in = nullptr, e_done = nullptr;  // cpc_count_async ordering
   // scratch
@@ -2446,9 +2447,8 @@ cpc_status sky_finish(cpc_ctx *c, SkyPlan &P, size_t k, cpc_engine engine, float
   return CPC_OK;
 }
 
-// Sky counts (coordinates 0) of one context: the fast engine runs every job in
-// one launch of the chunked warp kernel, then the fixed-point blocks are
-// converted and each job's host edge tier runs; the FP64 engine runs the plain
+// Sky counts (coordinates 0) of one context: the fast engine runs the units of
+// every job (sky_tile_kernel), then the fixed-point blocks are converted and each job's host edge tier runs; the FP64 engine runs the plain
 // kernel per job.
 cpc_status sky_run(cpc_ctx *c, std::vector<SkyPlan> &plans, cpc_engine engine) {
   const cpc_params &p = c->p;
@@ -2478,26 +2478,29 @@ cpc_status sky_run(cpc_ctx *c, std::vector<SkyPlan> &plans, cpc_engine engine) {
       }
     } else {
       // the units of every job, split until each block finds about six of them:
-      // first a key pair's tiles, then the redshift range of its candidates
-      size_t hist_words = 1;
-      int set = 0;
+      // first a key pair's tiles, then the redshift range of its candidates.  Each
+      // instantiation (0 counts, 1 shape x density, 2 shape x shape) has its range of
+      // the list, counts first: their units (randoms against randoms) are the longest,
+      // and last they cost 5% in few regions.
       std::vector<SkyUnit> units;
+      size_t end[3] = {0, 0, 0};  // of the units of each
+      auto set_of = [&](const JobDev &J) {
+        return J.corel == COREL_DD ? 0 : J.corel == COREL_SD ? 1 : 2;
+      };
       auto build = [&](int parts, int slices) {
         size_t pairs = 0;
         units.clear();
-        for (size_t m = 0; m < jd.size(); m++) {
-          const SkyPlan &P = plans[idx[m]];
-          pairs += sky_units(c->slots[P.s1], c->slots[P.s2], *P.keys, (int)m, parts, slices,
-                             jd[m].sk.guard, jd[m].sk.flip != 0, P.all, units);
+        for (int q = 0; q < 3; q++) {
+          for (size_t m = 0; m < jd.size(); m++) {
+            const SkyPlan &P = plans[idx[m]];
+            if (set_of(jd[m]) == q)
+              pairs += sky_units(c->slots[P.s1], c->slots[P.s2], *P.keys, (int)m, parts, slices,
+                                 jd[m].sk.guard, jd[m].sk.flip != 0, P.all, units);
+          }
+          end[q] = units.size();
         }
         return pairs;
       };
-      for (size_t m = 0; m < jd.size(); m++) {
-        const int cl = jd[m].corel;
-        set = std::max(set, cl == COREL_DD ? 0 : cl == COREL_SD ? 1 : 2);
-        if (jd[m].sk.hist_smem)
-          hist_words = std::max(hist_words, sky_hist_words(cl, jd[m].unit_w, p.n_bins * p.n_p_bin));
-      }
       const size_t want = (size_t)c->sm_count * 24;
       const size_t pairs = build(1, 1);
       if (pairs && units.size() < want) {
@@ -2506,15 +2509,55 @@ cpc_status sky_run(cpc_ctx *c, std::vector<SkyPlan> &plans, cpc_engine engine) {
         if (units.size() < want / 2)
           build(parts, (int)std::min<size_t>(4, want / std::max<size_t>(1, units.size())));
       }
+      // A launch per instantiation: counts keep four blocks per SM of 64 registers,
+      // shape terms three of 80 (20k x 200k: 30.6 ms in one launch, 28.6 in two).  The
+      // second goes on a stream of its own, so that its blocks follow the first's as
+      // they end.  Ranges of fewer than about eight units a block share a launch: a
+      // coarse list leaves blocks idle at the end of each (8k x 53k in 25 regions,
+      // 1,300 units of counts: 2.45 ms in one, 2.73 in two).
+      const size_t kRange = (size_t)c->sm_count * 32;
+      struct Range {
+        size_t first, n;
+        int set;
+      };
+      std::vector<Range> ranges;
+      for (int q = 0; q < 3; q++) {
+        const size_t first = q ? end[q - 1] : 0, n = end[q] - first;
+        if (n == 0) continue;
+        if (!ranges.empty() && (ranges.back().n < kRange || n < kRange)) {
+          ranges.back().n += n;
+          ranges.back().set = q;
+        } else {
+          ranges.push_back(Range{first, n, q});
+        }
+      }
       CK(c->d_sky_units.alloc(units.size()), "alloc units");
-      CK(c->d_sky_ctr.alloc(1), "alloc");
+      CK(c->d_sky_ctr.alloc(3), "alloc");
       if (!units.empty())
         CK(cudaMemcpyAsync(c->d_sky_units.p, units.data(), sizeof(SkyUnit) * units.size(),
                            cudaMemcpyHostToDevice, st), "H2D");
-      CK(cudaMemsetAsync(c->d_sky_ctr.p, 0, sizeof(unsigned long long), st), "memset");
-      CK(launch_sky_tile(c->d_jobs.p, c->d_sky_units.p, (int)units.size(), set, hist_words,
-                         c->d_sky_ctr.p, kSkyHostQueue, esum, c->sm_count, st), "sky kernel");
-      c->launches += 1;
+      CK(cudaMemsetAsync(c->d_sky_ctr.p, 0, 3 * sizeof(unsigned long long), st), "memset");
+      if (ranges.size() > 1) {
+        if (!c->st2) CK(cudaStreamCreateWithFlags(&c->st2, cudaStreamNonBlocking), "stream");
+        CK(cudaEventRecord(c->e_in, st), "event");
+        CK(cudaStreamWaitEvent(c->st2, c->e_in, 0), "stream wait");
+      }
+      std::reverse(ranges.begin(), ranges.end());  // (counts, of the small blocks, fill in)
+      for (size_t q = 0; q < ranges.size(); q++) {
+        size_t hist_words = 1;
+        for (const JobDev &J : jd)
+          if (J.sk.hist_smem && set_of(J) <= ranges[q].set)
+            hist_words = std::max(hist_words,
+                                  sky_hist_words(J.corel, J.unit_w, p.n_bins * p.n_p_bin));
+        CK(launch_sky_tile(c->d_jobs.p, c->d_sky_units.p + ranges[q].first, (int)ranges[q].n,
+                           ranges[q].set, hist_words, c->d_sky_ctr.p + q, kSkyHostQueue, esum,
+                           c->sm_count, q & 1 ? c->st2 : st), "sky kernel");
+        c->launches += 1;
+      }
+      if (ranges.size() > 1) {
+        CK(cudaEventRecord(c->e_done, c->st2), "event");
+        CK(cudaStreamWaitEvent(st, c->e_done, 0), "stream wait");
+      }
       for (size_t m = 0; m < jd.size(); m++) {
         const SkyPlan &P = plans[idx[m]];
         CK(launch_sky_finish((int64_t)P.n_fix, jd[m].acc_fix, jd[m].acc_fixh, jd[m].acc_sums,
@@ -2605,6 +2648,7 @@ cpc_status cpc_destroy(cpc_ctx *c) try {
   if (c->e_in) cudaEventDestroy(c->e_in);
   if (c->e_done) cudaEventDestroy(c->e_done);
   if (c->st) cudaStreamDestroy(c->st);
+  if (c->st2) cudaStreamDestroy(c->st2);
   delete c;
   return CPC_OK;
 } catch (...) {

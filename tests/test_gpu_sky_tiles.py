@@ -87,3 +87,15 @@ def test_sky_rows_shards_and_auto_match_fp64_engine():
     assert np.array_equal(sum(q["num"] for q in parts), ref["num"])
     _same(ctx.count_auto("SS", 0), ctx.count_auto("SS", 0, engine="fp64"), "SS")
     ctx.close()
+
+
+@pytest.mark.parametrize("which", [1, 2])
+def test_sky_terms_in_several_launches_match_fp64_engine(which):
+    """Enough region pairs for a launch per group of corels, beside one another."""
+    ctx, terms = _run(5000, 20000, which=which, side=10, nrp=2, npi=2)
+    l0 = ctx.launches()
+    batch = _lib.count_batch([(ctx, *t) for t in terms])
+    assert ctx.launches() - l0 > 1 + len(terms)  # the sums' launches, and more than one
+    for t, b in zip(terms, batch):
+        _same(b, ctx.count(*t, engine="fp64"), t[0])
+    ctx.close()
