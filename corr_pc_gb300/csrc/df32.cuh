@@ -216,15 +216,5 @@ DF_HD void f_to_words(float v, float qs, unsigned &hi, unsigned &lo) {
   hi = magic_bits(a);
   lo = magic_bits(rn_add(rn_fma(rn_sub(a, kMagic), -32768.0f, t), kMagic));
 }
-// the same for a float term (one rounding conversion)
-DF_HD void f_to_fixed15(float v, float qs, unsigned &lo15, unsigned &hi) {
-#ifdef __CUDA_ARCH__
-  const int u = __float2int_rn(v * qs);
-#else
-  const int u = (int)rintf(v * qs);
-#endif
-  lo15 = (unsigned)u & 0x7FFFu;
-  hi = (unsigned)(u >> 15);
-}
 
 }  // namespace cpc
