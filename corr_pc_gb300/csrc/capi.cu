@@ -601,6 +601,10 @@ void box_consts(const cpc_ctx *c, const Slot &g1, const Slot &g2, JobDev &J) {
 // rewritten, with the model 1.7 to 1.9; kappa of 20,000 rows in 288 buckets 0.86 ->
 // 0.17 ms, a batch of w++ boxes of up to 9,000 rows 4.0 -> 1.3; the 200k wg+ box,
 // whose tiles are full either way, 13.8 -> 13.5.
+// The model sees the catalogues, the binning and a fixed number of SMs (a GB300's),
+// never the device: contexts that count shards of the same pairs (cpc_set_shard)
+// must cut them into the same units.
+constexpr int kModelSMs = 152;
 struct ChunkModel {
   double kap, heavy, zw, ps, n, slots, unit, scale;
   int npi, wpi;
@@ -618,7 +622,7 @@ struct ChunkModel {
     wpi = w;
     rmu = p.coordinates == 7;
     narrow = !rmu && wpi < npi;
-    slots = (double)c->sm_count * fast_variant_blocks(variant);
+    slots = (double)kModelSMs * fast_variant_blocks(variant);
     unit = 500.0 * 4 / fast_variant_blocks(variant);
     scale = variant == 1 ? 1.0 : variant == 2 ? 1.05 : 1.1;  // wider blocks wait for one another
   }
@@ -698,6 +702,14 @@ int preferred_cells(cpc_ctx *c, int64_t n = 0) {
   return c->pref_k;
 }
 
+// The automatic cell width.  Of a context that counts shards it is r_max / 2,
+// whatever the context holds: the units that the shards share out are those of the
+// cell lists, and each shard's context may hold other catalogues beside the counted
+// ones.  (Shards pay for large catalogues, which take r_max / 2 anyway.)
+int automatic_cells(cpc_ctx *c, int64_t n = 0) {
+  return c->n_shards > 1 ? 2 : preferred_cells(c, n);
+}
+
 cpc_status rebuild_cells(cpc_ctx *c, Slot &s, int k);
 
 // allow_twin: false for the cell-list FP64 comparison engine, which counts every
@@ -722,7 +734,7 @@ cpc_status plan_job(cpc_ctx *c, cpc_pair_kind kind, int slot_g1, int slot_g2, in
   jp.s2 = jp.rule.swapped ? slot_g1 : slot_g2;
   Slot &g1 = c->slots[jp.s1], &g2 = c->slots[jp.s2];
   if (c->tune_k == 0 && !g1.sky && !g2.sky) {
-    const int k = preferred_cells(c);
+    const int k = automatic_cells(c);
     for (Slot *s : {&g1, &g2})
       if (s->kcells != k) {
         const cpc_status st = rebuild_cells(c, *s, k);
@@ -2752,7 +2764,7 @@ cpc_status cpc_upload(cpc_ctx *c, int slot, const cpc_catalog *cat) try {
     CK(cudaMemcpyAsync(&c->h_ustats, c->d_ustats.p, sizeof(UploadStats), cudaMemcpyDeviceToHost,
                        st), "D2H");
   }
-  return build_cells(c, s, n, c->tune_k > 0 ? c->tune_k : preferred_cells(c, n), nullptr, true);
+  return build_cells(c, s, n, c->tune_k > 0 ? c->tune_k : automatic_cells(c, n), nullptr, true);
 } catch (...) {
   return host_exception(c);
 }

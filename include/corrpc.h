@@ -236,8 +236,11 @@ cpc_status cpc_autotune_batch(int n_jobs, cpc_ctx *const *ctxs, const cpc_pair_k
  * cpc_count_batch) process only the work units i with i % n_shards == shard.
  * A unit is a tile of outer rows against one slice of its candidates, and the
  * units partition the pairs, so the RAW blocks of shards 0 .. n_shards-1 (one
- * per GPU, each on its own context with the same catalogues) sum to the whole
- * count: counts exactly, sums up to the order of FP64 additions.  Unlike
+ * per GPU, each on its own context) sum to the whole count: counts exactly, sums
+ * up to the order of FP64 additions.  The contexts need the same parameters, the
+ * same two catalogues in the counted slots and the same tuning (cpc_set_tuning;
+ * an autotuner's choice on one of them has to be set on all) and twin switch; what
+ * their other slots hold does not matter.  Unlike
  * row_stride, whose skipped rows still pass through every unit, each shard does
  * about 1/n_shards of the work.  Fast sky counts take the outer rows at
  * redshift-ordered positions k with k % n_shards == shard (the shards again

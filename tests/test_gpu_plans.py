@@ -1,0 +1,47 @@
+"""Counts whose plan depends on what else a context holds or was told."""
+import pytest
+
+from corr_pc_gb300 import _lib, host
+from test_gpu_box_tiles import _cat, _params, _same
+
+pytestmark = pytest.mark.gpu
+
+L = 250.0
+
+
+def _box(which=0, n_s=900, n_d=12000):
+    """A small pair of samples, and the density sample of 150,000 rows whose
+    presence changes the automatic cell width (r_max to r_max / 2)."""
+    s, d, big = _cat(n_s, 1, L, which=which), _cat(n_d, 2, L, which=which), _cat(150000, 3, L)
+    out = []
+    for c in (d, big):
+        p = _params(which, n_s, L=L, rmax=20.0, npi=20, pmax=100.0)
+        p.n_density = c.n
+        out.append((p, host.prepare(p, [("S", s), ("D", c)])))
+    (p, prep), (_, prep_big) = out
+    return p, s, d, prep["S"], prep["D"], prep_big["D"]
+
+
+@pytest.mark.parametrize("when", ["before", "after"])
+@pytest.mark.parametrize("which", [0, 1])
+def test_shards_on_contexts_of_other_contents_sum_to_the_whole_count(which, when):
+    """Each shard on its own context, one of which also holds a larger catalogue
+    in a slot that the count does not read."""
+    p, s, d, ps, pd, pbig = _box(which)
+    parts = []
+    for sh in range(3):
+        ctx = _lib.Context(p)
+        if sh == 1 and when == "before":
+            ctx.upload(5, pbig)
+        ctx.upload(0, ps)
+        ctx.upload(1, pd)
+        if sh == 1 and when == "after":
+            ctx.upload(5, pbig)
+        if sh == 0:
+            ref = ctx.count("SD", 1, 0, engine="fp64")
+            ctx.count("SD", 1, 0)  # whole, with a plan of its own
+        ctx.set_shard(sh, 3)
+        parts.append(ctx.count("SD", 1, 0))
+        ctx.close()
+    total = {k: sum(q[k] for q in parts) for k in ("n_binned", "n_window", "num", "sums")}
+    _same(total, ref, s, d)
