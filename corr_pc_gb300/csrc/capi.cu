@@ -73,6 +73,7 @@ struct Slot {
   uint64_t version = 0;
   // grid this cell list was built with
   int ncx = 0, ncy = 0, n_reg = 1, kcells = 0;
+  bool auto_k = true;  // kcells is automatic, not a width that the caller set
   double cw_x = 0, cw_y = 0, row_density = 0;
   // device, cell order
   DevBuf<float4> pos, shp, ewt, aux;
@@ -712,11 +713,30 @@ int automatic_cells(cpc_ctx *c, int64_t n = 0) {
 
 cpc_status rebuild_cells(cpc_ctx *c, Slot &s, int k);
 
+// The box catalogues in these slots on one grid: that of the first whose width the
+// caller set at its upload, else the automatic one (counts do not depend on it).
+cpc_status same_grid(cpc_ctx *c, const std::vector<int> &slots) {
+  int k = 0;
+  for (int q : slots)
+    if (!k && !c->slots[q].auto_k) k = c->slots[q].kcells;
+  if (!k) k = automatic_cells(c);
+  for (int q : slots) {
+    Slot &s = c->slots[q];
+    if (s.valid && !s.sky && s.kcells != k) {
+      const cpc_status st = rebuild_cells(c, s, k);
+      if (st != CPC_OK) return st;
+    }
+  }
+  return CPC_OK;
+}
+
 // allow_twin: false for the cell-list FP64 comparison engine, which counts every
-// order and keeps the plain job's window
+// order and keeps the plain job's window.  one_grid: same_grid was called for every
+// job of the context (a batch plans them all before it counts: none may rebuild a
+// slot that another one was planned on).
 cpc_status plan_job(cpc_ctx *c, cpc_pair_kind kind, int slot_g1, int slot_g2, int64_t rs,
                     int64_t ro, cpc_accum *out, JobPlan &jp, int auto_mode = 0,
-                    bool allow_twin = true) {
+                    bool allow_twin = true, bool one_grid = false) {
   if (slot_g1 < 0 || slot_g1 >= kMaxSlots || slot_g2 < 0 || slot_g2 >= kMaxSlots)
     return fail(c, CPC_ERR_INVALID, "slot out of range");
   Slot &A = c->slots[slot_g1], &B = c->slots[slot_g2];
@@ -733,13 +753,9 @@ cpc_status plan_job(cpc_ctx *c, cpc_pair_kind kind, int slot_g1, int slot_g2, in
   jp.s1 = jp.rule.swapped ? slot_g2 : slot_g1;
   jp.s2 = jp.rule.swapped ? slot_g1 : slot_g2;
   Slot &g1 = c->slots[jp.s1], &g2 = c->slots[jp.s2];
-  if (c->tune_k == 0 && !g1.sky && !g2.sky) {
-    const int k = automatic_cells(c);
-    for (Slot *s : {&g1, &g2})
-      if (s->kcells != k) {
-        const cpc_status st = rebuild_cells(c, *s, k);
-        if (st != CPC_OK) return st;
-      }
+  if (!one_grid) {
+    const cpc_status st = same_grid(c, {jp.s1, jp.s2});
+    if (st != CPC_OK) return st;
   }
   if (g1.ncx != g2.ncx || g1.ncy != g2.ncy || g1.n_reg != g2.n_reg)
     return fail(c, CPC_ERR_STATE, "catalogues were uploaded with different cell grids");
@@ -1585,6 +1601,13 @@ cpc_status rebuild_cells(cpc_ctx *c, Slot &s, int k) {
   s.zbuilt = false;
   s.version = ++c->version_ctr;
   return build_cells(c, s, n, k, c->u_orig.p, false);
+}
+
+// A box slot on cells r_max / k wide that no later upload changes (the autotuners).
+cpc_status set_cells(cpc_ctx *c, Slot &s, int k) {
+  const cpc_status st = s.kcells == k ? CPC_OK : rebuild_cells(c, s, k);
+  if (st == CPC_OK) s.auto_k = false;
+  return st;
 }
 
 // ---------------------------------------------------------------------------
@@ -2764,7 +2787,8 @@ cpc_status cpc_upload(cpc_ctx *c, int slot, const cpc_catalog *cat) try {
     CK(cudaMemcpyAsync(&c->h_ustats, c->d_ustats.p, sizeof(UploadStats), cudaMemcpyDeviceToHost,
                        st), "D2H");
   }
-  return build_cells(c, s, n, c->tune_k > 0 ? c->tune_k : automatic_cells(c, n), nullptr, true);
+  s.auto_k = c->tune_k == 0;
+  return build_cells(c, s, n, s.auto_k ? automatic_cells(c, n) : c->tune_k, nullptr, true);
 } catch (...) {
   return host_exception(c);
 }
@@ -2932,12 +2956,9 @@ cpc_status cpc_autotune(cpc_ctx *c, cpc_pair_kind kind, int slot_g1, int slot_g2
   int bk = c->slots[slot_g1].kcells, bw = c->tune_wpi;
   for (int k : ks) {
     cpc_status s;
-    c->tune_k = k;  // (a count would choose its own width)
-    if (c->slots[slot_g1].kcells != k && (s = rebuild_cells(c, c->slots[slot_g1], k)) != CPC_OK)
-      return s;
-    if (slot_g2 != slot_g1 && c->slots[slot_g2].kcells != k &&
-        (s = rebuild_cells(c, c->slots[slot_g2], k)) != CPC_OK)
-      return s;
+    c->tune_k = k;
+    if ((s = set_cells(c, c->slots[slot_g1], k)) != CPC_OK) return s;
+    if ((s = set_cells(c, c->slots[slot_g2], k)) != CPC_OK) return s;
     for (int w : ws) {
       c->tune_wpi = w;
       // first run builds the work units, the next two are timed (the faster counts)
@@ -2960,8 +2981,8 @@ cpc_status cpc_autotune(cpc_ctx *c, cpc_pair_kind kind, int slot_g1, int slot_g2
   c->tune_wpi = bw;
   for (int q = 0; q < kMaxSlots; q++) {
     Slot &sl = c->slots[q];
-    if (sl.valid && !sl.sky && sl.kcells != bk) {
-      const cpc_status s = rebuild_cells(c, sl, bk);
+    if (sl.valid && !sl.sky) {
+      const cpc_status s = set_cells(c, sl, bk);
       if (s != CPC_OK) return s;
     }
   }
@@ -2976,11 +2997,20 @@ cpc_status cpc_autotune(cpc_ctx *c, cpc_pair_kind kind, int slot_g1, int slot_g2
 cpc_status count_batch_rows(int n_jobs, cpc_ctx *const *ctxs, const cpc_pair_kind *kinds,
                             const int *slots_g1, const int *slots_g2, cpc_accum *outs,
                             int64_t row_stride) {
-  std::vector<JobPlan> jobs(n_jobs);
+  std::map<cpc_ctx *, std::vector<int>> used;  // the slots that each context's jobs read
   for (int k = 0; k < n_jobs; k++) {
     if (ctxs[k]->device != ctxs[0]->device) return fail(ctxs[k], CPC_ERR_INVALID, "batch spans devices");
-    cpc_status s = plan_job(ctxs[k], kinds[k], slots_g1[k], slots_g2[k], row_stride, 0, &outs[k],
-                            jobs[k]);
+    for (const int q : {slots_g1[k], slots_g2[k]})
+      if (q >= 0 && q < kMaxSlots) used[ctxs[k]].push_back(q);
+  }
+  for (const auto &u : used) {
+    const cpc_status s = same_grid(u.first, u.second);
+    if (s != CPC_OK) return s;
+  }
+  std::vector<JobPlan> jobs(n_jobs);
+  for (int k = 0; k < n_jobs; k++) {
+    const cpc_status s = plan_job(ctxs[k], kinds[k], slots_g1[k], slots_g2[k], row_stride, 0,
+                                  &outs[k], jobs[k], 0, true, true);
     if (s != CPC_OK) return s;
   }
   return run_fast(jobs);
@@ -3047,14 +3077,11 @@ cpc_status cpc_autotune_batch(int n_jobs, cpc_ctx *const *ctxs, const cpc_pair_k
   }
   // every slot a job reads, on cells r_max / kc
   auto regrid = [&](int kc) -> cpc_status {
-    for (int k = 0; k < n_jobs; k++) ctxs[k]->tune_k = kc;  // (a count would choose its own)
+    for (int k = 0; k < n_jobs; k++) ctxs[k]->tune_k = kc;
     for (int k = 0; k < n_jobs; k++)
       for (int sl : {slots_g1[k], slots_g2[k]}) {
-        Slot &s = ctxs[k]->slots[sl];
-        if (s.kcells != kc) {
-          const cpc_status st = rebuild_cells(ctxs[k], s, kc);
-          if (st != CPC_OK) return st;
-        }
+        const cpc_status st = set_cells(ctxs[k], ctxs[k]->slots[sl], kc);
+        if (st != CPC_OK) return st;
       }
     return CPC_OK;
   };

@@ -45,3 +45,27 @@ def test_shards_on_contexts_of_other_contents_sum_to_the_whole_count(which, when
         ctx.close()
     total = {k: sum(q[k] for q in parts) for k in ("n_binned", "n_window", "num", "sums")}
     _same(total, ref, s, d)
+
+
+@pytest.mark.parametrize("k", [1, 2, 3])
+@pytest.mark.parametrize("order", ["set first", "set second"])
+def test_set_and_automatic_cell_widths_count_together(order, k):
+    """A catalogue uploaded with a set cell width against one uploaded with the
+    automatic width."""
+    p, s, d, ps, pd, _ = _box()
+    ctx = _lib.Context(p)
+    if order == "set first":
+        ctx.set_tuning(k)
+        ctx.upload(0, ps)
+        ctx.set_tuning(0)
+        ctx.upload(1, pd)
+    else:
+        ctx.upload(0, ps)
+        ctx.set_tuning(k)
+        ctx.upload(1, pd)
+    got = ctx.count("SD", 1, 0)
+    _same(got, ctx.count("SD", 1, 0, engine="fp64"), s, d)
+    ctx.set_tuning(4)
+    ctx.upload(1, pd)
+    _same(ctx.count("SD", 1, 0), got, s, d)
+    ctx.close()
