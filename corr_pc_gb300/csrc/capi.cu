@@ -730,6 +730,17 @@ cpc_status same_grid(cpc_ctx *c, const std::vector<int> &slots) {
   return CPC_OK;
 }
 
+// Every catalogue of automatic width on the width that the context's state asks for
+// now: after an upload or a shard, so that no count has to rebuild a list.
+cpc_status settle_cells(cpc_ctx *c) {
+  for (Slot &s : c->slots) {
+    if (!s.valid || s.sky || !s.auto_k || s.kcells == automatic_cells(c)) continue;
+    const cpc_status st = rebuild_cells(c, s, automatic_cells(c));
+    if (st != CPC_OK) return st;
+  }
+  return CPC_OK;
+}
+
 // allow_twin: false for the cell-list FP64 comparison engine, which counts every
 // order and keeps the plain job's window.  one_grid: same_grid was called for every
 // job of the context (a batch plans them all before it counts: none may rebuild a
@@ -2788,7 +2799,9 @@ cpc_status cpc_upload(cpc_ctx *c, int slot, const cpc_catalog *cat) try {
                        st), "D2H");
   }
   s.auto_k = c->tune_k == 0;
-  return build_cells(c, s, n, s.auto_k ? automatic_cells(c, n) : c->tune_k, nullptr, true);
+  const cpc_status built =
+      build_cells(c, s, n, s.auto_k ? automatic_cells(c, n) : c->tune_k, nullptr, true);
+  return built == CPC_OK ? settle_cells(c) : built;
 } catch (...) {
   return host_exception(c);
 }
@@ -3183,14 +3196,16 @@ cpc_status cpc_host_rp_thresholds(const cpc_params *p, double *thr) try {
   return host_exception(nullptr);
 }
 
-cpc_status cpc_set_shard(cpc_ctx *c, int shard, int n_shards) {
+cpc_status cpc_set_shard(cpc_ctx *c, int shard, int n_shards) try {
   if (!c) return fail(nullptr, CPC_ERR_INVALID, "null context");
   if (busy(c)) return CPC_ERR_STATE;
   if (n_shards < 1 || shard < 0 || shard >= n_shards)
     return fail(c, CPC_ERR_INVALID, "shard must satisfy 0 <= shard < n_shards");
   c->shard = shard;
   c->n_shards = n_shards;
-  return CPC_OK;
+  return settle_cells(c);
+} catch (...) {
+  return host_exception(c);
 }
 
 cpc_status cpc_set_graph_replay(cpc_ctx *c, int enable) try {

@@ -149,7 +149,9 @@ const char *cpc_last_error(const cpc_ctx *ctx);
 
 /* Copy a catalogue into slot `slot` (0..7) and build its on-device cell list
  * (radix sort by (column, region, z)).  Replaces any previous catalogue in the
- * slot.  Validates labels (0 <= jk < n_jk when do_jk) and finite positions. */
+ * slot.  Validates labels (0 <= jk < n_jk when do_jk) and finite positions.  An
+ * upload that changes the automatic cell width (cpc_set_tuning) rebuilds the other
+ * slots' cell lists, so that no later count has to. */
 cpc_status cpc_upload(cpc_ctx *ctx, int slot, const cpc_catalog *cat);
 
 /* Count one pair type between the catalogues in slots slot_g1, slot_g2 --
@@ -246,7 +248,8 @@ cpc_status cpc_autotune_batch(int n_jobs, cpc_ctx *const *ctxs, const cpc_pair_k
  * about 1/n_shards of the work.  Fast sky counts take the outer rows at
  * redshift-ordered positions k with k % n_shards == shard (the shards again
  * partition the pairs); the FP64 engine shards by rows (row_stride /
- * row_offset), which it skips cheaply.  Default: shard 0 of 1. */
+ * row_offset), which it skips cheaply.  Default: shard 0 of 1.  May rebuild cell
+ * lists when sharding starts or ends (shards use cells of r_max / 2). */
 cpc_status cpc_set_shard(cpc_ctx *ctx, int shard, int n_shards);
 
 /* Number of GPU kernels this context has launched so far (all entry points;

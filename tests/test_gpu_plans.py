@@ -69,3 +69,19 @@ def test_set_and_automatic_cell_widths_count_together(order, k):
     ctx.upload(1, pd)
     _same(ctx.count("SD", 1, 0), got, s, d)
     ctx.close()
+
+
+def test_a_count_after_a_larger_upload_only_counts():
+    """The cell lists follow the automatic width at the upload that changes it: a
+    count enqueued later runs its own two kernels, no sort."""
+    p, s, d, ps, pd, pbig = _box()
+    ctx = _lib.Context(p)
+    ctx.upload(0, ps)
+    ctx.upload(1, pd)
+    ref = ctx.count("SD", 1, 0)
+    ctx.upload(2, pbig)
+    n = ctx.launches()
+    ctx.count_async("SD", 1, 0)
+    _same(ctx.finish(), ref, s, d)
+    assert ctx.launches() - n == 2
+    ctx.close()
