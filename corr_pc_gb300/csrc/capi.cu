@@ -131,6 +131,12 @@ struct SkyJobBufs {
   DevBuf<SkyTileRows> tiles;
 };
 
+// a box job's histogram block and counters
+struct AccumBufs {
+  DevBuf<unsigned long long> num, counters;
+  DevBuf<double> sums;
+};
+
 struct UnitCache {
   uint64_t v1 = 0, v2 = 0;
   int s1 = -1, s2 = -1, wpi = 0, tile = 0, twin = 0, variant = 0;
@@ -171,9 +177,7 @@ struct cpc_ctx {
   unsigned long long qcap = 0;
   double q_per_unit = 0;  // most pairs any count queued per work unit (queue sizing)
   size_t last_units = 0;  // work units of the last fast launch
-  DevBuf<unsigned long long> d_num;
-  DevBuf<double> d_sums;
-  DevBuf<unsigned long long> d_counters;
+  std::vector<std::unique_ptr<AccumBufs>> accum;  // one per job of this context in a launch
   // sky launches: one buffer set per job of the launch, the unit queue
   std::vector<std::unique_ptr<SkyJobBufs>> sky_bufs;
   DevBuf<SkyUnit> d_sky_units;
@@ -1028,23 +1032,33 @@ cpc_status ensure_scratch(cpc_ctx *c, size_t n_units, size_t n_jobs) {
   return CPC_OK;
 }
 
-cpc_status alloc_accum(cpc_ctx *c) {
+size_t accum_cells(const cpc_ctx *c) {
   const cpc_params &p = c->p;
-  const size_t n_hist = 1 + (p.do_jk ? p.n_jk : 0);
-  const size_t cells = n_hist * p.n_bins * p.n_p_bin;
-  CK(c->d_num.alloc(cells), "alloc accum");
-  CK(c->d_sums.alloc(cells * kNF), "alloc accum");
-  CK(c->d_counters.alloc(4), "alloc counters");
+  return (size_t)(1 + (p.do_jk ? p.n_jk : 0)) * p.n_bins * p.n_p_bin;
+}
+
+// The histogram block and counters of a box job: the context's q-th (the jobs of one
+// context in a batch have one each)
+cpc_status alloc_accum(JobPlan &jp, size_t q) {
+  cpc_ctx *c = jp.c;
+  const size_t cells = accum_cells(c);
+  while (c->accum.size() <= q) c->accum.emplace_back(new AccumBufs());
+  AccumBufs &a = *c->accum[q];
+  CK(a.num.alloc(cells), "alloc accum");
+  CK(a.sums.alloc(cells * kNF), "alloc accum");
+  CK(a.counters.alloc(4), "alloc counters");
+  jp.jd.acc_num = a.num.p;
+  jp.jd.acc_sums = a.sums.p;
+  jp.jd.counters = a.counters.p;
   return CPC_OK;
 }
 
-cpc_status zero_accum(cpc_ctx *c, cudaStream_t st) {
-  const cpc_params &p = c->p;
-  const size_t n_hist = 1 + (p.do_jk ? p.n_jk : 0);
-  const size_t cells = n_hist * p.n_bins * p.n_p_bin;
-  CK(cudaMemsetAsync(c->d_num.p, 0, sizeof(unsigned long long) * cells, st), "memset");
-  CK(cudaMemsetAsync(c->d_sums.p, 0, sizeof(double) * cells * kNF, st), "memset");
-  CK(cudaMemsetAsync(c->d_counters.p, 0, sizeof(unsigned long long) * 4, st), "memset");
+cpc_status zero_accum(const JobPlan &jp, cudaStream_t st) {
+  cpc_ctx *c = jp.c;
+  const size_t cells = accum_cells(c);
+  CK(cudaMemsetAsync(jp.jd.acc_num, 0, sizeof(unsigned long long) * cells, st), "memset");
+  CK(cudaMemsetAsync(jp.jd.acc_sums, 0, sizeof(double) * cells * kNF, st), "memset");
+  CK(cudaMemsetAsync(jp.jd.counters, 0, sizeof(unsigned long long) * 4, st), "memset");
   return CPC_OK;
 }
 
@@ -1071,8 +1085,8 @@ cpc_status fetch_accum_from(cpc_ctx *c, const unsigned long long *num, const dou
   return CPC_OK;
 }
 
-cpc_status fetch_accum(cpc_ctx *c, cpc_accum *out, cudaStream_t st, int unit_w) {
-  return fetch_accum_from(c, c->d_num.p, c->d_sums.p, c->d_counters.p, out, st, unit_w);
+cpc_status fetch_accum(const JobPlan &jp, cudaStream_t st, int unit_w) {
+  return fetch_accum_from(jp.c, jp.jd.acc_num, jp.jd.acc_sums, jp.jd.counters, jp.out, st, unit_w);
 }
 
 cpc_status build_zorder(cpc_ctx *c, Slot &s) {
@@ -1120,8 +1134,8 @@ DCat zview(Slot &s) {
 cpc_status enqueue_plain(JobPlan &jp) {
   cpc_ctx *c = jp.c;
   cpc_status s;
-  if ((s = alloc_accum(c)) != CPC_OK) return s;
-  if ((s = zero_accum(c, c->st)) != CPC_OK) return s;
+  if ((s = alloc_accum(jp, 0)) != CPC_OK) return s;
+  if ((s = zero_accum(jp, c->st)) != CPC_OK) return s;
   CK(cudaEventRecord(c->e0, c->st), "event");
   if (jp.empty) {
     CK(cudaEventRecord(c->e1, c->st), "event");
@@ -1131,9 +1145,6 @@ cpc_status enqueue_plain(JobPlan &jp) {
   if ((s = build_zorder(c, g1)) != CPC_OK) return s;
   if ((s = build_zorder(c, g2)) != CPC_OK) return s;
   if ((s = ensure_scratch(c, 1, 1)) != CPC_OK) return s;
-  jp.jd.acc_num = c->d_num.p;
-  jp.jd.acc_sums = c->d_sums.p;
-  jp.jd.counters = c->d_counters.p;
   DCat a = zview(g1), b = zview(g2);
   jp.jd.d1 = a;
   jp.jd.d2 = b;
@@ -1147,7 +1158,7 @@ cpc_status enqueue_plain(JobPlan &jp) {
 cpc_status finish_plain(JobPlan &jp) {
   cpc_ctx *c = jp.c;
   cpc_status s;
-  if ((s = fetch_accum(c, jp.out, c->st, 0)) != CPC_OK) return s;
+  if ((s = fetch_accum(jp, c->st, 0)) != CPC_OK) return s;
   float ms = 0;
   CK(cudaEventElapsedTime(&ms, c->e0, c->e1), "event time");
   jp.out->kernel_ms = ms;
@@ -1174,11 +1185,6 @@ struct FastGroup {
   int twin;        // the group's jobs are twin jobs (their own kernel)
 };
 
-size_t accum_cells(const cpc_ctx *c) {
-  const cpc_params &p = c->p;
-  return (size_t)(1 + (p.do_jk ? p.n_jk : 0)) * p.n_bins * p.n_p_bin;
-}
-
 // The device work of one fast count, in stream order on st: zero every job's
 // histogram block and counters, the edge-queue counter, then per group the
 // unit counter and the persistent kernel, then the FP64 recheck.  rec_flags
@@ -1188,7 +1194,7 @@ cpc_status fast_body(cpc_ctx *c0, std::vector<JobPlan> &jobs, const std::vector<
                      cudaStream_t st, unsigned rec_flags) {
   cpc_ctx *c = c0;
   for (size_t k = 0; k < jobs.size(); k++) {
-    const cpc_status s = zero_accum(jobs[k].c, st);
+    const cpc_status s = zero_accum(jobs[k], st);
     if (s != CPC_OK) return s;
   }
   CK(cudaMemsetAsync(c0->d_qcount.p, 0, sizeof(unsigned long long), st), "memset");
@@ -1224,9 +1230,9 @@ std::vector<uint64_t> fast_graph_key(cpc_ctx *c0, const std::vector<JobPlan> &jo
   put((uint64_t)c0->sm_count);
   put(jobs.size());
   for (const JobPlan &jp : jobs) {
-    put((uint64_t)(uintptr_t)jp.c->d_num.p);
-    put((uint64_t)(uintptr_t)jp.c->d_sums.p);
-    put((uint64_t)(uintptr_t)jp.c->d_counters.p);
+    put((uint64_t)(uintptr_t)jp.jd.acc_num);
+    put((uint64_t)(uintptr_t)jp.jd.acc_sums);
+    put((uint64_t)(uintptr_t)jp.jd.counters);
     put(accum_cells(jp.c));
   }
   put(gs.size());
@@ -1302,12 +1308,10 @@ cpc_status enqueue_fast(std::vector<JobPlan> &jobs) {
   cpc_ctx *c0 = jobs[0].c;
   cpc_ctx *c = c0;
   cudaStream_t st = c0->st;
-  for (size_t k = 0; k < jobs.size(); k++) {
-    cpc_status s;
-    if ((s = alloc_accum(jobs[k].c)) != CPC_OK) return s;
-    jobs[k].jd.acc_num = jobs[k].c->d_num.p;
-    jobs[k].jd.acc_sums = jobs[k].c->d_sums.p;
-    jobs[k].jd.counters = jobs[k].c->d_counters.p;
+  std::map<cpc_ctx *, size_t> n_of;  // jobs of each context so far
+  for (JobPlan &jp : jobs) {
+    const cpc_status s = alloc_accum(jp, n_of[jp.c]++);
+    if (s != CPC_OK) return s;
   }
   // group by kernel instantiation: corel, jackknife, twin, variant
   using Inst = std::tuple<int, int, int, int>;
@@ -1441,7 +1445,7 @@ cpc_status finish_fast(std::vector<JobPlan> &jobs, int grow_attempt) {
     return run_fast(jobs, 1);
   }
   for (size_t k = 0; k < jobs.size(); k++) {
-    if ((s = fetch_accum(jobs[k].c, jobs[k].out, st, jobs[k].jd.unit_w)) != CPC_OK) return s;
+    if ((s = fetch_accum(jobs[k], st, jobs[k].jd.unit_w)) != CPC_OK) return s;
     jobs[k].out->kernel_ms = ms;
     jobs[k].out->pair_kernel_ms = pms;
   }

@@ -196,12 +196,13 @@ cpc_status cpc_accum_shape(const cpc_ctx *ctx, int *n_hist, int *n_bins, int *n_
 /* Batched counting: run n_jobs pair types, possibly on different contexts
  * (e.g. many periodic sub-boxes), in ONE persistent launch of the fast
  * kernel that drains a single device work queue.  ctxs[k], kinds[k],
- * slots_g1[k], slots_g2[k] and outs[k] describe job k.  All contexts must
- * live on the current device.  Sky jobs (coordinates 0) that share one
- * context -- the SRd, RsRd, SD and DRs terms of a sky run, do_corr.cpp:103-131
- * -- share one list of work units (pairs of jackknife regions) of the fast sky
- * kernel, in one launch or, when it is long, one per group of corels; sky jobs on
- * several contexts run one after another.  Synchronous. */
+ * slots_g1[k], slots_g2[k] and outs[k] describe job k; jobs of one context may
+ * count any of its pairs.  All contexts must live on the current device.  Sky
+ * jobs (coordinates 0) that share one context -- the SRd, RsRd, SD and DRs terms
+ * of a sky run, do_corr.cpp:103-131 -- share one list of work units (pairs of
+ * jackknife regions) of the fast sky kernel, in one launch or, when it is long,
+ * one per group of corels; sky jobs on several contexts run one after another.
+ * Synchronous. */
 cpc_status cpc_count_batch(int n_jobs, cpc_ctx *const *ctxs, const cpc_pair_kind *kinds,
                            const int *slots_g1, const int *slots_g2, cpc_accum *outs);
 

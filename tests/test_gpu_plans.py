@@ -85,3 +85,25 @@ def test_a_count_after_a_larger_upload_only_counts():
     _same(ctx.finish(), ref, s, d)
     assert ctx.launches() - n == 2
     ctx.close()
+
+
+def test_a_batch_of_pairs_of_one_context():
+    """More pair types of one context in a batch than it keeps unit lists of: each
+    job has its own block, the first call's and the next one's."""
+    p, s, d, ps, pd, _ = _box(1)
+    ctx = _lib.Context(p)
+    cats = [(0, s, ps), (1, d, pd)]
+    for k in range(2, 7):
+        c = _cat(400 + 211 * k, 10 + k, L, which=1)
+        q = _params(1, 900, L=L, rmax=20.0, npi=20, pmax=100.0)
+        q.n_density = c.n
+        cats.append((k, c, host.prepare(q, [("S", s), ("D", c)])["D"]))
+    for k, _, g in cats:
+        ctx.upload(k, g)
+    pairs = [(k, 0) for k in range(1, 7)] + [(k, 1) for k in range(2, 7)]
+    refs = [ctx.count("SD", a, b, engine="fp64") for a, b in pairs]
+    for _ in range(2):
+        rs = _lib.count_batch([(ctx, "SD", a, b) for a, b in pairs])
+        for (a, b), r, ref in zip(pairs, rs, refs):
+            _same(r, ref, cats[a][1], cats[b][1], f"{a},{b}")
+    ctx.close()
