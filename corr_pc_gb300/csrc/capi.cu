@@ -890,15 +890,22 @@ cpc_status plan_job(cpc_ctx *c, cpc_pair_kind kind, int slot_g1, int slot_g2, in
   return CPC_OK;
 }
 
-// tiles of g1 rows and their units (cached per slot versions and window)
-const UnitCache &build_units(JobPlan &jp) {
+// tiles of g1 rows and their units (cached per slot versions and window).  The
+// context keeps the lists last used, 8 or those of the `jobs` jobs that the present
+// launch has of it: a list goes only when newer ones fill the cache.
+const UnitCache &build_units(JobPlan &jp, size_t jobs) {
   cpc_ctx *c = jp.c;
-  for (auto &uc : c->unit_cache)
+  for (auto it = c->unit_cache.begin(); it != c->unit_cache.end(); ++it) {
+    const UnitCache &uc = *it;
     if (uc.s1 == jp.s1 && uc.s2 == jp.s2 && uc.v1 == c->slots[jp.s1].version &&
         uc.v2 == c->slots[jp.s2].version && uc.wpi == jp.wpi && uc.tile == jp.tile &&
-        uc.twin == jp.jd.twin && uc.variant == jp.variant)
-      return uc;
-  if (c->unit_cache.size() >= 8) c->unit_cache.erase(c->unit_cache.begin());
+        uc.twin == jp.jd.twin && uc.variant == jp.variant) {
+      std::rotate(it, it + 1, c->unit_cache.end());
+      return c->unit_cache.back();
+    }
+  }
+  while (c->unit_cache.size() >= std::max<size_t>(8, jobs))
+    c->unit_cache.erase(c->unit_cache.begin());
   c->unit_cache.emplace_back();
   UnitCache &uc = c->unit_cache.back();
   uc.s1 = jp.s1;
@@ -1331,7 +1338,7 @@ cpc_status enqueue_fast(std::vector<JobPlan> &jobs) {
   for (auto &g : groups) {
     const size_t b = total_units;
     for (int k : g.second) {
-      const UnitCache &uc = build_units(jobs[k]);
+      const UnitCache &uc = build_units(jobs[k], n_of[jobs[k].c]);
       // this context's shard of the units (cpc_set_shard): every n_shards-th
       // unit from `shard`; the units partition the pairs, so the shards' blocks
       // sum to the whole count
@@ -1352,7 +1359,7 @@ cpc_status enqueue_fast(std::vector<JobPlan> &jobs) {
     all.reserve(total_units);
     for (const auto &m : members)
       for (int k : m) {
-        const std::vector<UnitDesc> &u = build_units(jobs[k]).units;
+        const std::vector<UnitDesc> &u = build_units(jobs[k], n_of[jobs[k].c]).units;
         const size_t nsh = (size_t)jobs[k].c->n_shards;
         for (size_t ui = (size_t)jobs[k].c->shard; ui < u.size(); ui += nsh) {
           UnitDesc d = u[ui];
