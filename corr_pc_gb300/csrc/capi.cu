@@ -1016,6 +1016,7 @@ const UnitCache &build_units(JobPlan &jp, size_t jobs) {
 }
 
 cpc_status ensure_scratch(cpc_ctx *c, size_t n_units, size_t n_jobs) {
+  if (n_units > c->d_units.n) c->units_key.clear();  // the list held goes, even if this fails
   CK(c->d_units.alloc(n_units), "alloc units");
   CK(c->d_jobs.alloc(n_jobs), "alloc jobs");
   CK(c->d_unit_ctr.alloc(1), "alloc counter");
@@ -1351,9 +1352,8 @@ cpc_status enqueue_fast(std::vector<JobPlan> &jobs) {
     members.push_back(g.second);
   }
   cpc_status s;
-  const UnitDesc *held = c0->d_units.p;
   if ((s = ensure_scratch(c0, std::max<size_t>(1, total_units), jobs.size())) != CPC_OK) return s;
-  if (held != c0->d_units.p || key != c0->units_key) {
+  if (key != c0->units_key) {
     c0->units_key.clear();
     std::vector<UnitDesc> all;
     all.reserve(total_units);
