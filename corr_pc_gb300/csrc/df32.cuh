@@ -216,5 +216,19 @@ DF_HD void f_to_words(float v, float qs, unsigned &hi, unsigned &lo) {
   hi = magic_bits(a);
   lo = magic_bits(rn_add(rn_fma(rn_sub(a, kMagic), -32768.0f, t), kMagic));
 }
+// The sum of n terms from their summed words, bias = n kMagicBits (mod 2^32): right
+// while each word less its bias stays within 31 bits.  For |t| < 2^29 a high part
+// is at most 2^14 and a low part the rest of t, at most 2^14, plus l 2^S.  The l of
+// pair_df.cuh's terms is made of roundings of 2^-24 (32 quanta at the bound) and, for
+// the rotated ones, of the l of cos and sin 2 theta, at most 13 of them (a reciprocal
+// of 2 ulps and the squares' roundings): 1450 quanta for the largest, a product of
+// two rotated ellipticities.  The sky kernel's terms, |t| <= 2^30 / (1 + 2^-12), have
+// high parts below 2^15 - 7 and an l of twice those quanta.
+constexpr int kLowTerm = (1 << 14) + (1 << 11);
+constexpr int kBinTerms = (1 << 17) - (1 << 14);  // terms a word of |t| < 2^29 may take
+static_assert((long long)kBinTerms * kLowTerm < 1ll << 31, "low words stay within 31 bits");
+DF_HD long long fixed_sum(const unsigned *w, unsigned bias) {
+  return (long long)(int)(w[0] - bias) * 32768ll + (int)(w[1] - bias);
+}
 
 }  // namespace cpc

@@ -150,21 +150,18 @@ size_t fast_smem_bytes(int corel, int do_jk, int nrp, int wpi, int auto_pairs, i
 
 // Fixed-point sums in 32-bit shared words.  A term v of field f becomes the
 // integer u = rint(v * 2^S_f), |u| < 2^29 (S_f from a bound on |v|), split into
-// a high part of at most 2^14 and a signed low part of at most 2^14 + 1, each
+// a high part of at most 2^14 and a signed low part of at most kLowTerm, each
 // added with its bias (df_to_words) to its own 32-bit word with a plain
 // reduction (no return value: no scoreboard wait).  A bin takes at most kBinTerms
 // pairs between flushes, so that a word, read as a signed integer after its
-// bin's count of biases is taken off, stays within 2^31: a block keeps a bound
+// bin's count of biases is taken off, stays within 2^31 (df32.cuh): a block keeps a bound
 // on the fullest bin (its last known maximum plus every pair tested since),
 // finds the maximum when the bound could pass kBinTerms and flushes when the
 // maximum itself could.  (Bounding the block's pair total instead flushed
 // almost every thousand candidates.)
-constexpr int kBinTerms = (1 << 17) - 64;
-// candidates a bin bound takes at a time: half of kBinTerms for a full tile
+// Candidates a bin bound takes at a time: half of kBinTerms for a full tile
 constexpr int kChunkTests = 1 << 16;
-__device__ __forceinline__ long long fixed_sum(const unsigned *w, unsigned bias) {
-  return (long long)(int)(w[0] - bias) * 32768ll + (int)(w[1] - bias);
-}
+static_assert(kChunkTests <= kBinTerms, "a chunk fits a bin's words after a flush");
 // Order of a lane's reductions.  Lanes of one instruction that hit the same bin
 // are serialised (a cycle each), and the pairs of a tile concentrate on a few
 // r_p bins: 32 pairs drawn from a (tile, group) of the 200k wg+ box put 6.2 on

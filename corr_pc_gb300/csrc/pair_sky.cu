@@ -161,8 +161,13 @@ constexpr int kSkySeg = 256;            // candidate buckets taken at a time
 // adds at most 32 of them each to fewer than 32 left over
 __host__ __device__ constexpr int sky_ring(int cand) { return 32 * cand; }
 // pairs a block may add to a bin between flushes: |u| < 2^30 splits into words
-// of at most 2^15, so 2^16 of them stay within a signed 32-bit word
+// below 2^15 - 7 and low ones within 2^14 + 2^12 (df32.cuh), so 2^16 of them stay
+// within a signed 32-bit word
 constexpr int kSkyFlushPairs = 1 << 16;
+static_assert((long long)kSkyFlushPairs * ((1 << 15) - 7) < 1ll << 31,
+              "high words stay within 31 bits");
+static_assert((long long)kSkyFlushPairs * ((1 << 14) + (1 << 12)) < 1ll << 31,
+              "low words stay within 31 bits");
 constexpr unsigned kSkyEdge = 0x8000u;  // queue entry: the window test is undecided
 
 // Jackknife attribution of a sky pair: jk_check_sky (jk.cpp:53-57), each
@@ -348,7 +353,7 @@ __device__ __noinline__ void sky_flush(const JobDev &J, unsigned *H, int xreg, i
     const unsigned bias = n * kMagicBits;
     for (int f = f0; f < F::FM; f++) {
       const int o = 1 + 2 * (f - f0), fld = F::m(f);
-      const long long x = (long long)(int)(h[o] - bias) * 32768ll + (int)(h[o + 1] - bias);
+      const long long x = fixed_sum(h + o, bias);
       h[o] = 0u;
       h[o + 1] = 0u;
       if (x == 0) continue;
