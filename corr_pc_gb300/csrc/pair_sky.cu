@@ -168,6 +168,10 @@ static_assert((long long)kSkyFlushPairs * ((1 << 15) - 7) < 1ll << 31,
               "high words stay within 31 bits");
 static_assert((long long)kSkyFlushPairs * ((1 << 14) + (1 << 12)) < 1ll << 31,
               "low words stay within 31 bits");
+// The same for counts of unit weights, which have no such words: what is pending and
+// the next candidates' pairs, each at most this many, stay within an int.
+constexpr int kSkyFlushCounts = 1 << 29;
+static_assert(2ll * kSkyFlushCounts <= INT_MAX, "pairs pending in a histogram fit an int");
 constexpr unsigned kSkyEdge = 0x8000u;  // queue entry: the window test is undecided
 
 // Jackknife attribution of a sky pair: jk_check_sky (jk.cpp:53-57), each
@@ -413,8 +417,7 @@ __device__ __forceinline__ void sky_unit(const SkyUnit &U, const JobDev &J, unsi
   // an upper bound of the pairs in the histogram, and the regions that take
   // them at the flush (the tile's, the candidates'; -1: none)
   int pending = 0, cur_x = -1, cur_y = -1;
-  // counts alone cannot overflow their words: only the fixed-point words can
-  const int flush_pairs = (F::FM > f0) ? kSkyFlushPairs : 1 << 30;
+  const int flush_pairs = (F::FM > f0) ? kSkyFlushPairs : kSkyFlushCounts;
   for (int ti = U.tile0; ti < U.tile1; ti++) {
   const SkyTileRows T = J.tiles[ti];
   const int W = (T.count + 31) >> 5;
