@@ -2600,21 +2600,25 @@ cpc_status sky_run(cpc_ctx *c, std::vector<SkyPlan> &plans, cpc_engine engine) {
         CK(cudaStreamWaitEvent(c->st2, c->e_in, 0), "stream wait");
       }
       std::reverse(ranges.begin(), ranges.end());  // (counts, of the small blocks, fill in)
-      for (size_t q = 0; q < ranges.size(); q++) {
+      cudaError_t launched = cudaSuccess;
+      for (size_t q = 0; q < ranges.size() && launched == cudaSuccess; q++) {
         size_t hist_words = 1;
         for (const JobDev &J : jd)
           if (J.sk.hist_smem && set_of(J) <= ranges[q].set)
             hist_words = std::max(hist_words,
                                   sky_hist_words(J.corel, J.unit_w, p.n_bins * p.n_p_bin));
-        CK(launch_sky_tile(c->d_jobs.p, c->d_sky_units.p + ranges[q].first, (int)ranges[q].n,
-                           ranges[q].set, hist_words, c->d_sky_ctr.p + q, kSkyHostQueue, esum,
-                           c->sm_count, q & 1 ? c->st2 : st), "sky kernel");
-        c->launches += 1;
+        launched = launch_sky_tile(c->d_jobs.p, c->d_sky_units.p + ranges[q].first,
+                                   (int)ranges[q].n, ranges[q].set, hist_words,
+                                   c->d_sky_ctr.p + q, kSkyHostQueue, esum, c->sm_count,
+                                   q & 1 ? c->st2 : st);
+        if (launched == cudaSuccess) c->launches += 1;
       }
+      // st goes on after st2, also where a launch failed: a later count reuses the buffers
       if (ranges.size() > 1) {
         CK(cudaEventRecord(c->e_done, c->st2), "event");
         CK(cudaStreamWaitEvent(st, c->e_done, 0), "stream wait");
       }
+      CK(launched, "sky kernel");
       for (size_t m = 0; m < jd.size(); m++) {
         const SkyPlan &P = plans[idx[m]];
         CK(launch_sky_finish((int64_t)P.n_fix, jd[m].acc_fix, jd[m].acc_fixh, jd[m].acc_sums,
@@ -2698,6 +2702,7 @@ cpc_status cpc_create(cpc_ctx **out, const cpc_params *params) try {
 cpc_status cpc_destroy(cpc_ctx *c) try {
   if (!c) return CPC_OK;
   cudaStreamSynchronize(c->st);
+  if (c->st2) cudaStreamSynchronize(c->st2);
   drop_graph(c);
   if (c->e0) cudaEventDestroy(c->e0);
   if (c->e1) cudaEventDestroy(c->e1);
