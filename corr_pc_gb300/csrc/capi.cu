@@ -107,6 +107,7 @@ struct Slot {
   double sky_mag = 0;         // largest window bound or coordinate of the float tests
   double sky_zw = 0;          // mean width of the rows' windows in scaled redshift
   double sky_fz = 0;          // mean share of the catalogue inside a row's redshift window
+  double sky_hw = 0, sky_area = 0;  // mean half width of the rows' Dec windows; area (degrees)
   int sky_nkey = 0;           // (region, keep flag) keys with galaxies
   std::vector<int> hc_zidx;   // redshift-ordered position of each cell-ordered row
   std::vector<float> hc_z;    // scaled redshift, cell order
@@ -1709,6 +1710,8 @@ void sky_cell_order(cpc_ctx *c, Slot &s, const std::vector<double> &zs,
   }
   s.sky_zw = zw * zk;
   s.sky_fz = fz;
+  s.sky_hw = hw;
+  s.sky_area = 0;
   int64_t cells = 0;
   for (Reg &r : reg) {
     r.base = cells;
@@ -1716,6 +1719,7 @@ void sky_cell_order(cpc_ctx *c, Slot &s, const std::vector<double> &zs,
       const double cosd = std::cos(0.5 * (r.d0 + r.d1) * M_PI / 180.0);
       const double ex = std::max((r.a1 - r.a0) * std::max(cosd, 1e-3), 1e-9);
       const double ey = std::max(r.d1 - r.d0, 1e-9);
+      s.sky_area += ex * ey;
       double sz = std::sqrt(96.0 * ex * ey / (std::max(1e-9, 0.25 * fz) * (double)r.n));
       sz = std::min(std::max(sz, hw / 8), 0.75 * hw);
       if (sz > 0) {
@@ -2274,6 +2278,17 @@ void sky_consts(const cpc_ctx *c, const Slot &g1, const Slot &g2, JobDev &J) {
   }
 }
 
+// Entries for the undecided pairs of `rows` rows of g1 against g2: their window pairs,
+// by the share of g2 in a mean window, times twice the rate met (pair_sky.cu).  Too
+// few cost time, not pairs: randoms x randoms of 1M rows leave 5e6, all but a fixed
+// 2^20 of which went to single lanes (304 ms, 292 with room for them).
+size_t sky_queue(const Slot &g1, const Slot &g2, double rows) {
+  const double sky = std::min(1.0, 4 * g1.sky_hw * g1.sky_hw / std::max(g2.sky_area, 1e-30));
+  const double want = rows * (double)g2.n * g1.sky_fz * sky / 4096;
+  if (!(want > (double)kSkyExactQueue)) return kSkyExactQueue;
+  return (size_t)std::min(want, (double)kSkyExactQueueMax);
+}
+
 // Plan job k of a sky launch: the corels2 rules, the bands and fixed-point
 // scales of the mixed-precision path, zeroed device buffers (set k), the row
 // sample as a list of g1 rows.
@@ -2427,7 +2442,13 @@ cpc_status sky_plan(cpc_ctx *c, cpc_pair_kind kind, int slot_g1, int slot_g2, in
       CK(cudaMemcpyAsync(Bf.tiles.p, P.tiles->data(), sizeof(SkyTileRows) * P.tiles->size(),
                          cudaMemcpyHostToDevice, st), "H2D");
     J.tiles = Bf.tiles.p;
-    CK(Bf.xq.alloc(kSkyExactQueue), "alloc undecided pairs");
+    {
+      const double rows = (double)g1.n / (double)std::max<int64_t>(1, rs) / W;
+      const size_t want = sky_queue(g1, g2, rows);
+      if (want > kSkyExactQueue && Bf.xq.alloc(want) != cudaSuccess) cudaGetLastError();
+      CK(Bf.xq.alloc(kSkyExactQueue), "alloc undecided pairs");
+      J.xq_cap = Bf.xq.n;
+    }
     CK(Bf.xq_n.alloc(1), "alloc");
     CK(cudaMemsetAsync(Bf.xq_n.p, 0, sizeof(unsigned long long), st), "memset");
     J.xq = Bf.xq.p;

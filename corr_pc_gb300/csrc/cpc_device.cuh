@@ -180,7 +180,7 @@ struct JobDev {
   const SkyTileRows *tiles;            // the fast sky kernel's row tiles of this job
   int2 *xq;                            // sky pairs left to the FP64 path (cell positions;
                                        // ~i1: the window test is undecided too)
-  unsigned long long *xq_n;            // their number
+  unsigned long long *xq_n, xq_cap;    // their number, and the most that xq holds
   int2 *hq;                            // sky host-tier queue of this job
   unsigned long long *hq_n;            // its length
 };

@@ -114,7 +114,8 @@ cudaError_t launch_plain_fp64(const JobDev *job, const DCat &a, const DCat &b, c
 // Sky pairs (coordinates 0) in FP64; pairs whose r_p may bin differently with
 // the C library's trigonometry are appended to hq (host edge tier).
 constexpr unsigned long long kSkyHostQueue = 1ull << 22;
-constexpr unsigned long long kSkyExactQueue = 1ull << 20;  // undecided pairs of a job
+// Undecided pairs that a job's queue takes, at least and at most (2 GB)
+constexpr unsigned long long kSkyExactQueue = 1ull << 20, kSkyExactQueueMax = 1ull << 28;
 // (SkyFast, SkyConst and SkyUnit are declared in cpc_device.cuh)
 // The fast sky kernel over the units of every job (pair types) of one launch;
 // ctr (zeroed) is the unit queue.  set: 0 every job counts (density_density),

@@ -284,11 +284,11 @@ __device__ __noinline__ void sky_pair_exact(const JobDev &J, int i1, int j2, boo
 // Undecided pairs (about 1 in 10^4) are queued and evaluated by
 // sky_finish_kernel with every lane busy: evaluated here, one lane of a warp at
 // a time, they kept the FP64 pipe 62% busy and took half of the kernel's time.
-// Past the queue's end they are evaluated here all the same.
+// Past the queue's end (sized by sky_queue) they are evaluated here all the same.
 __device__ __forceinline__ void sky_undecided(const JobDev &J, int i1, int j2, bool edge,
                                               unsigned long long hq_cap, double esum) {
   const unsigned long long pos = atomicAdd(J.xq_n, 1ull);
-  if (pos < kSkyExactQueue) J.xq[pos] = make_int2(edge ? ~i1 : i1, j2);
+  if (pos < J.xq_cap) J.xq[pos] = make_int2(edge ? ~i1 : i1, j2);
   else sky_pair_exact(J, i1, j2, edge, hq_cap, esum);
 }
 
@@ -921,7 +921,7 @@ __global__ void sky_finish_kernel(int64_t n, const unsigned long long *__restric
   const JobDev &J = *jobp;
   const int64_t step = (int64_t)gridDim.x * blockDim.x;
   const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const unsigned long long nx = min(*J.xq_n, kSkyExactQueue);
+  const unsigned long long nx = min(*J.xq_n, J.xq_cap);
   for (int64_t i = i0; i < (int64_t)nx; i += step) {
     const int2 e = J.xq[i];
     const bool edge = e.x < 0;

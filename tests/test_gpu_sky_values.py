@@ -1,0 +1,37 @@
+"""The fast sky kernel against the plain FP64 sky kernel on pairs that it leaves to
+double precision: separations too small for single precision, galaxies at one
+distance."""
+import numpy as np
+import pytest
+
+from corr_pc_gb300 import _lib, host, synth
+from test_gpu_sky_tiles import _same
+
+pytestmark = pytest.mark.gpu
+
+
+def _context(p, t, cats):
+    ctx = _lib.Context(p, table=t)
+    for k, c in enumerate(host.prepare(p, cats, table=t).values()):
+        ctx.upload(k, c)
+    return ctx
+
+
+def test_more_undecided_pairs_than_their_queue_holds():
+    """1.44 million pairs closer than the separations that single precision can
+    bin: past the 2^20 queued ones they are evaluated in the pair kernel."""
+    p = synth._sky_params(which_corr=1, rmin=1e-3, rmax=1.0, nrp=9, npi=8, pmax=40.0, njk=4)
+    t = synth.flat_lcdm_table(p.z_max, p.dz)
+    cats = []
+    for role, seed in (("S", 3), ("D", 4)):
+        c = synth.sky_patch(1200, seed, t, nside_jk=2, with_shapes=True, weights=True)
+        rng = np.random.default_rng(seed)
+        c.x[:] = 5.0 + rng.uniform(-2e-3, 2e-3, c.n)
+        c.y[:] = 5.0 + rng.uniform(-2e-3, 2e-3, c.n)
+        c.z[:] = np.sort(rng.uniform(0.25, 0.252, c.n))
+        cats.append((role, c))
+    ctx = _context(p, t, cats)
+    got, ref = ctx.count("SD", 1, 0), ctx.count("SD", 1, 0, engine="fp64")
+    assert ref["n_window"] > 1 << 20
+    _same(got, ref, "undecided")
+    ctx.close()
