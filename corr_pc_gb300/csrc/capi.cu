@@ -2279,12 +2279,12 @@ void sky_consts(const cpc_ctx *c, const Slot &g1, const Slot &g2, JobDev &J) {
 }
 
 // Entries for the undecided pairs of `rows` rows of g1 against g2: their window pairs,
-// by the share of g2 in a mean window, times twice the rate met (pair_sky.cu).  Too
+// by the share of g2 in a mean window, times twice the rates met (pair_sky.cu).  Too
 // few cost time, not pairs: randoms x randoms of 1M rows leave 5e6, all but a fixed
 // 2^20 of which went to single lanes (304 ms, 292 with room for them).
-size_t sky_queue(const Slot &g1, const Slot &g2, double rows) {
+size_t sky_queue(const Slot &g1, const Slot &g2, double rows, bool counts) {
   const double sky = std::min(1.0, 4 * g1.sky_hw * g1.sky_hw / std::max(g2.sky_area, 1e-30));
-  const double want = rows * (double)g2.n * g1.sky_fz * sky / 4096;
+  const double want = rows * (double)g2.n * g1.sky_fz * sky * (counts ? 1.0 / 4096 : 1.0 / 200);
   if (!(want > (double)kSkyExactQueue)) return kSkyExactQueue;
   return (size_t)std::min(want, (double)kSkyExactQueueMax);
 }
@@ -2444,7 +2444,7 @@ cpc_status sky_plan(cpc_ctx *c, cpc_pair_kind kind, int slot_g1, int slot_g2, in
     J.tiles = Bf.tiles.p;
     {
       const double rows = (double)g1.n / (double)std::max<int64_t>(1, rs) / W;
-      const size_t want = sky_queue(g1, g2, rows);
+      const size_t want = sky_queue(g1, g2, rows, J.corel == COREL_DD && J.unit_w);
       if (want > kSkyExactQueue && Bf.xq.alloc(want) != cudaSuccess) cudaGetLastError();
       CK(Bf.xq.alloc(kSkyExactQueue), "alloc undecided pairs");
       J.xq_cap = Bf.xq.n;

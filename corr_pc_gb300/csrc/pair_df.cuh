@@ -43,16 +43,6 @@ DF_HD float ephi32(float phi, float theta) {  // ephi_calc (calcs.cpp:97-105)
   const float t = fabsf(phi - theta);
   return t > 1.5707963267948966f ? 3.14159265358979f - t : t;
 }
-// The same rounded once, from double-floats: with phi = -10 (a galaxy read
-// without shapes) the plain form's roundings, on a coarse grid, add up to 3e-7.
-DF_HD float ephi32_fine(float phi, float theta) {
-  const df32 d = two_diff(phi, theta);
-  const float s = d.h < 0.0f ? -1.0f : 1.0f, h = s * d.h, l = s * d.l;
-  const float pi_h = 3.14159274101257f, pi_l = -8.74227766e-8f;
-  if (!(h > 1.5707963267948966f)) return rn_add(h, l);
-  const df32 v = two_diff(pi_h, h);
-  return rn_add(v.h, rn_add(v.l, rn_sub(pi_l, l)));
-}
 
 // Terms of one binned pair for corel C.  d[q]: double-float terms of the
 // fields df_field(C, q); f[q]: float terms of the others (f[0] is set by the
@@ -62,12 +52,10 @@ DF_HD float ephi32_fine(float phi, float theta) {
 // of the same pair in the other order (g2, g1), the only ones that differ when
 // both galaxies carry the same data in either role (the orientation angle and
 // the rotations are those of the pair; the products are symmetric).
-// fine: the phi terms by ephi32_fine.
 template <int C>
 DF_HD void df_pair_terms(df32 c, df32 s, float theta, const DfGal &g1, const DfGal &g2, int gws,
                          bool unit_w, df32 *d, float *f, df32 *dm = nullptr,
-                         float *fm = nullptr, bool fine = false) {
-  auto ephi = [&](float phi) { return fine ? ephi32_fine(phi, theta) : ephi32(phi, theta); };
+                         float *fm = nullptr) {
   if (C == kDfDK) {  // density_convergence (corels.cpp:79-90): wt kappa of the shape holder
     const df32 z{0.0f, 0.0f};
     if (gws == 1) d[1] = unit_w ? g1.e1 : df_mul(g2.w, g1.e1);
@@ -96,7 +84,7 @@ DF_HD void df_pair_terms(df32 c, df32 s, float theta, const DfGal &g1, const DfG
     d[3] = unit_w ? ex : df_mul(go.w, ex);
     f[2] = d[1].h * d[1].h;
     f[4] = d[3].h * d[3].h;
-    f[11] = ephi(g1.phi);
+    f[11] = ephi32(g1.phi, theta);
     f[12] = f[11] * f[11];
     return;
   }
@@ -108,7 +96,7 @@ DF_HD void df_pair_terms(df32 c, df32 s, float theta, const DfGal &g1, const DfG
     // the shape holder's terms for the holder in role 2 (g2) and in role 1 (g1);
     // the other order (g2, g1) swaps them
     const df32 e_of2 = unit_w ? ej0 : df_mul(g1.w, ej0), e_of1 = unit_w ? ei0 : df_mul(g2.w, ei0);
-    const float t_of2 = ephi(g2.phi), t_of1 = ephi(g1.phi);
+    const float t_of2 = ephi32(g2.phi, theta), t_of1 = ephi32(g1.phi, theta);
     if (gws == 2) {
       d[1] = e_of2;
       f[11] = t_of2;
@@ -143,7 +131,7 @@ DF_HD void df_pair_terms(df32 c, df32 s, float theta, const DfGal &g1, const DfG
     const float ha = 0.5f * pa.h, hb = 0.5f * pb.h, ka = 0.5f * qa.h, kb = 0.5f * qb.h;
     f[2] = ha * ha + hb * hb;
     f[4] = ka * ka + kb * kb;
-    const float ta = ephi(g1.phi), tb = ephi(g2.phi);
+    const float ta = ephi32(g1.phi, theta), tb = ephi32(g2.phi, theta);
     f[11] = ta + tb;
     f[12] = ta * ta + tb * tb;
   }

@@ -20,8 +20,9 @@
 // queue and binned there with the C library.  All other pairs are binned here
 // against the exact host-derived thresholds, so the integer counts equal the
 // reference's.  D_C is a row of the distance table, so 0.2% of the pairs have
-// Pi = 0 exactly, often a bin edge: the fast kernel recognises them by equal
-// D_C (three float parts) and takes their bin from the host.  Shape sums use CUDA's atan/cos/sin (within 1e-6).
+// Pi = 0 exactly, often a bin edge: counts of unit weights recognise them by equal
+// D_C (three float parts) and take their bin from the host, else they take the FP64
+// path.  Shape sums use CUDA's atan/cos/sin (within 1e-6).
 //
 // Two kernels:
 //  * sky_fp64_kernel -- the plain FP64 kernel: one thread per g1 row, every
@@ -281,10 +282,11 @@ __device__ __noinline__ void sky_pair_exact(const JobDev &J, int i1, int j2, boo
   sky_pair_fp64(J, i, j, hq_cap, esum);
 }
 
-// Undecided pairs (about 1 in 10^4) are queued and evaluated by
-// sky_finish_kernel with every lane busy: evaluated here, one lane of a warp at
-// a time, they kept the FP64 pipe 62% busy and took half of the kernel's time.
-// Past the queue's end (sized by sky_queue) they are evaluated here all the same.
+// Undecided pairs (about 1 in 10^4, and with weights or shapes those of equal D_C, 1
+// in 400) are queued and evaluated by sky_finish_kernel with every lane busy:
+// evaluated here, one lane of a warp at a time, they kept the FP64 pipe 62% busy and
+// took half of the kernel's time.  Past the queue's end (sized by sky_queue) they
+// are evaluated here all the same.
 __device__ __forceinline__ void sky_undecided(const JobDev &J, int i1, int j2, bool edge,
                                               unsigned long long hq_cap, double esum) {
   const unsigned long long pos = atomicAdd(J.xq_n, 1ull);
@@ -734,11 +736,11 @@ __device__ __forceinline__ void sky_unit(const SkyUnit &U, const JobDev &J, unsi
               const float m2 = v2 + kMagic;
               int n2 = __float_as_int(m2) - (int)kMagicBits;
               bool pi_ok = fabsf(v2 - (m2 - kMagic)) <= S.k.pi_in;
-              // equal D_C (all three parts: common, as D_C is a distance-table row):
-              // Pi is exactly 0, here a bin edge
-              const bool zero_pi =
-                  !pi_ok && pf == 0.0f && w1.w == w2.w && l1.w == l2.w && S.d3[a1] == S.d3[a2];
-              if (zero_pi) {
+              // equal D_C (all three parts: common, as D_C is a distance-table row): Pi is
+              // exactly 0, here a bin edge.  Where the pair adds a count and nothing else,
+              // its bin is all there is to know; other pairs' values stay FP64
+              if (!kShapes && uw && !pi_ok && pf == 0.0f && w1.w == w2.w && l1.w == l2.w &&
+                  S.d3[a1] == S.d3[a2]) {
                 n2 = S.k.pi_zero;
                 pi_ok = true;
               }
@@ -804,9 +806,7 @@ __device__ __forceinline__ void sky_unit(const SkyUnit &U, const JobDev &J, unsi
                   const float2 p1 = v_p[a1], p2 = v_p[a2];
                   const DfGal g1{{e1.x, e1.z}, {e1.y, e1.w}, {x1.w, p1.y}, p1.x};
                   const DfGal g2{{e2.x, e2.z}, {e2.y, e2.w}, {x2.w, p2.y}, p2.x};
-                  // (pairs at Pi = 0, one bin's share of which is large, would reach the
-                  // FP64 path but for their exact bin: their phi terms stay as exact)
-                  df_pair_terms<C>(c, sn, theta, g1, g2, gws, uw, vd, v, nullptr, nullptr, zero_pi);
+                  df_pair_terms<C>(c, sn, theta, g1, g2, gws, uw, vd, v);
                 }
                 unsigned wh[F::FM], wl[F::FM];
 #pragma unroll

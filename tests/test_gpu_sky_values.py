@@ -17,6 +17,26 @@ def _context(p, t, cats):
     return ctx
 
 
+@pytest.mark.parametrize("which", [0, 1, 2])
+def test_pairs_of_equal_distance_keep_the_fp64_values(which):
+    """Every pair has Pi = 0, an edge of the Pi bins: the values added are those of
+    the FP64 engine.  The sums differ by the order of n additions alone, each
+    within 2^-53 of the largest partial sum."""
+    p = synth._sky_params(which_corr=which, rmin=0.3, rmax=40.0, nrp=12, npi=16, pmax=40.0, njk=9)
+    t = synth.flat_lcdm_table(p.z_max, p.dz)
+    a = synth.sky_patch(700, 3, t, nside_jk=3, with_shapes=True, weights=True)
+    b = synth.sky_patch(1900, 4, t, nside_jk=3, with_shapes=True, weights=True)
+    for c in (a, b):
+        c.z[:] = 0.25
+    ctx = _context(p, t, [("S", a), ("D", b)])
+    got, ref = ctx.count("SD", 1, 0), ctx.count("SD", 1, 0, engine="fp64")
+    assert np.array_equal(got["num"], ref["num"]) and got["n_window"] == ref["n_window"]
+    bound = np.array([2.25, 2.25, 5.1, 2.25, 5.1, 2.25, 2.25, 5.1, 2.25, 5.1, 5.1, 27.0, 400.0])
+    n = ref["num"][..., None].astype(float)
+    assert (np.abs(got["sums"] - ref["sums"]) <= 2 * n * n * bound * 2.0 ** -53).all()
+    ctx.close()
+
+
 def test_more_undecided_pairs_than_their_queue_holds():
     """1.44 million pairs closer than the separations that single precision can
     bin: past the 2^20 queued ones they are evaluated in the pair kernel."""
