@@ -1626,6 +1626,36 @@ cpc_status rebuild_cells(cpc_ctx *c, Slot &s, int k) {
   return build_cells(c, s, n, k, c->u_orig.p, false);
 }
 
+// A context's tuning and cell widths during the autotuners' trials: put back when the
+// trials end without a choice (an error return).  A slot whose rebuild fails stays
+// invalid, as after a failed upload.
+struct TuneTrials {
+  cpc_ctx *c;
+  int k, wpi;
+  bool active = true;
+  struct Cells {
+    int k;
+    bool automatic;
+  } cells[kMaxSlots];
+  explicit TuneTrials(cpc_ctx *ctx) : c(ctx), k(ctx->tune_k), wpi(ctx->tune_wpi) {
+    for (int q = 0; q < kMaxSlots; q++) cells[q] = {c->slots[q].kcells, c->slots[q].auto_k};
+  }
+  ~TuneTrials() {
+    if (!active) return;
+    c->tune_k = k;
+    c->tune_wpi = wpi;
+    for (int q = 0; q < kMaxSlots; q++) {
+      Slot &s = c->slots[q];
+      s.auto_k = cells[q].automatic;
+      try {
+        if (s.valid && !s.sky && s.kcells != cells[q].k) rebuild_cells(c, s, cells[q].k);
+      } catch (...) {
+        s.valid = false;
+      }
+    }
+  }
+};
+
 // A box slot on cells r_max / k wide that no later upload changes (the autotuners).
 cpc_status set_cells(cpc_ctx *c, Slot &s, int k) {
   const cpc_status st = s.kcells == k ? CPC_OK : rebuild_cells(c, s, k);
@@ -3002,6 +3032,7 @@ cpc_status cpc_autotune(cpc_ctx *c, cpc_pair_kind kind, int slot_g1, int slot_g2
   // tiles, so each trial's per-unit costs are those of the full count)
   const int64_t stride = std::max<int64_t>(1, sample_stride);
   ShardOverride so(c, 0, (int)std::min<int64_t>(stride, 1 << 30));
+  TuneTrials trials(c);
   double best = INFINITY;
   int bk = c->slots[slot_g1].kcells, bw = c->tune_wpi;
   for (int k : ks) {
@@ -3026,6 +3057,10 @@ cpc_status cpc_autotune(cpc_ctx *c, cpc_pair_kind kind, int slot_g1, int slot_g2
     }
   }
   so.restore();
+  if (cells_per_rmax) *cells_per_rmax = bk;
+  if (pi_window) *pi_window = bw;
+  if (best == INFINITY) return CPC_OK;  // no trial ran: as before
+  trials.active = false;
   // keep the best: every box slot on the chosen grid (counts pair slots of one grid)
   c->tune_k = bk;
   c->tune_wpi = bw;
@@ -3036,8 +3071,6 @@ cpc_status cpc_autotune(cpc_ctx *c, cpc_pair_kind kind, int slot_g1, int slot_g2
       if (s != CPC_OK) return s;
     }
   }
-  if (cells_per_rmax) *cells_per_rmax = bk;
-  if (pi_window) *pi_window = bw;
   return CPC_OK;
 } catch (...) {
   return host_exception(c);
@@ -3119,11 +3152,13 @@ cpc_status cpc_autotune_batch(int n_jobs, cpc_ctx *const *ctxs, const cpc_pair_k
   // count)
   const int64_t stride = std::max<int64_t>(1, sample_stride);
   std::vector<std::unique_ptr<ShardOverride>> sos;
+  std::vector<std::unique_ptr<TuneTrials>> trials;
   for (int k = 0; k < n_jobs; k++) {
     bool seen = false;
     for (const auto &so : sos) seen = seen || so->c == ctxs[k];
-    if (!seen)
-      sos.emplace_back(new ShardOverride(ctxs[k], 0, (int)std::min<int64_t>(stride, 1 << 30)));
+    if (seen) continue;
+    sos.emplace_back(new ShardOverride(ctxs[k], 0, (int)std::min<int64_t>(stride, 1 << 30)));
+    trials.emplace_back(new TuneTrials(ctxs[k]));
   }
   // every slot a job reads, on cells r_max / kc
   auto regrid = [&](int kc) -> cpc_status {
@@ -3159,15 +3194,15 @@ cpc_status cpc_autotune_batch(int n_jobs, cpc_ctx *const *ctxs, const cpc_pair_k
     }
   }
   sos.clear();  // the contexts' own shards again
+  if (cells_per_rmax) *cells_per_rmax = bk;
+  if (pi_window) *pi_window = bw;
+  if (best == INFINITY) return CPC_OK;  // no trial ran: as before
+  for (const auto &t : trials) t->active = false;
   for (int k = 0; k < n_jobs; k++) {
     ctxs[k]->tune_k = bk;
     ctxs[k]->tune_wpi = bw;
   }
-  const cpc_status s = regrid(bk);
-  if (s != CPC_OK) return s;
-  if (cells_per_rmax) *cells_per_rmax = bk;
-  if (pi_window) *pi_window = bw;
-  return CPC_OK;
+  return regrid(bk);
 } catch (...) {
   return host_exception(n_jobs > 0 && ctxs ? ctxs[0] : nullptr);
 }
