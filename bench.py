@@ -533,11 +533,13 @@ def main() -> None:
         n_rows = wls[0].density.n
         k, w = ctxs[0].autotune("SD", 0, 1, sample_stride=max(1, n_rows // 25000))
         tuning = {"cells_per_rmax": k, "pi_window": w if w else "automatic (every mu bin that fits)",
-                  "by": "cpc_autotune on a shard of the work units"}
+                  "by": "cpc_autotune on a shard of the work units (the fastest pair; the "
+                        "automatic plan is kept where it is as fast)"}
     elif len(ctxs) > 1 and not args.no_tune and not args.tune:
         k, w = _lib.autotune_batch([(c, "SD", 0, 1) for c in ctxs])
         tuning = {"cells_per_rmax": k, "pi_window": w,
-                  "by": "cpc_autotune_batch on a shard of every box's work units"}
+                  "by": "cpc_autotune_batch on a shard of every box's work units (the fastest "
+                        "pair; the automatic plans are kept where they are as fast)"}
     # the uploads (copy, device checks, radix sort into the cell list, gather of
     # the SoA streams, host bucket tables), wall clock, outside the timed steps
     cell_list = {"upload_wall_ms_per_catalog": 1e3 * upload_s / (2 * len(ctxs)),

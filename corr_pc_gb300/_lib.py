@@ -193,7 +193,8 @@ class Context:
 
     def autotune(self, kind: str, slot_g1: int, slot_g2: int, sample_stride: int = 8):
         """Pick the fastest cell width and Pi window for this pair type on every
-        sample_stride-th work unit; returns (cells_per_rmax, pi_window)."""
+        sample_stride-th work unit; returns (cells_per_rmax, pi_window), and keeps
+        the automatic plan where no pair is faster."""
         k, w = ctypes.c_int(), ctypes.c_int()
         check(self.lib.cpc_autotune(self.h, PAIR[kind], slot_g1, slot_g2, sample_stride,
                                     ctypes.byref(k), ctypes.byref(w)), self.h)
@@ -308,7 +309,8 @@ def autotune_batch(jobs, sample_stride: int = 0) -> tuple:
     """jobs: list of (Context, kind, slot_g1, slot_g2) as for count_batch.
     Times batched launches on every sample_stride-th work unit of every job
     for the cell widths and Pi windows the single-job autotuner tries, keeps
-    the fastest on every context and returns (cells_per_rmax, pi_window).
+    the fastest on every context (or the automatic plans, where they are as fast)
+    and returns (cells_per_rmax, pi_window).
     sample_stride 0: the largest job's g1 rows // 25,000."""
     lib = load()
     n = len(jobs)

@@ -3031,36 +3031,48 @@ cpc_status cpc_autotune(cpc_ctx *c, cpc_pair_kind kind, int slot_g1, int slot_g2
   // the trials count every sample_stride-th work unit (a unit shard: whole
   // tiles, so each trial's per-unit costs are those of the full count)
   const int64_t stride = std::max<int64_t>(1, sample_stride);
+  const int automatic = automatic_cells(c);
   ShardOverride so(c, 0, (int)std::min<int64_t>(stride, 1 << 30));
   TuneTrials trials(c);
-  double best = INFINITY;
-  int bk = c->slots[slot_g1].kcells, bw = c->tune_wpi;
-  for (int k : ks) {
+  // time of a pair on cells r_max / k (w 0: the automatic window and variant); the
+  // first run builds the work units, the next two are timed (the faster counts)
+  auto trial = [&](int k, int w, double &t) -> cpc_status {
     cpc_status s;
+    t = INFINITY;
     c->tune_k = k;
+    c->tune_wpi = w;
     if ((s = set_cells(c, c->slots[slot_g1], k)) != CPC_OK) return s;
     if ((s = set_cells(c, c->slots[slot_g2], k)) != CPC_OK) return s;
+    for (int rep = 0; rep < 3; rep++) {
+      if (cpc_count(c, kind, slot_g1, slot_g2, CPC_ENGINE_FAST, 1, 0, &acc) != CPC_OK) break;
+      if (rep) t = std::min(t, (double)acc.pair_kernel_ms);
+    }
+    return CPC_OK;
+  };
+  cpc_status s;
+  double untuned, best = INFINITY;
+  if ((s = trial(automatic, 0, untuned)) != CPC_OK) return s;
+  int bk = automatic, bw = 0;
+  for (int k : ks)
     for (int w : ws) {
-      c->tune_wpi = w;
-      // first run builds the work units, the next two are timed (the faster counts)
-      if (cpc_count(c, kind, slot_g1, slot_g2, CPC_ENGINE_FAST, 1, 0, &acc) != CPC_OK) continue;
-      double t = INFINITY;
-      for (int rep = 0; rep < 2; rep++) {
-        if (cpc_count(c, kind, slot_g1, slot_g2, CPC_ENGINE_FAST, 1, 0, &acc) != CPC_OK) break;
-        t = std::min(t, (double)acc.pair_kernel_ms);
-      }
+      double t;
+      if ((s = trial(k, w, t)) != CPC_OK) return s;
       if (t < best) {
         best = t;
         bk = k;
         bw = w;
       }
     }
-  }
   so.restore();
   if (cells_per_rmax) *cells_per_rmax = bk;
   if (pi_window) *pi_window = bw;
-  if (best == INFINITY) return CPC_OK;  // no trial ran: as before
+  if (std::min(untuned, best) == INFINITY) return CPC_OK;  // no trial ran: as before
   trials.active = false;
+  if (untuned <= best) {  // no pair is faster
+    c->tune_k = c->tune_wpi = 0;
+    for (Slot &sl : c->slots) sl.auto_k = true;
+    return settle_cells(c);
+  }
   // keep the best: every box slot on the chosen grid (counts pair slots of one grid)
   c->tune_k = bk;
   c->tune_wpi = bw;
@@ -3151,6 +3163,8 @@ cpc_status cpc_autotune_batch(int n_jobs, cpc_ctx *const *ctxs, const cpc_pair_k
   // shards: whole tiles, so each trial's per-unit costs are those of the full
   // count)
   const int64_t stride = std::max<int64_t>(1, sample_stride);
+  std::vector<int> automatic;  // cell width of each job's context
+  for (int k = 0; k < n_jobs; k++) automatic.push_back(automatic_cells(ctxs[k]));
   std::vector<std::unique_ptr<ShardOverride>> sos;
   std::vector<std::unique_ptr<TuneTrials>> trials;
   for (int k = 0; k < n_jobs; k++) {
@@ -3160,49 +3174,56 @@ cpc_status cpc_autotune_batch(int n_jobs, cpc_ctx *const *ctxs, const cpc_pair_k
     sos.emplace_back(new ShardOverride(ctxs[k], 0, (int)std::min<int64_t>(stride, 1 << 30)));
     trials.emplace_back(new TuneTrials(ctxs[k]));
   }
-  // every slot a job reads, on cells r_max / kc
-  auto regrid = [&](int kc) -> cpc_status {
-    for (int k = 0; k < n_jobs; k++) ctxs[k]->tune_k = kc;
-    for (int k = 0; k < n_jobs; k++)
+  // every slot a job reads, on cells r_max / kc (0: each context's automatic width)
+  auto regrid = [&](int kc, int w) -> cpc_status {
+    for (int k = 0; k < n_jobs; k++) {
+      ctxs[k]->tune_k = kc ? kc : automatic[k];
+      ctxs[k]->tune_wpi = w;
       for (int sl : {slots_g1[k], slots_g2[k]}) {
-        const cpc_status st = set_cells(ctxs[k], ctxs[k]->slots[sl], kc);
+        const cpc_status st = set_cells(ctxs[k], ctxs[k]->slots[sl], ctxs[k]->tune_k);
         if (st != CPC_OK) return st;
       }
+    }
     return CPC_OK;
   };
-  double best = INFINITY;
-  int bk = ctxs[0]->slots[slots_g1[0]].kcells, bw = ctxs[0]->tune_wpi;
-  for (int kc : {2, 3, 4, 5, 6}) {
-    cpc_status s = regrid(kc);
-    if (s != CPC_OK) return s;
-    for (int w : ws) {
-      for (int k = 0; k < n_jobs; k++) ctxs[k]->tune_wpi = w;
-      // first run builds the work units, the next two are timed (the faster counts)
+  // time of the batch so; the first run builds the work units, the next two are timed
+  // (the faster counts)
+  auto trial = [&](int kc, int w, double &t) -> cpc_status {
+    t = INFINITY;
+    const cpc_status s = regrid(kc, w);
+    for (int rep = 0; rep < 3 && s == CPC_OK; rep++) {
       if (count_batch_rows(n_jobs, ctxs, kinds, slots_g1, slots_g2, accs.data(), 1) != CPC_OK)
-        continue;
-      double t = INFINITY;
-      for (int rep = 0; rep < 2; rep++) {
-        if (count_batch_rows(n_jobs, ctxs, kinds, slots_g1, slots_g2, accs.data(), 1) != CPC_OK)
-          break;
-        t = std::min(t, (double)accs[0].pair_kernel_ms);
-      }
+        break;
+      if (rep) t = std::min(t, (double)accs[0].pair_kernel_ms);
+    }
+    return s;
+  };
+  cpc_status s;
+  double untuned, best = INFINITY;
+  if ((s = trial(0, 0, untuned)) != CPC_OK) return s;
+  int bk = automatic[0], bw = 0;
+  for (int kc : {2, 3, 4, 5, 6})
+    for (int w : ws) {
+      double t;
+      if ((s = trial(kc, w, t)) != CPC_OK) return s;
       if (t < best) {
         best = t;
         bk = kc;
         bw = w;
       }
     }
-  }
   sos.clear();  // the contexts' own shards again
   if (cells_per_rmax) *cells_per_rmax = bk;
   if (pi_window) *pi_window = bw;
-  if (best == INFINITY) return CPC_OK;  // no trial ran: as before
+  if (std::min(untuned, best) == INFINITY) return CPC_OK;  // no trial ran: as before
   for (const auto &t : trials) t->active = false;
-  for (int k = 0; k < n_jobs; k++) {
-    ctxs[k]->tune_k = bk;
-    ctxs[k]->tune_wpi = bw;
+  if (!(untuned <= best)) return regrid(bk, bw);
+  for (int k = 0; k < n_jobs; k++) {  // no pair is faster
+    ctxs[k]->tune_k = ctxs[k]->tune_wpi = 0;
+    for (Slot &sl : ctxs[k]->slots) sl.auto_k = true;
+    if ((s = settle_cells(ctxs[k])) != CPC_OK) return s;
   }
-  return regrid(bk);
+  return CPC_OK;
 } catch (...) {
   return host_exception(n_jobs > 0 && ctxs ? ctxs[0] : nullptr);
 }

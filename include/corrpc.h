@@ -217,8 +217,9 @@ cpc_status cpc_set_tuning(cpc_ctx *ctx, int cells_per_rmax, int pi_window, int t
  * full count; twin counts run as twins) of this pair type, the faster of two
  * timed runs per candidate, for cell widths r_max / k (k = 2 .. 6; the cell lists are
  * rebuilt on the device) and block-local Pi windows (for 256, 512 and 1024 threads a
- * block, the largest window that fits and three quarters of it), keeps the
- * fastest for this context (as cpc_set_tuning would) and returns it.  Results
+ * block, the largest window that fits and three quarters of it) and for the
+ * automatic plan.  Returns the fastest pair and keeps it for this context (as
+ * cpc_set_tuning would), or the automatic plan where no pair is faster.  Results
  * never depend on the choice.  With coordinates 7 (r-mu) only the cell width is
  * tuned and pi_window returns 0 (the mu window stays automatic).  Box runs only
  * (sky runs return zeros). */
@@ -227,8 +228,9 @@ cpc_status cpc_autotune(cpc_ctx *ctx, cpc_pair_kind kind, int slot_g1, int slot_
 
 /* Autotuner of a batch (the jobs of cpc_count_batch, box runs with one binning
  * and which_corr): the same cell widths and Pi windows, each trial one batched
- * launch over every `sample_stride`-th work unit of every job; the fastest is
- * kept for every context of the batch and returned.  No counterpart in the
+ * launch over every `sample_stride`-th work unit of every job; the fastest pair is
+ * returned, and kept for every context of the batch unless the automatic plans are
+ * as fast.  No counterpart in the
  * reference (its sub-boxes are separate runs, corr.cpp:219). */
 cpc_status cpc_autotune_batch(int n_jobs, cpc_ctx *const *ctxs, const cpc_pair_kind *kinds,
                               const int *slots_g1, const int *slots_g2, int64_t sample_stride,

@@ -107,3 +107,28 @@ def test_a_batch_of_pairs_of_one_context():
         for (a, b), r, ref in zip(pairs, rs, refs):
             _same(r, ref, cats[a][1], cats[b][1], f"{a},{b}")
     ctx.close()
+
+
+def test_autotuned_counts_keep_up_with_untuned_ones():
+    """Sparse boxes, whose automatic cells of r_max no pair of the autotuners has: the
+    pair kernel with what they keep takes at most a fifth longer than without them
+    (cells of r_max / 2 take 1.4 times as long)."""
+    n = 20000
+    c = _cat(n, 4, L, which=0)
+    p = _params(0, n, L=L, rmin=0.1, rmax=20.0, nrp=10, npi=20, pmax=100.0)
+    prep = host.prepare(p, [("S", c), ("D", c)])
+    ctxs = [_lib.Context(p) for _ in range(3)]
+    for ctx in ctxs:
+        ctx.upload(0, prep["D"])
+        ctx.upload(1, prep["S"])
+
+    def ms(ctx):
+        return min(ctx.count("SD", 0, 1)["pair_kernel_ms"] for _ in range(20))
+
+    ref, untuned = ctxs[0].count("SD", 0, 1), ms(ctxs[0])
+    ctxs[0].autotune("SD", 0, 1, sample_stride=1)
+    _lib.autotune_batch([(ctx, "SD", 0, 1) for ctx in ctxs[1:]], sample_stride=1)
+    for ctx in ctxs:
+        assert ms(ctx) <= 1.2 * untuned
+        _same(ctx.count("SD", 0, 1), ref, c, c)
+        ctx.close()
