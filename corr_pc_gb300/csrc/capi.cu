@@ -194,10 +194,6 @@ struct cpc_ctx {
   DevBuf<int64_t> u_orig;
   DevBuf<UploadStats> d_ustats;
   UploadStats h_ustats{};
-  // sky: fixed-point sums of the fast kernel, host edge queue
-  DevBuf<unsigned long long> d_fix;
-  DevBuf<int2> d_hq;
-  DevBuf<unsigned long long> d_hq_n;
   std::vector<UnitCache> unit_cache;
   // a count enqueued by cpc_count_async, collected by cpc_count_finish
   int pending = 0;  // 0 none, 1 fast engine, 2 FP64 engine
@@ -886,7 +882,6 @@ cpc_status plan_job(cpc_ctx *c, cpc_pair_kind kind, int slot_g1, int slot_g2, in
       J.inv_qscale[f] = std::ldexp(1.0, -S);
     }
   }
-  J.qbias = 1 << 29;
   J.unit_w = unit_weights(g1, g2);
   return CPC_OK;
 }
@@ -2556,8 +2551,8 @@ cpc_status sky_finish(cpc_ctx *c, SkyPlan &P, size_t k, cpc_engine engine, float
 }
 
 // Sky counts (coordinates 0) of one context: the fast engine runs the units of
-// every job (sky_tile_kernel), then the fixed-point blocks are converted and each job's host edge tier runs; the FP64 engine runs the plain
-// kernel per job.
+// every job (sky_tile_kernel), then the fixed-point blocks are converted and each
+// job's host edge tier runs; the FP64 engine runs the plain kernel per job.
 cpc_status sky_run(cpc_ctx *c, std::vector<SkyPlan> &plans, cpc_engine engine) {
   const cpc_params &p = c->p;
   cudaStream_t st = c->st;
@@ -2881,7 +2876,7 @@ cpc_status cpc_count(cpc_ctx *c, cpc_pair_kind kind, int slot_g1, int slot_g2, c
     return fail(c, CPC_ERR_INVALID, "unknown engine");
   if (kind == CPC_PAIR_SS)
     return fail(c, CPC_ERR_INVALID, "CPC_PAIR_SS pairs one catalogue: use cpc_count_auto");
-  // sky: FP32-prefiltered warp kernel (fast) or plain FP64 kernel, both with
+  // sky: mixed-precision tile kernel (fast) or plain FP64 kernel, both with
   // the FP64 path and the host edge tier for the pairs that can bin
   if (c->p.coordinates == 0) {
     if (engine == CPC_ENGINE_CELL_FP64)

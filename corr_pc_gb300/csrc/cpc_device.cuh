@@ -158,7 +158,6 @@ struct JobDev {
   float Lf;
   BoxConst bc;
   float qscale[kNF];                   // per-field fixed-point scale 2^S_f
-  int qbias;                           // fixed-point bound: |v_f| 2^S_f <= qbias
   int unit_w;                          // every weight is 1: wt_num = count
   // ---- FP64 exact constants ----
   double L, rmin, rmax, pmin, pmax, ps, rsize;

@@ -213,7 +213,7 @@ __device__ __forceinline__ void sky_accumulate_exact(const JobDev &J, int r1, in
 // (0 .. 2^15 - 1) into word lo, its arithmetic shift x >> 15 into word hi.
 // Terms have |x| < 2^30 and a block's partial sum holds fewer than 2^33 of them,
 // so a bin takes 2^48 terms before either word can overflow; the value is
-// hi 2^15 + lo (fix_to_sums_kernel).
+// hi 2^15 + lo (sky_finish_kernel).
 __device__ __forceinline__ void fix_add(unsigned long long *lo, unsigned long long *hi,
                                         long long x) {
   const unsigned long long l = (unsigned long long)x & 0x7FFFull;
@@ -442,7 +442,7 @@ __device__ __forceinline__ void sky_unit(const SkyUnit &U, const JobDev &J, unsi
       v_l[t] = fa.sl[i1];
       v_x[t] = fa.sx[i1];
       S.pos[t] = i1;
-      S.d3[t] = fa.dl[i1];
+      if (!kShapes && uw) S.d3[t] = fa.dl[i1];
       if (kShapes) {
         v_s[t] = fa.ss[i1];
         v_h[t] = fa.sh[i1];
@@ -602,7 +602,7 @@ __device__ __forceinline__ void sky_unit(const SkyUnit &U, const JobDev &J, unsi
             const int j2 = S.seg_a[lo] + (p - S.seg_pre[lo]);
             S.key[slot - kSkyTile] = S.seg_key[lo];
             S.pos[slot] = j2;
-            S.d3[slot] = fb.dl[j2];
+            if (!kShapes && uw) S.d3[slot] = fb.dl[j2];
             v_u[slot] = fb.su[j2];
             v_w[slot] = fb.sw[j2];
             v_l[slot] = fb.sl[j2];
