@@ -184,25 +184,30 @@ __device__ __forceinline__ int sky_regions(int r1, int keep1, int r2, int keep2,
   return n;
 }
 
-// FP64 values of a pair from the FP64 path: global FP64 atomics (rare pairs),
-// corel_jk1 (jk.cpp:138-171) for the regions.
-__device__ __forceinline__ void sky_accumulate_exact(const JobDev &J, int r1, int keep1, int r2,
-                                                     int keep2, int64_t cell,
-                                                     const double f[kNF]) {
+// n pairs of one bin whose FP64 values sum to f, into the full sample: global FP64
+// atomics (rare pairs)
+__device__ __forceinline__ void sky_add_full(const JobDev &J, int64_t cell, unsigned n,
+                                             const double f[kNF]) {
   const int nf = J.corel == COREL_DD ? 1 : kNF;
-  atomicAdd(&J.acc_num[cell], 1ull);
+  atomicAdd(&J.acc_num[cell], (unsigned long long)n);
   for (int q = 0; q < nf; q++)
     if (f[q] != 0) atomicAdd(&J.acc_sums[cell * kNF + q], f[q]);
+}
+// A pair's FP64 values into its jackknife regions (corel_jk1, jk.cpp:138-171); i, j:
+// redshift-ordered positions.
+__device__ __forceinline__ void sky_add_regions(const JobDev &J, int64_t i, int64_t j,
+                                                int64_t cell, const double f[kNF]) {
   if (!J.do_jk) return;
+  const DCat &a = J.sky1.d, &b = J.sky2.d;
   const int64_t hstride = (int64_t)J.nrp * J.npi;
   int rs[2];
-  const int nr = sky_regions(r1, keep1, r2, keep2, rs);
+  const int nr = sky_regions(a.jk[i], a.keep[i], b.jk[j], b.keep[j], rs);
   for (int t = 0; t < nr; t++) {
     const int64_t hc = (int64_t)(1 + rs[t]) * hstride + cell;
     atomicAdd(&J.acc_num[hc], 1ull);
     double *sj = J.acc_sums + hc * kNF;
     if (f[0] != 0) atomicAdd(&sj[0], f[0]);
-    if (J.which_corr == 0 || nf == 1) continue;
+    if (J.which_corr == 0 || J.corel == COREL_DD) continue;
     for (int q = 1; q < kNF; q += 2)
       if (f[q] != 0) atomicAdd(&sj[q], f[q]);
   }
@@ -222,15 +227,15 @@ __device__ __forceinline__ void fix_add(unsigned long long *lo, unsigned long lo
   if (h) atomicAdd(hi, (unsigned long long)h);
 }
 
-// FP64 path of one window pair whose Pi and r_p may fall in the bins: exact
-// Pi bin, great-circle r_p, ambiguity test, values and accumulation.  i, j:
-// redshift-ordered positions.
-__device__ __noinline__ void sky_pair_fp64(const JobDev &J, int64_t i, int64_t j,
-                                           unsigned long long hq_cap, double esum) {
+// FP64 path of one window pair whose Pi and r_p may fall in the bins: exact Pi bin,
+// great-circle r_p, ambiguity test.  The pair's bin, or -1: none, or left to the host
+// tier.  i, j: redshift-ordered positions.
+__device__ __forceinline__ int sky_bin_fp64(const JobDev &J, int64_t i, int64_t j,
+                                            unsigned long long hq_cap, double esum) {
   const SkyView &a = J.sky1, &b = J.sky2;
   const double dP = __dsub_rn(b.dc[j], a.dc[i]);
   const double v2 = floor(__ddiv_rn(__dsub_rn(dP, J.pmin), J.ps));
-  if (!(v2 >= 0.0) || v2 >= (double)J.npi) return;
+  if (!(v2 >= 0.0) || v2 >= (double)J.npi) return -1;
   const double cdel = cos(__dsub_rn(a.rar[i], b.rar[j]));
   const double sum =
       __dadd_rn(__dmul_rn(a.sd[i], b.sd[j]), __dmul_rn(__dmul_rn(a.cd[i], b.cd[j]), cdel));
@@ -249,37 +254,47 @@ __device__ __noinline__ void sky_pair_fp64(const JobDev &J, int64_t i, int64_t j
   if (amb) {
     const unsigned long long q = atomicAdd(J.hq_n, 1ull);
     if (q < hq_cap) J.hq[q] = make_int2((int)i, (int)j);
-    return;
+    return -1;
   }
-  if (k < 1 || k > J.nrp) return;
+  return k < 1 || k > J.nrp ? -1 : (k - 1) * J.npi + (int)v2;
+}
+__device__ __forceinline__ void sky_values_fp64(const JobDev &J, int64_t i, int64_t j,
+                                                double f[kNF]) {
+  const SkyView &a = J.sky1, &b = J.sky2;
   const double wt = __dmul_rn(a.d.w[i], b.d.w[j]);
   double theta = 0.0;
   if (J.corel != COREL_DD)
     theta = atan((b.d.y[j] - a.d.y[i]) /
                  ((b.d.x[j] - a.d.x[i]) * cos((a.decr[i] + b.decr[j]) / 2.0)));
-  double f[kNF];
   pair_values(J.corel, J.gws, wt, theta, PairGal{a.d.e1[i], a.d.e2[i], a.d.phi[i]},
               PairGal{b.d.e1[j], b.d.e2[j], b.d.phi[j]}, f);
-  sky_accumulate_exact(J, a.d.jk[i], a.d.keep[i], b.d.jk[j], b.d.keep[j],
-                       (int64_t)(k - 1) * J.npi + (int)v2, f);
 }
 
-// A pair the mixed-precision path leaves undecided (cell positions i1, j2): the
-// exact double window first when that test is the undecided one (edge), then
-// the FP64 path.
-__device__ __noinline__ void sky_pair_exact(const JobDev &J, int i1, int j2, bool edge,
-                                            unsigned long long hq_cap, double esum) {
-  const int64_t i = J.sf1.zidx[i1], j = J.sf2.zidx[j2];
+// A pair the mixed-precision path leaves undecided (positions i, j): the exact double
+// window first when that test is the undecided one (edge), then the FP64 path.
+__device__ __forceinline__ int sky_exact_bin(const JobDev &J, int64_t i, int64_t j, bool edge,
+                                             unsigned long long hq_cap, double esum) {
   if (edge) {
     const double *win = J.sky1.win;
     const int64_t n1 = J.sky1.d.n;
     const double z2 = J.sky2.d.z[j], dec2 = J.sky2.d.y[j], ra2 = J.sky2.d.x[j];
-    if (z2 < win[i] || z2 > win[n1 + i]) return;
-    if (dec2 > win[5 * n1 + i] || dec2 < win[4 * n1 + i]) return;
-    if (ra2 < win[2 * n1 + i] || ra2 > win[3 * n1 + i]) return;  // NaN bounds pass
+    if (z2 < win[i] || z2 > win[n1 + i]) return -1;
+    if (dec2 > win[5 * n1 + i] || dec2 < win[4 * n1 + i]) return -1;
+    if (ra2 < win[2 * n1 + i] || ra2 > win[3 * n1 + i]) return -1;  // NaN bounds pass
     atomicAdd(&J.counters[1], 1ull);
   }
-  sky_pair_fp64(J, i, j, hq_cap, esum);
+  return sky_bin_fp64(J, i, j, hq_cap, esum);
+}
+// The same pair (cell positions i1, j2) binned and added.
+__device__ __noinline__ void sky_pair_exact(const JobDev &J, int i1, int j2, bool edge,
+                                            unsigned long long hq_cap, double esum) {
+  const int64_t i = J.sf1.zidx[i1], j = J.sf2.zidx[j2];
+  const int cell = sky_exact_bin(J, i, j, edge, hq_cap, esum);
+  if (cell < 0) return;
+  double f[kNF];
+  sky_values_fp64(J, i, j, f);
+  sky_add_full(J, cell, 1, f);
+  sky_add_regions(J, i, j, cell, f);
 }
 
 // Undecided pairs (about 1 in 10^4, and with weights or shapes those of equal D_C, 1
@@ -921,11 +936,46 @@ __global__ void sky_finish_kernel(int64_t n, const unsigned long long *__restric
   const JobDev &J = *jobp;
   const int64_t step = (int64_t)gridDim.x * blockDim.x;
   const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const unsigned long long nx = min(*J.xq_n, J.xq_cap);
-  for (int64_t i = i0; i < (int64_t)nx; i += step) {
-    const int2 e = J.xq[i];
-    const bool edge = e.x < 0;
-    sky_pair_exact(J, edge ? ~e.x : e.x, e.y, edge, hq_cap, esum);
+  // The pairs of equal D_C fall in one Pi bin: a warp adds its pairs of one bin
+  // together, else the few addresses of that bin's full sample take turns, 2.5 ns
+  // a pair (100k x 1M shape x density, 6.6e6 such pairs: 114 ms in all, added so 102).
+  // A few thousand pairs do not wait longer than the adding takes (8 us a job).
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const bool shapes = J.corel != COREL_DD;
+  const int64_t nx = (int64_t)min(*J.xq_n, J.xq_cap);
+  const bool together = nx >= 8192;
+  for (int64_t base = i0 - lane; base < nx; base += step) {
+    int cell = -1;
+    double f[kNF];
+    for (int q = 0; q < kNF; q++) f[q] = 0.0;
+    if (base + lane < nx) {
+      const int2 e = J.xq[base + lane];
+      const bool edge = e.x < 0;
+      const int64_t i = J.sf1.zidx[edge ? ~e.x : e.x], j = J.sf2.zidx[e.y];
+      cell = sky_exact_bin(J, i, j, edge, hq_cap, esum);
+      if (cell >= 0) {
+        sky_values_fp64(J, i, j, f);
+        sky_add_regions(J, i, j, cell, f);
+      }
+    }
+    unsigned same = together ? __match_any_sync(FULL, cell) : 1u << lane;
+    if (cell < 0) same = 0u;
+    const bool first = same && lane == __ffs(same) - 1;
+    // the first lane of a bin adds the others' values, one of them a turn
+    unsigned rest = first ? same & (same - 1) : 0u;
+    while (__any_sync(FULL, rest != 0u)) {
+      const int l = rest ? __ffs(rest) - 1 : lane;
+      const bool add = rest != 0u;
+#pragma unroll
+      for (int q = 0; q < kNF; q++) {
+        if (q > 0 && !shapes) break;
+        const double v = __shfl_sync(FULL, f[q], l);
+        if (add) f[q] += v;
+      }
+      rest &= rest - 1;
+    }
+    if (first) sky_add_full(J, cell, __popc(same), f);
   }
   for (int64_t i = i0; i < n; i += step) {
     const unsigned long long l = lo[i];
