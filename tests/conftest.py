@@ -12,6 +12,11 @@ sys.path.insert(0, os.path.dirname(os.path.abspath(__file__)))
 
 def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA GPU (runs the sm_103a kernels)")
+    # an empty reference tree is an absent one (oracle.build_reference has the same
+    # rule): the test that compiles against its sources then skips
+    import oracle
+    if os.path.isdir(oracle.REF_DIR) and not os.listdir(oracle.REF_DIR):
+        os.environ["CPC_REFERENCE_DIR"] = os.path.join(ROOT, "oracle", "no_reference")
 
 
 @pytest.fixture(scope="session", autouse=True)
