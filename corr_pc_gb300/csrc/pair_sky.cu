@@ -768,8 +768,10 @@ __device__ __forceinline__ void sky_unit(const SkyUnit &U, const JobDev &J, unsi
               float th2 = fmaf(c2, fmaf(c2, fmaf(c2, 1.0f / 560.0f, 1.0f / 90.0f), 1.0f / 12.0f),
                                1.0f) * c2;
               if (c2 > 0.0625f) {
+                // (within 0.32 rad of the antipode the chord's rounding is too much of
+                // theta: undecided)
                 const float th = 2.0f * asinf(0.5f * sqrtf(c2));
-                th2 = th * th;
+                th2 = c2 < 3.9f ? th * th : __int_as_float(0x7fc00000);
               }
               const float ds = u1.w + u2.w;
               const float r4 = th2 * (ds * ds);  // (2 r_p)^2

@@ -55,3 +55,26 @@ def test_more_undecided_pairs_than_their_queue_holds():
     assert ref["n_window"] > 1 << 20
     _same(got, ref, "undecided")
     ctx.close()
+
+
+def test_nearly_antipodal_pairs():
+    """Galaxies so near that r_p bins reach half the sky, where the chord hardly
+    changes with the angle: two caps on opposite sides, 64 fine bins below pi D_A."""
+    t = synth.flat_lcdm_table(1.0, 0.0001)
+    da = float(t.transverse[35])
+    p = synth._sky_params(which_corr=1, rmin=(np.pi - 0.005) * da,
+                          rmax=(np.pi + 0.0002) * da, nrp=64, npi=5, pmax=1.0, njk=4)
+    p.lin_bin = 1
+    cats = []
+    for role, seed, ra, dec in (("S", 3, 10.0, 60.0), ("D", 4, 190.0, -60.0)):
+        c = synth.sky_patch(400, seed, t, nside_jk=2, with_shapes=True, weights=True)
+        rng = np.random.default_rng(seed)
+        c.x[:] = ra + rng.uniform(-0.15, 0.15, c.n)
+        c.y[:] = dec + rng.uniform(-0.08, 0.08, c.n)
+        c.z[:] = 0.00355
+        cats.append((role, c))
+    ctx = _context(p, t, cats)
+    got, ref = ctx.count("SD", 1, 0), ctx.count("SD", 1, 0, engine="fp64")
+    assert ref["n_binned"] > 100000
+    _same(got, ref, "antipodal")
+    ctx.close()
