@@ -42,13 +42,13 @@
 //    Undecided windows and bins go to a queue that sky_finish_kernel evaluates
 //    in FP64 (behind it the host tier).
 //
-//    Counts (RsRd) are bound by instruction issue (77% of issue slots: 34
+//    Counts (RsRd) are bound by instruction issue (81% of issue slots: 34
 //    instructions per 32 window tests, 120 per 32 binned pairs), data against
-//    randoms by the latency of bucket searches and staging (53%).  Four terms of
-//    20k data and 200k randoms, 100 regions, 1.44e9 binned pairs: 111.6 ms before (a
+//    randoms by the latency of bucket searches and staging (61%).  Four terms of
+//    20k data and 200k randoms, 100 regions, 1.44e9 binned pairs: 113.8 ms before (a
 //    warp per row scanning its whole redshift range, every corel in one
-//    128-register kernel, the partner's region by global atomics per pair), 28.6 ms
-//    now; counts alone 8.3e10 pairs/s.
+//    128-register kernel, the partner's region by global atomics per pair), 29.1 ms
+//    now; counts alone 8.4e10 pairs/s.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
