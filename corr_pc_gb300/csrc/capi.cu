@@ -714,19 +714,20 @@ int automatic_cells(cpc_ctx *c, int64_t n = 0) {
 
 cpc_status rebuild_cells(cpc_ctx *c, Slot &s, int k);
 
-// The box catalogues in these slots on one grid: that of the first whose width the
-// caller set at its upload, else the automatic one (counts do not depend on it).
+// The box catalogues in these slots on one grid: where their widths differ, that of
+// the context's present setting, which they then keep, so that no two counts rebuild
+// a slot in turn (results do not depend on it).
 cpc_status same_grid(cpc_ctx *c, const std::vector<int> &slots) {
-  int k = 0;
-  for (int q : slots)
-    if (!k && !c->slots[q].auto_k) k = c->slots[q].kcells;
-  if (!k) k = automatic_cells(c);
+  bool same = true;
+  for (int q : slots) same = same && c->slots[q].kcells == c->slots[slots[0]].kcells;
+  if (same) return CPC_OK;
+  const int k = c->tune_k > 0 ? c->tune_k : automatic_cells(c);
   for (int q : slots) {
     Slot &s = c->slots[q];
-    if (s.valid && !s.sky && s.kcells != k) {
-      const cpc_status st = rebuild_cells(c, s, k);
-      if (st != CPC_OK) return st;
-    }
+    if (!s.valid || s.sky) continue;
+    const cpc_status st = s.kcells == k ? CPC_OK : rebuild_cells(c, s, k);
+    if (st != CPC_OK) return st;
+    s.auto_k = c->tune_k == 0;
   }
   return CPC_OK;
 }

@@ -208,8 +208,8 @@ cpc_status cpc_count_batch(int n_jobs, cpc_ctx *const *ctxs, const cpc_pair_kind
 
 /* Tuning knobs of the fast kernel (0 = automatic).  cells_per_rmax: column
  * width = r_max / k, k <= 9, of later uploads (a count of catalogues of two widths
- * rebuilds one: a width set here goes before an automatic one); pi_window: Pi bins
- * held per block; tile: g1 rows per block (0 or 128). */
+ * rebuilds them with the present one); pi_window: Pi bins held per block; tile: g1
+ * rows per block (0 or 128). */
 cpc_status cpc_set_tuning(cpc_ctx *ctx, int cells_per_rmax, int pi_window, int tile);
 
 /* Autotuner: times the fast kernel on every `sample_stride`-th work unit (a

@@ -68,6 +68,13 @@ def test_set_and_automatic_cell_widths_count_together(order, k):
     ctx.set_tuning(4)
     ctx.upload(1, pd)
     _same(ctx.count("SD", 1, 0), got, s, d)
+    # from here on the three slots share one width: no count rebuilds a list
+    ctx.upload(2, pd)
+    for _ in range(2):
+        n = ctx.launches()
+        _same(ctx.count("SD", 1, 0), got, s, d)
+        _same(ctx.count("SD", 2, 0), got, s, d)
+    assert ctx.launches() - n == 4
     ctx.close()
 
 
